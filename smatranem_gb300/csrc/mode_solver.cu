@@ -17,8 +17,8 @@
  * come from Chebyshev-filtered block subspace iteration:
  *   - the filter p(A) = T_d((A - c)/e) damps the interval [a, b] that holds
  *     the unwanted spectrum (a: below the spectral radius estimate, b: the
- *     smallest Ritz value of the block) and is fused into the two stencil
- *     kernels (three-term recurrence in the mbb kernel's epilogue);
+ *     smallest Ritz value of the block) and runs inside the stencil kernel
+ *     (three-term recurrence in its epilogue);
  *   - Rayleigh-Ritz on an orthonormal basis of the filtered block, the small
  *     non-symmetric problem solved on the host by a complex Schur
  *     decomposition.  mbb*maa is self-adjoint only in the indefinite form
@@ -94,12 +94,14 @@ __global__ void k_maa(Op op, const T *__restrict__ Vt, const T *__restrict__ X, 
 /* out = mbb W (W = maa Ycur), then Ynew = alpha*(out - c*Ycur) - beta*Yprev.
  *     u = (1/(w mu22)) (Ddown0 w0 + Ddown1 w1),
  *     out0 = V3 w0 + Dup0 u,   out1 = V4 w1 + Dup1 u.
- * alpha = 1, c = 0, beta = 0 gives the plain product A Ycur = mbb maa Ycur.
+ * alpha = 1, c = 0, beta = 0 gives the plain product A Ycur = mbb maa Ycur;
+ * ascale: alpha read from device memory instead.
  * Ynew may alias Yprev (each thread reads its own entries before writing). */
 template <class T>
 __global__ void k_mbb(Op op, const T *__restrict__ Vt, const T *__restrict__ W, const T *Ycur, const T *Yprev, T *Ynew,
-                      long long ld, T alpha, T c, T beta)
+                      long long ld, T alpha, T c, T beta, const double *__restrict__ ascale)
 {
+    if (ascale) alpha = (T)*ascale;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= op.NA1) return;
     const int L0 = op.L0, L1 = op.L1, NA1 = op.NA1;
@@ -189,8 +191,10 @@ __global__ void k_div(Op op, const T *__restrict__ Vt, const T *__restrict__ W, 
 
 template <class T>
 __global__ void k_mbb2(Op op, const T *__restrict__ Vt, const T *__restrict__ W, const T *__restrict__ Uc,
-                       const T *Ycur, const T *Yprev, T *Ynew, long long ld, T alpha, T c, T beta)
+                       const T *Ycur, const T *Yprev, T *Ynew, long long ld, T alpha, T c, T beta,
+                       const double *__restrict__ ascale)
 {
+    if (ascale) alpha = (T)*ascale;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= op.NA1) return;
     const int L0 = op.L0, L1 = op.L1, NA1 = op.NA1;
@@ -215,6 +219,105 @@ __global__ void k_mbb2(Op op, const T *__restrict__ Vt, const T *__restrict__ W,
     yn[p + NA1] = r1;
 }
 
+/* Ynew = alpha (mbb maa Ycur - c Ycur) - beta Yprev in one launch: each block
+ * stages a tile of Ycur with two halo points per side in shared memory and
+ * evaluates w, maa Y, u and mbb there, one halo ring fewer each stage.  The
+ * same operations as k_curl, k_maa2, k_div and k_mbb2 in turn, so the same
+ * bits: a link across the lattice's edge carries its wrap coefficient, a link
+ * inside 1, and a product by -1, 0 or 1 is exact, so s x + c x' is the one
+ * fused multiply-add c x' - x (s = -1: both axes have more than one cell).
+ *
+ * The stencils are bound by the FP64 pipe (1.7 operations a clock and SM
+ * measured): 22 operations a point against the four launches' 30, and 14 %
+ * more points in the halos of a 32 x 16 tile.  A solve of the 256 x 192 layer
+ * (1150 products of 12 columns): 70.3 ms with four launches a product, 48.1 ms
+ * with one; of a 40 x 30 layer, where launches count: 10.5 and 6.8 ms.  Tiles of 8 rows where 16 would leave SMs without
+ * a block: small layers are bound by one block's latency.
+ * ascale: alpha read from device memory instead (the power iteration). */
+constexpr int PX = 32; /* tile columns */
+template <class T, int PY>
+__global__ void __launch_bounds__(256) k_product(Op op, const T *__restrict__ Vt, const T *Ycur, const T *Yprev,
+                                                 T *Ynew, long long ld, T alpha, T c, T beta,
+                                                 const double *__restrict__ ascale)
+{
+    constexpr int XW = PX + 4, XH = PY + 4, WW = PX + 3, WH = PY + 3, MW = PX + 2, MH = PY + 2, UW = PX + 1, UH = PY + 1;
+    __shared__ T xs[2][XH * XW], ws[WH * WW], ms[2][MH * MW], us[UH * UW];
+    __shared__ int rx[XW], ry[XH]; /* lattice index of each tile column and row */
+    __shared__ T lx[XW], ly[XH];   /* coefficient of the link from it to the next */
+    const int L0 = op.L0, L1 = op.L1, NA1 = op.NA1, tid = threadIdx.x;
+    const int ntx = (L0 + PX - 1) / PX, x0 = (int)(blockIdx.x % ntx) * PX, y0 = (int)(blockIdx.x / ntx) * PY;
+    const int nx = min(PX, L0 - x0), ny = min(PY, L1 - y0);
+    const long long col = (long long)blockIdx.y * ld;
+    if (tid < XW) {
+        const int r = ((x0 - 2 + tid) % L0 + L0) % L0;
+        rx[tid] = r;
+        lx[tid] = r < L0 - 1 ? (T)1 : (T)op.e0;
+    } else if (tid >= 64 && tid < 64 + XH) {
+        const int r = ((y0 - 2 + tid - 64) % L1 + L1) % L1;
+        ry[tid - 64] = r;
+        ly[tid - 64] = r < L1 - 1 ? (T)1 : (T)op.e1;
+    }
+    if (ascale) alpha = (T)*ascale;
+    __syncthreads();
+    for (int t = tid; t < XW * XH; t += 256) {
+        const int i = t % XW, j = t / XW;
+        if (i < nx + 4 && j < ny + 4) {
+            const T *y = Ycur + col + rx[i] + L0 * ry[j];
+            xs[0][t] = y[0];
+            xs[1][t] = y[NA1];
+        }
+    }
+    __syncthreads();
+    for (int t = tid; t < WW * WH; t += 256) { /* w at tile point (i, j) of the staged tile */
+        const int i = t % WW, j = t / WW;
+        if (i < nx + 3 && j < ny + 3) {
+            const T *a = xs[0] + j * XW + i, *b = xs[1] + j * XW + i;
+            const T d1 = fma(ly[j], a[XW], -a[0]), d0 = fma(lx[i], b[1], -b[0]);
+            ws[t] = __ldg(Vt + 2 * (long long)NA1 + rx[i] + L0 * ry[j]) * (d1 - d0);
+        }
+    }
+    __syncthreads();
+    for (int t = tid; t < MW * MH; t += 256) { /* maa Y at (i + 1, j + 1) */
+        const int i = t % MW, j = t / MW;
+        if (i < nx + 2 && j < ny + 2) {
+            const T *w = ws + (j + 1) * WW + i + 1;
+            const T *v = Vt + rx[i + 1] + L0 * ry[j + 1];
+            const int x = (j + 1) * XW + i + 1;
+            ms[0][t] = fma(__ldg(v), xs[0][x], fma(-ly[j], w[-WW], w[0]));
+            ms[1][t] = fma(__ldg(v + NA1), xs[1][x], -fma(-lx[i], w[-1], w[0]));
+        }
+    }
+    __syncthreads();
+    for (int t = tid; t < UW * UH; t += 256) { /* u at (i + 2, j + 2) */
+        const int i = t % UW, j = t / UW;
+        if (i < nx + 1 && j < ny + 1) {
+            const T *a = ms[0] + (j + 1) * MW + i + 1, *b = ms[1] + (j + 1) * MW + i + 1;
+            const T a0 = fma(-lx[i + 1], a[-1], a[0]), a1 = fma(-ly[j + 1], b[-MW], b[0]);
+            us[t] = __ldg(Vt + 5 * (long long)NA1 + rx[i + 2] + L0 * ry[j + 2]) * (a0 + a1);
+        }
+    }
+    __syncthreads();
+    for (int t = tid; t < PX * PY; t += 256) {
+        const int i = t % PX, j = t / PX;
+        if (i < nx && j < ny) {
+            const int p = x0 + i + L0 * (y0 + j), m = (j + 1) * MW + i + 1;
+            const T *u = us + j * UW + i;
+            const T o0 = fma(__ldg(Vt + 3 * (long long)NA1 + p), ms[0][m], fma(lx[i + 2], u[1], -u[0]));
+            const T o1 = fma(__ldg(Vt + 4 * (long long)NA1 + p), ms[1][m], fma(ly[j + 2], u[UW], -u[0]));
+            const int x = (j + 2) * XW + i + 2;
+            T r0 = alpha * (o0 - c * xs[0][x]), r1 = alpha * (o1 - c * xs[1][x]);
+            if (beta != (T)0) {
+                const T *yp = Yprev + col;
+                r0 -= beta * yp[p];
+                r1 -= beta * yp[p + NA1];
+            }
+            T *yn = Ynew + col;
+            yn[p] = r0;
+            yn[p + NA1] = r1;
+        }
+    }
+}
+
 /* column-major block conversion between FP64 and FP32 */
 template <class A, class B>
 __global__ void k_cvt(const A *__restrict__ in, B *__restrict__ out, long long count)
@@ -227,11 +330,16 @@ constexpr int GT = 256;       // threads of the reduction kernels
 constexpr int GROWS = 32;     // rows staged per pass of k_gram
 constexpr int MAXB = 128;     // largest block the kernels accept
 
-/* partial Gram blocks: P[blk][i][j] = sum over this CTA's rows of X[r,i] Y[r,j] */
-__global__ void k_gram(const double *__restrict__ X, const double *__restrict__ Y, long long n, long long ld, int mx,
-                       int my, double *__restrict__ P)
+/* partial Gram blocks: P[blk][i][j] = sum over this CTA's rows of X[r,i] Y[r,j],
+ * Y = Ya (blockIdx.y = 0) or Yb (1, its partials after the first's): the two
+ * products of a Rayleigh-Ritz step in one launch, whose blocks balance over
+ * the SMs better than two launches of 1.3 blocks an SM */
+__global__ void k_gram(const double *__restrict__ X, const double *__restrict__ Ya, const double *__restrict__ Yb,
+                       long long n, long long ld, int mx, int my, double *__restrict__ P)
 {
     extern __shared__ double sm[];
+    const double *__restrict__ Y = blockIdx.y ? Yb : Ya;
+    P += (long long)blockIdx.y * gridDim.x * mx * my;
     double *xs = sm, *ys = sm + GROWS * mx;
     const int nout = mx * my;
     const int per = (nout + GT - 1) / GT;  // <= MAXB*MAXB/GT = 64
@@ -266,12 +374,17 @@ __global__ void k_gram(const double *__restrict__ X, const double *__restrict__ 
     }
 }
 
-/* G[o] = sum over blocks of P[blk][o], blocks in order (deterministic) */
+/* G[o] = sum over blocks of P[blk][o], blocks in order (deterministic);
+ * blockIdx.y: one such sum after another in P and G.  The loads of several
+ * blocks leave together; the additions are a chain either way. */
 __global__ void k_sum_blocks(const double *__restrict__ P, int nblk, int nout, double *__restrict__ G)
 {
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= nout) return;
+    P += (long long)blockIdx.y * nblk * nout;
+    G += (long long)blockIdx.y * nout;
     double s = 0.0;
+#pragma unroll 16
     for (int b = 0; b < nblk; b++) s += P[(long long)b * nout + o];
     G[o] = s;
 }
@@ -302,8 +415,8 @@ __global__ void k_gemm(const double *__restrict__ X, const double *__restrict__ 
         if (j0 + j < mo) Y[r + ld * (j0 + j)] = acc[j];
 }
 
-/* per column j: sum_r (A[r,j] - lam[j] B[r,j])^2 (lam == nullptr: sum A^2),
- * partial sums per CTA into P[blk][j] */
+/* per column j (blockIdx.y): sum_r (A[r,j] - lam[j] B[r,j])^2 (lam == nullptr:
+ * sum A^2), partial sums per CTA into P[blk][j] */
 template <class T>
 __global__ void k_colres(const T *__restrict__ A, const T *__restrict__ B, const double *__restrict__ lam,
                          long long n, long long ld, int m, double *__restrict__ P)
@@ -311,36 +424,50 @@ __global__ void k_colres(const T *__restrict__ A, const T *__restrict__ B, const
     __shared__ double red[GT];
     const long long chunk = (n + gridDim.x - 1) / gridDim.x;
     const long long r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
-    for (int j = 0; j < m; j++) {
-        const double l = lam ? lam[j] : 0.0;
-        double s = 0.0;
-        for (long long r = r0 + threadIdx.x; r < r1; r += GT) {
-            const double v = lam ? (double)A[r + ld * j] - l * (double)B[r + ld * j] : (double)A[r + ld * j];
-            s = fma(v, v, s);
-        }
-        red[threadIdx.x] = s;
-        __syncthreads();
-        for (int h = GT / 2; h > 0; h >>= 1) {
-            if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) P[(long long)blockIdx.x * m + j] = red[0];
+    const int j = blockIdx.y;
+    const double l = lam ? lam[j] : 0.0;
+    double s = 0.0;
+    for (long long r = r0 + threadIdx.x; r < r1; r += GT) {
+        const double v = lam ? (double)A[r + ld * j] - l * (double)B[r + ld * j] : (double)A[r + ld * j];
+        s = fma(v, v, s);
+    }
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int h = GT / 2; h > 0; h >>= 1) {
+        if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
         __syncthreads();
     }
+    if (threadIdx.x == 0) P[(long long)blockIdx.x * m + j] = red[0];
 }
 
-/* column j of A and of B scaled by s[j] (keeps the Chebyshev recurrence's
- * last two terms bounded; the recurrence is linear per column) */
+/* one step of the power iteration from the squared norm s: est = {1/norm of
+ * the vector (the next product's scale), largest norm ratio so far, nonzero
+ * where a norm was not finite}; first: the starting vector's norm */
+__global__ void k_power(const double *__restrict__ s, double *est, int first)
+{
+    const double r = sqrt(s[0]);
+    if (first) {
+        est[1] = est[2] = 0.0;
+    } else {
+        if (!isfinite(r)) est[2] = 1.0;
+        if (est[1] < r) est[1] = r;
+    }
+    est[0] = 1.0 / r;
+}
+
+/* column j (blockIdx.y) of A and of B divided by the norm whose square is
+ * s[j] (keeps the Chebyshev recurrence's last two terms bounded; the
+ * recurrence is linear per column) */
 template <class T>
-__global__ void k_scale2(T *A, T *B, const double *__restrict__ s, long long n, long long ld, int m)
+__global__ void k_scale2(T *A, T *B, const double *__restrict__ s, long long n, long long ld)
 {
     const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y;
     if (r >= n) return;
-    for (int j = 0; j < m; j++) {
-        const T f = (T)s[j];
-        A[r + ld * j] *= f;
-        B[r + ld * j] *= f;
-    }
+    const double v = s[j];
+    const T f = (T)(v > 0 && isfinite(v) ? 1.0 / sqrt(v) : 1.0);
+    A[r + ld * j] *= f;
+    B[r + ld * j] *= f;
 }
 
 /* deterministic uniform(-1, 1) fill (splitmix64 of seed and index) */
@@ -585,26 +712,18 @@ struct Solver {
     Op op{};
     cudaStream_t st = nullptr;
     long long n = 0, ld = 0;
-    int mb = 0, nblk = 0;
-    double *dV = nullptr, *bufs[7] = {}, *dP = nullptr, *dG = nullptr, *dC = nullptr, *dL = nullptr;
+    int mb = 0, nblk = 0, sms = 0;
+    double *dV = nullptr, *bufs[7] = {}, *dP = nullptr, *dG = nullptr, *dC = nullptr, *dL = nullptr, *dE = nullptr;
     float *dVf = nullptr, *fbufs[4] = {};  /* FP32 copy of the coefficients; FP32 filter buffers */
     double *aux = nullptr;                 /* w or u of every point and column (two-pass stencils) */
     float *auxf = nullptr;
+    void *slab = nullptr;                  /* the one allocation that holds them all */
     long long matvecs = 0, matvecs32 = 0;
 
     ~Solver()
     {
         if (st) cudaStreamSynchronize(st);
-        cudaFree(dV);
-        cudaFree(dVf);
-        for (double *b : bufs) cudaFree(b);
-        for (float *b : fbufs) cudaFree(b);
-        cudaFree(aux);
-        cudaFree(auxf);
-        cudaFree(dP);
-        cudaFree(dG);
-        cudaFree(dC);
-        cudaFree(dL);
+        cudaFree(slab);
         if (st) cudaStreamDestroy(st);
     }
     dim3 pgrid(int m) const { return dim3((unsigned)((op.NA1 + 127) / 128), (unsigned)m); }
@@ -626,36 +745,61 @@ struct Solver {
         return cudaPeekAtLastError() == cudaSuccess ? SMAT_OK : smat_fail(SMAT_ECUDA, "k_maa launch");
     }
     template <class T>
-    int mbb(const T *W, const T *Yc, const typename nd<T>::type *Yp, T *Yn, int m, double alpha, double c, double beta)
+    int mbb(const T *W, const T *Yc, const typename nd<T>::type *Yp, T *Yn, int m, double alpha, double c, double beta,
+            const double *ascale = nullptr)
     {
         if (two_pass) {
             T *u = scratch(W);
             k_div<T><<<pgrid(m), 128, 0, st>>>(op, coef(W), W, u, ld);
-            k_mbb2<T><<<pgrid(m), 128, 0, st>>>(op, coef(W), W, u, Yc, Yp, Yn, ld, (T)alpha, (T)c, (T)beta);
+            k_mbb2<T><<<pgrid(m), 128, 0, st>>>(op, coef(W), W, u, Yc, Yp, Yn, ld, (T)alpha, (T)c, (T)beta, ascale);
         } else {
-            k_mbb<T><<<pgrid(m), 128, 0, st>>>(op, coef(W), W, Yc, Yp, Yn, ld, (T)alpha, (T)c, (T)beta);
+            k_mbb<T><<<pgrid(m), 128, 0, st>>>(op, coef(W), W, Yc, Yp, Yn, ld, (T)alpha, (T)c, (T)beta, ascale);
         }
         return cudaPeekAtLastError() == cudaSuccess ? SMAT_OK : smat_fail(SMAT_ECUDA, "k_mbb launch");
     }
+    /* Yn = alpha (mbb maa Yc - c Yc) - beta Yp; W: room for maa Yc where the
+     * stencils run one after the other (one-cell axes, SMATRAN_MODE_ONE_PASS) */
+    template <class T>
+    int product(const T *Yc, const typename nd<T>::type *Yp, T *Yn, T *W, int m, double alpha, double c, double beta,
+                const double *ascale = nullptr)
+    {
+        if (!fused()) {
+            int rc = maa(Yc, W, m);
+            return rc ? rc : mbb(W, Yc, Yp, Yn, m, alpha, c, beta, ascale);
+        }
+        const int ntx = (op.L0 + PX - 1) / PX, n16 = ntx * ((op.L1 + 15) / 16);
+        if (n16 * m >= 2 * sms)
+            k_product<T, 16><<<dim3(n16, m), 256, 0, st>>>(op, coef(Yc), Yc, Yp, Yn, ld, (T)alpha, (T)c, (T)beta, ascale);
+        else
+            k_product<T, 8><<<dim3(ntx * ((op.L1 + 7) / 8), m), 256, 0, st>>>(op, coef(Yc), Yc, Yp, Yn, ld, (T)alpha, (T)c,
+                                                                             (T)beta, ascale);
+        return cudaPeekAtLastError() == cudaSuccess ? SMAT_OK : smat_fail(SMAT_ECUDA, "k_product launch");
+    }
+    bool fused() const { return two_pass && op.L0 > 1 && op.L1 > 1; }
     template <class A, class B> int convert(const A *in, B *out, int m)
     {
         const long long count = n * m;
         k_cvt<A, B><<<(unsigned)((count + 255) / 256), 256, 0, st>>>(in, out, count);
         return cudaPeekAtLastError() == cudaSuccess ? SMAT_OK : smat_fail(SMAT_ECUDA, "k_cvt launch");
     }
-    /* G (host, mx x my row-major by i*my + j) = X^T Y */
-    int gram(const double *X, const double *Y, int mx, int my, std::vector<double> &G)
+    /* G, H (host, m x m row-major) = X^T Ya, X^T Yb */
+    int gram(const double *X, const double *Ya, const double *Yb, int m, std::vector<double> &G, std::vector<double> &H)
     {
-        const size_t smem = (size_t)GROWS * (mx + my) * sizeof(double);
-        k_gram<<<nblk, GT, smem, st>>>(X, Y, n, ld, mx, my, dP);
-        k_sum_blocks<<<(mx * my + 255) / 256, 256, 0, st>>>(dP, nblk, mx * my, dG);
-        std::vector<double> g((size_t)mx * my);
+        const size_t smem = (size_t)GROWS * 2 * m * sizeof(double);
+        const int nout = m * m;
+        k_gram<<<dim3(nblk, 2), GT, smem, st>>>(X, Ya, Yb, n, ld, m, m, dP);
+        k_sum_blocks<<<dim3((nout + 63) / 64, 2), 64, 0, st>>>(dP, nblk, nout, dG);
+        std::vector<double> g(2 * (size_t)nout);
         if (cudaMemcpyAsync(g.data(), dG, g.size() * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
             return smat_fail(SMAT_ECUDA, "gram: %s", cudaGetErrorString(cudaGetLastError()));
-        G.assign((size_t)mx * my, 0.0);
-        for (int j = 0; j < my; j++)
-            for (int i = 0; i < mx; i++) G[(size_t)i * my + j] = g[i + (size_t)mx * j];
+        G.resize(nout);
+        H.resize(nout);
+        for (int j = 0; j < m; j++)
+            for (int i = 0; i < m; i++) {
+                G[(size_t)i * m + j] = g[i + (size_t)m * j];
+                H[(size_t)i * m + j] = g[nout + i + (size_t)m * j];
+            }
         return SMAT_OK;
     }
     /* Y = X C with C host row-major m x mo */
@@ -669,6 +813,12 @@ struct Solver {
         if (cudaStreamSynchronize(st) != cudaSuccess) return smat_fail(SMAT_ECUDA, "k_gemm");
         return SMAT_OK;
     }
+    /* the same into dG, on the stream */
+    template <class T> void norms(const T *A, const T *B, const double *dlam, int m)
+    {
+        k_colres<T><<<dim3(nblk, m), GT, 0, st>>>(A, B, dlam, n, ld, m, dP);
+        k_sum_blocks<<<(m + 31) / 32, 32, 0, st>>>(dP, nblk, m, dG);
+    }
     /* per column: ||A_j - lam_j B_j||^2 (lam empty: ||A_j||^2) */
     template <class T>
     int colres(const T *A, const typename nd<T>::type *B, const std::vector<double> &lam, int m,
@@ -677,8 +827,7 @@ struct Solver {
         if (!lam.empty() &&
             cudaMemcpyAsync(dL, lam.data(), (size_t)m * sizeof(double), cudaMemcpyHostToDevice, st) != cudaSuccess)
             return smat_fail(SMAT_ECUDA, "colres upload");
-        k_colres<T><<<nblk, GT, 0, st>>>(A, B, lam.empty() ? nullptr : dL, n, ld, m, dP);
-        k_sum_blocks<<<(m + 255) / 256, 256, 0, st>>>(dP, nblk, m, dG);
+        norms<T>(A, B, lam.empty() ? nullptr : dL, m);
         out.resize(m);
         if (cudaMemcpyAsync(out.data(), dG, (size_t)m * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
@@ -688,15 +837,9 @@ struct Solver {
     /* rescale columns of cur (and prev alike) to unit norm */
     template <class T> int rescale(T *cur, T *prev, int m)
     {
-        std::vector<double> nv;
-        int rc = colres<T>(cur, nullptr, {}, m, nv);
-        if (rc) return rc;
-        for (double &v : nv) v = (v > 0 && std::isfinite(v)) ? 1.0 / std::sqrt(v) : 1.0;
-        if (cudaMemcpyAsync(dL, nv.data(), (size_t)m * sizeof(double), cudaMemcpyHostToDevice, st) != cudaSuccess)
-            return smat_fail(SMAT_ECUDA, "rescale upload");
-        k_scale2<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(cur, prev, dL, n, ld, m);
-        if (cudaStreamSynchronize(st) != cudaSuccess) return smat_fail(SMAT_ECUDA, "k_scale2");
-        return SMAT_OK;
+        norms<T>(cur, nullptr, nullptr, m);
+        k_scale2<T><<<dim3((unsigned)((n + 255) / 256), m), 256, 0, st>>>(cur, prev, dG, n, ld);
+        return cudaPeekAtLastError() == cudaSuccess ? SMAT_OK : smat_fail(SMAT_ECUDA, "k_scale2 launch");
     }
     void random(double *X, int j0, int m, unsigned long long seed)
     {
@@ -713,10 +856,10 @@ int chebyshev(Solver &S, const T *X0, T *Fa, T *Fb, T *Wt, int mb, int degree, d
     int rc;
     const T *prev = X0;
     T *cur = Fa;
-    if ((rc = S.maa(prev, Wt, mb)) || (rc = S.mbb(Wt, prev, nullptr, cur, mb, 1.0 / e, c, 0.0))) return rc;
+    if ((rc = S.product(prev, nullptr, cur, Wt, mb, 1.0 / e, c, 0.0))) return rc;
     for (int k = 1; k < degree; k++) {
         T *nxt = (prev == X0) ? Fb : const_cast<T *>(prev);
-        if ((rc = S.maa(cur, Wt, mb)) || (rc = S.mbb(Wt, cur, prev, nxt, mb, 2.0 / e, c, 1.0))) return rc;
+        if ((rc = S.product(cur, prev, nxt, Wt, mb, 2.0 / e, c, 1.0))) return rc;
         prev = cur;
         cur = nxt;
         if (k % 32 == 0 && k + 1 < degree && (rc = S.rescale(cur, const_cast<T *>(prev), mb))) return rc;
@@ -762,32 +905,45 @@ int setup(Solver &S, int L0, int L1, const int *bc, const std::vector<double> &V
     S.op.e1 = L1 > 1 ? (double)bc[1] : 0.0;
     S.n = S.ld = 2LL * S.op.NA1;
     S.mb = mb;
-    int dev = 0, sms = 148;
+    int dev = 0;
     MCK(cudaGetDevice(&dev));
-    MCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    S.nblk = (int)std::min<long long>(2LL * sms, std::max<long long>(1, (S.n + 1023) / 1024));
+    MCK(cudaDeviceGetAttribute(&S.sms, cudaDevAttrMultiProcessorCount, dev));
+    S.nblk = (int)std::min<long long>(2LL * S.sms, std::max<long long>(1, (S.n + 1023) / 1024));
     MCK(cudaStreamCreateWithFlags(&S.st, cudaStreamNonBlocking));
-    MCK(cudaMalloc(&S.dV, V.size() * sizeof(double)));
-    MCK(cudaMemcpyAsync(S.dV, V.data(), V.size() * sizeof(double), cudaMemcpyHostToDevice, S.st));
-    S.op.V = S.dV;
     {   /* SMATRAN_MODE_ONE_PASS=1: the one-pass stencils (same results, for comparison) */
         const char *env = getenv("SMATRAN_MODE_ONE_PASS");
         S.two_pass = !(env && env[0] == '1');
     }
-    for (double *&b : S.bufs) MCK(cudaMalloc(&b, (size_t)S.n * mb * sizeof(double)));
-    for (float *&b : S.fbufs) MCK(cudaMalloc(&b, (size_t)S.n * mb * sizeof(float)));
-    MCK(cudaMalloc(&S.aux, (size_t)S.n * mb * sizeof(double)));
-    MCK(cudaMalloc(&S.auxf, (size_t)S.n * mb * sizeof(float)));
-    MCK(cudaMalloc(&S.dVf, V.size() * sizeof(float)));
+    {   /* every buffer from one allocation: twenty of them cost a small layer's
+         * solve 1 ms */
+        size_t used = 0;
+        std::vector<std::pair<void **, size_t>> want;
+        auto buf = [&](auto *&p, size_t count) {
+            want.push_back({(void **)&p, used});
+            used += (count * sizeof(*p) + 255) / 256 * 256;
+        };
+        const size_t blk = (size_t)S.n * mb, mm = (size_t)mb * mb;
+        buf(S.dV, V.size());
+        buf(S.dVf, V.size());
+        for (double *&p : S.bufs) buf(p, blk);
+        for (float *&p : S.fbufs) buf(p, blk);
+        buf(S.aux, blk);
+        buf(S.auxf, blk);
+        buf(S.dP, 2 * S.nblk * mm);
+        buf(S.dG, 2 * mm);
+        buf(S.dC, mm);
+        buf(S.dL, mb);
+        buf(S.dE, 3);
+        MCK(cudaMalloc(&S.slab, used));
+        for (auto &w : want) *w.first = (char *)S.slab + w.second;
+    }
+    MCK(cudaMemcpyAsync(S.dV, V.data(), V.size() * sizeof(double), cudaMemcpyHostToDevice, S.st));
+    S.op.V = S.dV;
     {
         std::vector<float> vf(V.begin(), V.end());
         MCK(cudaMemcpyAsync(S.dVf, vf.data(), vf.size() * sizeof(float), cudaMemcpyHostToDevice, S.st));
         MCK(cudaStreamSynchronize(S.st));
     }
-    MCK(cudaMalloc(&S.dP, (size_t)S.nblk * mb * mb * sizeof(double)));
-    MCK(cudaMalloc(&S.dG, (size_t)mb * mb * sizeof(double)));
-    MCK(cudaMalloc(&S.dC, (size_t)mb * mb * sizeof(double)));
-    MCK(cudaMalloc(&S.dL, (size_t)mb * sizeof(double)));
     {
         int smem_optin = 0;
         MCK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -837,7 +993,7 @@ extern "C" int smat_mode_apply(int L0, int L1, const int BoundC[2], double omega
         if ((rc = S.mbb(dX, dX, nullptr, dZ, m, 1.0, 0.0, 0.0))) return rc;
         out = dZ;
     } else {
-        if ((rc = S.maa(dX, dW, m)) || (rc = S.mbb(dW, dX, nullptr, dZ, m, 1.0, 0.0, 0.0))) return rc;
+        if ((rc = S.product(dX, nullptr, dZ, dW, m, 1.0, 0.0, 0.0))) return rc;
         out = dZ;
     }
     if (cudaMemcpyAsync(Y, out, bytes, cudaMemcpyDeviceToHost, S.st) != cudaSuccess ||
@@ -875,20 +1031,23 @@ extern "C" int smat_mode_solve(int L0, int L1, const int BoundC[2], double omega
     /* spectral radius by power iteration on one column */
     double rho = 0.0;
     {
+        /* on the stream throughout: the norms stay on the device */
         S.random(F[0], 0, 1, seed ^ 0xabcdefull);
-        std::vector<double> nv;
-        if ((rc = S.colres(F[0], nullptr, {}, 1, nv))) return rc;
-        double nrm = std::sqrt(nv[0]);
+        S.norms<double>(F[0], nullptr, nullptr, 1);
+        k_power<<<1, 1, 0, S.st>>>(S.dG, S.dE, 1);
         for (int it = 0; it < 80; it++) {
-            if ((rc = S.maa(F[0], W, 1)) || (rc = S.mbb(W, F[0], nullptr, F[1], 1, 1.0 / nrm, 0.0, 0.0))) return rc;
+            if ((rc = S.product(F[0], nullptr, F[1], W, 1, 1.0, 0.0, 0.0, S.dE))) return rc;
             S.matvecs++;
-            if ((rc = S.colres(F[1], nullptr, {}, 1, nv))) return rc;
-            const double r = std::sqrt(nv[0]);  // ||A v|| / ||v||
-            if (!std::isfinite(r)) return smat_fail(SMAT_ENUMERIC, "mode solver: non-finite operator norm");
-            rho = std::max(rho, r);
-            nrm = r;
+            S.norms<double>(F[1], nullptr, nullptr, 1);
+            k_power<<<1, 1, 0, S.st>>>(S.dG, S.dE, 0); /* ||A v|| / ||v|| */
             std::swap(F[0], F[1]);
         }
+        double est[3];
+        if (cudaMemcpyAsync(est, S.dE, sizeof est, cudaMemcpyDeviceToHost, S.st) != cudaSuccess ||
+            cudaStreamSynchronize(S.st) != cudaSuccess)
+            return smat_fail(SMAT_ECUDA, "mode solver: %s", cudaGetErrorString(cudaGetLastError()));
+        if (est[2] != 0.0) return smat_fail(SMAT_ENUMERIC, "mode solver: non-finite operator norm");
+        rho = est[1];
     }
     double a = -1.25 * rho, b = 0.0;
     S.random(X, 0, mb, seed);
@@ -930,10 +1089,10 @@ extern "C" int smat_mode_solve(int L0, int L1, const int BoundC[2], double omega
          * Q = Y T (T from the Gram matrix's eigen-decomposition, directions
          * below 1e-13 of the largest dropped), B = Q^T A Q, Ritz pairs from
          * the small non-symmetric eigenproblem */
-        if ((rc = S.maa(Y, W, mb)) || (rc = S.mbb(W, Y, nullptr, Z, mb, 1.0, 0.0, 0.0))) return rc;
+        if ((rc = S.product(Y, nullptr, Z, W, mb, 1.0, 0.0, 0.0))) return rc;
         S.matvecs += mb;
         std::vector<double> G, Fm;
-        if ((rc = S.gram(Y, Y, mb, mb, G)) || (rc = S.gram(Y, Z, mb, mb, Fm))) return rc;
+        if ((rc = S.gram(Y, Y, Z, mb, G, Fm))) return rc;
         std::vector<double> d(mb);
         for (int i = 0; i < mb; i++) d[i] = G[(size_t)i * mb + i] > 0 ? 1.0 / std::sqrt(G[(size_t)i * mb + i]) : 0.0;
         for (int i = 0; i < mb; i++)

@@ -239,3 +239,17 @@ def test_one_and_two_pass_stencils_agree_bit_for_bit(built):
         out[flag] = np.load(path)
         os.remove(path)
     assert np.array_equal(out["0"], out["1"])
+
+
+@pytest.mark.parametrize("L0,L1", [(2, 2), (3, 40), (31, 15), (32, 16), (33, 17), (64, 9), (65, 8), (130, 70)])
+@pytest.mark.parametrize("bc", [(0, 0), (1, -1), (-1, 1)])
+def test_tiled_product_equals_the_stencils_in_turn(built, L0, L1, bc):
+    """mbb*maa in one launch (tiles of 32 x 8 or 16 points, by the number of
+    blocks) against maa then mbb by themselves: the same operations, so the
+    same bits, at sizes around the tiles and under every kind of wrap."""
+    rng = np.random.default_rng(L0 * 100 + L1)
+    med = W.port_layer(L0, L1, core=(max(1, L0 // 3), max(1, L1 // 3)), seed=1, metric=0.2)
+    for m in (1, 13):
+        X = rng.standard_normal((2 * L0 * L1, m))
+        want = modes.apply(med, 0.405, L0, L1, bc, 1, modes.apply(med, 0.405, L0, L1, bc, 0, X))
+        assert np.array_equal(modes.apply(med, 0.405, L0, L1, bc, 2, X), want)
