@@ -2,7 +2,7 @@
  * FP64 split-field FDTD step, bit-identical to the reference main_calc
  * (FDTDcalc/FDTDsplitfieldMetal.c:242-329).
  *
- * One thread per cell and excitation.  Every floating-point expression keeps
+ * One thread per cell and component.  Every floating-point expression keeps
  * the reference's operands and order, and the file is compiled with
  * -fmad=false so that no multiply-add is fused: each result is the same IEEE
  * double the reference computes.  The two sweeps have no intra-sweep
@@ -11,8 +11,9 @@
  *
  * Deliberate differences that change no value: the boundary factor iBc in
  * {-1, 0, 1} multiplies by sign manipulation instead of a DMUL (bp*x for
- * finite x); an ordinary cell with no special neighbour skips the curl of the
- * aux arrays, which the reference evaluates as a sum of zeros; the 0.0 the
+ * finite x); products by the coefficients A and B are rounded on the integer
+ * pipes (the same bits); an ordinary cell with no special neighbour skips the
+ * curl of the aux arrays, which the reference evaluates as a sum of zeros; the 0.0 the
  * reference starts each curl sum from is dropped.  These can only flip the
  * sign of a zero.
  */
@@ -42,73 +43,35 @@ __device__ __forceinline__ double bmul(double x, Sel s)
     return __longlong_as_double((long long)((((unsigned long long)__double_as_longlong(x)) & s.keep) ^ s.flip));
 }
 
-struct Stn {
-    long long o[3]; /* offset of the neighbour along each axis (wrapped) */
-    Sel s[3];       /* its boundary factor */
+/* What the curl of component c of a field [3][n3] reads at cell l, a1 = c+1,
+ * a2 = c+2: components a1 and a2 of the cell, a2 of its neighbour along a1,
+ * a1 of its neighbour along a2 (offsets o1, o2).  A component array holds
+ * under 2^31 / 3 entries, so indexes are 32-bit. */
+struct Near {
+    double h1, h2, n2, n1;
 };
 
-/* neighbours of ope_R (forward, :374-381) or ope_Rd (backward, :395-402) */
-__device__ __forceinline__ Stn make_stn(const Geo &g, int j0, int j1, int j2, bool fwd)
+__device__ __forceinline__ Near load_near(const double *__restrict__ F, int i1, int i2, int o1, int o2)
 {
-    Stn st;
-    const int j[3] = {j0, j1, j2};
-    const int L[3] = {g.L0, g.L1, g.L2};
-    long long stride = 1;
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const bool edge = fwd ? (j[a] + 1 == L[a]) : (j[a] == 0);
-        const int jn = fwd ? (edge ? 0 : j[a] + 1) : (edge ? L[a] - 1 : j[a] - 1);
-        st.o[a] = (long long)(jn - j[a]) * stride;
-        st.s[a] = make_sel(g.bc[a], edge);
-        stride *= L[a];
-    }
-    return st;
+    return Near{F[i1], F[i2], F[i2 + o1], F[i1 + o2]};
 }
 
-/* Half curls of the main array F ([3][n3]) at cell l.  pl[c]: the term
- * differentiated along axis c+1 ("+" half), mi[c]: along axis c+2. */
+/* The half curls from them.  pl: the term differentiated along axis a1 ("+"
+ * half), mi: along a2; wrap: a neighbour lies across a face, with its
+ * boundary factor s1, s2. */
 template <bool FWD>
-__device__ __forceinline__ void curl_main(const double *__restrict__ F, long long n3, long long l,
-                                          const Stn &st, double pl[3], double mi[3])
+__device__ __forceinline__ void curl_near(Near v, bool wrap, Sel s1, Sel s2, double &pl, double &mi)
 {
-    const double h0 = F[l], h1 = F[n3 + l], h2 = F[2 * n3 + l];
-    const double here[3] = {h0, h1, h2};
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        const int a1 = (c + 1) % 3, a2 = (c + 2) % 3;
-        const double n2 = bmul(F[a2 * n3 + l + st.o[a1]], st.s[a1]);
-        const double n1 = bmul(F[a1 * n3 + l + st.o[a2]], st.s[a2]);
-        if (!FWD) {
-            pl[c] = here[a2] - n2; /* +E - Bp*E(j-1)   (:407) */
-            mi[c] = -here[a1] + n1; /* -E + Bp*E(j-1)  (:410) */
-        } else {
-            pl[c] = n2 - here[a2]; /* +Bp*H(j+1) - H   (:386) */
-            mi[c] = -n1 + here[a1]; /* -Bp*H(j+1) + H  (:389) */
-        }
+    if (__any_sync(__activemask(), wrap)) {
+        v.n2 = bmul(v.n2, s1);
+        v.n1 = bmul(v.n1, s2);
     }
-}
-
-/* The same on the aux arrays through address_notn (ope_Rmap :330-350,
- * ope_Rdmap :351-371); Fa is [3][lnotn+1] with a zero sentinel. */
-template <bool FWD>
-__device__ __forceinline__ void curl_aux(const double *__restrict__ Fa, long long as, const int *__restrict__ addr,
-                                         long long l, const Stn &st, double pl[3], double mi[3])
-{
-    const int ah = addr[l];
-    const int an[3] = {addr[l + st.o[0]], addr[l + st.o[1]], addr[l + st.o[2]]};
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        const int a1 = (c + 1) % 3, a2 = (c + 2) % 3;
-        const double here2 = Fa[a2 * as + ah], here1 = Fa[a1 * as + ah];
-        const double n2 = bmul(Fa[a2 * as + an[a1]], st.s[a1]);
-        const double n1 = bmul(Fa[a1 * as + an[a2]], st.s[a2]);
-        if (!FWD) {
-            pl[c] = here2 - n2;
-            mi[c] = -here1 + n1;
-        } else {
-            pl[c] = n2 - here2;
-            mi[c] = -n1 + here1;
-        }
+    if (!FWD) {
+        pl = v.h2 - v.n2;  /* +E - Bp*E(j-1)   (:407) */
+        mi = -v.h1 + v.n1; /* -E + Bp*E(j-1)   (:410) */
+    } else {
+        pl = v.n2 - v.h2;  /* +Bp*H(j+1) - H   (:386) */
+        mi = -v.n1 + v.h1; /* -Bp*H(j+1) + H   (:389) */
     }
 }
 
@@ -122,183 +85,234 @@ __device__ __forceinline__ double sheet(const Src &s, int pl, int b, int k, bool
     return sc[0] * t;                                /* (2*env) * ... */
 }
 
-/* H sweep, main_calc :255-286 */
-__global__ void __launch_bounds__(128) k_h64(const P64 p, const int rel)
+/* A x for an update factor A = (a)(1/b) of main :118-127.  Where a == b (no
+ * loss, no stretch) that is x' * fl(1/x'), which rounds to 1 or to its
+ * predecessor 1 - 2^-53, by the division's last bit; and (1 - 2^-53) x rounds
+ * to the double next below |x| for every x above the smallest normal number
+ * (x - x 2^-53 lies more than half a unit of the last place below x, or at
+ * the next number itself where x is a power of two), to x for x at or below
+ * it, for zeros, infinities and NaNs.  So for those two factors the product
+ * is a subtraction on the bits, off the FP64 pipe. */
+__device__ __forceinline__ double amul(double A, double x)
 {
-    const int j0 = blockIdx.x * 32 + threadIdx.x, j1 = blockIdx.y * 4 + threadIdx.y, j2 = blockIdx.z;
-    const Geo &g = p.g;
-    if (j0 >= g.L0 || j1 >= g.L1) return;
-    const long long n3 = g.n3, l = j0 + (long long)g.L0 * (j1 + (long long)g.L1 * j2);
-    const uint8_t fl = p.flags[l];
-    const int cls = fl & 7;
-    if (cls == CLS_E) return; /* the H of an 'e' cell is never updated */
-    const Stn st = make_stn(g, j0, j1, j2, false);
-    const int k = *p.s.base + rel;
-    const long long as = p.lnotn + 1;
-    const double *Ah = p.cm, *Bh = p.cm + 3 * n3;
-    const double *Aha = p.ca, *Bha = p.ca + 3 * (long long)p.lnotn;
-    for (int b = 0; b < p.batch; b++) {
-        double *__restrict__ H = p.H + (long long)b * 3 * n3;
-        const double *__restrict__ E = p.E + (long long)b * 3 * n3;
-        double *__restrict__ Ha = p.Ha + (long long)b * 3 * as;
-        const double *__restrict__ Ea = p.Ea + (long long)b * 3 * as;
-        double pl[3], mi[3];
-        curl_main<false>(E, n3, l, st, pl, mi);
-        if (cls == CLS_N) {
-            double W[3] = {pl[0] + mi[0], pl[1] + mi[1], pl[2] + mi[2]};
-            if (j2 == p.s.iI[b]) {
-                const int px = j0 + g.L0 * j1;
-                W[0] += p.s.sgn[b] * sheet(p.s, g.pl, b, k, true, 1, px);
-                W[1] -= p.s.sgn[b] * sheet(p.s, g.pl, b, k, true, 0, px);
-            }
-            double h[3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) h[c] = Ah[c * n3 + l] * H[c * n3 + l] + Bh[c * n3 + l] * (-W[c]);
-            if (fl & FL_BWD) {
-                double pa[3], ma[3];
-                curl_aux<false>(Ea, as, p.addr, l, st, pa, ma);
-#pragma unroll
-                for (int c = 0; c < 3; c++) h[c] += Bh[c * n3 + l] * (-(pa[c] + ma[c]));
-            }
-#pragma unroll
-            for (int c = 0; c < 3; c++) H[c * n3 + l] = h[c];
-        } else if (cls == CLS_A) {
-            double pa[3], ma[3];
-            curl_aux<false>(Ea, as, p.addr, l, st, pa, ma);
-            const int a = p.addr[l];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                double h = Ah[c * n3 + l] * H[c * n3 + l] + Bh[c * n3 + l] * (-pl[c]);
-                h += Bh[c * n3 + l] * (-pa[c]);
-                H[c * n3 + l] = h;
-                double x = Aha[c * p.lnotn + a] * Ha[c * as + a] + Bha[c * p.lnotn + a] * (-mi[c]);
-                x += Bha[c * p.lnotn + a] * (-ma[c]);
-                Ha[c * as + a] = x;
-            }
-        } else { /* 'h' or 'b': stable form, main-array curl only (:277-283) */
-            const int a = p.addr[l];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const double W = pl[c] + mi[c];
-                double h = H[c * n3 + l];
-                double x = Ha[c * as + a];
-                h += 0.5 * x;
-                x = Aha[c * p.lnotn + a] * x + Bha[c * p.lnotn + a] * (-W);
-                h += 0.5 * x;
-                Ha[c * as + a] = x;
-                H[c * n3 + l] = h;
-            }
-        }
-    }
+    const unsigned long long near1 = (unsigned long long)__double_as_longlong(A) - 0x3fefffffffffffffull;
+    if (__any_sync(__activemask(), near1 > 1ull)) return A * x; /* a branch of the whole warp: no DMUL issued for it */
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x), lo = 0x0010000000000001ull;
+    const bool dec = near1 == 0ull && (u & 0x7fffffffffffffffull) - lo < 0x7ff0000000000000ull - lo;
+    return __longlong_as_double((long long)(u - (dec ? 1ull : 0ull)));
 }
 
-/* E sweep, main_calc :287-317 */
-__global__ void __launch_bounds__(128) k_e64(const P64 p, const int rel)
+/* a b rounded to nearest (ties to even) on the integer pipes: the 53 x 53-bit
+ * product of the mantissas, normalised by at most one place, rounded on its
+ * low 64 bits; operands and results outside the normal range go through the
+ * FP64 unit.  The same bits as a * b.  By itself 2.0 products a clock and SM
+ * against the FP64 pipe's 1.7, and beside it 2.7 operations where half are
+ * these products (measured): the update kernels send their products by B here
+ * and keep the FP64 pipe for the additions. */
+template <bool NEG = false> /* -a b: the sign bit (a negated double as an operand would cost a DADD) */
+__device__ __forceinline__ double imul(double a, double b)
 {
-    const int j0 = blockIdx.x * 32 + threadIdx.x, j1 = blockIdx.y * 4 + threadIdx.y, j2 = blockIdx.z;
-    const Geo &g = p.g;
-    if (j0 >= g.L0 || j1 >= g.L1) return;
-    const long long n3 = g.n3, l = j0 + (long long)g.L0 * (j1 + (long long)g.L1 * j2);
-    const uint8_t fl = p.flags[l];
-    const int cls = fl & 7;
-    if (cls == CLS_H) return; /* the E of an 'h' cell is never updated */
-    const bool stable = (cls == CLS_E || cls == CLS_B);
-    /* the stable form takes the BACKWARD difference of H (:310) */
-    const Stn st = make_stn(g, j0, j1, j2, !stable);
-    const int k = *p.s.base + rel;
-    const long long as = p.lnotn + 1;
-    const double *Ae = p.cm + 6 * n3, *Be = p.cm + 9 * n3;
-    const double *Aea = p.ca + 6 * (long long)p.lnotn, *Bea = p.ca + 9 * (long long)p.lnotn;
-    for (int b = 0; b < p.batch; b++) {
-        double *__restrict__ E = p.E + (long long)b * 3 * n3;
-        const double *__restrict__ H = p.H + (long long)b * 3 * n3;
-        double *__restrict__ Ea = p.Ea + (long long)b * 3 * as;
-        const double *__restrict__ Ha = p.Ha + (long long)b * 3 * as;
-        double pl[3], mi[3];
-        if (stable) {
-            curl_main<false>(H, n3, l, st, pl, mi);
-            const int a = p.addr[l];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const double W = pl[c] + mi[c];
-                double e = E[c * n3 + l];
-                double x = Ea[c * as + a];
-                e += 0.5 * x;
-                x = Aea[c * p.lnotn + a] * x + Bea[c * p.lnotn + a] * W;
-                e += 0.5 * x;
-                Ea[c * as + a] = x;
-                E[c * n3 + l] = e;
-            }
-            continue;
-        }
-        curl_main<true>(H, n3, l, st, pl, mi);
-        if (cls == CLS_N) {
-            double W[3] = {pl[0] + mi[0], pl[1] + mi[1], pl[2] + mi[2]};
-            if (j2 == p.s.iI[b]) {
-                const int px = j0 + g.L0 * j1;
-                W[0] += p.s.sgn[b] * sheet(p.s, g.pl, b, k, false, 1, px);
-                W[1] -= p.s.sgn[b] * sheet(p.s, g.pl, b, k, false, 0, px);
-            }
-            double e[3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) e[c] = Ae[c * n3 + l] * E[c * n3 + l] + Be[c * n3 + l] * W[c];
-            if (fl & FL_FWD) {
-                double pa[3], ma[3];
-                curl_aux<true>(Ha, as, p.addr, l, st, pa, ma);
-#pragma unroll
-                for (int c = 0; c < 3; c++) e[c] += Be[c * n3 + l] * (pa[c] + ma[c]);
-            }
-#pragma unroll
-            for (int c = 0; c < 3; c++) E[c * n3 + l] = e[c];
-        } else { /* 'a' */
-            double pa[3], ma[3];
-            curl_aux<true>(Ha, as, p.addr, l, st, pa, ma);
-            const int a = p.addr[l];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                double e = Ae[c * n3 + l] * E[c * n3 + l] + Be[c * n3 + l] * pl[c];
-                e += Be[c * n3 + l] * pa[c];
-                E[c * n3 + l] = e;
-                double x = Aea[c * p.lnotn + a] * Ea[c * as + a] + Bea[c * p.lnotn + a] * mi[c];
-                x += Bea[c * p.lnotn + a] * ma[c];
-                Ea[c * as + a] = x;
-            }
-        }
+    const unsigned ah = (unsigned)__double2hiint(a), bh = (unsigned)__double2hiint(b);
+    const unsigned ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
+    const unsigned long long ma = ((unsigned long long)((ah & 0xfffffu) | 0x100000u) << 32 | (unsigned)__double2loint(a)) << 11;
+    const unsigned long long mb = (unsigned long long)((bh & 0xfffffu) | 0x100000u) << 32 | (unsigned)__double2loint(b);
+    unsigned long long hi = __umul64hi(ma, mb), lo = ma * mb; /* hi in [2^51, 2^53) */
+    const unsigned up = (unsigned)(hi >> 52);
+    const unsigned e = ea + eb - 1024u + up; /* the biased exponent less one: hi's leading bit adds it */
+    if (!up) {
+        hi = hi << 1 | lo >> 63;
+        lo <<= 1;
     }
+    const unsigned r = (unsigned)(lo >> 63) & (unsigned)(((lo << 1) != 0) | ((unsigned)hi & 1u));
+    const unsigned sign = ((ah ^ bh) & 0x80000000u) ^ (NEG ? 0x80000000u : 0u);
+    if (ea - 1u >= 2046u || eb - 1u >= 2046u || e >= 2045u) {
+        /* zero times a finite number: fields that no wave has reached yet */
+        const bool za = ((ah << 1) | (unsigned)__double2loint(a)) == 0, zb = ((bh << 1) | (unsigned)__double2loint(b)) == 0;
+        if ((za && eb != 2047u) || (zb && ea != 2047u)) return __hiloint2double((int)sign, 0);
+        return NEG ? -(a * b) : a * b;
+    }
+    return __longlong_as_double((long long)(((unsigned long long)(sign + (e << 20)) << 32) + hi + r));
 }
 
-/* running DFT on the monitor planes (main_calc :318-328), FP64 accumulators.
- * acc += phase * x computed as (re += pr*x, im += pi*x), the value of the
- * reference's complex product with a real factor. */
-__global__ void k_dft64(const P64 p, const int rel)
+__device__ __forceinline__ int monitor_index64(const Dft &d, int j2)
 {
-    const int px = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y, b = blockIdx.z;
+    int q = -1;
+#pragma unroll
+    for (int i = 0; i < MAX_PLANES; i++)
+        if (i < d.nq && d.planes[i] == j2) q = i;
+    return q;
+}
+
+__device__ __forceinline__ double *ring64_at(const Dft &d, int pl, int b, int k, int q, int v)
+{
+    return d.ring64 + ((((long long)b * d.ringK + k % d.ringK) * d.nq + q) * 4 + v) * (long long)pl;
+}
+
+/* Component c of a cell of class 'h', 'e' or 'b' in a sweep: frozen (the H of
+ * an 'e' cell, the E of an 'h' cell), else the stable form, which reads the
+ * main array only and takes the backward difference also of H (:277-283,
+ * :308-314).  f: its main slot; returns the new one.  Out of line: such cells
+ * are rare. */
+template <bool EF>
+__device__ __noinline__ double metal_cell(const P64 &p, int cls, int b, int c, int j2, int px, double f)
+{
+    if (cls == (EF ? CLS_H : CLS_E)) return f;
     const Geo &g = p.g;
-    if (px >= g.pl) return;
-    const long long n3 = g.n3, off = (long long)p.d.planes[q] * g.pl + px;
-    const double *H = p.H + (long long)b * 3 * n3, *E = p.E + (long long)b * 3 * n3;
-    double x[4] = {H[off], H[n3 + off], E[off], E[n3 + off]};
-    if ((p.flags[off] & 7) == CLS_A) {
+    const int n3 = (int)g.n3, l = px + g.pl * j2, a = p.addr[l];
+    const int j[3] = {px % g.L0, px / g.L0, j2}, L[3] = {g.L0, g.L1, g.L2}, step[3] = {1, g.L0, g.pl};
+    int o[3];
+    Sel s[3];
+    bool wrap = false;
+    for (int x = 0; x < 3; x++) {
+        const bool e = j[x] == 0;
+        o[x] = (e ? L[x] - 1 : -1) * step[x];
+        s[x] = make_sel(g.bc[x], e);
+        wrap |= e;
+    }
+    const int a1 = (c + 1) % 3, a2 = (c + 2) % 3;
+    double pl, mi;
+    curl_near<false>(load_near((EF ? p.H : p.E) + (long long)b * 3 * n3, a1 * n3 + l, a2 * n3 + l, o[a1], o[a2]), wrap,
+                     s[a1], s[a2], pl, mi);
+    const double W = pl + mi;
+    double *x = (EF ? p.Ea : p.Ha) + ((long long)b * 3 + c) * n3 + l;
+    const double *ca = p.ca + (long long)(EF ? 6 + c : c) * p.lnotn + a;
+    double v = *x;
+    f += 0.5 * v;
+    v = ca[0] * v + ca[3LL * p.lnotn] * (EF ? W : -W);
+    f += 0.5 * v;
+    *x = v;
+    return f;
+}
+
+/* One sweep: EF = false H from E (main_calc :255-286), EF = true E from H
+ * (:287-317).
+ *
+ * Two things bound it.  The FP64 pipe runs 1.7 operations a clock and SM
+ * (measured), a warp's instruction holding it for 19 clocks however few of
+ * its lanes take part: an ordinary cell costs 12 additions, a split cell 26,
+ * an ordinary cell next to a split one 21 (products by B and A are taken off
+ * it, imul and amul).  So what counts is warps whose cells take one path: with
+ * 32 consecutive x in a warp every warp at an x face ran two or three paths;
+ * here the cells of a plane are taken in the order p.ord of the host: the
+ * columns x that lie in a PML, row by row, then the columns next to one in
+ * the direction of this sweep's differences, column by column, then the
+ * others, row by row.  And latency, of the loads and of the FP64 pipe (67
+ * clocks): a thread takes one component of a cell, a block's three warps the
+ * three components of 32 cells, which share the loaded lines in L1, so that
+ * 39 warps fit an SM where 16 of whole cells did; cells that the host knows
+ * to be split issue their aux loads with the others, before the class byte
+ * has come back; the aux slots are dense, so that no address is fetched
+ * first.  Excitations are fastest in the grid: the coefficients are shared
+ * through L2.
+ *
+ * Measured a sweep, against one thread per cell with 32 consecutive x a warp
+ * and every operation on the FP64 pipe: 96^3 cube (12-cell PML) 60 us, from
+ * 85; 130 x 98 x 81 bend, two excitations, 129 us, from 211 (70 % of the
+ * pipe's peak); 24 x 20 x 40 guide 3.2 us, from 5.  Blocks of 32 cells rather
+ * than 64 or 128: 3 % and 10 % on the cube, 10 % and 30 % on the guide, whose
+ * plane fills 15 of them.  13 resident blocks (48 registers): 10 and 15 are
+ * within 7 %, 17 spills. */
+template <bool EF>
+__global__ void __launch_bounds__(96, 13) k_sweep64(const P64 p, const int rel)
+{
+    const Geo &g = p.g;
+    const int b = blockIdx.x % p.batch, i = blockIdx.x / p.batch * 32 + threadIdx.x;
+    const int j2 = blockIdx.y, c = threadIdx.y;
+    if (i >= g.pl) return;
+    const int2 od = p.ord[(EF ? g.pl : 0) + i]; /* pixel; 1: wraps along x, 2: along y, 4: split */
+    const int px = od.x, n3 = (int)g.n3, l = px + g.pl * j2;
+    const bool sp = (od.y & 4) | p.smask[j2];
+    const bool ex = od.y & 1, ey = od.y & 2, ez = j2 == (EF ? g.L2 - 1 : 0);
+    const int sd = EF ? 1 : -1;
+    const int ox = ex ? -sd * (g.L0 - 1) : sd, oy = (ey ? -sd * (g.L1 - 1) : sd) * g.L0;
+    const int oz = (ez ? -sd * (g.L2 - 1) : sd) * g.pl;
+    /* axes a1 = c+1, a2 = c+2 */
+    const int o1 = c == 0 ? oy : c == 1 ? oz : ox, o2 = c == 0 ? oz : c == 1 ? ox : oy;
+    const bool w1 = c == 0 ? ey : c == 1 ? ez : ex, w2 = c == 0 ? ez : c == 1 ? ex : ey;
+    const Sel s1 = make_sel(g.bc[c == 2 ? 0 : c + 1], w1), s2 = make_sel(g.bc[c == 0 ? 2 : c - 1], w2);
+    const int i0 = c * n3 + l, i1 = (c == 2 ? 0 : c + 1) * n3 + l, i2 = (c == 0 ? 2 : c - 1) * n3 + l;
+    const long long bo = (long long)b * 3 * n3;
+    double *__restrict__ F = (EF ? p.E : p.H) + bo, *__restrict__ Fa = (EF ? p.Ea : p.Ha) + bo;
+    const double *__restrict__ G = (EF ? p.H : p.E) + bo, *__restrict__ Ga = (EF ? p.Ha : p.Ea) + bo;
+    const double *__restrict__ cm = p.cm + (EF ? 6 : 0) * g.n3, *__restrict__ ca = p.ca + (EF ? 6 + c : c) * (long long)p.lnotn;
+    const int fl = p.flags[l], cls = fl & 7;
+    const double A = cm[i0], B = cm[3 * g.n3 + i0];
+    double f = F[i0];
+    const Near v = load_near(G, i1, i2, o1, o2);
+    double fa = 0.0, Aa, Ba;
+    Near va;
+    auto load_aux = [&]() {
+        const int a = p.addr[l];
+        fa = Fa[i0];
+        Aa = ca[a];
+        Ba = ca[3LL * p.lnotn + a];
+        va = load_near(Ga, i1, i2, o1, o2);
+    };
+    if (sp) load_aux();
+    double pl, mi, pa, ma;
+    if (cls == CLS_N) {
+        curl_near<EF>(v, w1 | w2, s1, s2, pl, mi);
+        double W = pl + mi;
+        if (j2 == p.s.iI[b] && c < 2) {
+            const double t = p.s.sgn[b] * sheet(p.s, g.pl, b, *p.s.base + rel, !EF, 1 - c, px);
+            W = c == 0 ? W + t : W - t;
+        }
+        f = amul(A, f) + imul<!EF>(B, W);
+        if (fl & (EF ? FL_FWD : FL_BWD)) {
+            curl_near<EF>(load_near(Ga, i1, i2, o1, o2), w1 | w2, s1, s2, pa, ma);
+            f += imul<!EF>(B, pa + ma);
+        }
+    } else if (cls == CLS_A) {
+        if (!sp) load_aux();
+        curl_near<EF>(v, w1 | w2, s1, s2, pl, mi);
+        curl_near<EF>(va, w1 | w2, s1, s2, pa, ma);
+        const double h = amul(A, f) + imul<!EF>(B, pl);
+        f = h + imul<!EF>(B, pa);
+        const double x = amul(Aa, fa) + imul<!EF>(Ba, mi);
+        fa = x + imul<!EF>(Ba, ma);
+        Fa[i0] = fa;
+    } else {
+        f = metal_cell<EF>(p, cls, b, c, j2, px, f);
+    }
+    F[i0] = f;
+    const int q = monitor_index64(p.d, j2);
+    if (q >= 0 && c < 2) {
         /* a plane through the PML (allowed for general schedules only; the
-         * reference exits, :320): sample the total field main + aux */
-        const long long as = p.lnotn + 1, a = p.addr[off];
-        const double *Ha = p.Ha + (long long)b * 3 * as, *Ea = p.Ea + (long long)b * 3 * as;
-        x[0] += Ha[a];
-        x[1] += Ha[as + a];
-        x[2] += Ea[a];
-        x[3] += Ea[as + a];
+         * reference exits, :320) samples the total field main + aux */
+        ring64_at(p.d, g.pl, b, *p.s.base + rel, q, (EF ? 2 : 0) + c)[px] = cls == CLS_A ? f + fa : f;
     }
-    const int k = *p.s.base + rel;
-    for (int f = 0; f < p.d.nfreq; f++) {
-        const double *ph = p.d.xphase ? p.d.xphase : p.d.phase + 4 * ((long long)k * p.d.nfreq + f);
-        double *acc = p.d.acc + 2 * ((((long long)b * p.d.nfreq + f) * p.d.nq + q) * 4 * g.pl + px);
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-            const double pr = ph[v < 2 ? 0 : 2], pi = ph[v < 2 ? 1 : 3];
-            double *a = acc + 2 * (long long)v * g.pl;
-            a[0] += pr * x[v];
-            a[1] += pi * x[v];
+}
+
+/* running DFT on the monitor planes (main_calc :318-328), FP64 accumulators:
+ * the samples of `count` steps ending at *base + rel_end, from the ring the
+ * sweeps fill, folded in step by step.  acc += phase * x computed as (re +=
+ * pr*x, im += pi*x), the value of the reference's complex product with a real
+ * factor, in the reference's order: the same bits as one pass over the
+ * accumulators every step, at 1/32 of their traffic and launches.  A thread
+ * takes one pixel and component of one plane and excitation and every
+ * gridDim.z / batch-th frequency.  96^3 cube, 11 wavelengths, 2 planes: 6.6 us
+ * a step (half of it the FP64 pipe's additions), from 32 us. */
+__global__ void __launch_bounds__(128) k_flush64(const P64 p, const int rel_end, const int count)
+{
+    const int px = blockIdx.x * 128 + threadIdx.x, q = blockIdx.y >> 2, v = blockIdx.y & 3;
+    const int b = blockIdx.z % p.batch, f0 = blockIdx.z / p.batch, nf = gridDim.z / p.batch;
+    const Geo &g = p.g;
+    const Dft &d = p.d;
+    if (px >= g.pl) return;
+    const int k0 = *p.s.base + rel_end - count;
+    const int qs = monitor_index64(d, d.planes[q]); /* the slot the sweeps fill, where a plane is listed twice */
+    for (int f = f0; f < d.nfreq; f += nf) {
+        double *acc = d.acc + 2 * (((((long long)b * d.nfreq + f) * d.nq + q) * 4 + v) * g.pl + px);
+        double re = acc[0], im = acc[1];
+#pragma unroll 4
+        for (int s = 0; s < count; s++) {
+            const double x = ring64_at(d, g.pl, b, k0 + s, qs, v)[px];
+            const double *ph = (d.xphase ? d.xphase : d.phase + 4 * ((long long)(k0 + s) * d.nfreq + f)) + (v < 2 ? 0 : 2);
+            re += imul(ph[0], x);
+            im += imul(ph[1], x);
         }
+        acc[0] = re;
+        acc[1] = im;
     }
 }
 
@@ -328,23 +342,24 @@ __global__ void k_maxabs(const void *x, long long n, int is_double, unsigned lon
     if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
-void launch_h64(const P64 &p, int rel, cudaStream_t st)
+template <bool EF> static void launch_sweep64(const P64 &p, int rel, cudaStream_t st)
 {
-    dim3 blk(32, 4, 1), grd((p.g.L0 + 31) / 32, (p.g.L1 + 3) / 4, p.g.L2);
-    k_h64<<<grd, blk, 0, st>>>(p, rel);
+    k_sweep64<EF><<<dim3((p.g.pl + 31) / 32 * p.batch, p.g.L2), dim3(32, 3), 0, st>>>(p, rel);
 }
 
-void launch_e64(const P64 &p, int rel, cudaStream_t st)
-{
-    dim3 blk(32, 4, 1), grd((p.g.L0 + 31) / 32, (p.g.L1 + 3) / 4, p.g.L2);
-    k_e64<<<grd, blk, 0, st>>>(p, rel);
-}
+void launch_h64(const P64 &p, int rel, cudaStream_t st) { launch_sweep64<false>(p, rel, st); }
 
-void launch_dft64(const P64 &p, int rel, cudaStream_t st)
+void launch_e64(const P64 &p, int rel, cudaStream_t st) { launch_sweep64<true>(p, rel, st); }
+
+/* the frequencies are spread over as many threads as fill the GPU's warps
+ * (a chain of two operations a step and frequency, 67 clocks each) */
+void launch_flush64(const P64 &p, int rel_end, int count, cudaStream_t st)
 {
-    if (p.d.nfreq <= 0 || p.d.nq <= 0) return;
-    dim3 blk(256), grd((p.g.pl + 255) / 256, p.d.nq, p.batch);
-    k_dft64<<<grd, blk, 0, st>>>(p, rel);
+    if (p.d.nfreq <= 0 || p.d.nq <= 0 || count <= 0) return;
+    const int nb = (p.g.pl + 127) / 128, used = nb * p.d.nq * 4 * p.batch;
+    int nf = used >= 1824 ? 1 : (1824 + used - 1) / used; /* 152 SMs x 12 blocks */
+    if (nf > p.d.nfreq) nf = p.d.nfreq;
+    k_flush64<<<dim3(nb, p.d.nq * 4, p.batch * nf), 128, 0, st>>>(p, rel_end, count);
 }
 
 void launch_bump(int *base, int by, cudaStream_t st) { k_bump<<<1, 1, 0, st>>>(base, by); }

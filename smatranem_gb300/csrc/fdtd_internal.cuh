@@ -8,8 +8,7 @@
  *
  *   FP64 (bit-identical path, the reference's representation):
  *     H, E   [3][L3D] doubles    main slot (total field of ordinary cells)
- *     Ha, Ea [3][Lnotn+1]        aux slot of each non-'n' cell, compact in
- *                                 address_notn order, then a zero sentinel
+ *     Ha, Ea [3][L3D]            aux slot of each non-'n' cell, zero elsewhere
  *     coefficients: main [4][3][L3D] (Ah, Bh, Ae, Be), aux [4][3][Lnotn]
  *     flags  [L3D] bytes: cell class + "a neighbour has an aux slot" bits
  *
@@ -64,8 +63,9 @@ struct Dft {
     const double *xphase; /* explicit {pH, pE} for smat_fdtd_step, or null */
     const float *xphase32; /* the same pairs of the explicit phases, [H, E][4] */
     double *acc;          /* [batch][nfreq][nq][4][pl] complex */
-    int ringK;            /* FP32: samples kept per flush */
+    int ringK;            /* samples kept per flush */
     float *ring;          /* FP32: [batch][ringK][nq][4][pl] */
+    double *ring64;       /* FP64: the same */
 };
 
 struct P64 {
@@ -76,7 +76,12 @@ struct P64 {
     const double *cm; /* [4][3][n3] */
     const double *ca; /* [4][3][lnotn] */
     double *H, *E;    /* [batch][3][n3] */
-    double *Ha, *Ea;  /* [batch][3][lnotn+1] */
+    double *Ha, *Ea;  /* [batch][3][n3], zero where a cell has no aux slot */
+    /* [2][pl]: the order in which the H and the E sweep take the pixels of a
+     * plane, each with what the sweep needs to know of it: 1, 2: its neighbour
+     * along x, y wraps, 4: no cell of its x or of its y is an ordinary one */
+    const int2 *ord;
+    const uint8_t *smask; /* [L2]: no cell of the plane is an ordinary one */
     Src s;
     Dft d;
 };
@@ -235,7 +240,7 @@ __device__ __forceinline__ void curl32(const Get &get, const Stn32 &st, float pl
 /* launchers (one translation unit per precision) */
 void launch_h64(const P64 &p, int rel, cudaStream_t st);
 void launch_e64(const P64 &p, int rel, cudaStream_t st);
-void launch_dft64(const P64 &p, int rel, cudaStream_t st);
+void launch_flush64(const P64 &p, int rel_end, int count, cudaStream_t st);
 void launch_h32(const P32 &p, int rel, int by, int z0, int z1, cudaStream_t st);
 void launch_e32(const P32 &p, int rel, int by, int z0, int z1, cudaStream_t st);
 void launch_flush32(const P32 &p, int rel_end, int count, cudaStream_t st);

@@ -56,6 +56,7 @@ Dft make_dft(const smat_fdtd_plan *p, bool explicit_phase)
     d.acc = p->d_acc;
     d.ringK = RING_K;
     d.ring = p->d_ring;
+    d.ring64 = p->d_ring64;
     return d;
 }
 
@@ -79,6 +80,8 @@ P64 make_p64(const smat_fdtd_plan *p, bool xp)
     q.lnotn = p->lnotn;
     q.flags = p->d_flags;
     q.addr = p->d_addr;
+    q.ord = p->d_ord;
+    q.smask = p->d_smask;
     q.cm = p->d_cm;
     q.ca = p->d_ca;
     q.H = p->d_H64;
@@ -159,8 +162,8 @@ void enqueue_steps(smat_fdtd_plan *p, int rel0, int n, bool xp)
         for (int i = 0; i < n; i++) {
             launch_h64(q, rel0 + i, p->stream);
             launch_e64(q, rel0 + i, p->stream);
-            launch_dft64(q, rel0 + i, p->stream);
         }
+        launch_flush64(q, rel0 + n, n, p->stream);
     } else if (p->fused == 6) {
         for (int i = 0; i < n; i++) launch_row_step(p, xp, rel0 + i, p->stream);
         launch_flush32(make_p32(p, xp), rel0 + n, n, p->stream);
@@ -297,7 +300,7 @@ int check_planes(const smat_fdtd_plan *p, int nq, const int *planes)
     return SMAT_OK;
 }
 
-/* (re)allocate DFT accumulators and the FP32 ring for nfreq x nq planes */
+/* (re)allocate DFT accumulators and the sample ring for nfreq x nq planes */
 int setup_dft(smat_fdtd_plan *p, int nfreq, int nq, const int *planes)
 {
     if (nq > MAX_PLANES) return smat_fail(SMAT_EINVAL, "at most %d monitor planes", MAX_PLANES);
@@ -307,9 +310,9 @@ int setup_dft(smat_fdtd_plan *p, int nfreq, int nq, const int *planes)
             return smat_fail(SMAT_EINVAL, "monitor plane %d outside 0..%d", planes[q], p->L[2] - 1);
     drop_graph(p);
     const size_t acc_n = (size_t)p->batch * nfreq * nq * 4 * p->pl * 2;
-    const size_t ring_n = p->precision == SMAT_FP32 ? (size_t)p->batch * RING_K * nq * 4 * p->pl : 0;
+    const size_t ring_n = (size_t)p->batch * RING_K * nq * 4 * p->pl;
     const size_t old_acc = (size_t)p->batch * p->nfreq * p->nq * 4 * p->pl * 2;
-    const size_t old_ring = p->precision == SMAT_FP32 ? (size_t)p->batch * RING_K * p->nq * 4 * p->pl : 0;
+    const size_t old_ring = (size_t)p->batch * RING_K * p->nq * 4 * p->pl;
     if (acc_n != old_acc || !p->d_acc) {
         if (p->d_acc) cudaFree(p->d_acc), p->dev_bytes -= old_acc * 8;
         p->d_acc = nullptr;
@@ -319,13 +322,20 @@ int setup_dft(smat_fdtd_plan *p, int nfreq, int nq, const int *planes)
             p->dev_bytes += acc_n * 8;
         }
     }
-    if (ring_n != old_ring || (!p->d_ring && ring_n)) {
-        if (p->d_ring) cudaFree(p->d_ring), p->dev_bytes -= old_ring * 4;
+    const bool f64 = p->precision == SMAT_FP64;
+    const size_t rs = f64 ? sizeof(double) : sizeof(float);
+    if (ring_n != old_ring || (!p->d_ring && !p->d_ring64 && ring_n)) {
+        if (p->d_ring || p->d_ring64) {
+            cudaFree(p->d_ring);
+            cudaFree(p->d_ring64);
+            p->dev_bytes -= old_ring * rs;
+        }
         p->d_ring = nullptr;
+        p->d_ring64 = nullptr;
         if (ring_n) {
-            rc = dalloc(&p->d_ring, ring_n, p->stream);
+            rc = f64 ? dalloc(&p->d_ring64, ring_n, p->stream) : dalloc(&p->d_ring, ring_n, p->stream);
             if (rc) return rc;
-            p->dev_bytes += ring_n * 4;
+            p->dev_bytes += ring_n * rs;
         }
     }
     p->nfreq = nfreq;
@@ -415,13 +425,47 @@ int upload_f64(smat_fdtd_plan *p, const double *Ah, const double *Bh, const doub
     const int ln = p->lnotn;
     std::vector<uint8_t> fl;
     build_flags(p, fl);
+    /* the sweeps' pixel order: columns x in a PML (no cell of them is an
+     * ordinary one) row by row; those whose neighbour in the sweep's direction
+     * is such a column, column by column; the others, row by row */
+    const int L0 = p->L[0], L1 = p->L[1], L2 = p->L[2];
+    std::vector<uint8_t> sx(L0, 1), sy(L1, 1), sz(L2, 1);
+    {
+        long long l = 0;
+        for (int z = 0; z < L2; z++)
+            for (int y = 0; y < L1; y++)
+                for (int x = 0; x < L0; x++, l++)
+                    if (p->cont[l] == 'n') sx[x] = sy[y] = sz[z] = 0;
+    }
+    std::vector<int2> ord;
+    ord.reserve(2 * (size_t)p->pl);
+    for (int ef = 0; ef < 2; ef++) {
+        std::vector<int> cols[3];
+        for (int x = 0; x < L0; x++) {
+            const int xn = ef ? (x + 1 == L0 ? 0 : x + 1) : (x == 0 ? L0 - 1 : x - 1);
+            cols[sx[x] ? 0 : sx[xn] ? 1 : 2].push_back(x);
+        }
+        auto put = [&](int x, int y) {
+            const int wx = x == (ef ? L0 - 1 : 0), wy = y == (ef ? L1 - 1 : 0);
+            ord.push_back(make_int2(x + L0 * y, wx | wy << 1 | (sx[x] || sy[y]) << 2));
+        };
+        for (int y = 0; y < L1; y++)
+            for (int x : cols[0]) put(x, y);
+        for (int x : cols[1])
+            for (int y = 0; y < L1; y++) put(x, y);
+        for (int y = 0; y < L1; y++)
+            for (int x : cols[2]) put(x, y);
+    }
+    if ((rc = p->alloc(&p->d_ord, ord.size())) || (rc = p->alloc(&p->d_smask, sz.size()))) return rc;
+    CK(p->cpy(p->d_ord, ord.data(), ord.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    CK(p->cpy(p->d_smask, sz.data(), sz.size(), cudaMemcpyHostToDevice));
     if ((rc = p->alloc(&p->d_flags, n3))) return rc;
     if ((rc = p->alloc(&p->d_addr, n3))) return rc;
     if ((rc = p->alloc(&p->d_cm, 12 * (size_t)n3))) return rc;
     if ((rc = p->alloc(&p->d_ca, 12 * (size_t)ln))) return rc;
-    const size_t fs = (size_t)p->batch * 3 * n3, as = (size_t)p->batch * 3 * (ln + 1);
+    const size_t fs = (size_t)p->batch * 3 * n3;
     if ((rc = p->alloc(&p->d_H64, fs)) || (rc = p->alloc(&p->d_E64, fs))) return rc;
-    if ((rc = p->alloc(&p->d_Ha64, as)) || (rc = p->alloc(&p->d_Ea64, as))) return rc;
+    if ((rc = p->alloc(&p->d_Ha64, fs)) || (rc = p->alloc(&p->d_Ea64, fs))) return rc;
     std::vector<double> cm(12 * (size_t)n3), ca(12 * (size_t)ln);
     const double *src[4] = {Ah, Bh, Ae, Be};
     for (int w = 0; w < 4; w++)
@@ -758,6 +802,7 @@ extern "C" int smat_fdtd_destroy(smat_fdtd_plan *p)
     for (void *a : p->allocations) cudaFree(a);
     if (p->d_acc) cudaFree(p->d_acc);
     if (p->d_ring) cudaFree(p->d_ring);
+    if (p->d_ring64) cudaFree(p->d_ring64);
     if (p->d_sched) cudaFree(p->d_sched);
     if (p->d_phase) cudaFree(p->d_phase);
     if (p->d_phase32) cudaFree(p->d_phase32);
@@ -783,17 +828,17 @@ extern "C" int smat_fdtd_set_fields(smat_fdtd_plan *p, int b, const double *H_t,
     smat_clear_error();
     if (!p || !H_t || !E_t || b < 0 || b >= p->batch) return smat_fail(SMAT_EINVAL, "set_fields: bad arguments");
     const long long n3 = p->n3;
-    const int ln = p->lnotn;
     for (int w = 0; w < 2; w++) {
         const double *src = w ? E_t : H_t;
         if (p->precision == SMAT_FP64) {
-            std::vector<double> m(3 * n3), a(3 * (size_t)(ln + 1), 0.0);
-            for (int c = 0; c < 3; c++) {
-                for (long long l = 0; l < n3; l++) m[c * n3 + l] = src[c + 3 * l];
-                for (int x = 0; x <= ln; x++) a[(size_t)c * (ln + 1) + x] = src[c + 3 * (n3 + x)];
-            }
+            std::vector<double> m(3 * n3), a(3 * n3, 0.0);
+            for (int c = 0; c < 3; c++)
+                for (long long l = 0; l < n3; l++) {
+                    m[c * n3 + l] = src[c + 3 * l];
+                    if (p->cont[l] != 'n') a[c * n3 + l] = src[c + 3 * (n3 + p->addr[l])];
+                }
             double *dm = (w ? p->d_E64 : p->d_H64) + (size_t)b * 3 * n3;
-            double *da = (w ? p->d_Ea64 : p->d_Ha64) + (size_t)b * 3 * (ln + 1);
+            double *da = (w ? p->d_Ea64 : p->d_Ha64) + (size_t)b * 3 * n3;
             CK(p->cpy(dm, m.data(), m.size() * 8, cudaMemcpyHostToDevice));
             CK(p->cpy(da, a.data(), a.size() * 8, cudaMemcpyHostToDevice));
             CK(cudaStreamSynchronize(p->stream));
@@ -827,15 +872,18 @@ extern "C" int smat_fdtd_get_fields(smat_fdtd_plan *p, int b, double *H_t, doubl
         double *dst = w ? E_t : H_t;
         if (!dst) continue;
         if (p->precision == SMAT_FP64) {
-            std::vector<double> m(3 * n3), a(3 * (size_t)(ln + 1));
+            std::vector<double> m(3 * n3), a(3 * n3);
             const double *dm = (w ? p->d_E64 : p->d_H64) + (size_t)b * 3 * n3;
-            const double *da = (w ? p->d_Ea64 : p->d_Ha64) + (size_t)b * 3 * (ln + 1);
+            const double *da = (w ? p->d_Ea64 : p->d_Ha64) + (size_t)b * 3 * n3;
             CK(p->cpy(m.data(), dm, m.size() * 8, cudaMemcpyDeviceToHost));
             CK(p->cpy(a.data(), da, a.size() * 8, cudaMemcpyDeviceToHost));
             CK(cudaStreamSynchronize(p->stream));
             for (int c = 0; c < 3; c++) {
-                for (long long l = 0; l < n3; l++) dst[c + 3 * l] = m[c * n3 + l];
-                for (int x = 0; x <= ln; x++) dst[c + 3 * (n3 + x)] = a[(size_t)c * (ln + 1) + x];
+                for (long long l = 0; l < n3; l++) {
+                    dst[c + 3 * l] = m[c * n3 + l];
+                    if (p->cont[l] != 'n') dst[c + 3 * (n3 + p->addr[l])] = a[c * n3 + l];
+                }
+                dst[c + 3 * (n3 + ln)] = 0.0; /* the sentinel */
             }
         } else {
             std::vector<float> t(3 * n3), a(3 * n3);
@@ -1052,10 +1100,10 @@ extern "C" int smat_fdtd_time_kernels(smat_fdtd_plan *p, int k_begin, int nsteps
             launch_e32v(q32, i, p->by32, p->sweep_mb, 0, p->L[2], p->d_egen, p->negen, p->stream);
         else if (p->fused == 0) launch_e32(q32, i, p->by32, 0, p->L[2], p->stream);
         CK(cudaEventRecord(ev[2], p->stream));
-        if (p->precision == SMAT_FP64) launch_dft64(q64, i, p->stream);
-        else if ((i + 1) % RING_K == 0 || i + 1 == nsteps) {
+        if ((i + 1) % RING_K == 0 || i + 1 == nsteps) {
             const int cnt = (i + 1) % RING_K == 0 ? RING_K : (i + 1) % RING_K;
-            launch_flush32(make_p32(p, false), i + 1, cnt, p->stream);
+            if (p->precision == SMAT_FP64) launch_flush64(q64, i + 1, cnt, p->stream);
+            else launch_flush32(make_p32(p, false), i + 1, cnt, p->stream);
         }
         CK(cudaEventRecord(ev[3], p->stream));
         CK(cudaEventSynchronize(ev[3]));
@@ -1348,11 +1396,10 @@ extern "C" int smat_fdtd_check_finite(smat_fdtd_plan *p, int *finite, double *ma
     CK(cudaMemsetAsync(p->d_scratch, 0, 8, p->stream));
     const bool d = p->precision == SMAT_FP64;
     const long long nf = (long long)p->batch * 3 * p->n3;
-    const long long na = d ? (long long)p->batch * 3 * (p->lnotn + 1) : nf;
     const P32 q = make_p32(p, false);
     const void *arr[4] = {d ? (void *)p->d_H64 : (void *)q.H, d ? (void *)p->d_E64 : (void *)q.E,
                           d ? (void *)p->d_Ha64 : (void *)q.Ha, d ? (void *)p->d_Ea64 : (void *)q.Ea};
-    for (int i = 0; i < 4; i++) launch_maxabs(arr[i], i < 2 ? nf : na, d, p->d_scratch, p->stream);
+    for (int i = 0; i < 4; i++) launch_maxabs(arr[i], nf, d, p->d_scratch, p->stream);
     unsigned long long bits = 0;
     CK(p->cpy(&bits, p->d_scratch, 8, cudaMemcpyDeviceToHost));
     CK(cudaStreamSynchronize(p->stream));
@@ -1399,28 +1446,61 @@ struct StateHeader {
 
 constexpr char STATE_MAGIC[8] = {'S', 'M', 'A', 'T', 'S', 'T', 'A', 'T'};
 
+/* a device array of a plan's state; compact: FP64 aux slots, dense on the
+ * device, are [batch][3][lnotn + 1] in the file (address_notn order, then a
+ * zero) */
+struct StateArray {
+    void *dev;
+    size_t bytes;
+    bool compact;
+};
+
 /* the device arrays that hold a plan's state, in file order */
-std::vector<std::pair<void *, size_t>> state_arrays(smat_fdtd_plan *p)
+std::vector<StateArray> state_arrays(smat_fdtd_plan *p)
 {
-    std::vector<std::pair<void *, size_t>> a;
+    std::vector<StateArray> a;
     const size_t b = (size_t)p->batch, n3 = (size_t)p->n3;
     if (p->precision == SMAT_FP64) {
-        const size_t main = b * 3 * n3 * 8, aux = b * 3 * ((size_t)p->lnotn + 1) * 8;
-        a.push_back({p->d_H64, main});
-        a.push_back({p->d_E64, main});
-        a.push_back({p->d_Ha64, aux});
-        a.push_back({p->d_Ea64, aux});
+        const size_t f = b * 3 * n3 * 8;
+        a.push_back({p->d_H64, f, false});
+        a.push_back({p->d_E64, f, false});
+        a.push_back({p->d_Ha64, f, true});
+        a.push_back({p->d_Ea64, f, true});
     } else {
         const P32 q = make_p32(p, false);
         const size_t f = b * 3 * n3 * 4;
-        a.push_back({q.H, f});
-        a.push_back({q.E, f});
-        a.push_back({q.Ha, f});
-        a.push_back({q.Ea, f});
+        a.push_back({q.H, f, false});
+        a.push_back({q.E, f, false});
+        a.push_back({q.Ha, f, false});
+        a.push_back({q.Ea, f, false});
     }
     if (p->d_acc && p->nq > 0 && p->nfreq > 0)
-        a.push_back({p->d_acc, b * (size_t)p->nfreq * p->nq * 4 * (size_t)p->pl * 16});
+        a.push_back({p->d_acc, b * (size_t)p->nfreq * p->nq * 4 * (size_t)p->pl * 16, false});
     return a;
+}
+
+/* bytes of a state array in the file */
+size_t file_bytes(const smat_fdtd_plan *p, const StateArray &a)
+{
+    return a.compact ? (size_t)p->batch * 3 * ((size_t)p->lnotn + 1) * 8 : a.bytes;
+}
+
+/* the aux slots between their dense and their compact form */
+void aux_compact(const smat_fdtd_plan *p, const double *dense, double *compact)
+{
+    for (size_t r = 0; r < (size_t)p->batch * 3; r++) {
+        double *c = compact + r * ((size_t)p->lnotn + 1);
+        for (long long l = 0; l < p->n3; l++)
+            if (p->cont[l] != 'n') c[p->addr[l]] = dense[r * p->n3 + l];
+        c[p->lnotn] = 0.0;
+    }
+}
+
+void aux_dense(const smat_fdtd_plan *p, const double *compact, double *dense)
+{
+    for (size_t r = 0; r < (size_t)p->batch * 3; r++)
+        for (long long l = 0; l < p->n3; l++)
+            dense[r * p->n3 + l] = p->cont[l] != 'n' ? compact[r * ((size_t)p->lnotn + 1) + p->addr[l]] : 0.0;
 }
 
 void fill_header(const smat_fdtd_plan *p, StateHeader &h)
@@ -1449,16 +1529,22 @@ extern "C" int smat_fdtd_save_state(smat_fdtd_plan *p, const char *path)
     FILE *f = fopen(path, "wb");
     if (!f) return smat_fail(SMAT_EINVAL, "save_state: cannot open %s", path);
     int rc = fwrite(&h, sizeof h, 1, f) == 1 ? SMAT_OK : smat_fail(SMAT_EINVAL, "save_state: write error");
-    std::vector<char> buf;
+    std::vector<char> buf, file;
     for (const auto &a : state_arrays(p)) {
         if (rc) break;
-        buf.resize(a.second);
-        p->d2h_bytes += (long long)a.second;
-        if (cudaMemcpy(buf.data(), a.first, a.second, cudaMemcpyDeviceToHost) != cudaSuccess) {
+        buf.resize(a.bytes);
+        p->d2h_bytes += (long long)a.bytes;
+        if (cudaMemcpy(buf.data(), a.dev, a.bytes, cudaMemcpyDeviceToHost) != cudaSuccess) {
             rc = cuda_fail(cudaGetLastError(), "save_state: copy");
             break;
         }
-        if (fwrite(buf.data(), 1, a.second, f) != a.second) rc = smat_fail(SMAT_EINVAL, "save_state: write error");
+        const size_t n = file_bytes(p, a);
+        if (a.compact) {
+            file.resize(n);
+            aux_compact(p, (const double *)buf.data(), (double *)file.data());
+        }
+        if (fwrite(a.compact ? file.data() : buf.data(), 1, n, f) != n)
+            rc = smat_fail(SMAT_EINVAL, "save_state: write error");
     }
     if (fclose(f) != 0 && !rc) rc = smat_fail(SMAT_EINVAL, "save_state: write error");
     return rc;
@@ -1485,16 +1571,19 @@ extern "C" int smat_fdtd_load_state(smat_fdtd_plan *p, const char *path)
     /* FP32: into the field set it was saved from, so that a run continues with
      * the same set parity (and so the same grouping of the DFT ring's sums) */
     if (!rc && p->precision == SMAT_FP32) p->cur = h.cur;
-    std::vector<char> buf;
+    std::vector<char> buf, file;
     for (const auto &a : state_arrays(p)) {
         if (rc) break;
-        buf.resize(a.second);
-        if (fread(buf.data(), 1, a.second, f) != a.second) {
+        const size_t n = file_bytes(p, a);
+        buf.resize(a.bytes);
+        if (a.compact) file.resize(n);
+        if (fread(a.compact ? file.data() : buf.data(), 1, n, f) != n) {
             rc = smat_fail(SMAT_EINVAL, "load_state: %s is truncated", path);
             break;
         }
-        p->h2d_bytes += (long long)a.second;
-        if (cudaMemcpy(a.first, buf.data(), a.second, cudaMemcpyHostToDevice) != cudaSuccess)
+        if (a.compact) aux_dense(p, (const double *)file.data(), (double *)buf.data());
+        p->h2d_bytes += (long long)a.bytes;
+        if (cudaMemcpy(a.dev, buf.data(), a.bytes, cudaMemcpyHostToDevice) != cudaSuccess)
             rc = cuda_fail(cudaGetLastError(), "load_state: copy");
     }
     if (!rc && fgetc(f) != EOF) rc = smat_fail(SMAT_EINVAL, "load_state: %s has trailing data", path);

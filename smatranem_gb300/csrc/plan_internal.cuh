@@ -75,6 +75,7 @@ struct smat_fdtd_plan {
     float *d_phase32 = nullptr;
     double *d_acc = nullptr;   /* [batch][nfreq][nq][4][pl] complex */
     float *d_ring = nullptr;
+    double *d_ring64 = nullptr;
     int nfreq = 0, nq = 0, planes[smat::MAX_PLANES] = {0};
     bool ref_dft = false;      /* DFT slot 0 on planes (iB, iT) is the reference one */
     bool ref_planes_ok = false; /* no PML cell on iB, iT (else the reference exits, :320) */
@@ -86,6 +87,8 @@ struct smat_fdtd_plan {
     /* FP64 */
     uint8_t *d_flags = nullptr;
     int *d_addr = nullptr;
+    int2 *d_ord = nullptr; /* [2][pl] pixel order of the two sweeps */
+    uint8_t *d_smask = nullptr;
     double *d_cm = nullptr, *d_ca = nullptr;
     double *d_H64 = nullptr, *d_E64 = nullptr, *d_Ha64 = nullptr, *d_Ea64 = nullptr;
 

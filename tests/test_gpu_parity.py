@@ -798,3 +798,46 @@ def test_fp32_dft_flush_is_compensated(built, runs):
     u = 2.0 ** -24
     assert np.max(err / scale) < 2 * u
     assert np.sqrt(np.mean(err ** 2)) < 0.5 * np.sqrt(np.mean(err_plain ** 2))
+
+
+@pytest.mark.parametrize("L,pml", [((5, 4, 6, 1), (1, 1, 1)), ((33, 3, 7, 1), (2, 0, 2)), ((64, 5, 6, 1), (3, 1, 1)),
+                                   ((31, 9, 5, 1), (0, 2, 1)), ((1, 8, 12, 2), (0, 2, 3)), ((9, 1, 12, 2), (2, 0, 3))])
+@pytest.mark.parametrize("scale", [1e-2, 1e-305, 1e290])
+def test_fp64_sweeps_bit_identical_at_edges(built, port, L, pml, scale):
+    """The FP64 sweeps (cells ordered by class, products on the integer pipes)
+    against the oracle, bit for bit: planes around the 32-cell blocks, one-cell
+    axes, PML on some axes only, lossy cells (update factors other than 1),
+    and fields near both ends of the exponent range, where products leave the
+    normal numbers.  The DFT, 35 steps (a full and a partial window) with one
+    plane listed twice, against numpy in step order."""
+    f = _fdtd()
+    from smatranem_gb300 import workloads as W
+    s = W.random_structure(L, seed=sum(L), pml=pml, lossy=0.1, iBc=(1, -1, 0))
+    pr = W.prepare(s)
+    H0, E0 = W.random_fields(s.n3, pr.lnotn, seed=3, scale=scale)
+    Ah, Bh, Ae, Be = pr.coefficients()
+    pl, iBTIin, n = L[0] * L[1], (L[2] // 2, L[2] // 2, L[2] // 2, 1), 35
+    Hinc, Einc = (a * scale for a in W.random_incident(pl, seed=2))
+    src, ph = (a[:n] for a in f.cw_schedule(pr.n2pi, (1, 1, 3)))
+    with f.Plan.create(L, s.iBc, iBTIin, pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma) as p:
+        p.set_fields(0, H0, E0)
+        p.set_incident(0, Hinc, Einc)
+        p.set_schedule(src, planes=(iBTIin[0], iBTIin[0]), phase=ph)
+        p.run(0, n)
+        got, dft = p.get_fields(0), [p.get_dft(0, 0, q) for q in range(2)]
+    H, E = H0.copy(), E0.copy()
+    mons = [np.zeros(2 * pl, np.complex128) for _ in range(4)]
+    re, im = np.zeros((4, pl)), np.zeros((4, pl))
+    z = slice(pl * iBTIin[0], pl * (iBTIin[0] + 1))
+    split = pr.cont[z] == ord("a")
+    for k in range(n):
+        port.time_loop(L, Ah, Bh, Ae, Be, s.iBc, H, E, iBTIin, Hinc, Einc, pr.n2pi, (1, 1, 3), k, k + 1, *mons, pr.cont,
+                       pr.addr)
+        for v in range(4):
+            x = (E if v > 1 else H).reshape(-1, 3)[:, v % 2]
+            x = np.where(split, x[z] + x[s.n3 + pr.addr[z]], x[z])
+            re[v] += ph[k, 0, 2 if v > 1 else 0] * x
+            im[v] += ph[k, 0, 3 if v > 1 else 1] * x
+    assert np.array_equal(got[0], H) and np.array_equal(got[1], E)
+    for d in dft:
+        assert np.array_equal(d.real, re) and np.array_equal(d.imag, im)
