@@ -1,14 +1,15 @@
 /*
  * Dense complex FP64 linear algebra on the GPU for the layer-transfer S matrix
  * (Smat/Scalc.c inv_process :316-400, which calls LAPACK zgesv and BLAS
- * zgemm): a blocked right-looking LU with partial pivoting, the solve with
- * many right-hand sides, a general multiply-add and a transpose.  Column-major
- * storage with leading dimensions, as LAPACK keeps it.
+ * zgemm): an in-place Gauss-Jordan sweep with partial pivoting, which does all
+ * of inv_process in one set of rank-32 updates (smat_scalc); a blocked
+ * right-looking LU and the solve with many right-hand sides (smat_zgesv); a
+ * general multiply-add.  Column-major storage with leading dimensions, as
+ * LAPACK keeps it.
  *
  * The sizes are those of the transfer: order NA = 2*L0*L1 (a few thousand at
- * most: Scalc's matrices are dense NA x NA), so every step is compute bound in
- * FP64 and the tiled multiply-add carries the O(NA^3) work.  The panel
- * factorisation runs in one CTA (NA x 32 complex values, L2 resident).
+ * most: Scalc's matrices are dense NA x NA).  The products carry the O(NA^3)
+ * work, on the tensor cores (zgemm_tc.cu) or with the FP64 kernel here.
  */
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -105,35 +106,6 @@ int zgemm_acc(int m, int n, int k, double2 alpha, const double2 *A, int lda, con
     return cudaPeekAtLastError() == cudaSuccess ? SMAT_OK : smat_fail(SMAT_ECUDA, "k_zgemm launch");
 }
 
-/* ---- out (n x m) = in^T (in: m x n), optionally conjugated -------------- */
-__global__ void k_transpose(int m, int n, const double2 *__restrict__ in, int ldi, double2 *__restrict__ out, int ldo,
-                            int conj)
-{
-    __shared__ double2 t[32][33];
-    const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-    for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-        const int r = bx + threadIdx.x, c = by + j;
-        if (r < m && c < n) t[j][threadIdx.x] = in[r + (long long)ldi * c];
-    }
-    __syncthreads();
-    for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-        const int r = by + threadIdx.x, c = bx + j;  // out row r (= in column), out column c (= in row)
-        if (r < n && c < m) {
-            double2 v = t[threadIdx.x][j];
-            if (conj) v.y = -v.y;
-            out[r + (long long)ldo * c] = v;
-        }
-    }
-}
-
-int transpose(int m, int n, const double2 *in, int ldi, double2 *out, int ldo, bool conj, cudaStream_t st)
-{
-    if (m <= 0 || n <= 0) return SMAT_OK;
-    const dim3 grid((unsigned)((m + 31) / 32), (unsigned)((n + 31) / 32));
-    k_transpose<<<grid, dim3(32, 8), 0, st>>>(m, n, in, ldi, out, ldo, conj ? 1 : 0);
-    return cudaPeekAtLastError() == cudaSuccess ? SMAT_OK : smat_fail(SMAT_ECUDA, "k_transpose launch");
-}
-
 /* ---- panel factorisation: rows [0, m) x columns [0, nb) of the panel at A
  * (the trailing part of the matrix from the current diagonal), partial
  * pivoting by |re| + |im| (LAPACK's izamax), first maximum on ties.
@@ -203,6 +175,7 @@ __global__ void __launch_bounds__(PT) k_panel(double2 *A, int lda, int m, int nb
 }
 
 constexpr int NBMAX = 32;
+constexpr size_t GJ_SMEM = 224 * 1024; /* dynamic shared memory of a sweep's panel CTA */
 
 /* X (nb x ncols at X, leading dimension ldx) <- T^{-1} X with T the nb x nb
  * triangle at T (unit lower if lower, else non-unit upper, nb <= 32): one
@@ -489,6 +462,270 @@ static int launch_panel(double2 *A, int lda, int m, int nb, int row0, int *ipiv,
     cfg.numAttrs = 1;
     if (cudaLaunchKernelEx(&cfg, k_panel_cl, A, lda, m, nb, row0, ipiv, info) != cudaSuccess)
         return smat_fail(SMAT_ECUDA, "k_panel_cl launch: %s", cudaGetErrorString(cudaGetLastError()));
+    return SMAT_OK;
+}
+
+/* ---- in-place Gauss-Jordan sweep ------------------------------------------
+ * M ((n + R) x (n + C)) = [A, F; B, G], A n x n.  Sweeping A out, 32 columns K
+ * at a time with partial pivoting among the rows of A not yet used,
+ *     A[K, J] <- D^-1 A[K, J] (D = A[K, K]; D^-1 itself in the columns K),
+ *     M[i, J] <- M[i, J] - M[i, K] D^-1 A[K, J] for every other row i
+ * (with M[i, K] taken as 0 on the left), leaves [X, X P F; -B X, G - B X P F]
+ * with X = (P A)^-1 = A^-1 P^-1: an inverse, its products from the left and
+ * the right and the Schur complement in n / 32 updates of rank 32 over the
+ * whole of M, where an LU, its two substitutions and a product of inner size n
+ * took three times as many and as many narrow ones between them.
+ *
+ * A step is four launches: k_gj_panel finds the pivots of 32 columns and D's
+ * factors; then in zgemm_tc.cu the rows M[i, K] are cut into slices, the
+ * columns are permuted, solved with D and cut, and one product updates M. */
+
+/* Pivots of columns [j, j + nb) of A (rows [j, n)) and the factors of the nb x
+ * nb block D that they select: an LU with partial pivoting of the panel in the
+ * shared memory of one cluster, of which only D's part is kept.
+ *   mv[c]:      row of A that becomes row j + c
+ *   mv[32 + r]: row that takes the contents of row j + r, or -1 where row
+ *               j + r is a pivot itself
+ *   lud:        [k][r], 32 x 32 (a unit matrix beyond nb): L below the
+ *               diagonal, the inverse of U's diagonal on it, U's rows divided
+ *               by theirs above it
+ * Per column: every thread's largest |re| + |im| among its rows (upper 32 bits
+ * of the double: enough to choose a pivot by) by warp and block; each CTA
+ * sends its candidate row to all others; one cluster barrier; all CTAs pick
+ * the same winner from their own copies.  The rank-1 update of a column's
+ * step is split: the thread that owns a row brings the next column up to date
+ * at once, for the next pivot, and a candidate row is brought up to date as
+ * it is sent; the other columns follow between arriving at the barrier and
+ * waiting for it, lane by lane, 32 / w rows a warp when they fit w lanes.  The
+ * FP64 pipe (20 clocks a warp instruction, whatever its lanes) bounds panels
+ * of many rows, 80 clocks a row and column and CTA; latency the others.
+ * 32 columns of 200 rows: 86 us, 1152 rows 122 us. */
+constexpr int GJT = 256;
+
+__device__ __forceinline__ double2 cfnma(double2 c, double2 a, double2 b) /* c - a b, four multiply-adds */
+{
+    return make_double2(fma(a.y, b.y, fma(-a.x, b.x, c.x)), fma(-a.y, b.x, fma(-a.x, b.y, c.y)));
+}
+
+/* 1 / d, 0 for d = 0: conj(d) / |d|^2, the real reciprocal by the cubic
+ * iteration x <- x + x (e + e^2), e = 1 - s x, from the hardware's 20-bit
+ * approximation (error e^3 < 2^-57); the FP64 division takes three times as
+ * long, on every column's critical path.  |d|^2 outside 2^+-1000: the
+ * division, scaled. */
+__device__ __forceinline__ double2 reciprocal(double2 d)
+{
+    const double s = fma(d.x, d.x, d.y * d.y);
+    const int e = (__double2hiint(s) >> 20) - 1023;
+    if (e < -1000 || e > 1000) { /* 0, tiny, huge or not a number */
+        if (d.x == 0.0 && d.y == 0.0) return make_double2(0.0, 0.0);
+        const double f = e > 0 ? 0x1p-600 : 0x1p600;
+        const double2 v = make_double2(d.x * f, d.y * f);
+        const double r = 1.0 / fma(v.x, v.x, v.y * v.y) * f;
+        return make_double2(v.x * r, -v.y * r);
+    }
+    double x;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(s));
+    const double t = fma(-s, x, 1.0);
+    x = fma(x, fma(t, t, t), x);
+    return make_double2(d.x * x, -d.y * x);
+}
+
+__host__ __device__ inline size_t gj_panel_smem(int R, int w)
+{
+    return sizeof(double2) * ((size_t)R * (w + 1) + 2 * 16 * NBMAX + (NBMAX + 1) * (NBMAX + 1) + R) + sizeof(int) * ((size_t)R + 64);
+}
+
+__global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *__restrict__ A, int lda, int j, int n, int nb, int w,
+                                                  double2 *__restrict__ lud, int *__restrict__ mv, int *info)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const int nc = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int m = n - j, R = (m + nc - 1) / nc, rbeg = rank * R, rn = max(0, min(m, rbeg + R) - rbeg), S = w + 1;
+    constexpr int LS = NBMAX + 1;
+    extern __shared__ __align__(16) unsigned char psm[];
+    double2 *a = reinterpret_cast<double2 *>(psm);   /* [R][S] this CTA's rows */
+    double2 *cand = a + (size_t)R * S;               /* [2][16][32] candidate rows, by column parity */
+    double2 *lu = cand + 2 * 16 * NBMAX;             /* [32][LS] the pivot rows: D's factors */
+    double2 *rd = lu + NBMAX * LS;                   /* [LS] reciprocals of U's diagonal */
+    double2 *lcol = rd + LS;                         /* [R] multipliers of this column */
+    int *used = reinterpret_cast<int *>(lcol + R);   /* [R] the row is a pivot */
+    int *ckey = used + R, *crow = ckey + 32;         /* [2][16] */
+    __shared__ unsigned wk[GJT / 32];
+    __shared__ int wr[GJT / 32], piv[NBMAX];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int t = tid; t < rn * nb; t += GJT) a[(t % rn) * S + t / rn] = A[(j + rbeg + t % rn) + (long long)lda * (j + t / rn)];
+    for (int i = tid; i < rn; i += GJT) used[i] = 0;
+    for (int t = tid; t < NBMAX * LS; t += GJT) lu[t] = make_double2(0.0, 0.0);
+    if (tid < LS) rd[tid] = make_double2(1.0, 0.0);
+    cl.sync();
+    unsigned key = 0;
+    int row = 0;
+    auto consider = [&](int i, double2 v) {
+        const unsigned k = (unsigned)__double2hiint(fabs(v.x) + fabs(v.y)) + 1u;
+        if (k > key) {
+            key = k;
+            row = i;
+        }
+    };
+    for (int i = tid; i < rn; i += GJT) consider(i, a[i * S]);
+    const double2 *prow = cand; /* the pivot row of the column before (none yet) */
+    for (int c = 0; c < nb; c++) {
+        const int par = c & 1;
+        {
+            const unsigned mk = __reduce_max_sync(0xffffffffu, key);
+            const int src = __ffs(__ballot_sync(0xffffffffu, key == mk)) - 1;
+            row = __shfl_sync(0xffffffffu, row, src);
+            if (lane == 0) {
+                wk[warp] = mk;
+                wr[warp] = row;
+            }
+        }
+        __syncthreads();
+        /* the CTA's candidate, up to date, sent by warp t to CTAs t and t + 8 */
+        if (warp < nc) {
+            key = lane < GJT / 32 ? wk[lane] : 0;
+            const unsigned mk = __reduce_max_sync(0xffffffffu, key);
+            const int src = __ffs(__ballot_sync(0xffffffffu, key == mk)) - 1;
+            row = wr[src];
+            double2 v = make_double2(0.0, 0.0);
+            if (mk && lane < nb) {
+                v = a[row * S + lane];
+                if (c > 0 && lane > c) v = cfnma(v, lcol[row], prow[lane]);
+            }
+            for (int t = warp; t < nc; t += GJT / 32) {
+                cl.map_shared_rank(cand, t)[(par * 16 + rank) * NBMAX + lane] = v;
+                if (lane == 0) {
+                    cl.map_shared_rank(ckey, t)[par * 16 + rank] = (int)mk;
+                    cl.map_shared_rank(crow, t)[par * 16 + rank] = rbeg + row;
+                }
+            }
+        }
+        /* columns beyond c of the step before; its pivot row is read before
+         * the barrier, after which another CTA may send over it */
+        const int rest = nb - c - 1, w2 = rest > 1 ? 1 << (32 - __clz(rest - 1)) : 1;
+        const int col = nb - w2 + (lane & (w2 - 1)), per = 32 / w2;
+        const bool live = c > 0 && rest > 0 && col > c;
+        const double2 pb = live ? prow[col] : make_double2(0.0, 0.0);
+        cl.barrier_arrive();
+        __syncthreads(); /* every warp has read the candidate row before it is updated */
+        if (live)
+            for (int i = warp * per + lane / w2; i < rn; i += GJT / 32 * per) a[i * S + col] = cfnma(a[i * S + col], lcol[i], pb);
+        cl.barrier_wait();
+        __syncthreads();
+        key = lane < nc ? (unsigned)ckey[par * 16 + lane] : 0;
+        const unsigned mk = __reduce_max_sync(0xffffffffu, key);
+        const int win = __ffs(__ballot_sync(0xffffffffu, key == mk)) - 1;
+        const int q = crow[par * 16 + win];
+        prow = cand + (par * 16 + win) * NBMAX;
+        key = 0;
+        if (tid < ((rn + 31) & ~31) || warp == 0) { /* every warp that has rows takes the reciprocal itself */
+            const double2 d = prow[c], inv = reciprocal(d);
+            const double2 next = c + 1 < nb ? prow[c + 1] : make_double2(0.0, 0.0);
+            for (int i = tid; i < rn; i += GJT) {
+                double2 l = make_double2(0.0, 0.0);
+                if (rbeg + i == q) used[i] = 1;
+                else if (!used[i]) {
+                    l = cmul(a[i * S + c], inv);
+                    a[i * S + c] = l;
+                    if (c + 1 < nb) {
+                        const double2 v = cfnma(a[i * S + c + 1], l, next);
+                        a[i * S + c + 1] = v;
+                        consider(i, v);
+                    }
+                }
+                lcol[i] = l;
+            }
+            if (warp == 0) {
+                if (lane < nb) lu[c * LS + lane] = prow[lane];
+                if (lane == 0) {
+                    rd[c] = inv;
+                    piv[c] = q;
+                    if (rank == 0 && inv.x == 0.0 && inv.y == 0.0 && *info == 0) *info = j + c + 1;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    /* D's factors: L below the diagonal, U's rows scaled to a unit diagonal
+     * above it, the reciprocals on it */
+    if (rank == 0)
+        for (int r = warp; r < NBMAX; r += GJT / 32) {
+            double2 v = lu[r * LS + lane];
+            if (lane > r) v = cmul(v, rd[r]);
+            else if (lane == r) v = rd[r];
+            lud[lane * NBMAX + r] = v;
+        }
+    if (rank == 0 && warp == 0) {
+        /* rows of D's place that are no pivots go where the pivots from below came from, in order */
+        const int q = lane < nb ? piv[lane] : -1;
+        const unsigned in = __reduce_or_sync(0xffffffffu, q >= 0 && q < nb ? 1u << q : 0u);
+        const unsigned out = __ballot_sync(0xffffffffu, q >= nb);
+        const bool free_row = lane < nb && !(in >> lane & 1u);
+        const unsigned fr = __ballot_sync(0xffffffffu, free_row);
+        int dst = -1;
+        if (free_row) {
+            unsigned o = out;
+            for (int t = __popc(fr & ((1u << lane) - 1)); t > 0; t--) o &= o - 1;
+            dst = j + piv[__ffs(o) - 1];
+        }
+        mv[lane] = lane < nb ? j + q : -1;
+        mv[32 + lane] = dst;
+    }
+    cl.sync(); /* no CTA leaves while another may still write to it */
+}
+
+/* the panel's width for matrices of order n: 32 columns where the rows of a
+ * full-height panel fit the shared memory of 16 CTAs (n up to about 5,500),
+ * else 16 or 8 */
+static int gj_width(int n)
+{
+    for (int w : {32, 16, 8})
+        if (gj_panel_smem((n + 15) / 16, w) <= GJ_SMEM) return w;
+    return 0;
+}
+
+static int launch_gj_panel(const double2 *A, int lda, int j, int n, int nb, int w, double2 *lud, int *mv, int *info,
+                           cudaStream_t st)
+{
+    /* 16 CTAs for panels of 128 rows and more; fewer rows synchronise fewer */
+    const int m = n - j, cs = m >= 128 ? 16 : m >= 64 ? 8 : m >= 32 ? 4 : 1;
+    static const bool ready = cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                              cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GJ_SMEM) == cudaSuccess;
+    if (!ready) return smat_fail(SMAT_ECUDA, "k_gj_panel: cluster of 16 CTAs refused");
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(cs);
+    cfg.blockDim = dim3(GJT);
+    cfg.dynamicSmemBytes = gj_panel_smem((m + cs - 1) / cs, w);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k_gj_panel, A, lda, j, n, nb, w, lud, mv, info) != cudaSuccess)
+        return smat_fail(SMAT_ECUDA, "k_gj_panel launch: %s", cudaGetErrorString(cudaGetLastError()));
+    return SMAT_OK;
+}
+
+__global__ void k_iota(int *p, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) p[i] = i;
+}
+
+int sweep(int n, int rows, int cols, double2 *M, int ld, const SweepWs &w, const GemmCtx &g, int *info, cudaStream_t st)
+{
+    const int width = gj_width(n);
+    if (!width) return smat_fail(SMAT_EINVAL, "sweep: order %d", n);
+    k_iota<<<(n + 255) / 256, 256, 0, st>>>(w.perm, n);
+    for (int j = 0; j < n; j += width) {
+        const int nb = std::min(width, n - j);
+        if (int rc = launch_gj_panel(M, ld, j, n, nb, width, w.lud, w.mv, info, st)) return rc;
+        if (int rc = sweep_update(rows, cols, j, nb, M, ld, w, g, st)) return rc;
+    }
     return SMAT_OK;
 }
 

@@ -39,14 +39,28 @@ int dense_mode();
 int gemm_ctx_alloc(GemmCtx &g, int m, int n, cudaStream_t st);
 int gemm_ctx_check(const GemmCtx &g);
 void gemm_ctx_release(GemmCtx &g);
-/* out (n x m) = in^T or in^H (in: m x n) */
-int transpose(int m, int n, const double2 *in, int ldi, double2 *out, int ldo, bool conj, cudaStream_t st);
 /* LU with partial pivoting in place (LAPACK zgetrf semantics: ipiv[k] = row
  * exchanged with k, 0-based; *info (device) = first zero pivot, 1-based, or 0) */
 int getrf(int n, double2 *A, int lda, int *ipiv, int *info, const GemmCtx *g, cudaStream_t st);
 /* B <- A^{-1} B from getrf's factors */
 int getrs(int n, int nrhs, const double2 *LU, int lda, const int *ipiv, double2 *B, int ldb, const GemmCtx *g,
           cudaStream_t st);
+
+/* Device buffers of a sweep: the factors of D of a step, the row moves of its pivots, the
+ * rows' permutation (perm[i] = row of A that pivoting moved to i), and for the
+ * FP64 kernel the step's rows and columns (rows x 32, 32 x cols). */
+struct SweepWs {
+    double2 *lud;
+    int *mv, *perm;
+    double2 *prow, *bcol;
+};
+/* The in-place Gauss-Jordan sweep of the leading n x n block A of M (rows x
+ * cols, column-major): [A, F; B, G] -> [X, X P F; -B X, G - B X P F], X P =
+ * A^-1, (X P)[:, perm[i]] = X[:, i]; *info: first zero pivot, 1-based, or 0.
+ * g: workspace for products up to rows x cols. */
+int sweep(int n, int rows, int cols, double2 *M, int ld, const SweepWs &w, const GemmCtx &g, int *info, cudaStream_t st);
+/* a step of it after its panel: columns [j, j + nb) (zgemm_tc.cu) */
+int sweep_update(int rows, int cols, int j, int nb, double2 *M, int ld, const SweepWs &w, const GemmCtx &g, cudaStream_t st);
 
 } // namespace dense
 } // namespace smat

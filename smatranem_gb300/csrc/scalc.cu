@@ -2,18 +2,26 @@
  * Frequency-domain S matrix by layer transfer on the GPU: the reference's
  * Smat/Scalc.c (main :74-96) with its dense steps on the device.
  *
- * State per direction (iway = +1 bottom -> top, -1 top -> bottom), NA =
- * 2*L0*L1, No = modes of the starting port: F01 ((No+NA) x No), B01
- * ((No+NA) x NA), F2 (NA x No), B2 (NA x NA), all complex FP64 in HBM.
+ * Per direction (iway = +1 bottom -> top, -1 top -> bottom; NA = 2*L0*L1, No
+ * modes of the starting port) the reference keeps F01 ((No+NA) x No), B01
+ * ((No+NA) x NA), F2 (NA x No) and B2 (NA x NA):
  *   set_iniMat (:407-458): the starting port's full mode matrix Phi;
  *   per half layer (initial_calc :192-221, scattering_calc :227-261,
  *   final_calc :269-306): F2 <- field rows of F01, B2 <- field rows of B01
  *   + i*iway*(maa or mbb of the layer), field rows of B01 <- 1, inv_process;
  *   set_finMat (:461-517): project on the ending port's dual modes;
- *   inv_process (:316-400): B01 <- B01 B2^{-1} (LU with partial pivoting of
- *   B2^T, the zgesv of the reference), F01 <- F01 - B01 F2, F2 = 0, B2 = 1.
- * maa / mbb are never formed: k_add_op adds each row's stencil coefficients
- * (those of set_M :716-790) straight into B2.
+ *   inv_process (:316-400): B01 <- B01 B2^{-1}, F01 <- F01 - B01 F2, F2 = 0,
+ *   B2 = 1.
+ * Here a direction's state is one matrix, complex FP64 in HBM,
+ *     M = [B2, F2; B, F]
+ * with the rows of B01 and F01 below, and inv_process one Gauss-Jordan sweep
+ * of B2 out of it (dense_z.cuh): every block that it needs comes out of the
+ * same updates of rank 32.  Where the field rows of B01 are 1, as in every
+ * half layer, the sweep's own block is that product and they are not kept:
+ * after it [X, X F2; -B X, F - B X F2] is, up to signs and the order of the
+ * columns, the next half layer's M but for the operator, which k_add_op adds
+ * (maa and mbb are never formed: each row's stencil coefficients, those of
+ * set_M :716-790).
  */
 #include <cuda_runtime.h>
 
@@ -32,9 +40,7 @@
 
 namespace {
 
-using smat::dense::getrf;
-using smat::dense::getrs;
-using smat::dense::transpose;
+using smat::dense::sweep;
 using smat::dense::zgemm_acc;
 
 struct Geo {
@@ -109,47 +115,100 @@ __global__ void k_add_op(double2 *B2, int ld, Geo g, const double2 *__restrict__
     }
 }
 
-/* dst (m x n, ldd) = src (ldsrc) */
-__global__ void k_copy2d(int m, int n, const double2 *__restrict__ src, int lds, double2 *__restrict__ dst, int ldd)
+/* entry (r, c) of the full mode matrix of set_Phi (:521-551) from Xi (2NA x
+ * 2NA, Mcalc's column order) */
+__device__ __forceinline__ double2 phi(const double2 *__restrict__ Xi, int NA, int iway, int r, int c)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)m * n) return;
-    const int r = (int)(t % m), c = (int)(t / m);
-    dst[r + (long long)ldd * c] = src[r + (long long)lds * c];
-}
-
-/* dst (m x n) = diag * identity (diag 0: zero) */
-__global__ void k_set2d(int m, int n, double2 *dst, int ldd, double diag)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)m * n) return;
-    const int r = (int)(t % m), c = (int)(t / m);
-    dst[r + (long long)ldd * c] = make_double2(r == c ? diag : 0.0, 0.0);
-}
-
-/* the full mode matrix of set_Phi (:521-551) / set_tilPhi (:555-595) from Xi
- * (2NA x 2NA, Mcalc's column order); kind 0: Phi, 1: tilPhi */
-__global__ void k_phi(const double2 *__restrict__ Xi, double2 *__restrict__ P, int NA, int iway, int nimag, int kind)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int N2 = 2 * NA;
-    if (t >= (long long)N2 * N2) return;
-    const int r = (int)(t % N2), col = (int)(t / N2);
-    const int j = col % NA, hi = col >= NA;
-    const int rr = (r + NA) % N2;  // the file row that lands on row r after the half rotation
-    auto X = [&](int row, int c) { return Xi[row + (long long)N2 * c]; };
-    auto neg = [](double2 v) { return make_double2(-v.x, -v.y); };
+    return iway == 1 ? Xi[r + (long long)N2 * c]
+                     : Xi[(r < NA ? r + NA : r - NA) + (long long)N2 * (c < NA ? c + NA : c - NA)];
+}
+
+/* conj of entry (r, c) of the dual mode matrix of set_tilPhi (:555-595) */
+__device__ __forceinline__ double2 dual(const double2 *__restrict__ Xi, int NA, int iway, int nimag, int r, int c)
+{
+    const int N2 = 2 * NA, j = c < NA ? c : c - NA;
+    const bool hi = c >= NA, real = j < nimag;
+    if (iway == 1) r = r < NA ? r + NA : r - NA;
+    /* the second half of Xi's columns: iway = 1, hi == real; -1, hi != real */
+    const bool second = (iway == 1) == (hi == real);
+    const bool neg = real && second;
+    double2 v = Xi[r + (long long)N2 * (second ? j + NA : j)];
+    if (neg) v.x = -v.x;
+    else v.y = -v.y;
+    return v;
+}
+
+/* set_iniMat (:407-458): M = [B2, F2; B0, F0; B1, F1] of the starting port,
+ * (2 NA + No) x (NA + No) */
+__global__ void k_start(double2 *__restrict__ M, const double2 *__restrict__ Xi, int NA, int No, int iway)
+{
+    const int rows = 2 * NA + No;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)rows * (NA + No)) return;
+    const int r = (int)(t % rows), c = (int)(t / rows);
+    const int pc = c < NA ? NA + c : c - NA; /* B: backward modes, F: forward ones */
     double2 v;
-    if (kind == 0) {
-        v = iway == 1 ? X(r, col) : X(rr, hi ? j : j + NA);
-    } else if (iway == 1) {
-        if (j < nimag) v = hi ? neg(X(rr, j + NA)) : X(rr, j);
-        else v = hi ? X(rr, j) : X(rr, j + NA);
+    if (r < NA) v = phi(Xi, NA, iway, NA + r, pc);
+    else if (r < NA + No) v = make_double2(r - NA == c ? 1.0 : 0.0, 0.0);
+    else v = phi(Xi, NA, iway, r - NA - No, pc);
+    M[t] = v;
+}
+
+/* The next half layer's M = [B1, F1; B0, F0] ((NA + No) x (NA + No)) from a
+ * swept matrix: rows r < NA of it are src rows r0 + r, the No others src rows
+ * r1 + r.  Columns c < NA go to perm[c].  own: the first rows are the swept
+ * block itself (X, X F2: sign + -), else extra rows (-B X, F - B X F2: - +),
+ * as the last No are. */
+__global__ void k_next(double2 *__restrict__ M, const double2 *__restrict__ X, int lds, int NA, int No, int r0, int r1,
+                       int own, const int *__restrict__ perm)
+{
+    const int n = NA + No;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)n * n) return;
+    const int r = (int)(t % n), c = (int)(t / n);
+    double2 v = X[(r < NA ? r0 + r : r1 + r - NA) + (long long)lds * c];
+    if ((c < NA) != (r < NA && own)) v = make_double2(-v.x, -v.y);
+    M[r + (long long)n * (c < NA ? perm[c] : c)] = v;
+}
+
+/* set_finMat (:461-517) before the product: with S = [B1, F1; B0, F0] the last
+ * half layer's state and T the dual modes, M = [lower rows of T^H [S1; 1], then
+ * its first nimag rows, then B0, F0]: the part of the unit block here (zero in
+ * the columns of F), B0 and F0 copied; LP ((NA + nimag) x NA): the factor of
+ * S1 = [B1, F1] */
+__global__ void k_final(double2 *__restrict__ M, double2 *__restrict__ LP, const double2 *__restrict__ S,
+                        const double2 *__restrict__ Xi, int NA, int No, int nimag, int iway)
+{
+    const int rows = NA + nimag + No, n = NA + No;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)rows * n) return;
+    const int r = (int)(t % rows), c = (int)(t / rows);
+    const int tc = r < NA ? NA + r : r - NA; /* the dual mode of a projected row */
+    double2 v = make_double2(0.0, 0.0);
+    if (r < NA + nimag) {
+        if (c < NA) {
+            v = dual(Xi, NA, iway, nimag, NA + c, tc);
+            LP[r + (long long)(NA + nimag) * c] = dual(Xi, NA, iway, nimag, c, tc);
+        }
     } else {
-        if (j < nimag) v = hi ? X(r, j) : neg(X(r, j + NA));
-        else v = hi ? X(r, j + NA) : X(r, j);
+        v = S[NA + (r - NA - nimag) + (long long)n * c];
     }
-    P[r + (long long)N2 * col] = v;
+    M[t] = v;
+}
+
+/* the rows Smat_calc reads: out = [F01, the first nimag columns of B01], rows
+ * [No of F0, B0; nimag of F1, B1], from the last swept matrix */
+__global__ void k_result(double2 *__restrict__ out, const double2 *__restrict__ X, int NA, int No, int nimag,
+                         const int *__restrict__ perm)
+{
+    const int N = No + nimag, lds = NA + N;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)N * (NA + No)) return;
+    const int r = (int)(t % N), c = (int)(t / N);
+    const double2 v = X[NA + (r < No ? nimag + r : r - No) + (long long)lds * c];
+    if (c >= NA) out[r + (long long)N * (c - NA)] = v;
+    else if (perm[c] < nimag) out[r + (long long)N * (No + perm[c])] = make_double2(-v.x, -v.y);
 }
 
 #define SCK(call)                                                                                                      \
@@ -165,69 +224,46 @@ __global__ void k_phi(const double2 *__restrict__ Xi, double2 *__restrict__ P, i
 
 struct Transfer {
     Geo g{};
-    int NA = 0, No = 0, ldF = 0;
+    int NA = 0, No = 0;
     cudaStream_t st = nullptr;
-    double2 *F01 = nullptr, *B01 = nullptr, *F2 = nullptr, *B2 = nullptr, *W1 = nullptr, *W2 = nullptr;
-    double2 *Xi = nullptr, *P = nullptr, *PH = nullptr, *FB = nullptr, *Cm = nullptr, *V = nullptr;
-    int *ipiv = nullptr, *dinfo = nullptr;
+    void *slab = nullptr; /* the one allocation that holds the matrices */
+    double2 *M[2] = {nullptr, nullptr}, *LP = nullptr, *out = nullptr;
+    smat::dense::SweepWs w{};
+    int *dinfo = nullptr;
     int solves = 0;
-    smat::dense::GemmCtx gm{0, nullptr, 0, nullptr}; /* how the multiply-adds run */
+    smat::dense::GemmCtx gm{0, nullptr, 0, nullptr}; /* how the products run */
 
     ~Transfer()
     {
         if (st) cudaStreamSynchronize(st);
         smat::dense::gemm_ctx_release(gm);
-        for (double2 *b : {F01, B01, F2, B2, W1, W2, Xi, P, PH, FB, Cm, V}) cudaFree(b);
-        cudaFree(ipiv);
-        cudaFree(dinfo);
+        cudaFree(slab);
         if (st) cudaStreamDestroy(st);
     }
     static unsigned blocks(long long n, int t) { return (unsigned)((n + t - 1) / t); }
-    int copy2d(int m, int n, const double2 *s, int lds, double2 *d, int ldd)
+    /* one inv_process on X = M[which] (rows x (NA + No)) */
+    int solve(int which, int rows)
     {
-        if ((long long)m * n == 0) return SMAT_OK;
-        k_copy2d<<<blocks((long long)m * n, 256), 256, 0, st>>>(m, n, s, lds, d, ldd);
-        return cudaPeekAtLastError() == cudaSuccess ? SMAT_OK : smat_fail(SMAT_ECUDA, "k_copy2d launch");
-    }
-    int set2d(int m, int n, double2 *d, int ldd, double diag)
-    {
-        if ((long long)m * n == 0) return SMAT_OK;
-        k_set2d<<<blocks((long long)m * n, 256), 256, 0, st>>>(m, n, d, ldd, diag);
-        return cudaPeekAtLastError() == cudaSuccess ? SMAT_OK : smat_fail(SMAT_ECUDA, "k_set2d launch");
-    }
-    /* inv_process :316-400 */
-    int inv_process()
-    {
-        RC(transpose(NA, NA, B2, NA, W1, NA, false, st));
-        RC(transpose(No + NA, NA, B01, ldF, W2, NA, false, st));
-        RC(getrf(NA, W1, NA, ipiv, dinfo, &gm, st));
-        RC(getrs(NA, No + NA, W1, NA, ipiv, W2, NA, &gm, st));
-        RC(transpose(NA, No + NA, W2, NA, B01, ldF, false, st));
-        RC(zgemm_acc(No + NA, No, NA, make_double2(-1.0, 0.0), B01, ldF, F2, NA, F01, ldF, &gm, st));
-        RC(set2d(NA, No, F2, NA, 0.0));
-        RC(set2d(NA, NA, B2, NA, 1.0));
         solves++;
-        return SMAT_OK;
+        return sweep(NA, rows, NA + No, M[which], rows, w, gm, dinfo, st);
     }
-    /* F2 <- field rows of F01, which become 0 */
-    int shift()
+    /* M[0] (k_next's arguments) <- M[1] */
+    int next(int lds, int r0, int r1, int own)
     {
-        RC(copy2d(NA, No, F01 + No, ldF, F2, NA));
-        return set2d(NA, No, F01 + No, ldF, 0.0);
-    }
-    /* B2 <- field rows of B01 + i*iway*M; field rows of B01 <- 1; eliminate */
-    int step(int which, int iway)
-    {
-        RC(copy2d(NA, NA, B01 + No, ldF, B2, NA));
-        k_add_op<<<blocks(NA, 128), 128, 0, st>>>(B2, NA, g, V, which, (double)iway);
+        const long long n = NA + No;
+        k_next<<<blocks(n * n, 256), 256, 0, st>>>(M[0], M[1], lds, NA, No, r0, r1, own, w.perm);
         SCK(cudaPeekAtLastError());
-        RC(set2d(NA, NA, B01 + No, ldF, 1.0));
-        return inv_process();
-    }
-    int upload_layer(const std::vector<std::complex<double>> &v)
-    {
-        SCK(cudaMemcpyAsync(V, v.data(), v.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
         return SMAT_OK;
+    }
+    /* a half layer: the operator into B2, eliminate */
+    int step(const double2 *V, int which, int iway)
+    {
+        const int n = NA + No;
+        k_add_op<<<blocks(NA, 128), 128, 0, st>>>(M[0], n, g, V, which, (double)iway);
+        SCK(cudaPeekAtLastError());
+        std::swap(M[0], M[1]);
+        RC(solve(1, n));
+        return next(n, 0, NA, 1);
     }
 };
 
@@ -247,76 +283,42 @@ int scalc_V(const double *med, long long NA1, double omega, std::vector<std::com
     return comp;
 }
 
-/* one direction (main :74-94); meds: nlayers layers starting at istart in the
- * direction of travel; Xs / Xe: start / end port Xi (host) */
-int one_way(Transfer &T, int iway, int nlayers, const double *const *meds, double omega, const double *Xs,
-            const double *Xe, int No, int Nimag, std::vector<std::complex<double>> &F01h,
-            std::vector<std::complex<double>> &B01h)
+/* one direction (main :74-94) of nlayers layers whose set_V values are at V
+ * (6*NA1 each), the first at istart, in the direction of travel; Xs / Xe:
+ * start / end port Xi (device) */
+int one_way(Transfer &T, int iway, int nlayers, const double2 *V, const double2 *Xs, const double2 *Xe, int No, int Nimag,
+            std::vector<std::complex<double>> &F01h, std::vector<std::complex<double>> &B01h)
 {
-    const int NA = T.NA, N2 = 2 * NA;
-    const long long NA1 = T.g.NA1;
+    const int NA = T.NA, n = NA + No, N = No + Nimag;
+    const long long lv = 6LL * T.g.NA1;
     T.No = No;
-    T.ldF = No + NA;
-    std::vector<std::complex<double>> v;
+    auto layer = [&](int l) { return V + lv * (iway > 0 ? l : nlayers - 1 - l); };
     /* set_iniMat :407-458 */
-    SCK(cudaMemcpyAsync(T.Xi, Xs, sizeof(double2) * (size_t)N2 * N2, cudaMemcpyHostToDevice, T.st));
-    k_phi<<<Transfer::blocks((long long)N2 * N2, 256), 256, 0, T.st>>>(T.Xi, T.P, NA, iway, 0, 0);
+    const int rows0 = 2 * NA + No;
+    k_start<<<Transfer::blocks((long long)rows0 * n, 256), 256, 0, T.st>>>(T.M[1], Xs, NA, No, iway);
     SCK(cudaPeekAtLastError());
-    RC(T.set2d(No, No, T.F01, T.ldF, 0.0));
-    RC(T.set2d(No, NA, T.B01, T.ldF, 1.0));  /* top rows of B01: identity in the first No columns */
-    RC(T.copy2d(NA, No, T.P, N2, T.F01 + No, T.ldF));
-    RC(T.copy2d(NA, No, T.P + NA, N2, T.F2, NA));
-    RC(T.copy2d(NA, NA, T.P + (long long)N2 * NA, N2, T.B01 + No, T.ldF));
-    RC(T.copy2d(NA, NA, T.P + NA + (long long)N2 * NA, N2, T.B2, NA));
-    RC(T.inv_process());
+    RC(T.solve(1, rows0));
+    RC(T.next(rows0, NA + No, NA, 0));
     /* initial_calc :192-221 */
-    RC(T.shift());
-    if (scalc_V(meds[0], NA1, omega, v)) return smat_fail(SMAT_EINVAL, "V is not real in initial_calc");
-    RC(T.upload_layer(v));
-    RC(T.step(iway > 0 ? 1 : 0, iway));
+    RC(T.step(layer(0), iway > 0 ? 1 : 0, iway));
     /* scattering_calc :227-261 */
-    for (int l = 1; l + 1 < nlayers; l++) {
-        scalc_V(meds[l], NA1, omega, v);  /* a lossy inner layer is allowed (a warning in the reference) */
-        RC(T.upload_layer(v));
-        for (int sub = 0; sub < 2; sub++) {
-            RC(T.shift());
-            const int i_shift = ((1 - iway) / 2 + sub) % 2;
-            RC(T.step(i_shift, iway));
-        }
-    }
+    for (int l = 1; l + 1 < nlayers; l++)
+        for (int sub = 0; sub < 2; sub++) RC(T.step(layer(l), ((1 - iway) / 2 + sub) % 2, iway));
     /* final_calc :269-306 */
-    RC(T.shift());
-    if (scalc_V(meds[nlayers - 1], NA1, omega, v)) return smat_fail(SMAT_EINVAL, "V is not real in final_calc");
-    RC(T.upload_layer(v));
-    RC(T.step(iway > 0 ? 0 : 1, iway));
-    /* set_finMat :461-517: C = tilPhi^H [F01 field rows, B01 field rows; F2, B2] */
-    SCK(cudaMemcpyAsync(T.Xi, Xe, sizeof(double2) * (size_t)N2 * N2, cudaMemcpyHostToDevice, T.st));
-    k_phi<<<Transfer::blocks((long long)N2 * N2, 256), 256, 0, T.st>>>(T.Xi, T.P, NA, iway, Nimag, 1);
+    RC(T.step(layer(nlayers - 1), iway > 0 ? 0 : 1, iway));
+    /* set_finMat :461-517 */
+    const int rows1 = NA + N;
+    k_final<<<Transfer::blocks((long long)rows1 * n, 256), 256, 0, T.st>>>(T.M[1], T.LP, T.M[0], Xe, NA, No, Nimag, iway);
     SCK(cudaPeekAtLastError());
-    RC(transpose(N2, N2, T.P, N2, T.PH, N2, true, T.st));
-    const int nc = No + NA;
-    RC(T.copy2d(NA, No, T.F01 + No, T.ldF, T.FB, N2));
-    RC(T.copy2d(NA, No, T.F2, NA, T.FB + NA, N2));
-    RC(T.copy2d(NA, NA, T.B01 + No, T.ldF, T.FB + (long long)N2 * No, N2));
-    RC(T.copy2d(NA, NA, T.B2, NA, T.FB + NA + (long long)N2 * No, N2));
-    RC(T.set2d(N2, nc, T.Cm, N2, 0.0));
-    RC(zgemm_acc(N2, nc, N2, make_double2(1.0, 0.0), T.PH, N2, T.FB, N2, T.Cm, N2, &T.gm, T.st));
-    RC(T.copy2d(NA, No, T.Cm, N2, T.F01 + No, T.ldF));
-    RC(T.copy2d(NA, No, T.Cm + NA, N2, T.F2, NA));
-    RC(T.copy2d(NA, NA, T.Cm + (long long)N2 * No, N2, T.B01 + No, T.ldF));
-    RC(T.copy2d(NA, NA, T.Cm + NA + (long long)N2 * No, N2, T.B2, NA));
-    RC(T.inv_process());
-    /* the rows Smat_calc reads: the top No + Nimag rows of F01 and B01 */
-    const int N = No + Nimag;
-    F01h.assign((size_t)N * No, 0.0);
-    B01h.assign((size_t)N * NA, 0.0);
-    for (int c = 0; c < No; c++)
-        SCK(cudaMemcpyAsync(&F01h[(size_t)N * c], T.F01 + (long long)T.ldF * c, sizeof(double2) * N,
-                            cudaMemcpyDeviceToHost, T.st));
-    for (int c = 0; c < Nimag && c < NA; c++)
-        SCK(cudaMemcpyAsync(&B01h[(size_t)N * c], T.B01 + (long long)T.ldF * c, sizeof(double2) * N,
-                            cudaMemcpyDeviceToHost, T.st));
+    RC(zgemm_acc(NA + Nimag, n, NA, make_double2(1.0, 0.0), T.LP, NA + Nimag, T.M[0], n, T.M[1], rows1, &T.gm, T.st));
+    RC(T.solve(1, rows1));
+    k_result<<<Transfer::blocks((long long)N * n, 256), 256, 0, T.st>>>(T.out, T.M[1], NA, No, Nimag, T.w.perm);
+    SCK(cudaPeekAtLastError());
+    std::vector<std::complex<double>> h((size_t)N * N);
+    SCK(cudaMemcpyAsync(h.data(), T.out, sizeof(double2) * h.size(), cudaMemcpyDeviceToHost, T.st));
     SCK(cudaStreamSynchronize(T.st));
+    F01h.assign(h.begin(), h.begin() + (size_t)N * No);
+    B01h.assign(h.begin() + (size_t)N * No, h.end());
     return SMAT_OK;
 }
 
@@ -337,7 +339,7 @@ extern "C" int smat_scalc(int L0, int L1, const int BoundC[2], double omega, int
     if (nB < 1 || nT < 1 || nB > NA || nT > NA) return smat_fail(SMAT_EINVAL, "smat_scalc: modes %d, %d", nB, nT);
     if (!(omega > 0) || !std::isfinite(omega)) return smat_fail(SMAT_EINVAL, "smat_scalc: omega = %g", omega);
     const int Nmax = std::max(nB, nT);
-    const size_t ldF = (size_t)Nmax + NA;
+    const size_t cols = (size_t)Nmax + NA, rows = cols + NA;
     /* one transfer state per direction: device matrices, stream, product workspace */
     auto setup = [&](Transfer &T) {
         T.NA = NA;
@@ -349,33 +351,63 @@ extern "C" int smat_scalc(int L0, int L1, const int BoundC[2], double omega, int
         T.g.e0 = L0 > 1 ? (double)BoundC[0] : 0.0;
         T.g.e1 = L1 > 1 ? (double)BoundC[1] : 0.0;
         SCK(cudaStreamCreateWithFlags(&T.st, cudaStreamNonBlocking));
-        auto alloc = [&](double2 **p, size_t n) {
-            if (cudaMalloc((void **)p, n * sizeof(double2)) != cudaSuccess) {
-                cudaGetLastError();
-                return smat_fail(SMAT_ENOMEM, "smat_scalc: %zu bytes of device memory", n * sizeof(double2));
-            }
-            return SMAT_OK;
+        /* products up to (2 NA + No) x (NA + No) (the first sweep) */
+        RC(smat::dense::gemm_ctx_alloc(T.gm, (int)rows, (int)cols, T.st));
+        size_t used = 0;
+        std::vector<std::pair<void **, size_t>> want;
+        auto buf = [&](auto *&p, size_t n) {
+            want.push_back({(void **)&p, used});
+            used += (n * sizeof(*p) + 255) / 256 * 256;
         };
-        RC(alloc(&T.F01, ldF * Nmax));
-        RC(alloc(&T.B01, ldF * NA));
-        RC(alloc(&T.F2, (size_t)NA * Nmax));
-        RC(alloc(&T.B2, (size_t)NA * NA));
-        RC(alloc(&T.W1, (size_t)NA * NA));
-        RC(alloc(&T.W2, (size_t)NA * ldF));
-        RC(alloc(&T.Xi, (size_t)N2 * N2));
-        RC(alloc(&T.P, (size_t)N2 * N2));
-        RC(alloc(&T.PH, (size_t)N2 * N2));
-        RC(alloc(&T.FB, (size_t)N2 * ldF));
-        RC(alloc(&T.Cm, (size_t)N2 * ldF));
-        RC(alloc(&T.V, 6 * (size_t)NA1));
-        SCK(cudaMalloc(&T.ipiv, sizeof(int) * NA));
-        SCK(cudaMalloc(&T.dinfo, sizeof(int)));
+        buf(T.M[0], rows * cols);
+        buf(T.M[1], rows * cols);
+        buf(T.LP, cols * NA);
+        buf(T.out, (size_t)(nB + nT) * (nB + nT));
+        buf(T.w.lud, 32 * 32);
+        buf(T.w.prow, T.gm.tc ? 0 : rows * 32);
+        buf(T.w.bcol, T.gm.tc ? 0 : cols * 32);
+        buf(T.w.mv, 64);
+        buf(T.w.perm, NA);
+        buf(T.dinfo, 1);
+        if (cudaMalloc(&T.slab, used) != cudaSuccess) {
+            cudaGetLastError();
+            return smat_fail(SMAT_ENOMEM, "smat_scalc: %zu bytes of device memory", used);
+        }
+        for (auto &w : want) *w.first = (char *)T.slab + w.second;
         SCK(cudaMemsetAsync(T.dinfo, 0, sizeof(int), T.st));
-        /* products up to 2NA x (Nmax + NA) (the projection on the dual modes) */
-        return smat::dense::gemm_ctx_alloc(T.gm, N2, (int)ldF, T.st);
+        return (int)SMAT_OK;
     };
+    /* both directions read the ports' modes and the layers' set_V values */
+    struct Inputs {
+        void *slab = nullptr;
+        double2 *XB = nullptr, *XT = nullptr, *V = nullptr;
+        ~Inputs() { cudaFree(slab); }
+    } in;
     Transfer T;
     RC(setup(T));
+    {
+        const size_t nx = (size_t)N2 * N2, nv = 6 * (size_t)NA1;
+        const bool same = XiB == XiT;
+        if (cudaMalloc(&in.slab, sizeof(double2) * (nx * (same ? 1 : 2) + nv * nlayers)) != cudaSuccess) {
+            cudaGetLastError();
+            return smat_fail(SMAT_ENOMEM, "smat_scalc: device memory for the port modes");
+        }
+        in.XB = static_cast<double2 *>(in.slab);
+        in.XT = same ? in.XB : in.XB + nx;
+        in.V = in.XT + nx;
+        std::vector<std::complex<double>> v, all;
+        for (int l = 0; l < nlayers; l++) {
+            /* a lossy inner layer is allowed (a warning in the reference) */
+            const int comp = scalc_V(meds + (size_t)2 * 6 * NA1 * l, NA1, omega, v);
+            if (comp && l == 0) return smat_fail(SMAT_EINVAL, "V is not real in initial_calc");
+            if (comp && l == nlayers - 1) return smat_fail(SMAT_EINVAL, "V is not real in final_calc");
+            all.insert(all.end(), v.begin(), v.end());
+        }
+        SCK(cudaMemcpyAsync(in.V, all.data(), sizeof(double2) * all.size(), cudaMemcpyHostToDevice, T.st));
+        SCK(cudaMemcpyAsync(in.XB, XiB, sizeof(double2) * nx, cudaMemcpyHostToDevice, T.st));
+        if (!same) SCK(cudaMemcpyAsync(in.XT, XiT, sizeof(double2) * nx, cudaMemcpyHostToDevice, T.st));
+        SCK(cudaStreamSynchronize(T.st));
+    }
     /* the backward pass on a state, stream and host thread of its own, so
      * that the two directions' latency-bound panel factorisations (a cluster
      * of 16 SMs) run beside each other's products; if the second state does
@@ -383,12 +415,6 @@ extern "C" int smat_scalc(int L0, int L1, const int BoundC[2], double omega, int
     Transfer T2;
     const bool concurrent = both_ways && setup(T2) == SMAT_OK;
     if (both_ways && !concurrent) smat_clear_error();
-    const size_t lstride = (size_t)2 * 6 * NA1;
-    std::vector<const double *> up(nlayers), down(nlayers);
-    for (int l = 0; l < nlayers; l++) {
-        up[l] = meds + lstride * l;
-        down[l] = meds + lstride * (nlayers - 1 - l);
-    }
     const int N = nB + nT;
     std::vector<std::complex<double>> Sm((size_t)N * N, 0.0), F01h, B01h, F01b, B01b;
     int rc_back = SMAT_OK;
@@ -399,12 +425,12 @@ extern "C" int smat_scalc(int L0, int L1, const int BoundC[2], double omega, int
         SCK(cudaGetDevice(&dev));
         back = std::thread([&, dev] {
             cudaSetDevice(dev);
-            rc_back = one_way(T2, -1, nlayers, down.data(), omega, XiT, XiB, nT, nB, F01b, B01b);
+            rc_back = one_way(T2, -1, nlayers, in.V, in.XT, in.XB, nT, nB, F01b, B01b);
             if (rc_back) msg_back = smat_last_error();
         });
     }
     /* forward: Smat_calc :148-158 */
-    const int rc_fwd = one_way(T, 1, nlayers, up.data(), omega, XiB, XiT, nB, nT, F01h, B01h);
+    const int rc_fwd = one_way(T, 1, nlayers, in.V, in.XB, in.XT, nB, nT, F01h, B01h);
     if (back.joinable()) back.join();
     RC(rc_fwd);
     if (rc_back) return smat_fail(rc_back, "%s", msg_back.c_str());
@@ -412,7 +438,7 @@ extern "C" int smat_scalc(int L0, int L1, const int BoundC[2], double omega, int
         for (int r = 0; r < N; r++)
             Sm[r + (size_t)N * c] = c < nB ? F01h[r + (size_t)N * c] : B01h[r + (size_t)N * (c - nB)];
     if (both_ways) { /* backward: Smat_calc :159-168 */
-        if (!concurrent) RC(one_way(T, -1, nlayers, down.data(), omega, XiT, XiB, nT, nB, F01b, B01b));
+        if (!concurrent) RC(one_way(T, -1, nlayers, in.V, in.XT, in.XB, nT, nB, F01b, B01b));
         for (int c = nB; c < N; c++) {
             for (int r = nB; r < N; r++) Sm[r + (size_t)N * c] = F01b[(r - nB) + (size_t)N * (c - nB)];
             for (int r = 0; r < nB; r++) Sm[r + (size_t)N * c] = F01b[(r + nT) + (size_t)N * (c - nB)];

@@ -156,6 +156,21 @@ __global__ void k_cut_rows(int m, int k, const double2 *__restrict__ A, int lda,
     }
 }
 
+/* the digits of row t of complex column j in the S images of its tile */
+__device__ __forceinline__ void write_col_slices(unsigned char *__restrict__ img, int ntc, int j, int t,
+                                                 const unsigned short dr[S], const unsigned short di[S])
+{
+    const int tc = j / BNC, jj = j % BNC;
+#pragma unroll
+    for (int l = 0; l < S; l++) {
+        unsigned char *base = img + (size_t)(l * ntc + tc) * BIMG;
+        *reinterpret_cast<unsigned short *>(base + img_off(jj, t)) = dr[l];
+        *reinterpret_cast<unsigned short *>(base + img_off(jj, KC + t)) = (unsigned short)(di[l] ? di[l] ^ 0x8000u : 0u);
+        *reinterpret_cast<unsigned short *>(base + img_off(BNC + jj, t)) = di[l];
+        *reinterpret_cast<unsigned short *>(base + img_off(BNC + jj, KC + t)) = dr[l];
+    }
+}
+
 /* Columns of B (k x n, k <= 32) cut into S slice images of the real
  * [[Br, Bi], [-Bi, Br]]: image (l * ntc + tc) holds, for the complex columns
  * j = 32 tc + jj, row jj = [Br | -Bi] (the Pr column) and row 32 + jj =
@@ -180,15 +195,122 @@ __global__ void k_cut_cols(int k, int n, const double2 *__restrict__ B, int ldb,
     unsigned short dr[S], di[S];
     cut_value(re, e, dr);
     cut_value(im, e, di);
-    const int tc = j / BNC, jj = j % BNC;
-#pragma unroll
-    for (int l = 0; l < S; l++) {
-        unsigned char *base = img + (size_t)(l * ntc + tc) * BIMG;
-        *reinterpret_cast<unsigned short *>(base + img_off(jj, t)) = dr[l];
-        *reinterpret_cast<unsigned short *>(base + img_off(jj, KC + t)) = (unsigned short)(di[l] ? di[l] ^ 0x8000u : 0u);
-        *reinterpret_cast<unsigned short *>(base + img_off(BNC + jj, t)) = di[l];
-        *reinterpret_cast<unsigned short *>(base + img_off(BNC + jj, KC + t)) = dr[l];
+    write_col_slices(img, ntc, j, t, dr, di);
+}
+
+/* ---- a sweep step's operands (dense_z.cu, sweep) --------------------------
+ * Rows: M[i, K] (K = columns [j, j + nb)) of every row after the step's row
+ * moves, cut into slice images as k_cut_rows does (or copied to prow for the
+ * FP64 kernel), and set to zero in M; rows of K itself count as zero.  One
+ * warp per row. */
+__global__ void k_gj_rows(int rows, int j, int nb, double2 *M, int ld, const int *__restrict__ mv,
+                          unsigned char *__restrict__ img, int *__restrict__ ea, int ntr, double2 *__restrict__ prow)
+{
+    const int r = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5), t = threadIdx.x & 31;
+    if (r >= ntr * BM) return;
+    const unsigned hit = __ballot_sync(0xffffffffu, mv[32 + t] == r); /* the row moved here, if any */
+    const int src = hit ? j + __ffs(hit) - 1 : r;
+    double re = 0.0, im = 0.0;
+    if (r < rows && (r < j || r >= j + nb) && t < nb) {
+        const double2 a = M[src + (long long)ld * (j + t)];
+        re = a.x;
+        im = a.y;
+        M[r + (long long)ld * (j + t)] = make_double2(0.0, 0.0);
     }
+    if (prow) {
+        if (r < rows) prow[r + (long long)rows * t] = make_double2(re, im);
+        return;
+    }
+    double mx = fmax(fabs(re), fabs(im));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const int e = row_exponent(mx);
+    if (t == 0 && r < rows) ea[r] = e;
+    unsigned short dr[S], di[S];
+    cut_value(re, e, dr);
+    cut_value(im, e, di);
+    const int tr = r / BM, rr = r % BM;
+#pragma unroll
+    for (int i = 0; i < S; i++) {
+        unsigned char *base = img + (size_t)(i * ntr + tr) * AIMG;
+        *reinterpret_cast<unsigned short *>(base + img_off(rr, t)) = dr[i];
+        *reinterpret_cast<unsigned short *>(base + img_off(rr, KC + t)) = di[i];
+    }
+}
+
+/* Columns: the row moves in every column outside K, then D^-1 (the factors
+ * lud) applied to its rows K (to the unit vectors in the columns K), in place
+ * and cut into slice images as k_cut_cols does (or copied to bcol).  One warp
+ * per column, lane t row j + t; one warp a block, which spreads the columns of
+ * a small matrix over the SMs (258 columns: 16 us, 22 with 8 warps a block;
+ * 1210 columns: 23 us, of which 20 is the FP64 pipe's 250 warp instructions a
+ * column).  Two triangular solves: a product by an explicit D^-1 takes half
+ * the instructions, but loses a digit or more of the result where D is near
+ * singular (1e-12 against 1e-13 on a 10 x 10 grating); several columns to a
+ * warp, which saves the instructions of rows a step no longer touches, has too
+ * few warps (25 us and more).  The first block also moves the entries of
+ * perm. */
+__global__ void __launch_bounds__(32) k_gj_cols(int cols, int j, int nb, double2 *M, int ld, const double2 *__restrict__ lud,
+                                                const int *__restrict__ mv, int *perm, unsigned char *__restrict__ img,
+                                                int *__restrict__ eb, int ntc, double2 *__restrict__ bcol)
+{
+    __shared__ double2 f[KC * KC];
+    const int t = threadIdx.x, c = (int)blockIdx.x;
+    const int from = mv[t], to = mv[32 + t];
+#pragma unroll
+    for (int k = 0; k < KC; k++) f[k * KC + t] = lud[k * KC + t];
+    if (c == 0) {
+        const int pk = t < nb ? perm[from] : 0, pd = t < nb ? perm[j + t] : 0;
+        __syncwarp();
+        if (t < nb) perm[j + t] = pk;
+        if (to >= 0) perm[to] = pd;
+    }
+    double2 *col = M + (long long)ld * c;
+    double2 x = make_double2(0.0, 0.0);
+    if (c >= j && c < j + nb) {
+        x.x = t == c - j ? 1.0 : 0.0;
+    } else if (c < cols) {
+        double2 moved = x;
+        if (t < nb) {
+            x = col[from];
+            moved = col[j + t];
+        }
+        __syncwarp();
+        if (to >= 0) col[to] = moved;
+    }
+    __syncwarp();
+    auto eliminate = [&](int k) { /* x less row t's factor times x_k */
+        const double2 l = f[k * KC + t];
+        const double2 b = make_double2(__shfl_sync(0xffffffffu, x.x, k), __shfl_sync(0xffffffffu, x.y, k));
+        return make_double2(fma(l.y, b.y, fma(-l.x, b.x, x.x)), fma(-l.y, b.x, fma(-l.x, b.y, x.y)));
+    };
+    for (int k = 0; k < nb - 1; k++) {
+        const double2 y = eliminate(k);
+        if (t > k) x = y;
+    }
+    {
+        const double2 d = f[t * (KC + 1)];
+        x = make_double2(fma(-x.y, d.y, x.x * d.x), fma(x.y, d.x, x.x * d.y));
+    }
+    for (int k = nb - 1; k > 0; k--) {
+        const double2 y = eliminate(k);
+        if (t < k) x = y;
+    }
+    if (t >= nb) x = make_double2(0.0, 0.0);
+    if (c < cols && t < nb) col[j + t] = x;
+    if (bcol) {
+        if (c < cols) bcol[t + (long long)KC * c] = x;
+        return;
+    }
+    double mx = fmax(fabs(x.x), fabs(x.y));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const int e = row_exponent(mx);
+    if (t == 0 && c < cols) eb[c] = e;
+    unsigned short dr[S], di[S];
+    cut_value(x.x, e, dr);
+    cut_value(x.y, e, di);
+    write_col_slices(img, ntc, c, t, dr, di);
 }
 
 /* X 2^E through FP64 arithmetic, for results outside the normal range (out
@@ -522,6 +644,33 @@ int zgemm_acc_tc(int m, int n, int k, double2 alpha, const double2 *A, int lda, 
         if (cudaPeekAtLastError() != cudaSuccess)
             return smat_fail(SMAT_ECUDA, "zgemm (tensor cores) launch: %s", cudaGetErrorString(cudaGetLastError()));
     }
+    return SMAT_OK;
+}
+
+int sweep_update(int rows, int cols, int j, int nb, double2 *M, int ld, const SweepWs &w, const GemmCtx &g, cudaStream_t st)
+{
+    const int ntr = (rows + BM - 1) / BM, ntc = (cols + BNC - 1) / BNC;
+    const double2 m1 = make_double2(-1.0, 0.0);
+    if (!g.tc) {
+        k_gj_rows<<<ntr * BM / 8, 256, 0, st>>>(rows, j, nb, M, ld, w.mv, nullptr, nullptr, ntr, w.prow);
+        k_gj_cols<<<ntc * BNC, 32, 0, st>>>(cols, j, nb, M, ld, w.lud, w.mv, w.perm, nullptr, nullptr, ntc, w.bcol);
+        return zgemm_acc(rows, cols, KC, m1, w.prow, rows, w.bcol, KC, M, ld, &g, st);
+    }
+    if (!g.ws || g.ws_bytes < tc_workspace_bytes(rows, cols) || !g.err)
+        return smat_fail(SMAT_EINVAL, "sweep: workspace of %zu bytes for %d x %d, %zu given", tc_workspace_bytes(rows, cols),
+                         rows, cols, g.ws_bytes);
+    if (cudaFuncSetAttribute(k_oz_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
+        return smat_fail(SMAT_ECUDA, "sweep: %d bytes of shared memory refused", SMEM);
+    unsigned char *aimg = static_cast<unsigned char *>(g.ws);
+    unsigned char *bimg = aimg + (size_t)S * ntr * AIMG;
+    int *ea = reinterpret_cast<int *>(bimg + (size_t)S * ntc * BIMG);
+    int *eb = ea + ntr * BM;
+    k_gj_rows<<<ntr * BM / 8, 256, 0, st>>>(rows, j, nb, M, ld, w.mv, aimg, ea, ntr, nullptr);
+    k_gj_cols<<<ntc * BNC, 32, 0, st>>>(cols, j, nb, M, ld, w.lud, w.mv, w.perm, bimg, eb, ntc, nullptr);
+    k_oz_mma<<<dim3((unsigned)ntr, (unsigned)ntc), MMA_THREADS, SMEM, st>>>(
+        rows, cols, m1, aimg, bimg, ea, eb, ntr, ntc, M, ld, g.err, g.wait_limit ? g.wait_limit : WAIT_LIMIT, g.skip_pair);
+    if (cudaPeekAtLastError() != cudaSuccess)
+        return smat_fail(SMAT_ECUDA, "sweep launch: %s", cudaGetErrorString(cudaGetLastError()));
     return SMAT_OK;
 }
 

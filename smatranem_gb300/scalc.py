@@ -40,7 +40,7 @@ def smatrix(meds, omega, L0, L1, bc, XiB, nB, XiT, nT, both_ways=True):
     iB..iT, each (6, L0*L1) complex; XiB / XiT: (4*L0*L1, 4*L0*L1) complex."""
     m = np.ascontiguousarray(np.asarray(meds, np.complex128).reshape(len(meds), 6 * L0 * L1))
     xb = np.asfortranarray(np.asarray(XiB, np.complex128))
-    xt = np.asfortranarray(np.asarray(XiT, np.complex128))
+    xt = xb if XiT is XiB else np.asfortranarray(np.asarray(XiT, np.complex128))  # one upload where the ports are alike
     bcv = np.ascontiguousarray(bc, np.int32)
     N = nB + nT
     S = np.zeros((N, N), np.complex128, order="F")
