@@ -160,19 +160,19 @@ __global__ void __launch_bounds__(256) k_adj_e(const Geo g, const int batch, con
     const int b = blockIdx.y;
     if (l >= g.n3) return;
     const long long n3 = g.n3, bs = 3 * n3;
-    const int x = (int)(l % g.L0), y = (int)((l / g.L0) % g.L1), z = (int)(l / g.pl);
+    const int x = (int)(l % g.P0), y = (int)((l / g.P0) % g.L1), z = (int)(l / g.ps);
+    if (x >= g.L0) return; /* padding */
     const T *PH = s.phiH + b * bs, *QH = s.psiH + b * bs;
     T *PE = s.phiE + b * bs, *QE = s.psiE + b * bs;
     const int j[3] = {x, y, z}, L[3] = {g.L0, g.L1, g.L2};
     long long o_[3];
     T f[3];
-    long long stride = 1;
+    const long long stride[3] = {1, g.P0, g.ps};
 #pragma unroll
     for (int a = 0; a < 3; a++) { /* forward neighbour along a, wrapped with iBc */
         const bool edge = j[a] + 1 == L[a];
-        o_[a] = (edge ? -(long long)(L[a] - 1) : 1LL) * stride;
+        o_[a] = (edge ? -(long long)(L[a] - 1) : 1LL) * stride[a];
         f[a] = edge ? (T)g.bc[a] : (T)1;
-        stride *= L[a];
     }
     T gs[2] = {0, 0};
     if (z == o.zq) {
@@ -210,19 +210,19 @@ __global__ void __launch_bounds__(256) k_adj_h(const Geo g, const int batch, con
     const int b = blockIdx.y;
     if (l >= g.n3) return;
     const long long n3 = g.n3, bs = 3 * n3;
-    const int x = (int)(l % g.L0), y = (int)((l / g.L0) % g.L1), z = (int)(l / g.pl);
+    const int x = (int)(l % g.P0), y = (int)((l / g.P0) % g.L1), z = (int)(l / g.ps);
+    if (x >= g.L0) return; /* padding */
     T *PH = s.phiH + b * bs, *QH = s.psiH + b * bs;
     const T *PE = s.phiE + b * bs, *QE = s.psiE + b * bs;
     const int j[3] = {x, y, z}, L[3] = {g.L0, g.L1, g.L2};
     long long o_[3];
     T f[3];
-    long long stride = 1;
+    const long long stride[3] = {1, g.P0, g.ps};
 #pragma unroll
     for (int a = 0; a < 3; a++) { /* backward neighbour along a, wrapped with iBc */
         const bool edge = j[a] == 0;
-        o_[a] = (edge ? (long long)(L[a] - 1) : -1LL) * stride;
+        o_[a] = (edge ? (long long)(L[a] - 1) : -1LL) * stride[a];
         f[a] = edge ? (T)g.bc[a] : (T)1;
-        stride *= L[a];
     }
     T gs[2] = {0, 0};
     if (z == o.zq) {
@@ -251,7 +251,7 @@ __global__ void k_adj_record(const Geo g, const int batch, const Box bx, const T
     const int b = blockIdx.y;
     if (i >= bx.n) return;
     const int u = (int)(i % bx.nx), v = (int)((i / bx.nx) % bx.ny), w = (int)(i / ((long long)bx.nx * bx.ny));
-    const long long l = (bx.x0 + u) + (long long)g.L0 * ((bx.y0 + v) + (long long)g.L1 * (bx.z0 + w));
+    const long long l = (bx.x0 + u) + (long long)g.P0 * ((bx.y0 + v) + (long long)g.L1 * (bx.z0 + w));
 #pragma unroll
     for (int c = 0; c < 3; c++) dst[((long long)b * 3 + c) * bx.n + i] = E[((long long)b * 3 + c) * g.n3 + l];
 }
@@ -501,7 +501,7 @@ StateView state_view(smat_fdtd_plan *p)
         v.ptr[1] = q.E;
         v.ptr[2] = q.Ha;
         v.ptr[3] = q.Ea;
-        v.bytes[0] = v.bytes[1] = v.bytes[2] = v.bytes[3] = b * 3 * p->n3 * 4;
+        v.bytes[0] = v.bytes[1] = v.bytes[2] = v.bytes[3] = b * 3 * p->n3p * 4;
     }
     return v;
 }
@@ -514,7 +514,7 @@ int zero_state(smat_fdtd_plan *p)
         StateView v = state_view(p);
         for (int i = 0; i < 4; i++) CK(cudaMemsetAsync(v.ptr[i], 0, v.bytes[i], p->stream));
     } else {
-        const size_t n = (size_t)p->batch * 3 * p->n3 * 4;
+        const size_t n = (size_t)p->batch * 3 * p->n3p * 4;
         float *arrs[8] = {p->d_H32, p->d_E32, p->d_Ha32, p->d_Ea32, p->d_H32b, p->d_E32b, p->d_Ha32b, p->d_Ea32b};
         for (float *a : arrs)
             if (a) CK(cudaMemsetAsync(a, 0, n, p->stream));
@@ -551,7 +551,7 @@ int adjoint_run(smat_fdtd_plan *p, const C &coef, int nsteps, int K, int f, int 
 {
     Scratch sc;
     sc.st = p->stream;
-    const long long n3 = p->n3;
+    const long long n3 = p->n3p;
     const int batch = p->batch, pl = p->pl;
     const int nseg = (nsteps + K - 1) / K;
     StateView sv = state_view(p);

@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(256) k_sweep32(const P32 p, const int rel, con
 
 /* ---------------------------------------------------------------------------
  * Vectorised sweep: four consecutive x-cells per thread (float4 loads and
- * stores), for L0 % 4 == 0.  Every element is updated with exactly the
+ * stores), for L0 % 4 == 0 or padded rows.  Every element is updated with exactly the
  * expressions of k_sweep32, so the two kernels give the same bits; what changes
  * is that a thread keeps four cells' worth of loads in flight, which is what
  * the HBM needs (the six curl neighbours of a cell are mostly cache hits, so a
@@ -443,18 +443,21 @@ __device__ __forceinline__ void quad_compute(const P32 &p, const int rel, const 
     }
 }
 
-/* one quad row segment: cells x = xr..xr+3 of row j1, plane j2, excitation b;
- * a warp covers 128 consecutive x-cells (lane = threadIdx.x) */
-template <bool EF, bool CG>
+/* one quad: cells x = xr..xr+3 of row j1, plane j2, excitation b; the lanes of a
+ * warp hold consecutive quads.  PAD: rows of padded length, whose last quad is
+ * cut off at L0 -- its cells past L0 neither wrap, nor take the source, nor are
+ * sampled; lanes that are not in repeat a live quad and store nothing. */
+template <bool EF, bool CG, bool PAD>
 __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const int b, const int j1, const int j2,
-                                              const int xr)
+                                              const int xr, const bool in)
 {
     const Geo &g = p.g;
-    if (j1 >= g.L1) return; /* uniform per warp */
-    const bool live = xr < g.L0;
-    const int x0 = live ? xr : g.L0 - 4; /* idle lanes load valid data, store nothing */
+    if (!PAD && j1 >= g.L1) return; /* uniform per warp */
+    const int P0 = PAD ? g.P0 : g.L0;
+    const bool live = PAD ? in : xr < g.L0;
+    const int x0 = PAD || live ? xr : g.L0 - 4; /* idle lanes load valid data, store nothing */
     const long long n3 = g.n3, bs = 3 * n3;
-    const long long l = x0 + (long long)g.L0 * (j1 + (long long)g.L1 * j2);
+    const long long l = x0 + (long long)P0 * (j1 + (long long)g.L1 * j2);
     const float *__restrict__ cf = EF ? p.be : p.bh;
     float *__restrict__ F = (EF ? p.E : p.H) + b * bs;
     float *__restrict__ Fa = (EF ? p.Ea : p.Ha) + b * bs;
@@ -466,14 +469,16 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
     /* neighbours along y and z (whole quads) with the boundary factor */
     const bool ey = EF ? (j1 + 1 == g.L1) : (j1 == 0);
     const bool ez = EF ? (j2 + 1 == g.L2) : (j2 == 0);
-    const long long oy = (long long)g.L0 * (EF ? (ey ? -(g.L1 - 1) : 1) : (ey ? g.L1 - 1 : -1));
-    const long long oz = (long long)g.pl * (EF ? (ez ? -(g.L2 - 1) : 1) : (ez ? g.L2 - 1 : -1));
+    const long long oy = (long long)P0 * (EF ? (ey ? -(g.L1 - 1) : 1) : (ey ? g.L1 - 1 : -1));
+    const long long oz = (long long)(PAD ? g.ps : g.pl) * (EF ? (ez ? -(g.L2 - 1) : 1) : (ez ? g.L2 - 1 : -1));
     const float fy = ey ? (float)g.bc[1] : 1.0f, fz = ez ? (float)g.bc[2] : 1.0f;
 
     /* split-PML quads need their aux slots: decided from the 1-D masks before
      * any load, so that those loads leave with the others (one DRAM round trip) */
     const bool pyz = p.pmask[s1 + j1] | p.pmask[s2 + j2];
-    const bool qsplit = pyz | p.pmask[x0] | p.pmask[x0 + 1] | p.pmask[x0 + 2] | p.pmask[x0 + 3];
+    const bool qsplit = PAD ? pyz | p.pmask[x0] | (x0 + 1 < g.L0 && p.pmask[x0 + 1]) |
+                                  (x0 + 2 < g.L0 && p.pmask[x0 + 2]) | (x0 + 3 < g.L0 && p.pmask[x0 + 3])
+                            : pyz | p.pmask[x0] | p.pmask[x0 + 1] | p.pmask[x0 + 2] | p.pmask[x0 + 3];
     float4 c[3], out[3], gh[3], aux[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) {
@@ -481,36 +486,39 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
         out[i] = ld4(F + i * n3 + l);
         gh[i] = ldG4<CG>(G + i * n3 + l);
     }
+    /* H sweep: Ex, Ez at y-1; Ex, Ey at z-1.  E sweep: Hx, Hz at y+1; Hx, Hy at z+1. */
+    float4 gy0 = ldG4<CG>(G + 0 * n3 + l + oy), gy2 = ldG4<CG>(G + 2 * n3 + l + oy);
+    float4 gz0 = ldG4<CG>(G + 0 * n3 + l + oz), gz1 = ldG4<CG>(G + 1 * n3 + l + oz);
+    /* the outer x neighbour (H sweep: Ey, Ez at x-1; E sweep: Hy, Hz at x+1) is
+     * the next lane's, or at the end of a warp or row loaded with the others */
+    const bool edge = EF ? x0 + 4 == P0 : x0 == 0, own_xn = edge | ((threadIdx.x & 31) == (EF ? 31 : 0));
+    float xn1 = 0.0f, xn2 = 0.0f; /* its components 1, 2 */
+    if (own_xn) {
+        const long long o = EF ? (edge ? -(P0 - 4) : 4) : (edge ? g.L0 - 1 : -1);
+        xn1 = ldG<CG>(G + 1 * n3 + l + o);
+        xn2 = ldG<CG>(G + 2 * n3 + l + o);
+    }
     if (qsplit) {
 #pragma unroll
         for (int i = 0; i < 3; i++) aux[i] = ld4(Fa + i * n3 + l);
     }
-    /* H sweep: Ex, Ez at y-1; Ex, Ey at z-1.  E sweep: Hx, Hz at y+1; Hx, Hy at z+1. */
-    const float4 gy0 = scale4(ldG4<CG>(G + 0 * n3 + l + oy), fy), gy2 = scale4(ldG4<CG>(G + 2 * n3 + l + oy), fy);
-    const float4 gz0 = scale4(ldG4<CG>(G + 0 * n3 + l + oz), fz), gz1 = scale4(ldG4<CG>(G + 1 * n3 + l + oz), fz);
-    /* x neighbours: H sweep needs Ey, Ez at x-1; E sweep Hy, Hz at x+1 */
+    gy0 = scale4(gy0, fy);
+    gy2 = scale4(gy2, fy);
+    gz0 = scale4(gz0, fz);
+    gz1 = scale4(gz1, fz);
     const unsigned full = 0xffffffffu;
-    float xn1, xn2; /* component 1, 2 of the outer neighbour of the quad */
-    if (!EF) {
-        xn1 = __shfl_up_sync(full, gh[1].w, 1);
-        xn2 = __shfl_up_sync(full, gh[2].w, 1);
-        if ((threadIdx.x & 31) == 0 || x0 == 0) {
-            const bool edge = x0 == 0;
-            const long long o = edge ? g.L0 - 1 : -1;
-            const float f = edge ? (float)g.bc[0] : 1.0f;
-            xn1 = f * ldG<CG>(G + 1 * n3 + l + o);
-            xn2 = f * ldG<CG>(G + 2 * n3 + l + o);
-        }
-    } else {
-        xn1 = __shfl_down_sync(full, gh[1].x, 1);
-        xn2 = __shfl_down_sync(full, gh[2].x, 1);
-        if ((threadIdx.x & 31) == 31 || x0 + 4 == g.L0) {
-            const bool edge = x0 + 4 == g.L0;
-            const long long o = edge ? -(g.L0 - 4) : 4;
-            const float f = edge ? (float)g.bc[0] : 1.0f;
-            xn1 = f * ldG<CG>(G + 1 * n3 + l + o);
-            xn2 = f * ldG<CG>(G + 2 * n3 + l + o);
-        }
+    const float s1n = EF ? __shfl_down_sync(full, gh[1].x, 1) : __shfl_up_sync(full, gh[1].w, 1);
+    const float s2n = EF ? __shfl_down_sync(full, gh[2].x, 1) : __shfl_up_sync(full, gh[2].w, 1);
+    const float fx = edge ? (float)g.bc[0] : 1.0f;
+    xn1 = own_xn ? fx * xn1 : s1n;
+    xn2 = own_xn ? fx * xn2 : s2n;
+    if (PAD && EF && edge) { /* the wrapped neighbour of cell L0-1 lies in the quad's own padding */
+#pragma unroll
+        for (int i = 1; i < 4; i++)
+            if (x0 + i == g.L0) {
+                set_el(gh[1], i, xn1);
+                set_el(gh[2], i, xn2);
+            }
     }
     if (!live) return;
     const bool on_src = j2 == p.s.iI[b];
@@ -550,6 +558,7 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
             any_aux = true;
             continue;
         }
+        if (PAD && xx >= g.L0) continue; /* padding: stays 0 */
         const bool split = p.pmask[xx] | pyz;
         const float bn[3] = {c0, el(c[1], i), el(c[2], i)};
         if (!split) {
@@ -576,7 +585,7 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
         for (int i = 0; i < 4; i++) {
             const int xx = x0 + i;
             const float c0 = el(c[0], i);
-            if (isnan(c0)) continue;
+            if (isnan(c0) || (PAD && xx >= g.L0)) continue;
             if (!(p.pmask[xx] | pyz)) continue;
             const float h0 = el(gh[0], i), h1 = el(gh[1], i), h2 = el(gh[2], i);
             float n1x, n2x;
@@ -627,8 +636,18 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
     }
     if (q >= 0) {
         /* split elements sample the total field, ordinary ones their field */
-        st4(ring_at(p.d, g.pl, b, k, q, EF ? 2 : 0) + px0, out[0]);
-        st4(ring_at(p.d, g.pl, b, k, q, EF ? 3 : 1) + px0, out[1]);
+        float *r0 = ring_at(p.d, g.pl, b, k, q, EF ? 2 : 0) + px0, *r1 = ring_at(p.d, g.pl, b, k, q, EF ? 3 : 1) + px0;
+        if (PAD) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (x0 + i < g.L0) {
+                    r0[i] = el(out[0], i);
+                    r1[i] = el(out[1], i);
+                }
+        } else {
+            st4(r0, out[0]);
+            st4(r1, out[1]);
+        }
     }
 }
 
@@ -641,7 +660,24 @@ __global__ void __launch_bounds__(128, MB) k_sweep32v(const P32 p, const int rel
     const int b = blockIdx.y % p.batch;
     const int xr = (blockIdx.x * 32 + threadIdx.x) * 4;
     const int j1 = (blockIdx.y / p.batch) * blockDim.y + threadIdx.y;
-    sweep32v_quad<EF, false>(p, rel, b, j1, z0 + blockIdx.z, xr);
+    sweep32v_quad<EF, false, false>(p, rel, b, j1, z0 + blockIdx.z, xr, true);
+}
+
+/* The vectorised sweep of padded rows (L0 % 4 != 0).  The quads of a plane are
+ * dealt out to the threads one after another, whatever their row: rows of any
+ * length fill the warps (in a warp per row piece, the 33 quads of 131 cells
+ * would fill 52 % of the lanes).  Bound by the latency of a quad's loads:
+ * 131 x 117 x 103 cells of two excitations 138 us a step before (one cell per
+ * thread), 83 us now, 3.2 TB/s of the compulsory 84 B a cell; 96 registers
+ * (128: 88 us, 80: 91 us).  Block x: quads of the plane x excitation
+ * (fastest, for the shared coefficients), y: the plane. */
+template <bool EF>
+__global__ void __launch_bounds__(128, 5) k_sweep32p(const P32 p, const int rel, const int z0)
+{
+    const int b = blockIdx.x % p.batch, nq = p.g.P0 >> 2;
+    const int i = blockIdx.x / p.batch * blockDim.x + threadIdx.x, last = nq * p.g.L1 - 1;
+    const int u = i <= last ? i : last, j1 = u / nq;
+    sweep32v_quad<EF, false, true>(p, rel, b, j1, z0 + blockIdx.y, 4 * (u - j1 * nq), i <= last);
 }
 
 /* general cells of the vectorised sweeps: one thread per record cell, run
@@ -651,7 +687,7 @@ __device__ void general32_cell(const P32 &p, const int rel, const int b, const l
 {
     const Geo &g = p.g;
     const long long n3 = g.n3, bs = 3 * n3;
-    const int j0 = (int)(l % g.L0), j1 = (int)((l / g.L0) % g.L1), j2 = (int)(l / g.pl);
+    const int j0 = (int)(l % g.P0), j1 = (int)((l / g.P0) % g.L1), j2 = (int)(l / g.ps);
     const float *__restrict__ cf = EF ? p.be : p.bh;
     float *F = (EF ? p.E : p.H) + b * bs, *Fa = (EF ? p.Ea : p.Ha) + b * bs;
     const float *G = (EF ? p.H : p.E) + b * bs, *Ga = (EF ? p.Ha : p.Ea) + b * bs;
@@ -746,7 +782,7 @@ __global__ void __launch_bounds__(128, 5) k_group32v(const int rel)
     const int yb = t % nyb, z = t / nyb;
     const int b = yb % p.batch;
     const int j1 = (yb / p.batch) * blockDim.y + threadIdx.y;
-    sweep32v_quad<EF, false>(p, rel, b, j1, z, (xb * 32 + threadIdx.x) * 4);
+    sweep32v_quad<EF, false, false>(p, rel, b, j1, z, (xb * 32 + threadIdx.x) * 4, true);
 }
 
 template <bool EF>
@@ -951,6 +987,25 @@ void launch_e32v(const P32 &p, int rel, int by, int mb, int z0, int z1, const in
 {
     launch_sweep32v<true>(p, rel, by, mb, z0, z1, st);
     if (nge > 0) k_general32<true><<<dim3((nge + 127) / 128, p.batch), 128, 0, st>>>(p, rel, gcells, nge);
+}
+
+template <bool EF>
+static void launch_sweep32p(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng,
+                            cudaStream_t st)
+{
+    const int nq = p.g.P0 / 4 * p.g.L1;
+    k_sweep32p<EF><<<dim3((nq + threads - 1) / threads * p.batch, z1 - z0), threads, 0, st>>>(p, rel, z0);
+    if (ng > 0) k_general32<EF><<<dim3((ng + 127) / 128, p.batch), 128, 0, st>>>(p, rel, gcells, ng);
+}
+
+void launch_h32p(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng, cudaStream_t st)
+{
+    launch_sweep32p<false>(p, rel, threads, z0, z1, gcells, ng, st);
+}
+
+void launch_e32p(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng, cudaStream_t st)
+{
+    launch_sweep32p<true>(p, rel, threads, z0, z1, gcells, ng, st);
 }
 
 void launch_flush32(const P32 &p, int rel_end, int count, cudaStream_t st)

@@ -21,6 +21,9 @@
  *                                 by 1-D sigma tables; cells needing anything else
  *                                 carry NaN in component 0 and a record index in
  *                                 component 1 ("general" cells, a short list)
+ *     Rows of L0 % 4 != 0 cells may be padded to P0 = the next multiple of 4
+ *     (padded_rows: l = j0 + P0*j1 + P0*L1*j2), for 16-byte loads.  The cells
+ *     past L0 have coefficients and fields 0, which every sweep leaves so.
  */
 #ifndef SMATRAN_FDTD_INTERNAL_CUH
 #define SMATRAN_FDTD_INTERNAL_CUH
@@ -38,7 +41,9 @@ constexpr int MAX_PLANES = 8;
 
 struct Geo {
     int L0, L1, L2, pl; /* pl = L0*L1 */
-    long long n3;       /* L0*L1*L2 */
+    int P0, ps;         /* cells from row to row and from plane to plane: L0 and
+                         * pl, or in FP32 plans of padded rows more */
+    long long n3;       /* ps*L2 */
     int bc[3];          /* iBc */
     int iI;             /* source plane */
     double sgn;         /* iBTIin[3]/|iBTIin[3]| */
@@ -205,14 +210,13 @@ __device__ __forceinline__ Stn32 make_stn32(const Geo &g, int j0, int j1, int j2
     Stn32 st;
     const int j[3] = {j0, j1, j2};
     const int L[3] = {g.L0, g.L1, g.L2};
-    long long stride = 1;
+    const long long stride[3] = {1, g.P0, g.ps};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         const bool edge = fwd ? (j[a] + 1 == L[a]) : (j[a] == 0);
         const int jn = fwd ? (edge ? 0 : j[a] + 1) : (edge ? L[a] - 1 : j[a] - 1);
-        st.o[a] = (long long)(jn - j[a]) * stride;
+        st.o[a] = (jn - j[a]) * stride[a];
         st.f[a] = edge ? (float)g.bc[a] : 1.0f;
-        stride *= L[a];
     }
     return st;
 }
@@ -243,6 +247,9 @@ void launch_e64(const P64 &p, int rel, cudaStream_t st);
 void launch_flush64(const P64 &p, int rel_end, int count, cudaStream_t st);
 void launch_h32(const P32 &p, int rel, int by, int z0, int z1, cudaStream_t st);
 void launch_e32(const P32 &p, int rel, int by, int z0, int z1, cudaStream_t st);
+/* the sweeps of padded rows, threads threads a block; gcells / ng as above */
+void launch_h32p(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng, cudaStream_t st);
+void launch_e32p(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng, cudaStream_t st);
 void launch_flush32(const P32 &p, int rel_end, int count, cudaStream_t st);
 /* mb: register bound of the vectorised sweep (minimum resident blocks: 5, 6 or 8) */
 void launch_h32v(const P32 &p, int rel, int by, int mb, int z0, int z1, const int *gcells, int ngh, cudaStream_t st);

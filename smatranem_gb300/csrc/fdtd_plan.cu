@@ -35,7 +35,9 @@ Geo make_geo(const smat_fdtd_plan *p)
     g.L1 = p->L[1];
     g.L2 = p->L[2];
     g.pl = p->pl;
-    g.n3 = p->n3;
+    g.P0 = p->P0;
+    g.ps = p->P0 * p->L[1];
+    g.n3 = p->n3p;
     for (int a = 0; a < 3; a++) g.bc[a] = p->iBc[a];
     g.iI = p->iBTIin[2];
     const int m = p->iBTIin[3];
@@ -195,6 +197,28 @@ void launch_row_step(smat_fdtd_plan *p, bool xp, int rel, cudaStream_t st)
     p->cur ^= 1;
 }
 
+/* threads of a block of the padded rows' sweeps: 32 x block_y, at most 128 */
+static int padded_threads(const smat_fdtd_plan *p) { return 32 * (p->by32 < 4 ? p->by32 : 4); }
+
+/* the H (E) sweep of kernel 0 or 2 on planes [z0, z1), with its general cells */
+static void sweep_h(const smat_fdtd_plan *p, const P32 &q, int rel, int z0, int z1, cudaStream_t st)
+{
+    const int *gen = p->d_hgen + p->hgen_z[z0];
+    const int n = p->hgen_z[z1] - p->hgen_z[z0];
+    if (p->fused == 2) launch_h32v(q, rel, p->by32, p->sweep_mb, z0, z1, gen, n, st);
+    else if (p->P0 != p->L[0]) launch_h32p(q, rel, padded_threads(p), z0, z1, gen, n, st);
+    else launch_h32(q, rel, p->by32, z0, z1, st);
+}
+
+static void sweep_e(const smat_fdtd_plan *p, const P32 &q, int rel, int z0, int z1, cudaStream_t st)
+{
+    const int *gen = p->d_egen + p->egen_z[z0];
+    const int n = p->egen_z[z1] - p->egen_z[z0];
+    if (p->fused == 2) launch_e32v(q, rel, p->by32, p->sweep_mb, z0, z1, gen, n, st);
+    else if (p->P0 != p->L[0]) launch_e32p(q, rel, padded_threads(p), z0, z1, gen, n, st);
+    else launch_e32(q, rel, p->by32, z0, z1, st);
+}
+
 /* One FP32 step as two sweeps (kernels 0 and 2), in z-chunks of szc planes:
  * H on planes [z0, z1), then E on [z0-1, z1-1) -- E of a plane needs H_new of
  * the plane above, H of a plane needs E_old of the plane below, and both
@@ -210,16 +234,8 @@ void sweep_step(smat_fdtd_plan *p, const P32 &q, int rel, cudaStream_t st)
     for (int z0 = 0; z0 < L2; z0 += zc) {
         const int z1 = z0 + zc < L2 ? z0 + zc : L2;
         const int e0 = z0 == 0 ? 0 : z0 - 1, e1 = z1 == L2 ? L2 : z1 - 1;
-        if (p->fused == 2) {
-            launch_h32v(q, rel, p->by32, p->sweep_mb, z0, z1, p->d_hgen + p->hgen_z[z0],
-                        p->hgen_z[z1] - p->hgen_z[z0], st);
-            if (e1 > e0)
-                launch_e32v(q, rel, p->by32, p->sweep_mb, e0, e1, p->d_egen + p->egen_z[e0],
-                            p->egen_z[e1] - p->egen_z[e0], st);
-        } else {
-            launch_h32(q, rel, p->by32, z0, z1, st);
-            if (e1 > e0) launch_e32(q, rel, p->by32, e0, e1, st);
-        }
+        sweep_h(p, q, rel, z0, z1, st);
+        if (e1 > e0) sweep_e(p, q, rel, e0, e1, st);
     }
 }
 
@@ -393,6 +409,18 @@ int validate_common(const int L[4], const int iBc[3], const int iBTIin[4], int b
     return SMAT_OK;
 }
 
+/* FP32 rows of L0 % 4 != 0 cells are padded for the vectorised sweeps, which
+ * a few warps' worth of quads cannot keep busy: small plans run the
+ * one-cell-per-thread sweeps.  The two meet near 220000 cells (us a step, one
+ * cell per thread / padded: 131 x 40 x 40 14.7 / 15.8, 33 x 60 x 60 of two
+ * excitations 19.8 / 16.0, 131 x 117 x 103 of two 138 / 83, 321 x 200 x 150
+ * 320 / 205).  Rows under 20 cells would grow by more than 15 %. */
+bool padded_rows(const int L[4], int batch)
+{
+    const long long n = (L[0] + 3LL) / 4 * 4 * L[1] * L[2];
+    return L[0] % 4 != 0 && L[0] >= 20 && n * batch >= 220000 && n < (1LL << 31) / 3;
+}
+
 smat_fdtd_plan *new_plan(const int L[4], const int iBc[3], const int iBTIin[4], int precision, int batch,
                          void *stream)
 {
@@ -405,6 +433,8 @@ smat_fdtd_plan *new_plan(const int L[4], const int iBc[3], const int iBTIin[4], 
     p->batch = batch;
     p->n3 = (long long)L[0] * L[1] * L[2];
     p->pl = L[0] * L[1];
+    p->P0 = precision == SMAT_FP32 && padded_rows(L, batch) ? (L[0] + 3) / 4 * 4 : L[0];
+    p->n3p = (long long)p->P0 * L[1] * L[2];
     if (stream) {
         p->stream = (cudaStream_t)stream;
     } else {
@@ -490,8 +520,15 @@ int upload_f32(smat_fdtd_plan *p, const smat_fdtd_desc *d, const double *Ah, con
     const long long n3 = p->n3;
     const double iR = d->invtau_R, iI = d->invtau_I;
     const double *mu = d->mu, *ep = d->epsi;
-    std::unique_ptr<float[]> bh(new (std::nothrow) float[3 * n3]), be(new (std::nothrow) float[3 * n3]);
+    const long long n3p = p->n3p; /* cells of the packed arrays: dl(l) of cell l */
+    const int L0 = p->L[0], P0 = p->P0;
+    auto dl = [=](long long l) { return P0 == L0 ? l : l + l / L0 * (P0 - L0); };
+    std::unique_ptr<float[]> bh(new (std::nothrow) float[3 * n3p]), be(new (std::nothrow) float[3 * n3p]);
     if (!bh || !be) return smat_fail(SMAT_ENOMEM, "create: out of host memory for the packed coefficients");
+    if (P0 != L0) { /* the padding */
+        memset(bh.get(), 0, 12 * (size_t)n3p);
+        memset(be.get(), 0, 12 * (size_t)n3p);
+    }
     auto aux = [&](long long l, int c) { return (size_t)c + 3 * (size_t)(n3 + p->addr[l]); };
     /* The cells go over host worker threads in runs of whole z planes.  Each
      * run numbers its records from 0 in cell order and keeps the cells they
@@ -527,7 +564,7 @@ int upload_f32(smat_fdtd_plan *p, const smat_fdtd_desc *d, const double *Ah, con
                 else if (k == 'a')
                     simple = lossless;
                 if (simple) {
-                    for (int c = 0; c < 3; c++) cf[c * n3 + l] = (float)(1. / (iR * m[2 * (3 * l + c)]));
+                    for (int c = 0; c < 3; c++) cf[c * n3p + dl(l)] = (float)(1. / (iR * m[2 * (3 * l + c)]));
                     continue;
                 }
                 /* a record: everything else (a few per mille of the cells) */
@@ -554,11 +591,12 @@ int upload_f32(smat_fdtd_plan *p, const smat_fdtd_desc *d, const double *Ah, con
                 }
                 /* the coefficient slot holds NaN, the next one the record number */
                 const int idx = (int)run.rec[side].size();
-                cf[l] = std::nanf("");
-                memcpy(&cf[n3 + l], &idx, 4);
-                cf[2 * n3 + l] = 0.0f;
+                const long long ld = dl(l);
+                cf[ld] = std::nanf("");
+                memcpy(&cf[n3p + ld], &idx, 4);
+                cf[2 * n3p + ld] = 0.0f;
                 run.rec[side].push_back(r);
-                run.cell[side].push_back((int)l);
+                run.cell[side].push_back((int)ld);
             }
         }
     };
@@ -583,7 +621,7 @@ int upload_f32(smat_fdtd_plan *p, const smat_fdtd_desc *d, const double *Ah, con
             if (base)
                 for (size_t i = 0; i < run.cell[side].size(); i++) {
                     const int idx = base + (int)i;
-                    memcpy(&cf[n3 + run.cell[side][i]], &idx, 4);
+                    memcpy(&cf[n3p + run.cell[side][i]], &idx, 4);
                 }
             recs.insert(recs.end(), run.rec[side].begin(), run.rec[side].end());
             gen.insert(gen.end(), run.cell[side].begin(), run.cell[side].end());
@@ -604,10 +642,10 @@ int upload_f32(smat_fdtd_plan *p, const smat_fdtd_desc *d, const double *Ah, con
             tab[3 * S + aoff[a] + j] = (float)(iR / (iR + iI * se));
             pmask[aoff[a] + j] = std::fabs(sh) > 10.0 * 2.220446049250313e-16 || std::fabs(se) > 10.0 * 2.220446049250313e-16;
         }
-    if ((rc = p->alloc(&p->d_bh, 3 * (size_t)n3)) || (rc = p->alloc(&p->d_be, 3 * (size_t)n3))) return rc;
+    if ((rc = p->alloc(&p->d_bh, 3 * (size_t)n3p)) || (rc = p->alloc(&p->d_be, 3 * (size_t)n3p))) return rc;
     if ((rc = p->alloc(&p->d_tab, 4 * (size_t)S)) || (rc = p->alloc(&p->d_pmask, (size_t)S))) return rc;
     if ((rc = p->alloc(&p->d_hrec, hrec.size() + 1)) || (rc = p->alloc(&p->d_erec, erec.size() + 1))) return rc;
-    const size_t fs = (size_t)p->batch * 3 * n3;
+    const size_t fs = (size_t)p->batch * 3 * n3p;
     if ((rc = p->alloc(&p->d_H32, fs)) || (rc = p->alloc(&p->d_E32, fs))) return rc;
     if ((rc = p->alloc(&p->d_Ha32, fs)) || (rc = p->alloc(&p->d_Ea32, fs))) return rc;
     if ((rc = p->alloc(&p->d_H32b, fs)) || (rc = p->alloc(&p->d_E32b, fs))) return rc;
@@ -621,7 +659,7 @@ int upload_f32(smat_fdtd_plan *p, const smat_fdtd_desc *d, const double *Ah, con
     p->hgen_z.assign(p->L[2] + 1, 0);
     p->egen_z.assign(p->L[2] + 1, 0);
     for (int z = 0; z <= p->L[2]; z++) {
-        const long long first = (long long)z * p->pl;
+        const long long first = (long long)z * P0 * p->L[1];
         p->hgen_z[z] = (int)(std::lower_bound(hgen.begin(), hgen.end(), first) - hgen.begin());
         p->egen_z[z] = (int)(std::lower_bound(egen.begin(), egen.end(), first) - egen.begin());
     }
@@ -668,8 +706,8 @@ int upload_f32(smat_fdtd_plan *p, const smat_fdtd_desc *d, const double *Ah, con
         if ((rc = p->alloc(&p->d_qorder, (size_t)nq))) return rc;
         CK(p->cpy(p->d_qorder, qorder.data(), nq * sizeof(int), cudaMemcpyHostToDevice));
     }
-    CK(p->cpy(p->d_bh, bh.get(), 3 * (size_t)n3 * 4, cudaMemcpyHostToDevice));
-    CK(p->cpy(p->d_be, be.get(), 3 * (size_t)n3 * 4, cudaMemcpyHostToDevice));
+    CK(p->cpy(p->d_bh, bh.get(), 3 * (size_t)n3p * 4, cudaMemcpyHostToDevice));
+    CK(p->cpy(p->d_be, be.get(), 3 * (size_t)n3p * 4, cudaMemcpyHostToDevice));
     CK(p->cpy(p->d_tab, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice));
     CK(p->cpy(p->d_pmask, pmask.data(), pmask.size(), cudaMemcpyHostToDevice));
     if (!hrec.empty())
@@ -823,6 +861,12 @@ extern "C" int smat_fdtd_info(const smat_fdtd_plan *p, int L[4], int *Lnotn, int
 
 extern "C" long long smat_fdtd_device_bytes(const smat_fdtd_plan *p) { return p ? p->dev_bytes : 0; }
 
+/* cell l of the grid in a device array */
+static long long device_cell(const smat_fdtd_plan *p, long long l)
+{
+    return p->P0 == p->L[0] ? l : l + l / p->L[0] * (p->P0 - p->L[0]);
+}
+
 extern "C" int smat_fdtd_set_fields(smat_fdtd_plan *p, int b, const double *H_t, const double *E_t)
 {
     smat_clear_error();
@@ -843,17 +887,19 @@ extern "C" int smat_fdtd_set_fields(smat_fdtd_plan *p, int b, const double *H_t,
             CK(p->cpy(da, a.data(), a.size() * 8, cudaMemcpyHostToDevice));
             CK(cudaStreamSynchronize(p->stream));
         } else {
-            std::vector<float> t(3 * n3), a(3 * n3, 0.0f);
+            const long long n3p = p->n3p;
+            std::vector<float> t(3 * n3p, 0.0f), a(3 * n3p, 0.0f);
             for (int c = 0; c < 3; c++)
                 for (long long l = 0; l < n3; l++) {
+                    const long long ld = c * n3p + device_cell(p, l);
                     double main = src[c + 3 * l], ax = 0.0;
                     if (p->cont[l] != 'n') ax = src[c + 3 * (n3 + p->addr[l])];
-                    t[c * n3 + l] = (float)(main + ax);
-                    a[c * n3 + l] = (float)ax;
+                    t[ld] = (float)(main + ax);
+                    a[ld] = (float)ax;
                 }
             const P32 q = make_p32(p, false);
-            float *dt = (w ? q.E : q.H) + (size_t)b * 3 * n3;
-            float *da = (w ? q.Ea : q.Ha) + (size_t)b * 3 * n3;
+            float *dt = (w ? q.E : q.H) + (size_t)b * 3 * n3p;
+            float *da = (w ? q.Ea : q.Ha) + (size_t)b * 3 * n3p;
             CK(p->cpy(dt, t.data(), t.size() * 4, cudaMemcpyHostToDevice));
             CK(p->cpy(da, a.data(), a.size() * 4, cudaMemcpyHostToDevice));
             CK(cudaStreamSynchronize(p->stream));
@@ -886,21 +932,23 @@ extern "C" int smat_fdtd_get_fields(smat_fdtd_plan *p, int b, double *H_t, doubl
                 dst[c + 3 * (n3 + ln)] = 0.0; /* the sentinel */
             }
         } else {
-            std::vector<float> t(3 * n3), a(3 * n3);
+            const long long n3p = p->n3p;
+            std::vector<float> t(3 * n3p), a(3 * n3p);
             const P32 q = make_p32(p, false);
-            const float *dt = (w ? q.E : q.H) + (size_t)b * 3 * n3;
-            const float *da = (w ? q.Ea : q.Ha) + (size_t)b * 3 * n3;
+            const float *dt = (w ? q.E : q.H) + (size_t)b * 3 * n3p;
+            const float *da = (w ? q.Ea : q.Ha) + (size_t)b * 3 * n3p;
             CK(p->cpy(t.data(), dt, t.size() * 4, cudaMemcpyDeviceToHost));
             CK(p->cpy(a.data(), da, a.size() * 4, cudaMemcpyDeviceToHost));
             CK(cudaStreamSynchronize(p->stream));
             memset(dst, 0, sizeof(double) * 3 * (size_t)(n3 + ln + 1));
             for (int c = 0; c < 3; c++)
                 for (long long l = 0; l < n3; l++) {
+                    const long long ld = c * n3p + device_cell(p, l);
                     if (p->cont[l] == 'n') {
-                        dst[c + 3 * l] = t[c * n3 + l];
+                        dst[c + 3 * l] = t[ld];
                     } else {
-                        const float ax = a[c * n3 + l];
-                        dst[c + 3 * l] = (double)(t[c * n3 + l] - ax);
+                        const float ax = a[ld];
+                        dst[c + 3 * l] = (double)(t[ld] - ax);
                         dst[c + 3 * (n3 + p->addr[l])] = ax;
                     }
                 }
@@ -1088,17 +1136,12 @@ extern "C" int smat_fdtd_time_kernels(smat_fdtd_plan *p, int k_begin, int nsteps
             launch_row_step(p, false, i, p->stream);
         } else if (p->szc > 0 && p->szc < p->L[2]) {
             sweep_step(p, q32, i, p->stream); /* chunked sweeps: the whole step in ms[0] */
-        } else if (p->fused == 2) {
-            launch_h32v(q32, i, p->by32, p->sweep_mb, 0, p->L[2], p->d_hgen, p->nhgen, p->stream);
         } else {
-            launch_h32(q32, i, p->by32, 0, p->L[2], p->stream);
+            sweep_h(p, q32, i, 0, p->L[2], p->stream);
         }
         CK(cudaEventRecord(ev[1], p->stream));
         if (p->precision == SMAT_FP64) launch_e64(q64, i, p->stream);
-        else if (p->fused == 6 || (p->szc > 0 && p->szc < p->L[2])) {
-        } else if (p->fused == 2)
-            launch_e32v(q32, i, p->by32, p->sweep_mb, 0, p->L[2], p->d_egen, p->negen, p->stream);
-        else if (p->fused == 0) launch_e32(q32, i, p->by32, 0, p->L[2], p->stream);
+        else if (p->fused != 6 && !(p->szc > 0 && p->szc < p->L[2])) sweep_e(p, q32, i, 0, p->L[2], p->stream);
         CK(cudaEventRecord(ev[2], p->stream));
         if ((i + 1) % RING_K == 0 || i + 1 == nsteps) {
             const int cnt = (i + 1) % RING_K == 0 ? RING_K : (i + 1) % RING_K;
@@ -1395,7 +1438,7 @@ extern "C" int smat_fdtd_check_finite(smat_fdtd_plan *p, int *finite, double *ma
     if (!p) return smat_fail(SMAT_EINVAL, "null plan");
     CK(cudaMemsetAsync(p->d_scratch, 0, 8, p->stream));
     const bool d = p->precision == SMAT_FP64;
-    const long long nf = (long long)p->batch * 3 * p->n3;
+    const long long nf = (long long)p->batch * 3 * p->n3p;
     const P32 q = make_p32(p, false);
     const void *arr[4] = {d ? (void *)p->d_H64 : (void *)q.H, d ? (void *)p->d_E64 : (void *)q.E,
                           d ? (void *)p->d_Ha64 : (void *)q.Ha, d ? (void *)p->d_Ea64 : (void *)q.Ea};
@@ -1446,13 +1489,14 @@ struct StateHeader {
 
 constexpr char STATE_MAGIC[8] = {'S', 'M', 'A', 'T', 'S', 'T', 'A', 'T'};
 
-/* a device array of a plan's state; compact: FP64 aux slots, dense on the
- * device, are [batch][3][lnotn + 1] in the file (address_notn order, then a
- * zero) */
+/* a device array of a plan's state and how the file holds it: as it is;
+ * FP64 aux slots, dense on the device, as [batch][3][lnotn + 1]
+ * (address_notn order, then a zero); FP32 fields without their rows' padding */
+enum class InFile { same, compact, unpadded };
 struct StateArray {
     void *dev;
     size_t bytes;
-    bool compact;
+    InFile form;
 };
 
 /* the device arrays that hold a plan's state, in file order */
@@ -1462,27 +1506,39 @@ std::vector<StateArray> state_arrays(smat_fdtd_plan *p)
     const size_t b = (size_t)p->batch, n3 = (size_t)p->n3;
     if (p->precision == SMAT_FP64) {
         const size_t f = b * 3 * n3 * 8;
-        a.push_back({p->d_H64, f, false});
-        a.push_back({p->d_E64, f, false});
-        a.push_back({p->d_Ha64, f, true});
-        a.push_back({p->d_Ea64, f, true});
+        a.push_back({p->d_H64, f, InFile::same});
+        a.push_back({p->d_E64, f, InFile::same});
+        a.push_back({p->d_Ha64, f, InFile::compact});
+        a.push_back({p->d_Ea64, f, InFile::compact});
     } else {
         const P32 q = make_p32(p, false);
-        const size_t f = b * 3 * n3 * 4;
-        a.push_back({q.H, f, false});
-        a.push_back({q.E, f, false});
-        a.push_back({q.Ha, f, false});
-        a.push_back({q.Ea, f, false});
+        const size_t f = b * 3 * (size_t)p->n3p * 4;
+        for (float *x : {q.H, q.E, q.Ha, q.Ea}) a.push_back({x, f, p->P0 == p->L[0] ? InFile::same : InFile::unpadded});
     }
     if (p->d_acc && p->nq > 0 && p->nfreq > 0)
-        a.push_back({p->d_acc, b * (size_t)p->nfreq * p->nq * 4 * (size_t)p->pl * 16, false});
+        a.push_back({p->d_acc, b * (size_t)p->nfreq * p->nq * 4 * (size_t)p->pl * 16, InFile::same});
     return a;
 }
 
 /* bytes of a state array in the file */
 size_t file_bytes(const smat_fdtd_plan *p, const StateArray &a)
 {
-    return a.compact ? (size_t)p->batch * 3 * ((size_t)p->lnotn + 1) * 8 : a.bytes;
+    if (a.form == InFile::compact) return (size_t)p->batch * 3 * ((size_t)p->lnotn + 1) * 8;
+    return a.form == InFile::unpadded ? (size_t)p->batch * 3 * p->n3 * 4 : a.bytes;
+}
+
+/* FP32 fields between padded and unpadded rows (padding: 0) */
+void rows_unpad(const smat_fdtd_plan *p, const float *padded, float *rows)
+{
+    const size_t L0 = p->L[0], n = (size_t)p->batch * 3 * p->L[1] * p->L[2];
+    for (size_t r = 0; r < n; r++) memcpy(rows + r * L0, padded + r * p->P0, L0 * 4);
+}
+
+void rows_pad(const smat_fdtd_plan *p, const float *rows, float *padded)
+{
+    const size_t L0 = p->L[0], n = (size_t)p->batch * 3 * p->L[1] * p->L[2];
+    memset(padded, 0, n * p->P0 * 4);
+    for (size_t r = 0; r < n; r++) memcpy(padded + r * p->P0, rows + r * L0, L0 * 4);
 }
 
 /* the aux slots between their dense and their compact form */
@@ -1539,11 +1595,10 @@ extern "C" int smat_fdtd_save_state(smat_fdtd_plan *p, const char *path)
             break;
         }
         const size_t n = file_bytes(p, a);
-        if (a.compact) {
-            file.resize(n);
-            aux_compact(p, (const double *)buf.data(), (double *)file.data());
-        }
-        if (fwrite(a.compact ? file.data() : buf.data(), 1, n, f) != n)
+        if (a.form != InFile::same) file.resize(n);
+        if (a.form == InFile::compact) aux_compact(p, (const double *)buf.data(), (double *)file.data());
+        if (a.form == InFile::unpadded) rows_unpad(p, (const float *)buf.data(), (float *)file.data());
+        if (fwrite(a.form != InFile::same ? file.data() : buf.data(), 1, n, f) != n)
             rc = smat_fail(SMAT_EINVAL, "save_state: write error");
     }
     if (fclose(f) != 0 && !rc) rc = smat_fail(SMAT_EINVAL, "save_state: write error");
@@ -1576,12 +1631,13 @@ extern "C" int smat_fdtd_load_state(smat_fdtd_plan *p, const char *path)
         if (rc) break;
         const size_t n = file_bytes(p, a);
         buf.resize(a.bytes);
-        if (a.compact) file.resize(n);
-        if (fread(a.compact ? file.data() : buf.data(), 1, n, f) != n) {
+        if (a.form != InFile::same) file.resize(n);
+        if (fread(a.form != InFile::same ? file.data() : buf.data(), 1, n, f) != n) {
             rc = smat_fail(SMAT_EINVAL, "load_state: %s is truncated", path);
             break;
         }
-        if (a.compact) aux_dense(p, (const double *)file.data(), (double *)buf.data());
+        if (a.form == InFile::compact) aux_dense(p, (const double *)file.data(), (double *)buf.data());
+        if (a.form == InFile::unpadded) rows_pad(p, (const float *)file.data(), (float *)buf.data());
         p->h2d_bytes += (long long)a.bytes;
         if (cudaMemcpy(a.dev, buf.data(), a.bytes, cudaMemcpyHostToDevice) != cudaSuccess)
             rc = cuda_fail(cudaGetLastError(), "load_state: copy");

@@ -56,6 +56,8 @@ struct smat_fdtd_plan {
     int precision, batch, lnotn;
     long long n3;
     int pl;
+    int P0;        /* cells from row to row on the device (L[0], or padded: FP32) */
+    long long n3p; /* P0 * L[1] * L[2] */
     double invtau_R = 0, invtau_I = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;

@@ -841,3 +841,114 @@ def test_fp64_sweeps_bit_identical_at_edges(built, port, L, pml, scale):
     assert np.array_equal(got[0], H) and np.array_equal(got[1], E)
     for d in dft:
         assert np.array_equal(d.real, re) and np.array_equal(d.imag, im)
+
+
+# ---- padded rows (L0 % 4 != 0) ---------------------------------------------------
+
+PADDED_CASES = [
+    # rows of 1, 2 and 3 cells past a multiple of 4, the PML's edge in the last
+    # quad and before it, every boundary factor, records at the row's end
+    ((21, 9, 30, 2), 81, dict(pml=(2, 2, 3), metals=0.03, lossy=0.05, pec=0.04, iBc=(-1, 0, 1)), (6, 20, 9, 1)),
+    ((22, 10, 28, 2), 82, dict(pml=(4, 0, 4), lossy=0.04, lossy_pml=0.2, iBc=(0, -1, 0)), (7, 19, 11, -1)),
+    ((23, 9, 30, 2), 83, dict(pml=(0, 0, 3), pml_z_only=True, pec=0.05, iBc=(1, 1, -1)), (6, 20, 9, 1)),
+]
+
+
+def _padded_structure(L, seed, kw):
+    from smatranem_gb300 import workloads as W
+    kw = dict(kw)
+    lossy_pml = kw.pop("lossy_pml", 0.0)
+    s = W.random_structure(L, seed=seed, **kw)
+    pr = W.prepare(s)
+    if lossy_pml:  # absorbing split cells: records, from the plan API only
+        cells = np.flatnonzero(np.asarray(pr.cont).view(np.uint8) == ord("a"))
+        pick = np.random.default_rng(seed).choice(cells, size=int(lossy_pml * cells.size), replace=False)
+        for c in range(3):
+            pr.epsi[3 * pick + c] += 0.1j * np.abs(pr.epsi[3 * pick + c].real)
+    return s, pr
+
+
+def _padded_setup(case, batch, tuning=None, path=None, resume=False):
+    """Excitations 0 and 35 of a plan of 36 (padded rows), or of plans of one
+    excitation each (a plan too small for padding): the same inputs."""
+    f = _fdtd()
+    from smatranem_gb300 import workloads as W
+    L, seed, kw, iBTIin = PADDED_CASES[case]
+    nsteps = 12 if kw.get("metals") else 37  # fields grow at metal cells
+    s, pr = _padded_structure(L, seed, kw)
+    src, ph = f.cw_schedule(pr.n2pi, (1, 1, 3))
+    out = []
+    for first in range(0, 36, batch):
+        if batch == 1 and first not in (0, 35):
+            continue
+        with f.Plan.create(s.L, s.iBc, iBTIin, pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma, precision=f.FP32,
+                           batch=batch, pec=s.pec) as p:
+            if tuning:
+                p.set_tuning(*tuning)
+            for b in range(batch):
+                p.set_fields(b, *W.random_fields(s.n3, pr.lnotn, seed=first + b, scale=1e-2))
+                p.set_incident(b, *W.random_incident(L[0] * L[1], seed=100 + first + b))
+                p.set_source_plane(b, iBTIin[2] + (first + b) % 3, 1 - 2 * ((first + b) % 2))
+            p.set_schedule(src, planes=(iBTIin[0], iBTIin[1], 0), phase=ph)
+            p.run(0, nsteps // 2)
+            if path:
+                p.save_state(path)
+                if resume:
+                    for b in range(batch):
+                        z = np.zeros(3 * (s.n3 + pr.lnotn + 1))
+                        p.set_fields(b, z, z)
+                    p.load_state(path)
+            p.run(nsteps // 2, nsteps)
+            assert p.check_finite()[0]
+            for b in ((0, 35) if batch == 36 else (0,)):
+                out += [*p.get_fields(b), *[p.get_dft(b, 0, q) for q in range(3)]]
+    return s, out
+
+
+@pytest.mark.parametrize("case", range(len(PADDED_CASES)))
+def test_padded_rows_are_bit_identical_to_the_scalar_sweeps(built, case, tmp_path):
+    """The sweeps of padded rows give the bits of the one-cell-per-thread
+    sweeps: whole grid and z chunks, fields through set/get and a state file
+    (which holds no padding)."""
+    _, ref = _padded_setup(case, 1)
+    sizes = []
+    for batch, kw in ((36, {}), (36, dict(tuning=(0, 1, 0, 0, 4))), (36, dict(tuning=(0, 4, 3, 0, 4))),
+                      (36, dict(path=str(tmp_path / "padded"), resume=True))):
+        s, got = _padded_setup(case, batch, **kw)
+        assert len(ref) == len(got) == 10
+        for a, b in zip(ref, got):
+            assert np.array_equal(a, b), kw
+    _padded_setup(case, 1, path=str(tmp_path / "plain"))
+    pl = s.L[0] * s.L[1]
+    for name, batch in (("padded", 36), ("plain", 1)):
+        sizes.append((tmp_path / name).stat().st_size - batch * (4 * 3 * s.n3 * 4 + 3 * 4 * pl * 16))
+    assert sizes[0] == sizes[1] > 0
+
+
+@pytest.mark.parametrize("case", [1, 2])
+def test_padded_rows_adjoint(built, case):
+    """The adjoint gradient of a plan of padded rows is the sum of those of
+    plans of one excitation (the same FP32 values, summed in FP64 in another
+    order: 1e-12)."""
+    f = _fdtd()
+    from smatranem_gb300 import workloads as W
+    L, seed, kw, iBTIin = PADDED_CASES[case]
+    s, pr = _padded_structure(L, seed, {**kw, "pec": 0.0, "lossy": 0.0, "lossy_pml": 0.0})
+    src, ph = f.cw_schedule(pr.n2pi, (1, 1, 3))
+    pl = L[0] * L[1]
+    rng = np.random.default_rng(seed)
+    cols = rng.standard_normal(4 * pl) + 1j * rng.standard_normal(4 * pl)
+    box = (8, 12, 3, 6, 12, 16)
+
+    def run(first, batch):
+        with f.Plan.create(s.L, s.iBc, iBTIin, pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma, precision=f.FP32,
+                           batch=batch) as p:
+            for b in range(batch):
+                p.set_incident(b, *W.random_incident(pl, seed=100 + first + b))
+            p.set_schedule(src, planes=(iBTIin[0], iBTIin[1], 0), phase=ph)
+            return p.adjoint_grad(12, 5, 0, 0, cols, box)
+
+    J, g = run(0, 36)[:2]
+    one = [run(b, 1)[:2] for b in range(36)]
+    assert _relerr(np.asarray(g), sum(np.asarray(o[1]) for o in one)) < 1e-12
+    assert abs(J - sum(o[0] for o in one)) <= 1e-12 * abs(J)
