@@ -150,7 +150,9 @@ __device__ __forceinline__ double sample_sens(const Obj &o, int b, int v, int px
 }
 
 /* transpose of the E sweep of step k; also accumulates the design gradient
- * -L_E^{k+1} (E^{k+1} - A E^k) on the box cells ([batch][3][nbox]) */
+ * -L_E^{k+1} (E^{k+1} - A E^k) on the box cells ([batch][3][nbox]), times the
+ * cell's B, which L_E = phi / B divides by: k_adj_scale, once after the last
+ * step (an FP64 division a step and cell otherwise) */
 template <class T, class C>
 __global__ void __launch_bounds__(256) k_adj_e(const Geo g, const int batch, const C coef, const AState<T> s,
                                                const Obj o, const int k, const Box bx, const T *__restrict__ rec1,
@@ -193,10 +195,9 @@ __global__ void __launch_bounds__(256) k_adj_e(const Geo g, const int batch, con
         const T phi = Ap * PE[c * n3 + l] + Bp * sv;
         PE[c * n3 + l] = phi;
         QE[c * n3 + l] = Am * QE[c * n3 + l] + Bm * sv;
-        if (design && Bp != (T)0) {
+        if (design) {
             const long long r = ((long long)b * 3 + c) * bx.n + bi;
-            const double lam = (double)phi / (double)Bp;
-            grad[r] -= lam * ((double)rec1[r] - (double)Ap * (double)rec0[r]);
+            grad[r] -= (double)phi * ((double)rec1[r] - (double)Ap * (double)rec0[r]);
         }
     }
 }
@@ -243,6 +244,24 @@ __global__ void __launch_bounds__(256) k_adj_h(const Geo g, const int batch, con
     }
 }
 
+/* the division by B of the accumulated design gradient (0 where B is 0) */
+template <class T, class C>
+__global__ void k_adj_scale(const Geo g, const C coef, const Box bx, double *__restrict__ grad)
+{
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int b = blockIdx.y;
+    if (i >= bx.n) return;
+    const int x = bx.x0 + (int)(i % bx.nx), y = bx.y0 + (int)((i / bx.nx) % bx.ny),
+              z = bx.z0 + (int)(i / ((long long)bx.nx * bx.ny));
+    const long long l = x + (long long)g.P0 * (y + (long long)g.L1 * z);
+    for (int c = 0; c < 3; c++) {
+        T Ap, Bp, Am, Bm;
+        coef.get(true, c, l, g.n3, x, y, z, Ap, Bp, Am, Bm);
+        double &v = grad[((long long)b * 3 + c) * bx.n + i];
+        v = Bp != (T)0 ? v / (double)Bp : 0.0;
+    }
+}
+
 /* E of the design cells: dst[b][c][i] = E[b][c][cell i] */
 template <class T>
 __global__ void k_adj_record(const Geo g, const int batch, const Box bx, const T *__restrict__ E, T *__restrict__ dst)
@@ -257,11 +276,10 @@ __global__ void k_adj_record(const Geo g, const int batch, const Box bx, const T
 }
 
 /* ---------------------------------------------------------------------------
- * Vectorised FP32 adjoint steps (L0 % 4 == 0): four x-cells per thread, as
+ * Vectorised FP32 adjoint steps (L0 % 4 == 0 or padded rows): four x-cells per thread, as
  * the forward sweep k_sweep32v -- float4 loads of the adjoint fields and the
  * coefficient stream, x neighbours by warp shuffle -- with the per-element
- * arithmetic of k_adj_e / k_adj_h.  A block is 32 x by threads; grid as
- * k_sweep32v's (x blocks, row blocks x excitations, planes).
+ * arithmetic of k_adj_e / k_adj_h.  Grid: quads of a plane x excitations, planes.
  * ------------------------------------------------------------------------- */
 __device__ __forceinline__ float4 ldf4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ void stf4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
@@ -309,47 +327,75 @@ __device__ __forceinline__ void coef32_elem(const Coef32 &cf, bool efield, const
     Bm = bn * tG[i2];
 }
 
-template <bool EF>
+/* Bound by the latency of a quad's loads, so they all leave before the first is
+ * used: the quads of a plane are dealt out to the threads row after row (in a
+ * warp per row piece the 40 quads of 160 cells fill 63 % of the lanes), the
+ * outer x neighbour at the end of a warp or row is loaded with the others, and
+ * the gradient needs no division (k_adj_scale).  160 x 160 x 120 cells with
+ * 72000 of design: 74 and 55 us before, 50 and 47 now (187 MB, 3.9 TB/s); 96
+ * registers instead of 128: 1 % more for the whole gradient.  PAD: padded rows
+ * (as sweep32v_quad of fdtd_f32.cu), with the sums in k_adj_e's and k_adj_h's
+ * order, so that the route does not show in the result. */
+template <bool EF, bool PAD>
 __global__ void __launch_bounds__(128, 4) k_adj32v(const Geo g, const int batch, const Coef32 cf,
                                                   const AState<float> s, const Obj o, const int k, const Box bx,
                                                   const float *__restrict__ rec1, const float *__restrict__ rec0,
                                                   double *__restrict__ grad)
 {
-    const int b = blockIdx.y % batch;
-    const int xr = (blockIdx.x * 32 + threadIdx.x) * 4;
-    const int y = (blockIdx.y / batch) * blockDim.y + threadIdx.y;
-    const int z = blockIdx.z;
-    if (y >= g.L1) return; /* uniform per warp */
-    const bool live = xr < g.L0;
-    const int x0 = live ? xr : g.L0 - 4;
+    const int P0 = PAD ? g.P0 : g.L0, nq = P0 >> 2;
+    const int b = blockIdx.x % batch, z = blockIdx.y;
+    const int iq = blockIdx.x / batch * blockDim.x + threadIdx.x, last = nq * g.L1 - 1;
+    const bool live = iq <= last; /* the others repeat the last quad and store nothing */
+    const int u = live ? iq : last, y = u / nq, x0 = 4 * (u - y * nq);
     const long long n3 = g.n3, bs = 3 * n3;
-    const long long l = x0 + (long long)g.L0 * (y + (long long)g.L1 * z);
+    const long long l = x0 + (long long)P0 * (y + (long long)g.L1 * z);
     /* EF: transpose of the E sweep (reads the H adjoint, forward neighbours);
      * else of the H sweep (reads the E adjoint, backward neighbours) */
     const float *PG = (EF ? s.phiH : s.phiE) + b * bs, *QG = (EF ? s.psiH : s.psiE) + b * bs;
     float *PF = (EF ? s.phiE : s.phiH) + b * bs, *QF = (EF ? s.psiE : s.psiH) + b * bs;
     const float *cfs = EF ? cf.be : cf.bh;
+    const bool ex = EF ? x0 + 4 == P0 : x0 == 0;
     const bool ey = EF ? (y + 1 == g.L1) : (y == 0);
     const bool ez = EF ? (z + 1 == g.L2) : (z == 0);
-    const long long oy = (long long)g.L0 * (EF ? (ey ? -(g.L1 - 1) : 1) : (ey ? g.L1 - 1 : -1));
-    const long long oz = (long long)g.pl * (EF ? (ez ? -(g.L2 - 1) : 1) : (ez ? g.L2 - 1 : -1));
+    const long long oy = (long long)P0 * (EF ? (ey ? -(g.L1 - 1) : 1) : (ey ? g.L1 - 1 : -1));
+    const long long oz = (long long)(PAD ? g.ps : g.pl) * (EF ? (ez ? -(g.L2 - 1) : 1) : (ez ? g.L2 - 1 : -1));
     const float fy = ey ? (float)g.bc[1] : 1.0f, fz = ez ? (float)g.bc[2] : 1.0f;
     /* In a quad with no split cell psi equals phi: both start at zero and take
      * the same coefficients (A- = A+, B- = B+) and the same source.  Such quads
      * neither read nor write psi, and neighbours read their phi in its place;
      * psi is kept (read and written) for quads with a split cell only. */
-    const bool pmx = cf.pmask[x0] | cf.pmask[x0 + 1] | cf.pmask[x0 + 2] | cf.pmask[x0 + 3];
-    const bool pmy = cf.pmask[cf.s1 + y], pmz = cf.pmask[cf.s2 + z];
+    auto quad_mask = [&](int q) -> unsigned { /* the split x indices of a quad */
+        unsigned m = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (!PAD || q + i < g.L0) m |= (unsigned)(cf.pmask[q + i] != 0) << i;
+        return m;
+    };
+    const unsigned xm = quad_mask(x0);
+    const bool pmx = xm != 0, pmy = cf.pmask[cf.s1 + y], pmz = cf.pmask[cf.s2 + z];
     const bool qsplit = pmx | pmy | pmz;
     const int yn = EF ? (ey ? 0 : y + 1) : (ey ? g.L1 - 1 : y - 1);
     const int zn = EF ? (ez ? 0 : z + 1) : (ez ? g.L2 - 1 : z - 1);
     const bool ysplit = pmx | cf.pmask[cf.s1 + yn] | pmz, zsplit = pmx | pmy | cf.pmask[cf.s2 + zn];
+    const bool own_xn = ex | ((threadIdx.x & 31) == (EF ? 31 : 0));
     float4 cq[3], pf[3], qf[3], pg[3], qg[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
         cq[c] = ldf4(cfs + c * n3 + l);
         pf[c] = ldf4(PF + c * n3 + l);
         pg[c] = ldf4(PG + c * n3 + l);
+    }
+    /* y and z neighbours: EF reads psi_z, phi_x at y+1 and phi_y, psi_x at z+1;
+     * the H transpose reads psi_z, phi_x at y-1 and phi_y, psi_x at z-1 */
+    float4 qyz = ldf4((ysplit ? QG : PG) + 2 * n3 + l + oy), pyx = ldf4(PG + 0 * n3 + l + oy);
+    float4 pzy = ldf4(PG + 1 * n3 + l + oz), qzx = ldf4((zsplit ? QG : PG) + 0 * n3 + l + oz);
+    /* x neighbours: phi_z and psi_y at x+1 (EF) or x-1 */
+    float xpz = 0.0f, xqy = 0.0f;
+    if (own_xn) {
+        const long long ox = EF ? (ex ? -(P0 - 4) : 4) : (ex ? g.L0 - 1 : -1);
+        const bool xsplit = pmy | pmz | (quad_mask(EF ? (ex ? 0 : x0 + 4) : (ex ? P0 - 4 : x0 - 4)) != 0);
+        xpz = PG[2 * n3 + l + ox];
+        xqy = (xsplit ? QG : PG)[1 * n3 + l + ox];
     }
     if (qsplit) {
 #pragma unroll
@@ -364,37 +410,19 @@ __global__ void __launch_bounds__(128, 4) k_adj32v(const Geo g, const int batch,
             qg[c] = pg[c];
         }
     }
-    /* y and z neighbours: EF reads psi_z, phi_x at y+1 and phi_y, psi_x at z+1;
-     * the H transpose reads psi_z, phi_x at y-1 and phi_y, psi_x at z-1 */
-    float4 qyz = ldf4((ysplit ? QG : PG) + 2 * n3 + l + oy), pyx = ldf4(PG + 0 * n3 + l + oy);
-    float4 pzy = ldf4(PG + 1 * n3 + l + oz), qzx = ldf4((zsplit ? QG : PG) + 0 * n3 + l + oz);
-    /* x neighbours: phi_z and psi_y at x+1 (EF) or x-1 */
     const unsigned full = 0xffffffffu;
-    float xpz, xqy;
-    if (EF) {
-        xpz = __shfl_down_sync(full, pg[2].x, 1);
-        xqy = __shfl_down_sync(full, qg[1].x, 1);
-        if ((threadIdx.x & 31) == 31 || x0 + 4 == g.L0) {
-            const bool edge = x0 + 4 == g.L0;
-            const long long ox = edge ? -(g.L0 - 4) : 4;
-            const float f = edge ? (float)g.bc[0] : 1.0f;
-            const int xq = edge ? 0 : x0 + 4; /* the neighbouring quad */
-            const bool xsplit = pmy | pmz | cf.pmask[xq] | cf.pmask[xq + 1] | cf.pmask[xq + 2] | cf.pmask[xq + 3];
-            xpz = f * PG[2 * n3 + l + ox];
-            xqy = f * (xsplit ? QG : PG)[1 * n3 + l + ox];
-        }
-    } else {
-        xpz = __shfl_up_sync(full, pg[2].w, 1);
-        xqy = __shfl_up_sync(full, qg[1].w, 1);
-        if ((threadIdx.x & 31) == 0 || x0 == 0) {
-            const bool edge = x0 == 0;
-            const long long ox = edge ? g.L0 - 1 : -1;
-            const float f = edge ? (float)g.bc[0] : 1.0f;
-            const int xq = edge ? g.L0 - 4 : x0 - 4; /* the neighbouring quad */
-            const bool xsplit = pmy | pmz | cf.pmask[xq] | cf.pmask[xq + 1] | cf.pmask[xq + 2] | cf.pmask[xq + 3];
-            xpz = f * PG[2 * n3 + l + ox];
-            xqy = f * (xsplit ? QG : PG)[1 * n3 + l + ox];
-        }
+    const float spz = EF ? __shfl_down_sync(full, pg[2].x, 1) : __shfl_up_sync(full, pg[2].w, 1);
+    const float sqy = EF ? __shfl_down_sync(full, qg[1].x, 1) : __shfl_up_sync(full, qg[1].w, 1);
+    const float fx = ex ? (float)g.bc[0] : 1.0f;
+    xpz = own_xn ? fx * xpz : spz;
+    xqy = own_xn ? fx * xqy : sqy;
+    if (PAD && EF && ex) { /* the wrapped neighbour of cell L0-1 lies in the quad's own padding */
+#pragma unroll
+        for (int i = 1; i < 4; i++)
+            if (x0 + i == g.L0) {
+                s4(pg[2], i, xpz);
+                s4(qg[1], i, xqy);
+            }
     }
     if (!live) return;
     const float fx_in = 1.0f;
@@ -403,6 +431,7 @@ __global__ void __launch_bounds__(128, 4) k_adj32v(const Geo g, const int batch,
     if (z == o.zq) {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
+            if (PAD && x0 + i >= g.L0) break;
             const int px = x0 + i + g.L0 * y;
             gs[0][i] = (float)sample_sens(o, b, EF ? 2 : 0, px, g.pl, k);
             gs[1][i] = (float)sample_sens(o, b, EF ? 3 : 1, px, g.pl, k);
@@ -411,7 +440,8 @@ __global__ void __launch_bounds__(128, 4) k_adj32v(const Geo g, const int batch,
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int x = x0 + i;
-        const bool split = cf.pmask[x] | pyzm;
+        if (PAD && x >= g.L0) break; /* padding: stays 0 */
+        const bool split = (xm >> i & 1u) | pyzm;
         /* neighbour along x of element i: phi_z, psi_y */
         const float npz = EF ? (i == 3 ? xpz : e4(pg[2], i + 1)) : (i == 0 ? xpz : e4(pg[2], i - 1));
         const float nqy = EF ? (i == 3 ? xqy : e4(qg[1], i + 1)) : (i == 0 ? xqy : e4(qg[1], i - 1));
@@ -437,13 +467,12 @@ __global__ void __launch_bounds__(128, 4) k_adj32v(const Geo g, const int batch,
         for (int c = 0; c < 3; c++) {
             float Ap, Bp, Am, Bm;
             coef32_elem(cf, EF, cq, i, c, split, x, y, z, Ap, Bp, Am, Bm);
-            const float phi = Ap * e4(pf[c], i) + Bp * sv[c];
+            const float phi = PAD ? fmaf(Bp, sv[c], __fmul_rn(Ap, e4(pf[c], i))) : Ap * e4(pf[c], i) + Bp * sv[c];
             s4(pf[c], i, phi);
-            s4(qf[c], i, Am * e4(qf[c], i) + Bm * sv[c]);
-            if (design && Bp != 0.0f) {
+            s4(qf[c], i, PAD ? fmaf(Bm, sv[c], __fmul_rn(Am, e4(qf[c], i))) : Am * e4(qf[c], i) + Bm * sv[c]);
+            if (design) {
                 const long long r = ((long long)b * 3 + c) * bx.n + bi;
-                const double lam = (double)phi / (double)Bp;
-                grad[r] -= lam * ((double)rec1[r] - (double)Ap * (double)rec0[r]);
+                grad[r] -= (double)phi * ((double)rec1[r] - (double)Ap * (double)rec0[r]);
             }
         }
     }
@@ -526,16 +555,21 @@ int zero_state(smat_fdtd_plan *p)
     return SMAT_OK;
 }
 
-/* the vectorised FP32 adjoint step where it applies (L0 % 4 == 0); false:
+/* the vectorised FP32 adjoint step where it applies (L0 % 4 == 0, or padded rows); false:
  * the caller launches the scalar kernels */
 bool adj_launch_vec(smat_fdtd_plan *p, const Geo &g, int batch, const Coef32 &cf, const AState<float> &as,
                     const Obj &o, int k, const Box &bx, const float *rec1, const float *rec0, double *grad)
 {
-    if (g.L0 % 4 != 0 || p->adj_scalar) return false;
-    const int by = 2;
-    const dim3 blk(32, by, 1), grd((g.L0 / 4 + 31) / 32, ((g.L1 + by - 1) / by) * batch, g.L2);
-    k_adj32v<true><<<grd, blk, 0, p->stream>>>(g, batch, cf, as, o, k, bx, rec1, rec0, grad);
-    k_adj32v<false><<<grd, blk, 0, p->stream>>>(g, batch, cf, as, o, k, bx, nullptr, nullptr, nullptr);
+    if (g.P0 % 4 != 0 || p->adj_scalar) return false;
+    const int threads = 64;
+    const dim3 grd((g.P0 / 4 * g.L1 + threads - 1) / threads * batch, g.L2);
+    if (g.P0 == g.L0) {
+        k_adj32v<true, false><<<grd, threads, 0, p->stream>>>(g, batch, cf, as, o, k, bx, rec1, rec0, grad);
+        k_adj32v<false, false><<<grd, threads, 0, p->stream>>>(g, batch, cf, as, o, k, bx, nullptr, nullptr, nullptr);
+    } else {
+        k_adj32v<true, true><<<grd, threads, 0, p->stream>>>(g, batch, cf, as, o, k, bx, rec1, rec0, grad);
+        k_adj32v<false, true><<<grd, threads, 0, p->stream>>>(g, batch, cf, as, o, k, bx, nullptr, nullptr, nullptr);
+    }
     return true;
 }
 
@@ -665,6 +699,7 @@ int adjoint_run(smat_fdtd_plan *p, const C &coef, int nsteps, int K, int f, int 
     p->nq = nq_save;
     drop_graph(p);
     if (rc) return rc;
+    k_adj_scale<T, C><<<gr, 256, 0, p->stream>>>(g, coef, bx, dgrad);
     std::vector<double> hg(rec_n);
     CK(cudaMemcpyAsync(hg.data(), dgrad, rec_n * 8, cudaMemcpyDeviceToHost, p->stream));
     CK(cudaStreamSynchronize(p->stream));
