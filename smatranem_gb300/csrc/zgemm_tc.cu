@@ -37,8 +37,9 @@
  * core matrices of 8 rows x 16 bytes), so one thread loads them with bulk
  * async copies (cp.async.bulk, completion on mbarriers: every B slice at
  * once, the A slices through a ring of three buffers) and issues the
- * tcgen05.mma (kind::f16, bf16 x bf16 -> f32, M = 128, N = 32, K = 16) of
- * slice i as soon as it has landed; the S accumulators (32 TMEM columns each)
+ * tcgen05.mma (kind::f16, bf16 x bf16 -> f32, M = 128, K = 16) of slice i
+ * with all the B slices it meets, side by side as N = 32 (S - i) columns, as
+ * soon as it has landed; the S accumulators (32 TMEM columns each)
  * are read back by all eight warps (tcgen05.ld, one row per thread) for an
  * integer epilogue (exact int64 sum of the digit levels, the double assembled
  * from its bits) with one FP64 multiply-add per output: GB300's FP64 pipe
@@ -74,7 +75,8 @@ constexpr int CTILE = BM * BNC * 16; /* bytes of a tile of C (32 KB) */
 constexpr int SMEM = RING * AIMG + S * BIMG + CTILE + 8 * (2 * RING + 2) + 16;
 constexpr unsigned WAIT_LIMIT = 1u << 24;
 
-static_assert(S * BN <= TMEM_COLS, "accumulators exceed the TMEM allocation");
+static_assert(S * BN <= TMEM_COLS && S * BN <= 256, "accumulators exceed the TMEM allocation or a product's columns");
+static_assert(BIMG == BN / 8 * 1024, "the B images continue each other's row groups");
 static_assert(S * KI * 128 * 128 < (1 << 24), "partial sums must stay exact in FP32");
 
 /* byte offset of element (row, kk) in an operand image: 8-row groups of 1024
@@ -314,53 +316,37 @@ __global__ void __launch_bounds__(32) k_gj_cols(int cols, int j, int nb, double2
     write_col_slices(img, ntc, c, t, dr, di);
 }
 
-/* X 2^E through FP64 arithmetic, for results outside the normal range (out
- * of line: the compiler would otherwise evaluate it, on GB300's narrow FP64
- * pipe, for every element) */
+/* X 2^E, X = xt 2^32 + xb (xt signed, |xt| < 2^42; xb in [0, 2^32)), through
+ * FP64 arithmetic, for results outside the normal range and X of a few bits
+ * (out of line: the compiler would otherwise evaluate it, on GB300's narrow
+ * FP64 pipe, for every element).  In the second case it is exact. */
 __device__ __noinline__ double fixed_to_double_slow(long long xt, unsigned xb, int E)
 {
     return ldexp(fma((double)xt, 4294967296.0, (double)xb), E);
 }
 
-/* The double nearest (ties to even) to X 2^E, X = xt 2^32 + xb (xt signed,
- * |xt| < 2^42; xb in [0, 2^32)), assembled with integer operations; a result
- * outside the normal range goes through FP64 arithmetic instead. */
-__device__ __forceinline__ double fixed_to_double(long long xt, unsigned xb, int E)
+/* The double nearest (ties to even) to X 2^E, assembled with integer
+ * operations and without a branch, so that a thread's values overlap; slow:
+ * one for fixed_to_double_slow. */
+__device__ __forceinline__ double fixed_to_double(long long xt, unsigned xb, int E, bool &slow)
 {
-    const bool neg = xt < 0;
-    unsigned long long hi, lo;
-    if (!neg) {
-        hi = (unsigned long long)xt;
-        lo = xb;
-    } else if (xb) {
-        hi = (unsigned long long)(~xt);
-        lo = 0x100000000ull - xb;
-    } else {
-        hi = (unsigned long long)(-xt);
-        lo = 0;
-    }
-    if ((hi | lo) == 0) return 0.0;
-    unsigned long long mm;
-    bool sticky = false;
-    int E2 = E;
-    if (hi >> 31) { /* more than 63 bits: the top 64, the rest sticky */
-        const int bh = 64 - __clzll((long long)hi), r = bh - 32;
-        mm = (hi << (64 - bh)) | (lo >> r);
-        sticky = (lo & ((1ull << r) - 1)) != 0;
-        E2 += r;
-    } else {
-        mm = (hi << 32) | lo;
-    }
-    const int lz = __clzll((long long)mm);
-    mm <<= lz;
-    E2 -= lz;
-    unsigned long long mant = mm >> 11;
-    const unsigned rem = (unsigned)(mm & 0x7FFu);
-    if ((rem & 0x400u) && ((rem & 0x3FFu) || sticky || (mant & 1ull))) mant++;
-    const int bexp = E2 + 11 + 52 + 1023;
-    if (bexp < 1 || bexp > 2046) return fixed_to_double_slow(xt, xb, E);
-    return __longlong_as_double(
-        (long long)(((unsigned long long)neg << 63) + ((unsigned long long)(bexp - 1) << 52) + mant));
+    const long long s = xt >> 63;
+    /* |X| = h 2^10 + its low 10 bits, h below 2^64 */
+    const unsigned lo = (xb ^ (unsigned)s) - (unsigned)s;
+    const unsigned long long hi = (unsigned long long)((xt ^ s) + (s != 0 && xb == 0));
+    const unsigned long long h = hi << 22 | lo >> 10, low = (unsigned long long)lo << 54;
+    const int lz = __clzll((long long)h), z = lz & 63;
+    const unsigned long long mm = h << z | low >> 1 >> (63 - z); /* the leading 64 bits */
+    const unsigned long long mant = mm >> 11;
+    /* the rest of them and whether any bit follows: up above a half, or at it from an odd mant */
+    const unsigned rem = ((unsigned)mm & 0x7FFu) << 1 | ((low << z) != 0);
+    const unsigned long long up = rem + ((unsigned)mant & 1u) > 0x800u;
+    const int bexp = E + 10 - lz + 11 + 52 + 1023;
+    const bool zero = (xt | (long long)xb) == 0;
+    slow = !zero && (h == 0 || bexp < 1 || bexp > 2046);
+    const unsigned long long bits =
+        ((unsigned long long)s & 0x8000000000000000ull) + ((unsigned long long)(bexp - 1) << 52) + mant + up;
+    return zero ? 0.0 : __longlong_as_double((long long)bits);
 }
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -393,16 +379,19 @@ __device__ __forceinline__ uint64_t op_desc(unsigned saddr)
 }
 
 /* instruction descriptor, kind::f16: f32 accumulator, bf16 A and B, both
- * K-major, N = 64, M = 128 */
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+ * K-major, N columns, M = 128 */
+__device__ __forceinline__ uint32_t instr_desc(int n)
+{
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+}
 
-__device__ __forceinline__ void mma_bf16(unsigned tmem, uint64_t a, uint64_t b, unsigned accumulate)
+__device__ __forceinline__ void mma_bf16(unsigned tmem, uint64_t a, uint64_t b, uint32_t idesc, unsigned accumulate)
 {
     asm volatile("{\n\t.reg .pred p;\n\t"
                  "setp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                  :
-                 : "r"(tmem), "l"(a), "l"(b), "r"(IDESC), "r"(accumulate)
+                 : "r"(tmem), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
                  : "memory");
 }
 
@@ -426,12 +415,17 @@ constexpr int MMA_THREADS = 256; /* 8 warps: two per TMEM lane quarter in the ep
  * B slice (one mbarrier) and streams the A slices through a ring of three
  * buffers (full / empty mbarriers per buffer; a buffer is refilled once the
  * products that read it have completed, tcgen05.commit); slice i is multiplied
- * with B_l, l = 0 .. S-1-i, into accumulator i + l.  Then the 8 warps read
+ * with B_l, l = 0 .. S-1-i, into accumulators i + l in one product of 32 (S - i)
+ * columns.  Then the 8 warps read
  * the accumulators back, warp w the TMEM lanes of quarter w % 4 and the
- * complex columns 8 (w / 4) .. + 7.  Bound by a tile's latency (load, 112
- * products of 32 columns, epilogue; two tiles a SM at a time), so a thread's
- * values of C come into shared memory beside the products instead of one by
- * one between its stores: 1210 x 1210 at k = 32 50 -> 40 us.  Every wait is bounded: on a timeout the
+ * complex columns 8 (w / 4) .. + 7.  Bound by a tile's latency (load,
+ * products, epilogue; two tiles a SM at a time: 21000 clocks once).  So the
+ * loads start before the TMEM allocation; 28 products of up to 224 columns take
+ * the place of 112 of 32 (75 clocks each, 8500 in all); a thread's values of C
+ * come into shared memory beside the products instead of one by one between
+ * its stores; and its 16 results are assembled without a branch, so that they
+ * overlap.  1210 x 1210 at k = 32: 50 us, 40 with C fetched early, 30 with all
+ * of it.  Every wait is bounded: on a timeout the
  * CTA records error 1, lets its copies in flight land (bounded) and returns
  * through the same epilogue. */
 __global__ void __launch_bounds__(MMA_THREADS, 2)
@@ -461,11 +455,32 @@ __global__ void __launch_bounds__(MMA_THREADS, 2)
     asm volatile("cp.async.commit_group;" ::: "memory");
     const int er = row < m ? ea[row] : 0, ec = lane < 8 && col0 + lane < n ? eb[col0 + lane] : 0;
 
+    int last[RING]; /* thread 0: the slice last loaded into each buffer (-1: none) */
+    auto load_a = [&](int i) {
+        const int slot = i % RING;
+        const unsigned b = smem_u32(a_full + slot);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(AIMG) : "memory");
+        last[slot] = i;
+        if (i == skip_slice) return; /* the timeout test: a slice that never arrives */
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         smem_u32(ring + slot * AIMG)),
+                     "l"(aimg + (size_t)(i * ntr + tr) * AIMG), "r"(AIMG), "r"(b)
+                     : "memory");
+    };
     if (threadIdx.x == 0) {
         for (int b = 0; b < 2 * RING + 2; b++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar + b)));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        const unsigned b = smem_u32(b_full);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(S * BIMG) : "memory");
+        for (int l = 0; l < S; l++)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             smem_u32(sB + l * BIMG)),
+                         "l"(bimg + (size_t)(l * ntc + tc) * BIMG), "r"(BIMG), "r"(b)
+                         : "memory");
+        for (int i = 0; i < RING; i++) load_a(i);
     }
+    __syncwarp();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
                      "r"(TMEM_COLS)
@@ -478,31 +493,6 @@ __global__ void __launch_bounds__(MMA_THREADS, 2)
     const unsigned tmem = *tslot;
 
     if (threadIdx.x == 0) {
-        int last[RING]; /* the slice last loaded into each buffer (-1: none) */
-#pragma unroll
-        for (int r = 0; r < RING; r++) last[r] = -1;
-        auto load_a = [&](int i) {
-            const int slot = i % RING;
-            const unsigned b = smem_u32(a_full + slot);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(AIMG) : "memory");
-            last[slot] = i;
-            if (i == skip_slice) return; /* the timeout test: a slice that never arrives */
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                             smem_u32(ring + slot * AIMG)),
-                         "l"(aimg + (size_t)(i * ntr + tr) * AIMG), "r"(AIMG), "r"(b)
-                         : "memory");
-        };
-        {
-            const unsigned b = smem_u32(b_full);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(S * BIMG) : "memory");
-            for (int l = 0; l < S; l++)
-                asm volatile(
-                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                        smem_u32(sB + l * BIMG)),
-                    "l"(bimg + (size_t)(l * ntc + tc) * BIMG), "r"(BIMG), "r"(b)
-                    : "memory");
-        }
-        for (int i = 0; i < RING && i < S; i++) load_a(i);
         bool ok = mbar_wait(smem_u32(b_full), 0, wait_limit);
         for (int i = 0; i < S && ok; i++) {
             const int slot = i % RING;
@@ -511,13 +501,12 @@ __global__ void __launch_bounds__(MMA_THREADS, 2)
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int l = 0; l + i < S; l++) {
-                const unsigned acc = tmem + (unsigned)((i + l) * BN);
+            /* slice i with B_0 .. B_(S-1-i), whose images lie one after
+             * another as the rows of one operand, into accumulators i .. S-1 */
 #pragma unroll
-                for (int ks = 0; ks < KI / 16; ks++)
-                    mma_bf16(acc, op_desc(smem_u32(ring + slot * AIMG + ks * 256)),
-                             op_desc(smem_u32(sB + l * BIMG + ks * 256)), (i > 0 || ks > 0) ? 1u : 0u);
-            }
+            for (int ks = 0; ks < KI / 16; ks++)
+                mma_bf16(tmem + (unsigned)(i * BN), op_desc(smem_u32(ring + slot * AIMG + ks * 256)),
+                         op_desc(smem_u32(sB + ks * 256)), instr_desc((S - i) * BN), (i > 0 || ks > 0) ? 1u : 0u);
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                              smem_u32(a_empty + slot))
                          : "memory");
@@ -544,7 +533,7 @@ __global__ void __launch_bounds__(MMA_THREADS, 2)
                      : "memory");
     }
     __syncwarp();
-    const bool done = mbar_wait(smem_u32(acc_full), 0, wait_limit);
+    const bool done = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc_full), 0, wait_limit));
     asm volatile("cp.async.wait_group 0;" ::: "memory"); /* its own values only: no barrier */
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (!done) {
@@ -580,28 +569,43 @@ __global__ void __launch_bounds__(MMA_THREADS, 2)
         /* C += alpha * value; a real alpha (the layer transfer's -1 and 1)
          * gets a loop of its own, so that no element evaluates the complex
          * form's extra FP64 multiply-adds */
+        double x[2][8];
+        unsigned slow = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int E = er + __shfl_sync(0xffffffffu, ec, j) - 14 - 8 * (S - 1);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const long long th = ((long long)a0[h][j] << 16) + p12[h][j];
+                const long long tl = ((long long)p34[h][j] << 16) + p56[h][j];
+                bool sl;
+                x[h][j] = fixed_to_double(th + (tl >> 32), (unsigned)tl, E, sl);
+                if (sl) slow |= 1u << (2 * j + h);
+            }
+        }
+        if (__any_sync(0xffffffffu, slow))
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int E = er + __shfl_sync(0xffffffffu, ec, j) - 14 - 8 * (S - 1);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const long long th = ((long long)a0[h][j] << 16) + p12[h][j];
+                    const long long tl = ((long long)p34[h][j] << 16) + p56[h][j];
+                    if (slow >> (2 * j + h) & 1u) x[h][j] = fixed_to_double_slow(th + (tl >> 32), (unsigned)tl, E);
+                }
+            }
         auto update = [&](auto real_alpha) {
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                const int col = col0 + j, E = er + __shfl_sync(0xffffffffu, ec, j) - 14 - 8 * (S - 1);
-                if (row < m && col < n) {
-                    double x[2];
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        const long long th = ((long long)a0[h][j] << 16) + p12[h][j];
-                        const long long tl = ((long long)p34[h][j] << 16) + p56[h][j];
-                        x[h] = fixed_to_double(th + (tl >> 32), (unsigned)tl, E);
-                    }
-                    double2 v = myc[j * BM];
-                    if (decltype(real_alpha)::value) {
-                        v.x = fma(alpha.x, x[0], v.x);
-                        v.y = fma(alpha.x, x[1], v.y);
-                    } else {
-                        v.x = fma(alpha.x, x[0], fma(-alpha.y, x[1], v.x));
-                        v.y = fma(alpha.x, x[1], fma(alpha.y, x[0], v.y));
-                    }
-                    C[row + (long long)ldc * col] = v;
+                double2 v = myc[j * BM];
+                if (decltype(real_alpha)::value) {
+                    v.x = fma(alpha.x, x[0][j], v.x);
+                    v.y = fma(alpha.x, x[1][j], v.y);
+                } else {
+                    v.x = fma(alpha.x, x[0][j], fma(-alpha.y, x[1][j], v.x));
+                    v.y = fma(alpha.x, x[1][j], fma(alpha.y, x[0][j], v.y));
                 }
+                if (row < m && col0 + j < n) C[row + (long long)ldc * (col0 + j)] = v;
             }
         };
         if (alpha.y == 0.0) update(std::true_type{});

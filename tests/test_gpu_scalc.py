@@ -197,3 +197,44 @@ def test_sweep_sizes_match_oracle(built, L0, L1, bc, layers, n, mode):
         scalc.dense_mode(1)
     assert info["solves"] == 4 * layers and np.array_equal(got, again)
     assert np.abs(got - want).max() <= 1e-9 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (130, 17, 5), (128, 16, 32), (257, 33, 40)])
+def test_zgemm_results_round_to_nearest(built, m, n, k):
+    """B of 8-bit entries (one digit: -128 would take two) meets every digit of A, so the product's integers are
+    exact and each result is the exact sum rounded once to the nearest double:
+    zeros, both signs, sums of a few bits beside a row's large entry, ties
+    (entries a half unit above and below), and results outside the normal range
+    (there within a unit of 2^-1074).  k > 32 adds the passes in turn."""
+    from fractions import Fraction
+    rng = np.random.default_rng(m * n + k)
+    ints = rng.integers(-2 ** 53, 2 ** 53, (m, k, 2))
+    ints[rng.random(ints.shape) < 0.3] = 0
+    ints >>= rng.integers(0, 53, ints.shape)  # entries of every size beside the largest
+    ints[:, 0, 0] = 2 ** 53  # the row's largest entry, which column 0 of B does not meet
+    bints = rng.integers(-127, 128, (k, n, 2))
+    bints[0, :, :] = 0
+    if k > 1:
+        bints[1:, 0, :] = 0
+        bints[1, 0, 0] = 1  # sums of a single entry
+    ea = rng.integers(-40, 40, m)
+    ea[m // 2] = -600
+    eb = rng.integers(-40, 40, n)
+    eb[n // 2] = -440
+    A = np.ldexp(ints[..., 0].astype(float), ea[:, None] - 53) + 1j * np.ldexp(ints[..., 1].astype(float), ea[:, None] - 53)
+    B = np.ldexp(bints[..., 0].astype(float), eb - 7) + 1j * np.ldexp(bints[..., 1].astype(float), eb - 7)
+    C = scalc.zgemm(A, B, mode=1)
+    a, b = ints.astype(object), bints.astype(object)
+    for r in range(0, m, max(1, m // 24)):
+        for c in range(n):
+            want = np.zeros(2)
+            for k0 in range(0, k, 32):
+                s = slice(k0, min(k, k0 + 32))
+                re = sum(a[r, s, 0] * b[s, c, 0] - a[r, s, 1] * b[s, c, 1])
+                im = sum(a[r, s, 0] * b[s, c, 1] + a[r, s, 1] * b[s, c, 0])
+                want += [float(Fraction(int(v)) * Fraction(2) ** int(ea[r] + eb[c] - 60)) for v in (re, im)]
+            got = np.array([C[r, c].real, C[r, c].imag])
+            if np.abs(want).max() < 2.0 ** -1000:
+                assert np.abs(got - want).max() <= 2.0 ** -1074, (r, c)
+            else:
+                assert np.array_equal(got, want), (r, c)
