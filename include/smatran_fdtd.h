@@ -494,6 +494,12 @@ int smat_scalc(int L0, int L1, const int BoundC[2], double omega, int nlayers, c
                const double *XiB, int nB, const double *XiT, int nT, int both_ways, double *S,
                smat_scalc_info *info);
 
+/* smat_scalc with either order of the port matrices' entries: rowsB, rowsT
+ * nonzero: XiB, XiT are row-major. */
+int smat_scalc_ordered(int L0, int L1, const int BoundC[2], double omega, int nlayers, const double *meds,
+                       const double *XiB, int nB, int rowsB, const double *XiT, int nT, int rowsT, int both_ways,
+                       double *S, smat_scalc_info *info);
+
 /* No counterpart in the reference: the GPU LU solve behind smat_scalc (zgesv
  * semantics) on host arrays, for testing.  A: n x n, B and X: n x nrhs, all
  * complex column-major; *info = first zero pivot (1-based) or 0. */

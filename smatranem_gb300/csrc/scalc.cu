@@ -115,25 +115,33 @@ __global__ void k_add_op(double2 *B2, int ld, Geo g, const double2 *__restrict__
     }
 }
 
+/* A port's modes on the device, as the caller holds them: entry (r, c) at
+ * r sr + c sc.  The kernels that read them take either order (each reads them
+ * once; turning 85 MB of a 24 x 24 lattice round on the host took 28 of 172
+ * ms). */
+struct Port {
+    const double2 *X;
+    long long sr, sc;
+    __device__ __forceinline__ double2 at(int r, int c) const { return X[r * sr + c * sc]; }
+};
+
 /* entry (r, c) of the full mode matrix of set_Phi (:521-551) from Xi (2NA x
  * 2NA, Mcalc's column order) */
-__device__ __forceinline__ double2 phi(const double2 *__restrict__ Xi, int NA, int iway, int r, int c)
+__device__ __forceinline__ double2 phi(const Port &Xi, int NA, int iway, int r, int c)
 {
-    const int N2 = 2 * NA;
-    return iway == 1 ? Xi[r + (long long)N2 * c]
-                     : Xi[(r < NA ? r + NA : r - NA) + (long long)N2 * (c < NA ? c + NA : c - NA)];
+    return iway == 1 ? Xi.at(r, c) : Xi.at(r < NA ? r + NA : r - NA, c < NA ? c + NA : c - NA);
 }
 
 /* conj of entry (r, c) of the dual mode matrix of set_tilPhi (:555-595) */
-__device__ __forceinline__ double2 dual(const double2 *__restrict__ Xi, int NA, int iway, int nimag, int r, int c)
+__device__ __forceinline__ double2 dual(const Port &Xi, int NA, int iway, int nimag, int r, int c)
 {
-    const int N2 = 2 * NA, j = c < NA ? c : c - NA;
+    const int j = c < NA ? c : c - NA;
     const bool hi = c >= NA, real = j < nimag;
     if (iway == 1) r = r < NA ? r + NA : r - NA;
     /* the second half of Xi's columns: iway = 1, hi == real; -1, hi != real */
     const bool second = (iway == 1) == (hi == real);
     const bool neg = real && second;
-    double2 v = Xi[r + (long long)N2 * (second ? j + NA : j)];
+    double2 v = Xi.at(r, second ? j + NA : j);
     if (neg) v.x = -v.x;
     else v.y = -v.y;
     return v;
@@ -141,7 +149,7 @@ __device__ __forceinline__ double2 dual(const double2 *__restrict__ Xi, int NA, 
 
 /* set_iniMat (:407-458): M = [B2, F2; B0, F0; B1, F1] of the starting port,
  * (2 NA + No) x (NA + No) */
-__global__ void k_start(double2 *__restrict__ M, const double2 *__restrict__ Xi, int NA, int No, int iway)
+__global__ void k_start(double2 *__restrict__ M, const Port Xi, int NA, int No, int iway)
 {
     const int rows = 2 * NA + No;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -178,7 +186,7 @@ __global__ void k_next(double2 *__restrict__ M, const double2 *__restrict__ X, i
  * the columns of F), B0 and F0 copied; LP ((NA + nimag) x NA): the factor of
  * S1 = [B1, F1] */
 __global__ void k_final(double2 *__restrict__ M, double2 *__restrict__ LP, const double2 *__restrict__ S,
-                        const double2 *__restrict__ Xi, int NA, int No, int nimag, int iway)
+                        const Port Xi, int NA, int No, int nimag, int iway)
 {
     const int rows = NA + nimag + No, n = NA + No;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -286,7 +294,7 @@ int scalc_V(const double *med, long long NA1, double omega, std::vector<std::com
 /* one direction (main :74-94) of nlayers layers whose set_V values are at V
  * (6*NA1 each), the first at istart, in the direction of travel; Xs / Xe:
  * start / end port Xi (device) */
-int one_way(Transfer &T, int iway, int nlayers, const double2 *V, const double2 *Xs, const double2 *Xe, int No, int Nimag,
+int one_way(Transfer &T, int iway, int nlayers, const double2 *V, const Port &Xs, const Port &Xe, int No, int Nimag,
             std::vector<std::complex<double>> &F01h, std::vector<std::complex<double>> &B01h)
 {
     const int NA = T.NA, n = NA + No, N = No + Nimag;
@@ -327,6 +335,13 @@ int one_way(Transfer &T, int iway, int nlayers, const double2 *V, const double2 
 extern "C" int smat_scalc(int L0, int L1, const int BoundC[2], double omega, int nlayers, const double *meds,
                           const double *XiB, int nB, const double *XiT, int nT, int both_ways, double *S,
                           smat_scalc_info *info)
+{
+    return smat_scalc_ordered(L0, L1, BoundC, omega, nlayers, meds, XiB, nB, 0, XiT, nT, 0, both_ways, S, info);
+}
+
+extern "C" int smat_scalc_ordered(int L0, int L1, const int BoundC[2], double omega, int nlayers, const double *meds,
+                                  const double *XiB, int nB, int rowsB, const double *XiT, int nT, int rowsT,
+                                  int both_ways, double *S, smat_scalc_info *info)
 {
     smat::TraceRange trace_("smat_scalc");
     const auto t0 = std::chrono::steady_clock::now();
@@ -387,7 +402,7 @@ extern "C" int smat_scalc(int L0, int L1, const int BoundC[2], double omega, int
     RC(setup(T));
     {
         const size_t nx = (size_t)N2 * N2, nv = 6 * (size_t)NA1;
-        const bool same = XiB == XiT;
+        const bool same = XiB == XiT; /* in whatever order */
         if (cudaMalloc(&in.slab, sizeof(double2) * (nx * (same ? 1 : 2) + nv * nlayers)) != cudaSuccess) {
             cudaGetLastError();
             return smat_fail(SMAT_ENOMEM, "smat_scalc: device memory for the port modes");
@@ -415,6 +430,8 @@ extern "C" int smat_scalc(int L0, int L1, const int BoundC[2], double omega, int
     Transfer T2;
     const bool concurrent = both_ways && setup(T2) == SMAT_OK;
     if (both_ways && !concurrent) smat_clear_error();
+    auto port = [N2](const double2 *X, int by_rows) { return by_rows ? Port{X, N2, 1} : Port{X, 1, N2}; };
+    const Port PB = port(in.XB, rowsB), PT = port(in.XT, rowsT);
     const int N = nB + nT;
     std::vector<std::complex<double>> Sm((size_t)N * N, 0.0), F01h, B01h, F01b, B01b;
     int rc_back = SMAT_OK;
@@ -425,12 +442,12 @@ extern "C" int smat_scalc(int L0, int L1, const int BoundC[2], double omega, int
         SCK(cudaGetDevice(&dev));
         back = std::thread([&, dev] {
             cudaSetDevice(dev);
-            rc_back = one_way(T2, -1, nlayers, in.V, in.XT, in.XB, nT, nB, F01b, B01b);
+            rc_back = one_way(T2, -1, nlayers, in.V, PT, PB, nT, nB, F01b, B01b);
             if (rc_back) msg_back = smat_last_error();
         });
     }
     /* forward: Smat_calc :148-158 */
-    const int rc_fwd = one_way(T, 1, nlayers, in.V, in.XB, in.XT, nB, nT, F01h, B01h);
+    const int rc_fwd = one_way(T, 1, nlayers, in.V, PB, PT, nB, nT, F01h, B01h);
     if (back.joinable()) back.join();
     RC(rc_fwd);
     if (rc_back) return smat_fail(rc_back, "%s", msg_back.c_str());
@@ -438,7 +455,7 @@ extern "C" int smat_scalc(int L0, int L1, const int BoundC[2], double omega, int
         for (int r = 0; r < N; r++)
             Sm[r + (size_t)N * c] = c < nB ? F01h[r + (size_t)N * c] : B01h[r + (size_t)N * (c - nB)];
     if (both_ways) { /* backward: Smat_calc :159-168 */
-        if (!concurrent) RC(one_way(T, -1, nlayers, in.V, in.XT, in.XB, nT, nB, F01b, B01b));
+        if (!concurrent) RC(one_way(T, -1, nlayers, in.V, PT, PB, nT, nB, F01b, B01b));
         for (int c = nB; c < N; c++) {
             for (int r = nB; r < N; r++) Sm[r + (size_t)N * c] = F01b[(r - nB) + (size_t)N * (c - nB)];
             for (int r = 0; r < nB; r++) Sm[r + (size_t)N * c] = F01b[(r + nT) + (size_t)N * (c - nB)];

@@ -24,8 +24,8 @@ class ScalcInfo(C.Structure):
 def _lib():
     L = fdtd.lib()
     if not getattr(L, "_scalc_bound", False):
-        L.smat_scalc.argtypes = [C.c_int, C.c_int, _P, C.c_double, C.c_int, _P, _P, C.c_int, _P, C.c_int, C.c_int,
-                                 _P, _P]
+        L.smat_scalc_ordered.argtypes = [C.c_int, C.c_int, _P, C.c_double, C.c_int, _P, _P, C.c_int, C.c_int, _P,
+                                         C.c_int, C.c_int, C.c_int, _P, _P]
         L.smat_zgesv.argtypes = [C.c_int, C.c_int, _P, _P, _P, _P]
         L.smat_zgemm.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, _P, _P, C.c_int, _P, C.c_int, _P, C.c_int]
         L.smat_dense_mode.argtypes = [C.c_int]
@@ -35,19 +35,28 @@ def _lib():
     return L
 
 
+def _port(Xi):
+    """A port's mode matrix as the library reads it: the array, whether its
+    entries are in row order (no copy of a contiguous array in either order)."""
+    x = np.asarray(Xi, np.complex128)
+    if x.flags.f_contiguous:
+        return x, 0
+    return (x, 1) if x.flags.c_contiguous else (np.asfortranarray(x), 0)
+
+
 def smatrix(meds, omega, L0, L1, bc, XiB, nB, XiT, nT, both_ways=True):
     """S ((nB+nT) x (nB+nT) complex) and the call's info dict.  meds: layers
     iB..iT, each (6, L0*L1) complex; XiB / XiT: (4*L0*L1, 4*L0*L1) complex."""
     m = np.ascontiguousarray(np.asarray(meds, np.complex128).reshape(len(meds), 6 * L0 * L1))
-    xb = np.asfortranarray(np.asarray(XiB, np.complex128))
-    xt = xb if XiT is XiB else np.asfortranarray(np.asarray(XiT, np.complex128))  # one upload where the ports are alike
+    xb, rb = _port(XiB)
+    xt, rt = (xb, rb) if XiT is XiB else _port(XiT)  # one upload where the ports are alike
     bcv = np.ascontiguousarray(bc, np.int32)
     N = nB + nT
     S = np.zeros((N, N), np.complex128, order="F")
     info = ScalcInfo()
-    fdtd._check(_lib().smat_scalc(L0, L1, bcv.ctypes.data_as(_P), float(omega), m.shape[0], m.ctypes.data_as(_P),
-                                  xb.ctypes.data_as(_P), nB, xt.ctypes.data_as(_P), nT, 1 if both_ways else 0,
-                                  S.ctypes.data_as(_P), C.byref(info)))
+    fdtd._check(_lib().smat_scalc_ordered(L0, L1, bcv.ctypes.data_as(_P), float(omega), m.shape[0], m.ctypes.data_as(_P),
+                                          xb.ctypes.data_as(_P), nB, rb, xt.ctypes.data_as(_P), nT, rt,
+                                          1 if both_ways else 0, S.ctypes.data_as(_P), C.byref(info)))
     return np.array(S), {f: getattr(info, f) for f, _ in ScalcInfo._fields_}
 
 

@@ -238,3 +238,23 @@ def test_zgemm_results_round_to_nearest(built, m, n, k):
                 assert np.abs(got - want).max() <= 2.0 ** -1074, (r, c)
             else:
                 assert np.array_equal(got, want), (r, c)
+
+
+def test_port_matrices_in_either_order(built):
+    """Row-major, column-major and strided port matrices, alike or mixed, give
+    the same bits."""
+    rng = np.random.default_rng(5)
+    L0, L1, n = 4, 3, 5
+    NA = 2 * L0 * L1
+    meds = rng.uniform(1, 4, (3, 6, L0 * L1)) + 0j
+    X = [rng.standard_normal((2 * NA, 2 * NA)) + 1j * rng.standard_normal((2 * NA, 2 * NA)) for _ in range(2)]
+    wide = np.zeros((2 * NA, 4 * NA), np.complex128)
+    wide[:, ::2] = X[0]
+    ref, _ = scalc.smatrix(meds, 0.4, L0, L1, (1, 1), np.asfortranarray(X[0]), n, np.asfortranarray(X[1]), n)
+    for b in (X[0], np.asfortranarray(X[0]), wide[:, ::2]):
+        for t in (X[1], np.asfortranarray(X[1])):
+            got, _ = scalc.smatrix(meds, 0.4, L0, L1, (1, 1), b, n, t, n)
+            assert np.array_equal(got, ref)
+    ref, _ = scalc.smatrix(meds, 0.4, L0, L1, (1, 1), np.asfortranarray(X[0]), n, np.asfortranarray(X[0]), n)
+    got, _ = scalc.smatrix(meds, 0.4, L0, L1, (1, 1), X[0], n, X[0], n)
+    assert np.array_equal(got, ref)
