@@ -496,11 +496,15 @@ static int launch_panel(double2 *A, int lda, int m, int nb, int row0, int *ipiv,
  * step is split: the thread that owns a row brings the next column up to date
  * at once, for the next pivot, and a candidate row is brought up to date as
  * it is sent; the other columns follow between arriving at the barrier and
- * waiting for it, lane by lane, 32 / w rows a warp when they fit w lanes.  The
+ * waiting for it.  The
  * FP64 pipe (20 clocks a warp instruction, whatever its lanes) bounds panels
  * of many rows, 80 clocks a row and column and CTA; latency the others.
- * 32 columns of 200 rows: 86 us, 1152 rows 122 us. */
-constexpr int GJT = 256;
+ * So two warps, not all eight, bring the candidate row up to date and send it,
+ * which leaves the others free to go on while the stores drain, and the
+ * trailing columns are dealt out by element (a row's columns rounded up to a
+ * power of two would idle a quarter of the lanes).  32 columns of 200 rows: 73
+ * us, 1152 rows 96 us (79 and 111 before). */
+constexpr int GJT = 256, GJS = 2; /* threads; warps that send */
 
 __device__ __forceinline__ double2 cfnma(double2 c, double2 a, double2 b) /* c - a b, four multiply-adds */
 {
@@ -582,8 +586,9 @@ __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *__restrict__ A,
             }
         }
         __syncthreads();
-        /* the CTA's candidate, up to date, sent by warp t to CTAs t and t + 8 */
-        if (warp < nc) {
+        /* the CTA's candidate, up to date, sent by two warps (each brings it up to
+         * date for itself: more of them would queue for the FP64 pipe) */
+        if (warp < GJS && warp < nc) {
             key = lane < GJT / 32 ? wk[lane] : 0;
             const unsigned mk = __reduce_max_sync(0xffffffffu, key);
             const int src = __ffs(__ballot_sync(0xffffffffu, key == mk)) - 1;
@@ -593,7 +598,7 @@ __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *__restrict__ A,
                 v = a[row * S + lane];
                 if (c > 0 && lane > c) v = cfnma(v, lcol[row], prow[lane]);
             }
-            for (int t = warp; t < nc; t += GJT / 32) {
+            for (int t = warp; t < nc; t += GJS) {
                 cl.map_shared_rank(cand, t)[(par * 16 + rank) * NBMAX + lane] = v;
                 if (lane == 0) {
                     cl.map_shared_rank(ckey, t)[par * 16 + rank] = (int)mk;
@@ -601,16 +606,20 @@ __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *__restrict__ A,
                 }
             }
         }
-        /* columns beyond c of the step before; its pivot row is read before
-         * the barrier, after which another CTA may send over it */
-        const int rest = nb - c - 1, w2 = rest > 1 ? 1 << (32 - __clz(rest - 1)) : 1;
-        const int col = nb - w2 + (lane & (w2 - 1)), per = 32 / w2;
-        const bool live = c > 0 && rest > 0 && col > c;
-        const double2 pb = live ? prow[col] : make_double2(0.0, 0.0);
+        __syncthreads(); /* the candidate row has been read: it may be updated */
         cl.barrier_arrive();
-        __syncthreads(); /* every warp has read the candidate row before it is updated */
-        if (live)
-            for (int i = warp * per + lane / w2; i < rn; i += GJT / 32 * per) a[i * S + col] = cfnma(a[i * S + col], lcol[i], pb);
+        /* columns beyond c of the step before, while the candidates travel (the
+         * pivot row from this CTA's own copy: cand may be sent over by now) */
+        const int rest = nb - c - 1;
+        if (c > 0 && rest > 0) {
+            const unsigned inv = 0xffffffffu / (unsigned)rest + 1u; /* t / rest = umulhi(t, inv), rest > 1 */
+            const double2 *pr = lu + (c - 1) * LS + c + 1;
+            for (int t = tid; t < rn * rest; t += GJT) {
+                const int i = rest > 1 ? (int)__umulhi((unsigned)t, inv) : t, k = t - i * rest;
+                double2 *v = a + i * S + c + 1 + k;
+                *v = cfnma(*v, lcol[i], pr[k]);
+            }
+        }
         cl.barrier_wait();
         __syncthreads();
         key = lane < nc ? (unsigned)ckey[par * 16 + lane] : 0;
