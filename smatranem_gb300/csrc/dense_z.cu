@@ -496,10 +496,8 @@ static int launch_panel(double2 *A, int lda, int m, int nb, int row0, int *ipiv,
  * step is split: the thread that owns a row brings the next column up to date
  * at once, for the next pivot, and a candidate row is brought up to date as
  * it is sent; the other columns follow between arriving at the barrier and
- * waiting for it.  The
- * FP64 pipe (20 clocks a warp instruction, whatever its lanes) bounds panels
- * of many rows, 80 clocks a row and column and CTA; latency the others.
- * So two warps, not all eight, bring the candidate row up to date and send it,
+ * waiting for it.  The FP64 pipe (20 clocks a warp instruction, whatever its
+ * lanes) bounds panels of many rows, latency the others.  So two warps, not all eight, bring the candidate row up to date and send it,
  * which leaves the others free to go on while the stores drain, and the
  * trailing columns are dealt out by element (a row's columns rounded up to a
  * power of two would idle a quarter of the lanes).  32 columns of 200 rows: 73

@@ -454,8 +454,8 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
     const Geo &g = p.g;
     if (!PAD && j1 >= g.L1) return; /* uniform per warp */
     const int P0 = PAD ? g.P0 : g.L0;
-    const bool live = PAD ? in : xr < g.L0;
-    const int x0 = PAD || live ? xr : g.L0 - 4; /* idle lanes load valid data, store nothing */
+    const bool live = in && xr < P0;
+    const int x0 = xr < P0 ? xr : P0 - 4; /* idle lanes load valid data, store nothing */
     const long long n3 = g.n3, bs = 3 * n3;
     const long long l = x0 + (long long)P0 * (j1 + (long long)g.L1 * j2);
     const float *__restrict__ cf = EF ? p.be : p.bh;
@@ -663,21 +663,24 @@ __global__ void __launch_bounds__(128, MB) k_sweep32v(const P32 p, const int rel
     sweep32v_quad<EF, false, false>(p, rel, b, j1, z0 + blockIdx.z, xr, true);
 }
 
-/* The vectorised sweep of padded rows (L0 % 4 != 0).  The quads of a plane are
- * dealt out to the threads one after another, whatever their row: rows of any
- * length fill the warps (in a warp per row piece, the 33 quads of 131 cells
- * would fill 52 % of the lanes).  Bound by the latency of a quad's loads:
- * 131 x 117 x 103 cells of two excitations 138 us a step before (one cell per
- * thread), 83 us now, 3.2 TB/s of the compulsory 84 B a cell; 96 registers
- * (128: 88 us, 80: 91 us).  Block x: quads of the plane x excitation
- * (fastest, for the shared coefficients), y: the plane. */
-template <bool EF>
-__global__ void __launch_bounds__(128, 5) k_sweep32p(const P32 p, const int rel, const int z0)
+/* The same with the quads of a plane dealt out to the threads one after
+ * another, whatever their row: rows of any length fill the warps, where a warp
+ * per row piece leaves lanes idle unless L0 % 128 == 0 (83 % of the lanes used
+ * at 320 cells, 63 % at 160, 52 % in padded rows of 131).  Bound by the latency
+ * of a quad's loads, then by HBM.  us a step, row pieces / dealt out: 320 x 320
+ * x 256 498 / 471 (5.3 TB/s), 160 x 160 x 120 90.6 / 77.9, 144 x 100 x 100 of
+ * two excitations 89.5 / 72.7; 256 x 192 x 64 of four, whose row pieces are
+ * whole warps, 247 / 250: those keep k_sweep32v (flat_quads).  PAD: rows of
+ * padded length, L0 % 4 != 0: 131 x 117 x 103 of two 138 with one cell a
+ * thread, 83 so; 96 registers (MB = 5; 128: 88, 80: 91).  Block x: quads of the
+ * plane x excitation (fastest, for the shared coefficients), y: the plane. */
+template <bool EF, bool PAD, int MB>
+__global__ void __launch_bounds__(128, MB) k_sweep32f(const P32 p, const int rel, const int z0)
 {
-    const int b = blockIdx.x % p.batch, nq = p.g.P0 >> 2;
+    const int b = blockIdx.x % p.batch, nq = (PAD ? p.g.P0 : p.g.L0) >> 2;
     const int i = blockIdx.x / p.batch * blockDim.x + threadIdx.x, last = nq * p.g.L1 - 1;
     const int u = i <= last ? i : last, j1 = u / nq;
-    sweep32v_quad<EF, false, true>(p, rel, b, j1, z0 + blockIdx.y, 4 * (u - j1 * nq), i <= last);
+    sweep32v_quad<EF, false, PAD>(p, rel, b, j1, z0 + blockIdx.y, 4 * (u - j1 * nq), i <= last);
 }
 
 /* general cells of the vectorised sweeps: one thread per record cell, run
@@ -760,8 +763,7 @@ __global__ void k_general32(const P32 p, const int rel, const int *cells, int nc
 /* ---------------------------------------------------------------------------
  * Groups: the vectorised H (E) sweep of every member plan in one launch.
  * Block i belongs to the member m with blk[m] <= i < blk[m+1]; inside it the
- * block decodes exactly as a k_sweep32v block (x block fastest, then row
- * block x excitation, then plane), so each member gets the same bits as
+ * block decodes exactly as a k_sweep32f or k_sweep32v block, so each member gets the same bits as
  * when it is stepped alone.  The member table lives in constant memory: a
  * block-uniform index into it is served by the constant cache, as kernel
  * parameters are, so a member's fields cost the sweep no extra registers.
@@ -776,7 +778,16 @@ __global__ void __launch_bounds__(128, 5) k_group32v(const int rel)
     while (m + 1 < c_group.n && (int)blockIdx.x >= c_group.blk[m + 1]) m++;
     const P32 &p = c_group.p[m];
     const int local = blockIdx.x - c_group.blk[m];
-    const int nxb = (p.g.L0 / 4 + 31) / 32;
+    const int nq = p.g.L0 / 4;
+    if (flat_quads(p.g.L0)) {
+        const int per = sweep32f_blocks(nq * p.g.L1, 32 * c_group.by) * p.batch;
+        const int z = local / per, t = local - z * per, b = t % p.batch;
+        const int i = t / p.batch * 32 * c_group.by + 32 * threadIdx.y + threadIdx.x, last = nq * p.g.L1 - 1;
+        const int u = i <= last ? i : last, j1 = u / nq;
+        sweep32v_quad<EF, false, false>(p, rel, b, j1, z, 4 * (u - j1 * nq), i <= last);
+        return;
+    }
+    const int nxb = (nq + 31) / 32;
     const int nyb = ((p.g.L1 + c_group.by - 1) / c_group.by) * p.batch;
     const int xb = local % nxb, t = local / nxb;
     const int yb = t % nyb, z = t / nyb;
@@ -968,11 +979,16 @@ static void launch_sweep32v(const P32 &p, int rel, int by, int mb, int z0, int z
         grd.z = (z1 - z0 + 1) / 2;
         if (mb == -3) k_sweep32v2<EF, 3><<<grd, blk, 0, st>>>(p, rel, z0, z1);
         else k_sweep32v2<EF, 4><<<grd, blk, 0, st>>>(p, rel, z0, z1);
-        return;
+    } else if (flat_quads(p.g.L0)) {
+        grd = dim3(sweep32f_blocks(p.g.L0 / 4 * p.g.L1, 32 * by) * p.batch, z1 - z0);
+        if (mb >= 8) k_sweep32f<EF, false, 8><<<grd, 32 * by, 0, st>>>(p, rel, z0);
+        else if (mb == 6) k_sweep32f<EF, false, 6><<<grd, 32 * by, 0, st>>>(p, rel, z0);
+        else k_sweep32f<EF, false, 5><<<grd, 32 * by, 0, st>>>(p, rel, z0);
+    } else {
+        if (mb >= 8) k_sweep32v<EF, 8><<<grd, blk, 0, st>>>(p, rel, z0);
+        else if (mb == 6) k_sweep32v<EF, 6><<<grd, blk, 0, st>>>(p, rel, z0);
+        else k_sweep32v<EF, 5><<<grd, blk, 0, st>>>(p, rel, z0);
     }
-    if (mb >= 8) k_sweep32v<EF, 8><<<grd, blk, 0, st>>>(p, rel, z0);
-    else if (mb == 6) k_sweep32v<EF, 6><<<grd, blk, 0, st>>>(p, rel, z0);
-    else k_sweep32v<EF, 5><<<grd, blk, 0, st>>>(p, rel, z0);
 }
 
 void launch_h32v(const P32 &p, int rel, int by, int mb, int z0, int z1, const int *gcells, int ngh,
@@ -993,8 +1009,8 @@ template <bool EF>
 static void launch_sweep32p(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng,
                             cudaStream_t st)
 {
-    const int nq = p.g.P0 / 4 * p.g.L1;
-    k_sweep32p<EF><<<dim3((nq + threads - 1) / threads * p.batch, z1 - z0), threads, 0, st>>>(p, rel, z0);
+    const int n = sweep32f_blocks(p.g.P0 / 4 * p.g.L1, threads);
+    k_sweep32f<EF, true, 5><<<dim3(n * p.batch, z1 - z0), threads, 0, st>>>(p, rel, z0);
     if (ng > 0) k_general32<EF><<<dim3((ng + 127) / 128, p.batch), 128, 0, st>>>(p, rel, gcells, ng);
 }
 

@@ -76,8 +76,10 @@ Group32 make_group(const smat_fdtd_group *g)
         gr.egen[i] = p->d_egen;
         gr.nhgen[i] = p->nhgen;
         gr.negen[i] = p->negen;
-        const int nxb = (p->L[0] / 4 + 31) / 32;
-        blk += nxb * ((p->L[1] + g->by - 1) / g->by) * p->batch * p->L[2];
+        const int nq = p->L[0] / 4;
+        const int plane = flat_quads(p->L[0]) ? sweep32f_blocks(nq * p->L[1], 32 * g->by)
+                                              : (nq + 31) / 32 * ((p->L[1] + g->by - 1) / g->by);
+        blk += plane * p->batch * p->L[2];
         gh += p->nhgen * p->batch;
         ge += p->negen * p->batch;
     }

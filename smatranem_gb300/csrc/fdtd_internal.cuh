@@ -254,6 +254,11 @@ void launch_flush32(const P32 &p, int rel_end, int count, cudaStream_t st);
 /* mb: register bound of the vectorised sweep (minimum resident blocks: 5, 6 or 8) */
 void launch_h32v(const P32 &p, int rel, int by, int mb, int z0, int z1, const int *gcells, int ngh, cudaStream_t st);
 void launch_e32v(const P32 &p, int rel, int by, int mb, int z0, int z1, const int *gcells, int nge, cudaStream_t st);
+/* whether a vectorised sweep deals out a plane's quads one after another
+ * (k_sweep32f, a block per excitation and `threads` quads) rather than by row
+ * pieces of a warp, which rows of whole warps fill as well */
+__host__ __device__ inline bool flat_quads(int L0) { return L0 % 128 != 0; }
+__host__ __device__ inline int sweep32f_blocks(int quads, int threads) { return (quads + threads - 1) / threads; }
 void load_group32(const Group32 *host_pinned, cudaStream_t st);
 void launch_group32v(const Group32 &gr, int rel, cudaStream_t st);
 /* form 6: threads of a CTA (one per quad of its ty + 1 rows, rounded up to

@@ -952,3 +952,46 @@ def test_padded_rows_adjoint(built, case):
     one = [run(b, 1)[:2] for b in range(36)]
     assert _relerr(np.asarray(g), sum(np.asarray(o[1]) for o in one)) < 1e-12
     assert abs(J - sum(o[0] for o in one)) <= 1e-12 * abs(J)
+
+
+@pytest.mark.parametrize("L", [(4, 7, 9, 2), (124, 5, 7, 2), (128, 6, 7, 2), (132, 5, 6, 2), (256, 3, 6, 2)])
+def test_quads_dealt_out_bit_identical(built, L):
+    """The vectorised sweeps whose quads go to the threads row after row (L0 not
+    a multiple of 128: a last block of idle lanes, warps across rows) and by row
+    pieces (128, 256), at every block size, register bound and z chunk, alone
+    and in a group, as the one-cell-per-thread sweeps."""
+    from smatranem_gb300 import workloads as W
+    f = _fdtd()
+    s = W.random_structure(L, seed=L[0], pml=(0, 0, 2), pml_z_only=True, lossy=0.05, pec=0.03, iBc=(1, -1, 0))
+    pr = W.prepare(s)
+    iBTIin = (3, L[2] - 2, 3, 1)
+    ref = _run_fp32(s, pr, iBTIin, (0, 4, 0, 0, 4), 33)
+    for tuning in [(2, 1, 0, 5, 4), (2, 4, 0, 5, 4), (2, 3, 0, 6, 4), (2, 2, 0, 8, 4), (2, 2, 3, 5, 4), (2, 2, 0, -3, 4)]:
+        for rb, gb in zip(ref, _run_fp32(s, pr, iBTIin, tuning, 33)):
+            for a, b in zip(rb, gb):
+                assert np.array_equal(a, b), tuning
+    src, ph = f.cw_schedule(pr.n2pi, (1, 1, 3))
+    plans = []
+    try:
+        for _ in range(2):
+            p = f.Plan.create(s.L, s.iBc, iBTIin, pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma, precision=f.FP32,
+                              batch=2, pec=s.pec)
+            plans.append(p)
+            for b in range(2):
+                p.set_fields(b, *W.random_fields(s.n3, pr.lnotn, seed=b, scale=1e-2))
+                p.set_incident(b, *W.random_incident(L[0] * L[1], seed=10 + b))
+                p.set_source_plane(b, iBTIin[2] + b, 1 - 2 * b)
+            p.set_schedule(src, planes=(iBTIin[0], iBTIin[1], 0), phase=ph)
+        with f.Group(plans) as g:
+            for by in (1, 3):
+                g.set_tuning(0, by)
+            g.run(0, 16)
+            g.run(16, 33)
+        for p in plans:
+            for b in range(2):
+                got = (*p.get_fields(b), *[p.get_dft(b, 0, q) for q in range(3)])
+                for x, y in zip(ref[b], got):
+                    assert np.array_equal(x, y)
+    finally:
+        for p in plans:
+            p.close()
