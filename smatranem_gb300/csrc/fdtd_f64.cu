@@ -51,8 +51,18 @@ struct Near {
     double h1, h2, n2, n1;
 };
 
+/* a load that does not count on the data standing still for the whole kernel */
+__device__ __forceinline__ double ld_coherent(const double *p)
+{
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+
+template <bool AFTER>
 __device__ __forceinline__ Near load_near(const double *__restrict__ F, int i1, int i2, int o1, int o2)
 {
+    if (AFTER) return Near{ld_coherent(F + i1), ld_coherent(F + i2), ld_coherent(F + i2 + o1), ld_coherent(F + i1 + o2)};
     return Near{F[i1], F[i2], F[i2 + o1], F[i1 + o2]};
 }
 
@@ -171,7 +181,7 @@ __device__ __noinline__ double metal_cell(const P64 &p, int cls, int b, int c, i
     }
     const int a1 = (c + 1) % 3, a2 = (c + 2) % 3;
     double pl, mi;
-    curl_near<false>(load_near((EF ? p.H : p.E) + (long long)b * 3 * n3, a1 * n3 + l, a2 * n3 + l, o[a1], o[a2]), wrap,
+    curl_near<false>(load_near<true>((EF ? p.H : p.E) + (long long)b * 3 * n3, a1 * n3 + l, a2 * n3 + l, o[a1], o[a2]), wrap,
                      s[a1], s[a2], pl, mi);
     const double W = pl + mi;
     double *x = (EF ? p.Ea : p.Ha) + ((long long)b * 3 + c) * n3 + l;
@@ -211,8 +221,11 @@ __device__ __noinline__ double metal_cell(const P64 &p, int cls, int b, int c, i
  * pipe's peak); 24 x 20 x 40 guide 3.2 us, from 5.  Blocks of 32 cells rather
  * than 64 or 128: 3 % and 10 % on the cube, 10 % and 30 % on the guide, whose
  * plane fills 15 of them.  13 resident blocks (48 registers): 10 and 15 are
- * within 7 %, 17 spills. */
-template <bool EF>
+ * within 7 %, 17 spills.
+ *
+ * AFTER: launched beside the sweep before (launch_after), with the coefficients
+ * loaded before that one has ended. */
+template <bool EF, bool AFTER>
 __global__ void __launch_bounds__(96, 13) k_sweep64(const P64 p, const int rel)
 {
     const Geo &g = p.g;
@@ -237,16 +250,24 @@ __global__ void __launch_bounds__(96, 13) k_sweep64(const P64 p, const int rel)
     const double *__restrict__ cm = p.cm + (EF ? 6 : 0) * g.n3, *__restrict__ ca = p.ca + (EF ? 6 + c : c) * (long long)p.lnotn;
     const int fl = p.flags[l], cls = fl & 7;
     const double A = cm[i0], B = cm[3 * g.n3 + i0];
-    double f = F[i0];
-    const Near v = load_near(G, i1, i2, o1, o2);
-    double fa = 0.0, Aa, Ba;
-    Near va;
-    auto load_aux = [&]() {
+    double Aa, Ba;
+    auto load_coef = [&]() {
         const int a = p.addr[l];
-        fa = Fa[i0];
         Aa = ca[a];
         Ba = ca[3LL * p.lnotn + a];
-        va = load_near(Ga, i1, i2, o1, o2);
+    };
+    if (AFTER) {
+        if (sp) load_coef();
+        prior_done();
+    }
+    double f = F[i0];
+    const Near v = load_near<AFTER>(G, i1, i2, o1, o2);
+    double fa = 0.0;
+    Near va;
+    auto load_aux = [&]() {
+        fa = Fa[i0];
+        if (!AFTER) load_coef();
+        va = load_near<AFTER>(Ga, i1, i2, o1, o2);
     };
     if (sp) load_aux();
     double pl, mi, pa, ma;
@@ -259,11 +280,14 @@ __global__ void __launch_bounds__(96, 13) k_sweep64(const P64 p, const int rel)
         }
         f = amul(A, f) + imul<!EF>(B, W);
         if (fl & (EF ? FL_FWD : FL_BWD)) {
-            curl_near<EF>(load_near(Ga, i1, i2, o1, o2), w1 | w2, s1, s2, pa, ma);
+            curl_near<EF>(load_near<AFTER>(Ga, i1, i2, o1, o2), w1 | w2, s1, s2, pa, ma);
             f += imul<!EF>(B, pa + ma);
         }
     } else if (cls == CLS_A) {
-        if (!sp) load_aux();
+        if (!sp) {
+            if (AFTER) load_coef();
+            load_aux();
+        }
         curl_near<EF>(v, w1 | w2, s1, s2, pl, mi);
         curl_near<EF>(va, w1 | w2, s1, s2, pa, ma);
         const double h = amul(A, f) + imul<!EF>(B, pl);
@@ -344,7 +368,13 @@ __global__ void k_maxabs(const void *x, long long n, int is_double, unsigned lon
 
 template <bool EF> static void launch_sweep64(const P64 &p, int rel, cudaStream_t st)
 {
-    k_sweep64<EF><<<dim3((p.g.pl + 31) / 32 * p.batch, p.g.L2), dim3(32, 3), 0, st>>>(p, rel);
+    const dim3 grid((p.g.pl + 31) / 32 * p.batch, p.g.L2), block(32, 3);
+    /* Small grids: a sweep is launched beside the one before, where the blocks
+     * of both are resident at once (13 a SM).  us a step, one after another /
+     * beside: 24 x 20 x 40 (600 blocks) 9.8 / 8.2, 32 x 24 x 40 (960) 11.8 /
+     * 10.0; 32 x 32 x 32 (1024) 11.8 / 14.2. */
+    if (2LL * grid.x * grid.y <= 13LL * plan::sm_count()) launch_after(k_sweep64<EF, true>, grid, block, 0, st, p, rel);
+    else k_sweep64<EF, false><<<grid, block, 0, st>>>(p, rel);
 }
 
 void launch_h64(const P64 &p, int rel, cudaStream_t st) { launch_sweep64<false>(p, rel, st); }

@@ -197,6 +197,35 @@ struct RowGroup32 {
 };
 
 
+/* Kernels of a step follow one another as programmatic dependents
+ * (launch_after): one may start when every block of the one before has passed
+ * prior_done, and runs up to its own prior_done beside it -- index arithmetic
+ * and loads of what no launch of a run changes (coefficients, masks, orders,
+ * records).  Fields, the ring and the step counter are touched after it only,
+ * and fields that the kernel before writes are read through coherent loads
+ * (no const __restrict__: such loads may count on data that stands still for the
+ * whole kernel).  Every thread that touches them calls it. */
+__device__ __forceinline__ void prior_done()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
+}
+
 /* The curl stencil of a cell: offsets of its forward (fwd) or backward
  * neighbour along each axis, wrapped at the grid's faces, and the boundary
  * factor iBc at a wrapped neighbour (else 1). */
@@ -241,6 +270,9 @@ __device__ __forceinline__ void curl32(const Get &get, const Stn32 &st, float pl
     }
 }
 
+namespace plan {
+int sm_count(); /* of the current device */
+}
 /* launchers (one translation unit per precision) */
 void launch_h64(const P64 &p, int rel, cudaStream_t st);
 void launch_e64(const P64 &p, int rel, cudaStream_t st);

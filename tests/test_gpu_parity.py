@@ -995,3 +995,33 @@ def test_quads_dealt_out_bit_identical(built, L):
     finally:
         for p in plans:
             p.close()
+
+
+@pytest.mark.parametrize("L,pml", [((20, 15, 12, 1), (3, 2, 3)), ((33, 7, 14, 1), (0, 0, 3))])
+def test_fp64_small_grids_beside_one_another(built, L, pml):
+    """FP64 sweeps of a small grid start beside the sweep before them, those of
+    a large one after it: excitations 0 and 11 of a plan of 12 (large) and plans
+    of one give the same bits, with split cells, sources and DFT planes, through
+    graphs, single launches and a state that goes on."""
+    f = _fdtd()
+    from smatranem_gb300 import workloads as W
+    s = W.random_structure(L, seed=91, pml=pml, lossy=0.05, pec=0.03, iBc=(1, -1, 0),
+                           **({"pml_z_only": True} if pml[0] == 0 else {}))
+    pr = W.prepare(s)
+    src, ph = f.cw_schedule(pr.n2pi, (1, 1, 3))
+    out = []
+    for batch in (12, 1):
+        for first in ((0,) if batch == 12 else (0, 11)):
+            with f.Plan.create(s.L, s.iBc, (4, L[2] - 4, 5, 1), pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma,
+                               precision=f.FP64, batch=batch, pec=s.pec) as p:
+                for b in range(batch):
+                    p.set_fields(b, *W.random_fields(s.n3, pr.lnotn, seed=first + b, scale=1e-2))
+                    p.set_incident(b, *W.random_incident(L[0] * L[1], seed=50 + first + b))
+                p.set_schedule(src, planes=(4, L[2] - 4), phase=ph)
+                for k in ((0, 5), (5, 70), (70, 71), (71, 110)):
+                    p.run(*k)
+                for b in ((0, 11) if batch == 12 else (0,)):
+                    out.append((*p.get_fields(b), p.get_dft(b, 0, 0), p.get_dft(b, 0, 1)))
+    for x, y in zip(out[:2], out[2:]):
+        for a, b in zip(x, y):
+            assert np.all(np.isfinite(a)) and np.array_equal(a, b)
