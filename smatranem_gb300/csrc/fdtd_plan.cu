@@ -1091,11 +1091,13 @@ extern "C" int smat_fdtd_run(smat_fdtd_plan *p, int k_begin, int k_end)
     if (k_end > p->nsched) return smat_fail(SMAT_EINVAL, "run: k_end %d beyond the %d-step schedule", k_end, p->nsched);
     launch_set(p->d_base, k_begin, p->stream);
     int n = k_end - k_begin;
-    if (p->precision == SMAT_FP32 && p->fused == 6 && p->cur != 0 && n >= GRAPH_STEPS + 1) {
-        /* graphs are captured from field set 0: take one step to get there */
-        enqueue_steps(p, 0, 1, false);
-        launch_bump(p->d_base, 1, p->stream);
-        n -= 1;
+    if (p->precision == SMAT_FP32 && p->fused == 6 && p->cur != 0 && n >= GRAPH_STEPS) {
+        /* graphs are captured from field set 0: take one step to get there, or
+         * all of them where a graph's worth is left */
+        const int first = n > GRAPH_STEPS ? 1 : n;
+        enqueue_steps(p, 0, first, false);
+        launch_bump(p->d_base, first, p->stream);
+        n -= first;
     }
     if (n >= GRAPH_STEPS) build_graph(p);
     while (n >= GRAPH_STEPS) {

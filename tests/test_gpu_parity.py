@@ -1025,3 +1025,29 @@ def test_fp64_small_grids_beside_one_another(built, L, pml):
     for x, y in zip(out[:2], out[2:]):
         for a, b in zip(x, y):
             assert np.all(np.isfinite(a)) and np.array_equal(a, b)
+
+
+def test_row_fused_run_of_one_graph_from_the_other_set(built):
+    """A run of exactly 32 steps (one graph) that starts from the second field
+    set, before and after a graph exists, as the sweeps."""
+    from smatranem_gb300 import workloads as W
+    f = _fdtd()
+    L, seed, kw, iBTIin = ROW_CASES[0]
+    s = W.random_structure(L, seed=seed, **kw)
+    pr = W.prepare(s)
+    src, ph = f.cw_schedule(pr.n2pi, (1, 1, 5))
+    out = []
+    for tuning in ((0, 4, 0, 0, 4), (6, 2, 0, 2, 0)):
+        with f.Plan.create(s.L, s.iBc, iBTIin, pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma, precision=f.FP32,
+                           batch=1, pec=s.pec) as p:
+            p.set_tuning(*tuning)
+            p.set_fields(0, *W.random_fields(s.n3, pr.lnotn, seed=1, scale=1e-2))
+            p.set_incident(0, *W.random_incident(L[0] * L[1], seed=2))
+            p.set_schedule(src, planes=(iBTIin[0], iBTIin[1]), phase=ph)
+            k = 0
+            for n in (1, 32, 1, 32, 33, 32, 3):  # from set 0, 1, 1, 0, 0, 1, 1
+                p.run(k, k + n)
+                k += n
+            out.append(p.get_fields(0))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
