@@ -339,9 +339,10 @@ __device__ __forceinline__ void coef32_elem(const Coef32 &cf, bool efield, const
 template <bool EF, bool PAD>
 __global__ void __launch_bounds__(128, 4) k_adj32v(const Geo g, const int batch, const Coef32 cf,
                                                   const AState<float> s, const Obj o, const int k, const Box bx,
-                                                  const float *__restrict__ rec1, const float *__restrict__ rec0,
+                                                  const float *rec1, const float *rec0,
                                                   double *__restrict__ grad)
 {
+    prior_done();
     const int P0 = PAD ? g.P0 : g.L0, nq = P0 >> 2;
     const int b = blockIdx.x % batch, z = blockIdx.y;
     const int iq = blockIdx.x / batch * blockDim.x + threadIdx.x, last = nq * g.L1 - 1;
@@ -564,11 +565,11 @@ bool adj_launch_vec(smat_fdtd_plan *p, const Geo &g, int batch, const Coef32 &cf
     const int threads = 64;
     const dim3 grd((g.P0 / 4 * g.L1 + threads - 1) / threads * batch, g.L2);
     if (g.P0 == g.L0) {
-        k_adj32v<true, false><<<grd, threads, 0, p->stream>>>(g, batch, cf, as, o, k, bx, rec1, rec0, grad);
-        k_adj32v<false, false><<<grd, threads, 0, p->stream>>>(g, batch, cf, as, o, k, bx, nullptr, nullptr, nullptr);
+        launch_after(k_adj32v<true, false>, grd, dim3(threads), 0, p->stream, g, batch, cf, as, o, k, bx, rec1, rec0, grad);
+        launch_after(k_adj32v<false, false>, grd, dim3(threads), 0, p->stream, g, batch, cf, as, o, k, bx, nullptr, nullptr, nullptr);
     } else {
-        k_adj32v<true, true><<<grd, threads, 0, p->stream>>>(g, batch, cf, as, o, k, bx, rec1, rec0, grad);
-        k_adj32v<false, true><<<grd, threads, 0, p->stream>>>(g, batch, cf, as, o, k, bx, nullptr, nullptr, nullptr);
+        launch_after(k_adj32v<true, true>, grd, dim3(threads), 0, p->stream, g, batch, cf, as, o, k, bx, rec1, rec0, grad);
+        launch_after(k_adj32v<false, true>, grd, dim3(threads), 0, p->stream, g, batch, cf, as, o, k, bx, nullptr, nullptr, nullptr);
     }
     return true;
 }

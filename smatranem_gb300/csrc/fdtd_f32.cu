@@ -58,6 +58,7 @@ __device__ __forceinline__ float *ring_at(const Dft &d, int pl, int b, int k, in
 template <bool EF>
 __global__ void __launch_bounds__(256) k_sweep32(const P32 p, const int rel, const int z0)
 {
+    prior_done();
     /* blockIdx.y = row block * batch + excitation: the blocks of one tile for
      * all excitations launch together and share the coefficient lines in L2 */
     const int b = blockIdx.y % p.batch;
@@ -69,8 +70,8 @@ __global__ void __launch_bounds__(256) k_sweep32(const P32 p, const int rel, con
     const float *__restrict__ cf = EF ? p.be : p.bh;
     float *__restrict__ F0 = EF ? p.E : p.H;   /* updated field (total form) */
     float *__restrict__ Fa0 = EF ? p.Ea : p.Ha;
-    const float *__restrict__ G0 = EF ? p.H : p.E; /* field whose curl drives it */
-    const float *__restrict__ Ga0 = EF ? p.Ha : p.Ea;
+    const float *G0 = EF ? p.H : p.E; /* field whose curl drives it */
+    const float *Ga0 = EF ? p.Ha : p.Ea;
     const float sg = EF ? 1.0f : -1.0f;
     const int k = *p.s.base + rel;
     const int q = monitor_index(p.d, j2);
@@ -461,7 +462,7 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
     const float *__restrict__ cf = EF ? p.be : p.bh;
     float *__restrict__ F = (EF ? p.E : p.H) + b * bs;
     float *__restrict__ Fa = (EF ? p.Ea : p.Ha) + b * bs;
-    const float *__restrict__ G = (EF ? p.H : p.E) + b * bs;
+    const float *G = (EF ? p.H : p.E) + b * bs;
     const float sg = EF ? 1.0f : -1.0f;
     const int k = *p.s.base + rel;
     const int px0 = x0 + g.L0 * j1;
@@ -657,6 +658,7 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
 template <bool EF, int MB>
 __global__ void __launch_bounds__(128, MB) k_sweep32v(const P32 p, const int rel, const int z0)
 {
+    prior_done();
     const int b = blockIdx.y % p.batch;
     const int xr = (blockIdx.x * 32 + threadIdx.x) * 4;
     const int j1 = (blockIdx.y / p.batch) * blockDim.y + threadIdx.y;
@@ -677,6 +679,7 @@ __global__ void __launch_bounds__(128, MB) k_sweep32v(const P32 p, const int rel
 template <bool EF, bool PAD, int MB>
 __global__ void __launch_bounds__(128, MB) k_sweep32f(const P32 p, const int rel, const int z0)
 {
+    prior_done();
     const int b = blockIdx.x % p.batch, nq = (PAD ? p.g.P0 : p.g.L0) >> 2;
     const int i = blockIdx.x / p.batch * blockDim.x + threadIdx.x, last = nq * p.g.L1 - 1;
     const int u = i <= last ? i : last, j1 = u / nq;
@@ -755,6 +758,7 @@ __device__ void general32_cell(const P32 &p, const int rel, const int b, const l
 template <bool EF>
 __global__ void k_general32(const P32 p, const int rel, const int *cells, int ncells)
 {
+    prior_done();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ncells) return;
     general32_cell<EF, false>(p, rel, blockIdx.y, cells[i]);
@@ -942,13 +946,13 @@ __global__ void __launch_bounds__(128, 6) k_flush32(const P32 p, const int rel_e
 void launch_h32(const P32 &p, int rel, int by, int z0, int z1, cudaStream_t st)
 {
     dim3 blk(32, by, 1), grd((p.g.L0 + 31) / 32, ((p.g.L1 + by - 1) / by) * p.batch, z1 - z0);
-    k_sweep32<false><<<grd, blk, 0, st>>>(p, rel, z0);
+    launch_after(k_sweep32<false>, grd, blk, 0, st, p, rel, z0);
 }
 
 void launch_e32(const P32 &p, int rel, int by, int z0, int z1, cudaStream_t st)
 {
     dim3 blk(32, by, 1), grd((p.g.L0 + 31) / 32, ((p.g.L1 + by - 1) / by) * p.batch, z1 - z0);
-    k_sweep32<true><<<grd, blk, 0, st>>>(p, rel, z0);
+    launch_after(k_sweep32<true>, grd, blk, 0, st, p, rel, z0);
 }
 
 /* gcells / ngh: the general cells of those planes */
@@ -981,13 +985,13 @@ static void launch_sweep32v(const P32 &p, int rel, int by, int mb, int z0, int z
         else k_sweep32v2<EF, 4><<<grd, blk, 0, st>>>(p, rel, z0, z1);
     } else if (flat_quads(p.g.L0)) {
         grd = dim3(sweep32f_blocks(p.g.L0 / 4 * p.g.L1, 32 * by) * p.batch, z1 - z0);
-        if (mb >= 8) k_sweep32f<EF, false, 8><<<grd, 32 * by, 0, st>>>(p, rel, z0);
-        else if (mb == 6) k_sweep32f<EF, false, 6><<<grd, 32 * by, 0, st>>>(p, rel, z0);
-        else k_sweep32f<EF, false, 5><<<grd, 32 * by, 0, st>>>(p, rel, z0);
+        if (mb >= 8) launch_after(k_sweep32f<EF, false, 8>, grd, dim3(32 * by), 0, st, p, rel, z0);
+        else if (mb == 6) launch_after(k_sweep32f<EF, false, 6>, grd, dim3(32 * by), 0, st, p, rel, z0);
+        else launch_after(k_sweep32f<EF, false, 5>, grd, dim3(32 * by), 0, st, p, rel, z0);
     } else {
-        if (mb >= 8) k_sweep32v<EF, 8><<<grd, blk, 0, st>>>(p, rel, z0);
-        else if (mb == 6) k_sweep32v<EF, 6><<<grd, blk, 0, st>>>(p, rel, z0);
-        else k_sweep32v<EF, 5><<<grd, blk, 0, st>>>(p, rel, z0);
+        if (mb >= 8) launch_after(k_sweep32v<EF, 8>, grd, blk, 0, st, p, rel, z0);
+        else if (mb == 6) launch_after(k_sweep32v<EF, 6>, grd, blk, 0, st, p, rel, z0);
+        else launch_after(k_sweep32v<EF, 5>, grd, blk, 0, st, p, rel, z0);
     }
 }
 
@@ -995,14 +999,14 @@ void launch_h32v(const P32 &p, int rel, int by, int mb, int z0, int z1, const in
                  cudaStream_t st)
 {
     launch_sweep32v<false>(p, rel, by, mb, z0, z1, st);
-    if (ngh > 0) k_general32<false><<<dim3((ngh + 127) / 128, p.batch), 128, 0, st>>>(p, rel, gcells, ngh);
+    if (ngh > 0) launch_after(k_general32<false>, dim3((ngh + 127) / 128, p.batch), dim3(128), 0, st, p, rel, gcells, ngh);
 }
 
 void launch_e32v(const P32 &p, int rel, int by, int mb, int z0, int z1, const int *gcells, int nge,
                  cudaStream_t st)
 {
     launch_sweep32v<true>(p, rel, by, mb, z0, z1, st);
-    if (nge > 0) k_general32<true><<<dim3((nge + 127) / 128, p.batch), 128, 0, st>>>(p, rel, gcells, nge);
+    if (nge > 0) launch_after(k_general32<true>, dim3((nge + 127) / 128, p.batch), dim3(128), 0, st, p, rel, gcells, nge);
 }
 
 template <bool EF>
@@ -1010,8 +1014,8 @@ static void launch_sweep32p(const P32 &p, int rel, int threads, int z0, int z1, 
                             cudaStream_t st)
 {
     const int n = sweep32f_blocks(p.g.P0 / 4 * p.g.L1, threads);
-    k_sweep32f<EF, true, 5><<<dim3(n * p.batch, z1 - z0), threads, 0, st>>>(p, rel, z0);
-    if (ng > 0) k_general32<EF><<<dim3((ng + 127) / 128, p.batch), 128, 0, st>>>(p, rel, gcells, ng);
+    launch_after(k_sweep32f<EF, true, 5>, dim3(n * p.batch, z1 - z0), dim3(threads), 0, st, p, rel, z0);
+    if (ng > 0) launch_after(k_general32<EF>, dim3((ng + 127) / 128, p.batch), dim3(128), 0, st, p, rel, gcells, ng);
 }
 
 void launch_h32p(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng, cudaStream_t st)

@@ -259,6 +259,7 @@ __global__ void __launch_bounds__(96, 13) k_sweep64(const P64 p, const int rel)
     if (AFTER) {
         if (sp) load_coef();
         prior_done();
+        next_may_start();
     }
     double f = F[i0];
     const Near v = load_near<AFTER>(G, i1, i2, o1, o2);

@@ -198,18 +198,17 @@ struct RowGroup32 {
 
 
 /* Kernels of a step follow one another as programmatic dependents
- * (launch_after): one may start when every block of the one before has passed
- * prior_done, and runs up to its own prior_done beside it -- index arithmetic
- * and loads of what no launch of a run changes (coefficients, masks, orders,
- * records).  Fields, the ring and the step counter are touched after it only,
- * and fields that the kernel before writes are read through coherent loads
- * (no const __restrict__: such loads may count on data that stands still for the
- * whole kernel).  Every thread that touches them calls it. */
-__device__ __forceinline__ void prior_done()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+ * (launch_after): one is set up while the one before ends and waits for its
+ * results in prior_done, which every thread that touches fields, the ring or
+ * the step counter calls first (half a microsecond a launch: 14.1 -> 12.6 us
+ * for a step of two sweeps at 48^3 cells, 21.0 -> 20.0 at 100^3, 71.9 -> 71.4
+ * at 160 x 160 x 120).  What the kernel before writes is read through coherent
+ * loads (no const __restrict__: such loads may count on data that stands still for
+ * the whole kernel).  After next_may_start in every block the next kernel may
+ * run up to its own prior_done beside this one -- index arithmetic and loads of
+ * what no launch of a run changes (coefficients, masks, orders, records). */
+__device__ __forceinline__ void prior_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>
 inline cudaError_t launch_after(void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
 {
