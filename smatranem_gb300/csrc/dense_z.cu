@@ -537,9 +537,10 @@ __host__ __device__ inline size_t gj_panel_smem(int R, int w)
     return sizeof(double2) * ((size_t)R * (w + 1) + 2 * 16 * NBMAX + (NBMAX + 1) * (NBMAX + 1) + R) + sizeof(int) * ((size_t)R + 64);
 }
 
-__global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *__restrict__ A, int lda, int j, int n, int nb, int w,
+__global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int j, int n, int nb, int w,
                                                   double2 *__restrict__ lud, int *__restrict__ mv, int *info)
 {
+    prior_done();
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     const int nc = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -700,19 +701,8 @@ static int launch_gj_panel(const double2 *A, int lda, int j, int n, int nb, int 
     static const bool ready = cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
                               cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GJ_SMEM) == cudaSuccess;
     if (!ready) return smat_fail(SMAT_ECUDA, "k_gj_panel: cluster of 16 CTAs refused");
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cs;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(cs);
-    cfg.blockDim = dim3(GJT);
-    cfg.dynamicSmemBytes = gj_panel_smem((m + cs - 1) / cs, w);
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_gj_panel, A, lda, j, n, nb, w, lud, mv, info) != cudaSuccess)
+    if (launch_after_in(cs, k_gj_panel, dim3(cs), dim3(GJT), gj_panel_smem((m + cs - 1) / cs, w), st, A, lda, j, n, nb, w, lud,
+                        mv, info) != cudaSuccess)
         return smat_fail(SMAT_ECUDA, "k_gj_panel launch: %s", cudaGetErrorString(cudaGetLastError()));
     return SMAT_OK;
 }

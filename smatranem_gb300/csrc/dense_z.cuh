@@ -6,6 +6,8 @@
 
 #include <cuda_runtime.h>
 
+#include "launch_after.cuh"
+
 namespace smat {
 namespace dense {
 

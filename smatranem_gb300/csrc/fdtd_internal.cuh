@@ -31,6 +31,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "launch_after.cuh"
+
 namespace smat {
 
 enum : uint8_t { CLS_N = 0, CLS_A = 1, CLS_H = 2, CLS_E = 3, CLS_B = 4 };
@@ -196,34 +198,6 @@ struct RowGroup32 {
     Row32 r[MAX_GROUP];
 };
 
-
-/* Kernels of a step follow one another as programmatic dependents
- * (launch_after): one is set up while the one before ends and waits for its
- * results in prior_done, which every thread that touches fields, the ring or
- * the step counter calls first (half a microsecond a launch: 14.1 -> 12.6 us
- * for a step of two sweeps at 48^3 cells, 21.0 -> 20.0 at 100^3, 71.9 -> 71.4
- * at 160 x 160 x 120).  What the kernel before writes is read through coherent
- * loads (no const __restrict__: such loads may count on data that stands still for
- * the whole kernel).  After next_may_start in every block the next kernel may
- * run up to its own prior_done beside this one -- index arithmetic and loads of
- * what no launch of a run changes (coefficients, masks, orders, records). */
-__device__ __forceinline__ void prior_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-template <class... P, class... A>
-inline cudaError_t launch_after(void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
-{
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
-}
 
 /* The curl stencil of a cell: offsets of its forward (fwd) or backward
  * neighbour along each axis, wrapped at the grid's faces, and the boundary

@@ -206,9 +206,10 @@ __global__ void k_cut_cols(int k, int n, const double2 *__restrict__ B, int ldb,
  * moves, cut into slice images as k_cut_rows does (or copied to prow for the
  * FP64 kernel), and set to zero in M; rows of K itself count as zero.  One
  * warp per row. */
-__global__ void k_gj_rows(int rows, int j, int nb, double2 *M, int ld, const int *__restrict__ mv,
+__global__ void k_gj_rows(int rows, int j, int nb, double2 *M, int ld, const int *mv,
                           unsigned char *__restrict__ img, int *__restrict__ ea, int ntr, double2 *__restrict__ prow)
 {
+    prior_done();
     const int r = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5), t = threadIdx.x & 31;
     if (r >= ntr * BM) return;
     const unsigned hit = __ballot_sync(0xffffffffu, mv[32 + t] == r); /* the row moved here, if any */
@@ -253,10 +254,11 @@ __global__ void k_gj_rows(int rows, int j, int nb, double2 *M, int ld, const int
  * warp, which saves the instructions of rows a step no longer touches, has too
  * few warps (25 us and more).  The first block also moves the entries of
  * perm. */
-__global__ void __launch_bounds__(32) k_gj_cols(int cols, int j, int nb, double2 *M, int ld, const double2 *__restrict__ lud,
-                                                const int *__restrict__ mv, int *perm, unsigned char *__restrict__ img,
+__global__ void __launch_bounds__(32) k_gj_cols(int cols, int j, int nb, double2 *M, int ld, const double2 *lud,
+                                                const int *mv, int *perm, unsigned char *__restrict__ img,
                                                 int *__restrict__ eb, int ntc, double2 *__restrict__ bcol)
 {
+    prior_done();
     __shared__ double2 f[KC * KC];
     const int t = threadIdx.x, c = (int)blockIdx.x;
     const int from = mv[t], to = mv[32 + t];
@@ -430,9 +432,10 @@ constexpr int MMA_THREADS = 256; /* 8 warps: two per TMEM lane quarter in the ep
  * through the same epilogue. */
 __global__ void __launch_bounds__(MMA_THREADS, 2)
     k_oz_mma(int m, int n, double2 alpha, const unsigned char *__restrict__ aimg, const unsigned char *__restrict__ bimg,
-             const int *__restrict__ ea, const int *__restrict__ eb, int ntr, int ntc, double2 *C, int ldc, int *err,
+             const int *ea, const int *eb, int ntr, int ntc, double2 *C, int ldc, int *err,
              unsigned wait_limit, int skip_slice)
 {
+    prior_done();
     extern __shared__ __align__(1024) unsigned char sm[];
     unsigned char *ring = sm, *sB = sm + RING * AIMG;
     double2 *sC = reinterpret_cast<double2 *>(sB + S * BIMG); /* [16][128] */
@@ -682,10 +685,10 @@ int sweep_update(int rows, int cols, int j, int nb, double2 *M, int ld, const Sw
     unsigned char *bimg = aimg + (size_t)S * ntr * AIMG;
     int *ea = reinterpret_cast<int *>(bimg + (size_t)S * ntc * BIMG);
     int *eb = ea + ntr * BM;
-    k_gj_rows<<<ntr * BM / 8, 256, 0, st>>>(rows, j, nb, M, ld, w.mv, aimg, ea, ntr, nullptr);
-    k_gj_cols<<<ntc * BNC, 32, 0, st>>>(cols, j, nb, M, ld, w.lud, w.mv, w.perm, bimg, eb, ntc, nullptr);
-    k_oz_mma<<<dim3((unsigned)ntr, (unsigned)ntc), MMA_THREADS, SMEM, st>>>(
-        rows, cols, m1, aimg, bimg, ea, eb, ntr, ntc, M, ld, g.err, g.wait_limit ? g.wait_limit : WAIT_LIMIT, g.skip_pair);
+    launch_after(k_gj_rows, dim3(ntr * BM / 8), dim3(256), 0, st, rows, j, nb, M, ld, w.mv, aimg, ea, ntr, nullptr);
+    launch_after(k_gj_cols, dim3(ntc * BNC), dim3(32), 0, st, cols, j, nb, M, ld, w.lud, w.mv, w.perm, bimg, eb, ntc, nullptr);
+    launch_after(k_oz_mma, dim3((unsigned)ntr, (unsigned)ntc), dim3(MMA_THREADS), SMEM, st, rows, cols, m1, aimg, bimg, ea, eb,
+                 ntr, ntc, M, ld, g.err, g.wait_limit ? g.wait_limit : WAIT_LIMIT, g.skip_pair);
     if (cudaPeekAtLastError() != cudaSuccess)
         return smat_fail(SMAT_ECUDA, "sweep launch: %s", cudaGetErrorString(cudaGetLastError()));
     return SMAT_OK;
