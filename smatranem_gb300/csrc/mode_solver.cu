@@ -237,144 +237,6 @@ __global__ void k_mbb2(Op op, const T *__restrict__ Vt, const T *__restrict__ W,
  * pipe (35 -> 31 us a product); of a 40 x 30 layer, where launches count: 10.5
  * and 6.8 ms.  Tiles of 8 rows where 16 would leave SMs without a block: small
  * layers are bound by one block's latency.
- * ascale: alpha read from device memory instead.
- * Ynew may alias Yprev (each thread reads its own entries before writing). */
-template <class T>
-__global__ void k_mbb(Op op, const T *__restrict__ Vt, const T *__restrict__ W, const T *Ycur, const T *Yprev, T *Ynew,
-                      long long ld, T alpha, T c, T beta, const double *__restrict__ ascale)
-{
-    if (ascale) alpha = (T)*ascale;
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= op.NA1) return;
-    const int L0 = op.L0, L1 = op.L1, NA1 = op.NA1;
-    const int i0 = p % L0, i1 = p / L0;
-    const T s0 = (T)op.s0, s1 = (T)op.s1, e0 = (T)op.e0, e1 = (T)op.e1;
-    const long long col = (long long)blockIdx.y * ld;
-    const T *w0 = W + col, *w1 = w0 + NA1;
-    const T *V5 = Vt + 5 * (long long)NA1;
-    auto cwt = [](int i, int La, T e) { return i < La - 1 ? (T)1 : e; };
-    auto div = [&](int j0, int j1) {  // u at (j0, j1)
-        const int q = j0 + L0 * j1;
-        const int j0m = j0 == 0 ? L0 - 1 : j0 - 1, j1m = j1 == 0 ? L1 - 1 : j1 - 1;
-        const T a0 = -s0 * __ldg(w0 + q) - cwt(j0m, L0, e0) * __ldg(w0 + j0m + L0 * j1);
-        const T a1 = -s1 * __ldg(w1 + q) - cwt(j1m, L1, e1) * __ldg(w1 + j0 + L0 * j1m);
-        return __ldg(V5 + q) * (a0 + a1);
-    };
-    const int i0p = i0 + 1 == L0 ? 0 : i0 + 1, i1p = i1 + 1 == L1 ? 0 : i1 + 1;
-    const T up = div(i0, i1), up0 = div(i0p, i1), up1 = div(i0, i1p);
-    const T o0 = __ldg(Vt + 3 * (long long)NA1 + p) * __ldg(w0 + p) + (s0 * up + cwt(i0, L0, e0) * up0);
-    const T o1 = __ldg(Vt + 4 * (long long)NA1 + p) * __ldg(w1 + p) + (s1 * up + cwt(i1, L1, e1) * up1);
-    const T *yc = Ycur + col;
-    T r0 = alpha * (o0 - c * yc[p]), r1 = alpha * (o1 - c * yc[p + NA1]);
-    if (beta != (T)0) {
-        const T *yp = Yprev + col;
-        r0 -= beta * yp[p];
-        r1 -= beta * yp[p + NA1];
-    }
-    T *yn = Ynew + col;
-    yn[p] = r0;
-    yn[p + NA1] = r1;
-}
-
-/* The same operators in two passes each, every curl w (resp. divergence u)
- * evaluated once per point instead of at three points: half the FP64
- * operations (the stencils are FP64-pipe bound), the same expressions, so
- * the results are bit-identical to k_maa / k_mbb. */
-template <class T>
-__global__ void k_curl(Op op, const T *__restrict__ Vt, const T *__restrict__ X, T *__restrict__ Wc, long long ld)
-{
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= op.NA1) return;
-    const int L0 = op.L0, L1 = op.L1, NA1 = op.NA1;
-    const int j0 = p % L0, j1 = p / L0;
-    const T s0 = (T)op.s0, s1 = (T)op.s1, e0 = (T)op.e0, e1 = (T)op.e1;
-    const T *x0 = X + (long long)blockIdx.y * ld, *x1 = x0 + NA1;
-    auto cwt = [](int i, int La, T e) { return i < La - 1 ? (T)1 : e; };
-    const int q0 = (j0 + 1 == L0 ? 0 : j0 + 1) + L0 * j1, q1 = j0 + L0 * (j1 + 1 == L1 ? 0 : j1 + 1);
-    const T d1 = s1 * __ldg(x0 + p) + cwt(j1, L1, e1) * __ldg(x0 + q1);
-    const T d0 = s0 * __ldg(x1 + p) + cwt(j0, L0, e0) * __ldg(x1 + q0);
-    Wc[(long long)blockIdx.y * ld + p] = __ldg(Vt + 2 * (long long)NA1 + p) * (d1 - d0);
-}
-
-template <class T>
-__global__ void k_maa2(Op op, const T *__restrict__ Vt, const T *__restrict__ X, const T *__restrict__ Wc,
-                       T *__restrict__ Y, long long ld)
-{
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= op.NA1) return;
-    const int L0 = op.L0, L1 = op.L1, NA1 = op.NA1;
-    const int i0 = p % L0, i1 = p / L0;
-    const int i0m = i0 == 0 ? L0 - 1 : i0 - 1, i1m = i1 == 0 ? L1 - 1 : i1 - 1;
-    const T s0 = (T)op.s0, s1 = (T)op.s1, e0 = (T)op.e0, e1 = (T)op.e1;
-    auto cwt = [](int i, int La, T e) { return i < La - 1 ? (T)1 : e; };
-    const long long col = (long long)blockIdx.y * ld;
-    const T *x0 = X + col, *x1 = x0 + NA1, *w = Wc + col;
-    const T wp = __ldg(w + p), wm0 = __ldg(w + i0m + L0 * i1), wm1 = __ldg(w + i0 + L0 * i1m);
-    T *y0 = Y + col, *y1 = y0 + NA1;
-    y0[p] = __ldg(Vt + p) * __ldg(x0 + p) + (-s1 * wp - cwt(i1m, L1, e1) * wm1);
-    y1[p] = __ldg(Vt + NA1 + p) * __ldg(x1 + p) - (-s0 * wp - cwt(i0m, L0, e0) * wm0);
-}
-
-template <class T>
-__global__ void k_div(Op op, const T *__restrict__ Vt, const T *__restrict__ W, T *__restrict__ U, long long ld)
-{
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= op.NA1) return;
-    const int L0 = op.L0, L1 = op.L1, NA1 = op.NA1;
-    const int j0 = p % L0, j1 = p / L0;
-    const T s0 = (T)op.s0, s1 = (T)op.s1, e0 = (T)op.e0, e1 = (T)op.e1;
-    auto cwt = [](int i, int La, T e) { return i < La - 1 ? (T)1 : e; };
-    const T *w0 = W + (long long)blockIdx.y * ld, *w1 = w0 + NA1;
-    const int j0m = j0 == 0 ? L0 - 1 : j0 - 1, j1m = j1 == 0 ? L1 - 1 : j1 - 1;
-    const T a0 = -s0 * __ldg(w0 + p) - cwt(j0m, L0, e0) * __ldg(w0 + j0m + L0 * j1);
-    const T a1 = -s1 * __ldg(w1 + p) - cwt(j1m, L1, e1) * __ldg(w1 + j0 + L0 * j1m);
-    U[(long long)blockIdx.y * ld + p] = __ldg(Vt + 5 * (long long)NA1 + p) * (a0 + a1);
-}
-
-template <class T>
-__global__ void k_mbb2(Op op, const T *__restrict__ Vt, const T *__restrict__ W, const T *__restrict__ Uc,
-                       const T *Ycur, const T *Yprev, T *Ynew, long long ld, T alpha, T c, T beta,
-                       const double *__restrict__ ascale)
-{
-    if (ascale) alpha = (T)*ascale;
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= op.NA1) return;
-    const int L0 = op.L0, L1 = op.L1, NA1 = op.NA1;
-    const int i0 = p % L0, i1 = p / L0;
-    const T s0 = (T)op.s0, s1 = (T)op.s1, e0 = (T)op.e0, e1 = (T)op.e1;
-    auto cwt = [](int i, int La, T e) { return i < La - 1 ? (T)1 : e; };
-    const long long col = (long long)blockIdx.y * ld;
-    const T *w0 = W + col, *w1 = w0 + NA1, *u = Uc + col;
-    const int i0p = i0 + 1 == L0 ? 0 : i0 + 1, i1p = i1 + 1 == L1 ? 0 : i1 + 1;
-    const T up = __ldg(u + p), up0 = __ldg(u + i0p + L0 * i1), up1 = __ldg(u + i0 + L0 * i1p);
-    const T o0 = __ldg(Vt + 3 * (long long)NA1 + p) * __ldg(w0 + p) + (s0 * up + cwt(i0, L0, e0) * up0);
-    const T o1 = __ldg(Vt + 4 * (long long)NA1 + p) * __ldg(w1 + p) + (s1 * up + cwt(i1, L1, e1) * up1);
-    const T *yc = Ycur + col;
-    T r0 = alpha * (o0 - c * yc[p]), r1 = alpha * (o1 - c * yc[p + NA1]);
-    if (beta != (T)0) {
-        const T *yp = Yprev + col;
-        r0 -= beta * yp[p];
-        r1 -= beta * yp[p + NA1];
-    }
-    T *yn = Ynew + col;
-    yn[p] = r0;
-    yn[p + NA1] = r1;
-}
-
-/* Ynew = alpha (mbb maa Ycur - c Ycur) - beta Yprev in one launch: each block
- * stages a tile of Ycur with two halo points per side in shared memory and
- * evaluates w, maa Y, u and mbb there, one halo ring fewer each stage.  The
- * same operations as k_curl, k_maa2, k_div and k_mbb2 in turn, so the same
- * bits: a link across the lattice's edge carries its wrap coefficient, a link
- * inside 1, and a product by -1, 0 or 1 is exact, so s x + c x' is the one
- * fused multiply-add c x' - x (s = -1: both axes have more than one cell).
- *
- * The stencils are bound by the FP64 pipe (1.7 operations a clock and SM
- * measured): 22 operations a point against the four launches' 30, and 14 %
- * more points in the halos of a 32 x 16 tile.  A solve of the 256 x 192 layer
- * (1150 products of 12 columns): 70.3 ms with four launches a product, 48.1 ms
- * with one; of a 40 x 30 layer, where launches count: 10.5 and 6.8 ms.  Tiles of 8 rows where 16 would leave SMs without
- * a block: small layers are bound by one block's latency.
  * ascale: alpha read from device memory instead (the power iteration). */
 constexpr int PX = 32; /* tile columns */
 __device__ __forceinline__ float mul(float a, float b) { return a * b; }
