@@ -790,6 +790,17 @@ extern "C" int smat_fdtd_create(const smat_fdtd_desc *d, void *stream, smat_fdtd
                 for (int c = 0; c < 3; c++) Ae[c + 3 * l] = Be[c + 3 * l] = 0.0;
     rc = p->precision == SMAT_FP64 ? upload_f64(p, Ah.get(), Bh.get(), Ae.get(), Be.get())
                                    : upload_f32(p, d, Ah.get(), Bh.get(), Ae.get(), Be.get());
+    if (rc == SMAT_ENOMEM && p->P0 != p->L[0]) { /* no room for the padding: without it */
+        cudaStreamSynchronize(p->stream);
+        for (void *a : p->allocations) cudaFree(a);
+        p->allocations.clear();
+        p->dev_bytes = 0;
+        p->nrec_metal = p->nrec_split = 0;
+        p->P0 = p->L[0];
+        p->n3p = p->n3;
+        smat_clear_error();
+        rc = upload_f32(p, d, Ah.get(), Bh.get(), Ae.get(), Be.get());
+    }
     return finish_create(p, rc, out);
 }
 

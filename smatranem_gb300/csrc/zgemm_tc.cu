@@ -2,7 +2,7 @@
  * FP64-accurate complex multiply-add on the tensor cores: C += alpha * A * B
  * with A (m x k), B (k x n), C (m x n) complex FP64, column-major -- the
  * zgemm_ of the layer transfer (Smat/Scalc.c inv_process :316-400 through the
- * blocked LU of dense_z.cu), computed by the Ozaki scheme (Ozaki, Ogita,
+ * sweeps and the LU of dense_z.cu), computed by the Ozaki scheme (Ozaki, Ogita,
  * Oishi, Rump, "Error-free transformations of matrix multiplication by using
  * fast routines of matrix multiplication and its applications", Numer.
  * Algorithms 59, 2012), in the tensor-core form of Mukunoki, Ozaki, Ogita and
