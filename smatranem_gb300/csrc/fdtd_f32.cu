@@ -447,8 +447,9 @@ __device__ __forceinline__ void quad_compute(const P32 &p, const int rel, const 
 /* one quad: cells x = xr..xr+3 of row j1, plane j2, excitation b; the lanes of a
  * warp hold consecutive quads.  PAD: rows of padded length, whose last quad is
  * cut off at L0 -- its cells past L0 neither wrap, nor take the source, nor are
- * sampled; lanes that are not in repeat a live quad and store nothing. */
-template <bool EF, bool CG, bool PAD>
+ * sampled; lanes that are not in repeat a live quad and store nothing.  GEN:
+ * other threads of the launch take the general cells. */
+template <bool EF, bool CG, bool PAD, bool GEN>
 __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const int b, const int j1, const int j2,
                                               const int xr, const bool in)
 {
@@ -525,6 +526,7 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
     const bool on_src = j2 == p.s.iI[b];
     const int q = monitor_index(p.d, j2);
     bool any_aux = false;
+    unsigned gen = 0; /* GEN: the quad's general cells, which it leaves alone */
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int xx = x0 + i;
@@ -555,8 +557,9 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
             mi[2] = h0 - el(gy0, i);
         }
         const float c0 = el(c[0], i);
-        if (isnan(c0)) { /* general cell: rewritten by k_general32 after this launch */
-            any_aux = true;
+        if (isnan(c0)) { /* general cell: k_general32 after this launch, or (GEN) others of it */
+            if (GEN) gen |= 1u << i;
+            else any_aux = true;
             continue;
         }
         if (PAD && xx >= g.L0) continue; /* padding: stays 0 */
@@ -629,6 +632,20 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
             }
         }
     }
+    if (GEN && gen) {
+        float *ring = q >= 0 ? ring_at(p.d, g.pl, b, k, q, EF ? 2 : 0) + px0 : nullptr;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (gen >> i & 1u || (PAD && x0 + i >= g.L0)) continue;
+#pragma unroll
+            for (int cc = 0; cc < 3; cc++) {
+                F[cc * n3 + l + i] = el(out[cc], i);
+                if (any_aux) Fa[cc * n3 + l + i] = el(aux[cc], i);
+                if (cc < 2 && ring) ring[(long long)cc * g.pl + i] = el(out[cc], i);
+            }
+        }
+        return;
+    }
 #pragma unroll
     for (int cc = 0; cc < 3; cc++) st4(F + cc * n3 + l, out[cc]);
     if (any_aux) {
@@ -662,34 +679,13 @@ __global__ void __launch_bounds__(128, MB) k_sweep32v(const P32 p, const int rel
     const int b = blockIdx.y % p.batch;
     const int xr = (blockIdx.x * 32 + threadIdx.x) * 4;
     const int j1 = (blockIdx.y / p.batch) * blockDim.y + threadIdx.y;
-    sweep32v_quad<EF, false, false>(p, rel, b, j1, z0 + blockIdx.z, xr, true);
+    sweep32v_quad<EF, false, false, false>(p, rel, b, j1, z0 + blockIdx.z, xr, true);
 }
 
-/* The same with the quads of a plane dealt out to the threads one after
- * another, whatever their row: rows of any length fill the warps, where a warp
- * per row piece leaves lanes idle unless L0 % 128 == 0 (83 % of the lanes used
- * at 320 cells, 63 % at 160, 52 % in padded rows of 131).  Bound by the latency
- * of a quad's loads, then by HBM.  us a step, row pieces / dealt out: 320 x 320
- * x 256 498 / 471 (5.3 TB/s), 160 x 160 x 120 90.6 / 77.9, 144 x 100 x 100 of
- * two excitations 89.5 / 72.7; 256 x 192 x 64 of four, whose row pieces are
- * whole warps, 247 / 250: those keep k_sweep32v (flat_quads).  PAD: rows of
- * padded length, L0 % 4 != 0: 131 x 117 x 103 of two 138 with one cell a
- * thread, 83 so; 96 registers (MB = 5; 128: 88, 80: 91).  Block x: quads of the
- * plane x excitation (fastest, for the shared coefficients), y: the plane. */
-template <bool EF, bool PAD, int MB>
-__global__ void __launch_bounds__(128, MB) k_sweep32f(const P32 p, const int rel, const int z0)
-{
-    prior_done();
-    const int b = blockIdx.x % p.batch, nq = (PAD ? p.g.P0 : p.g.L0) >> 2;
-    const int i = blockIdx.x / p.batch * blockDim.x + threadIdx.x, last = nq * p.g.L1 - 1;
-    const int u = i <= last ? i : last, j1 = u / nq;
-    sweep32v_quad<EF, false, PAD>(p, rel, b, j1, z0 + blockIdx.y, 4 * (u - j1 * nq), i <= last);
-}
-
-/* general cells of the vectorised sweeps: one thread per record cell, run
- * after k_sweep32v of the same field (the quads skipped them) */
+/* general cells of the vectorised sweeps: one thread per record cell, after
+ * the sweep of the same field or beside it (the quads skip them) */
 template <bool EF, bool CG>
-__device__ void general32_cell(const P32 &p, const int rel, const int b, const long long l)
+__device__ __noinline__ void general32_cell(const P32 &p, const int rel, const int b, const long long l)
 {
     const Geo &g = p.g;
     const long long n3 = g.n3, bs = 3 * n3;
@@ -755,6 +751,34 @@ __device__ void general32_cell(const P32 &p, const int rel, const int b, const l
     }
 }
 
+/* The same with the quads of a plane dealt out to the threads one after
+ * another, whatever their row: rows of any length fill the warps, where a warp
+ * per row piece leaves lanes idle unless L0 % 128 == 0 (83 % of the lanes used
+ * at 320 cells, 63 % at 160, 52 % in padded rows of 131).  Bound by the latency
+ * of a quad's loads, then by HBM.  us a step, row pieces / dealt out: 320 x 320
+ * x 256 498 / 471 (5.3 TB/s), 160 x 160 x 120 90.6 / 77.9, 144 x 100 x 100 of
+ * two excitations 89.5 / 72.7; 256 x 192 x 64 of four, whose row pieces are
+ * whole warps, 247 / 250: those keep k_sweep32v (flat_quads).  PAD: rows of
+ * padded length, L0 % 4 != 0: 131 x 117 x 103 of two 138 with one cell a
+ * thread, 83 so; 96 registers (MB = 5; 128: 88, 80: 91).  Block x: quads of the
+ * plane x excitation (fastest, for the shared coefficients), y: the
+ * plane.  GEN: plans with general cells, which the blocks of y = 0 take
+ * (launch_sweep32f). */
+template <bool EF, bool PAD, int MB, bool GEN>
+__global__ void __launch_bounds__(128, MB) k_sweep32f(const P32 p, const int rel, const int z0, const int *cells, const int ncells)
+{
+    prior_done();
+    if (GEN && blockIdx.y == 0) {
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncells * p.batch; i += gridDim.x * blockDim.x)
+            general32_cell<EF, false>(p, rel, i % p.batch, cells[i / p.batch]);
+        return;
+    }
+    const int b = blockIdx.x % p.batch, nq = (PAD ? p.g.P0 : p.g.L0) >> 2;
+    const int i = blockIdx.x / p.batch * blockDim.x + threadIdx.x, last = nq * p.g.L1 - 1;
+    const int u = i <= last ? i : last, j1 = u / nq;
+    sweep32v_quad<EF, false, PAD, GEN>(p, rel, b, j1, z0 + blockIdx.y - GEN, 4 * (u - j1 * nq), i <= last);
+}
+
 template <bool EF>
 __global__ void k_general32(const P32 p, const int rel, const int *cells, int ncells)
 {
@@ -788,7 +812,7 @@ __global__ void __launch_bounds__(128, 5) k_group32v(const int rel)
         const int z = local / per, t = local - z * per, b = t % p.batch;
         const int i = t / p.batch * 32 * c_group.by + 32 * threadIdx.y + threadIdx.x, last = nq * p.g.L1 - 1;
         const int u = i <= last ? i : last, j1 = u / nq;
-        sweep32v_quad<EF, false, false>(p, rel, b, j1, z, 4 * (u - j1 * nq), i <= last);
+        sweep32v_quad<EF, false, false, false>(p, rel, b, j1, z, 4 * (u - j1 * nq), i <= last);
         return;
     }
     const int nxb = (nq + 31) / 32;
@@ -797,7 +821,7 @@ __global__ void __launch_bounds__(128, 5) k_group32v(const int rel)
     const int yb = t % nyb, z = t / nyb;
     const int b = yb % p.batch;
     const int j1 = (yb / p.batch) * blockDim.y + threadIdx.y;
-    sweep32v_quad<EF, false, false>(p, rel, b, j1, z, (xb * 32 + threadIdx.x) * 4, true);
+    sweep32v_quad<EF, false, false, false>(p, rel, b, j1, z, (xb * 32 + threadIdx.x) * 4, true);
 }
 
 template <bool EF>
@@ -975,8 +999,27 @@ __global__ void __launch_bounds__(128, MB) k_sweep32v2(const P32 p, const int re
     if (two) quad_compute<EF>(p, rel, b, j1, za + 1, qb);
 }
 
+/* The sweep of quads dealt out (96 registers), with the general cells: in the
+ * same launch up to 4.5 million cells and excitations, where the launch they
+ * save counts for more than the quads' extra branch.  us a step of a plan with
+ * metal patches, in a launch of their own / in the sweep's: 48 x 48 x 64 18.8 /
+ * 16.4, 116 x 52 x 67 20.6 / 18.4, 131 x 120 x 90 of two 82.0 / 77.8, 160 x 160
+ * x 160 98.6 / 97.7; 160 x 160 x 120 of two 133.4 / 134.9, 320 x 320 x 256 472 /
+ * 487. */
+template <bool EF, bool PAD>
+static void launch_sweep32f(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng, cudaStream_t st)
+{
+    const int n = sweep32f_blocks((PAD ? p.g.P0 : p.g.L0) / 4 * p.g.L1, threads) * p.batch;
+    const bool inside = ng > 0 && (long long)p.g.ps * (z1 - z0) * p.batch <= 4500000;
+    if (inside) launch_after(k_sweep32f<EF, PAD, 5, true>, dim3(n, z1 - z0 + 1), dim3(threads), 0, st, p, rel, z0, gcells, ng);
+    else launch_after(k_sweep32f<EF, PAD, 5, false>, dim3(n, z1 - z0), dim3(threads), 0, st, p, rel, z0, gcells, 0);
+    if (ng > 0 && !inside)
+        launch_after(k_general32<EF>, dim3((ng + 127) / 128, p.batch), dim3(128), 0, st, p, rel, gcells, ng);
+}
+
+/* with the general cells gcells[0 .. ng) of those planes */
 template <bool EF>
-static void launch_sweep32v(const P32 &p, int rel, int by, int mb, int z0, int z1, cudaStream_t st)
+static void launch_sweep32v(const P32 &p, int rel, int by, int mb, int z0, int z1, const int *gcells, int ng, cudaStream_t st)
 {
     dim3 blk(32, by, 1), grd((p.g.L0 / 4 + 31) / 32, ((p.g.L1 + by - 1) / by) * p.batch, z1 - z0);
     if (mb < 0) { /* two planes per thread: -mb = register bound */
@@ -985,47 +1028,37 @@ static void launch_sweep32v(const P32 &p, int rel, int by, int mb, int z0, int z
         else k_sweep32v2<EF, 4><<<grd, blk, 0, st>>>(p, rel, z0, z1);
     } else if (flat_quads(p.g.L0)) {
         grd = dim3(sweep32f_blocks(p.g.L0 / 4 * p.g.L1, 32 * by) * p.batch, z1 - z0);
-        if (mb >= 8) launch_after(k_sweep32f<EF, false, 8>, grd, dim3(32 * by), 0, st, p, rel, z0);
-        else if (mb == 6) launch_after(k_sweep32f<EF, false, 6>, grd, dim3(32 * by), 0, st, p, rel, z0);
-        else launch_after(k_sweep32f<EF, false, 5>, grd, dim3(32 * by), 0, st, p, rel, z0);
+        if (mb >= 8) launch_after(k_sweep32f<EF, false, 8, false>, grd, dim3(32 * by), 0, st, p, rel, z0, gcells, 0);
+        else if (mb == 6) launch_after(k_sweep32f<EF, false, 6, false>, grd, dim3(32 * by), 0, st, p, rel, z0, gcells, 0);
+        else return launch_sweep32f<EF, false>(p, rel, 32 * by, z0, z1, gcells, ng, st);
     } else {
         if (mb >= 8) launch_after(k_sweep32v<EF, 8>, grd, blk, 0, st, p, rel, z0);
         else if (mb == 6) launch_after(k_sweep32v<EF, 6>, grd, blk, 0, st, p, rel, z0);
         else launch_after(k_sweep32v<EF, 5>, grd, blk, 0, st, p, rel, z0);
     }
+    if (ng > 0) launch_after(k_general32<EF>, dim3((ng + 127) / 128, p.batch), dim3(128), 0, st, p, rel, gcells, ng);
 }
 
 void launch_h32v(const P32 &p, int rel, int by, int mb, int z0, int z1, const int *gcells, int ngh,
                  cudaStream_t st)
 {
-    launch_sweep32v<false>(p, rel, by, mb, z0, z1, st);
-    if (ngh > 0) launch_after(k_general32<false>, dim3((ngh + 127) / 128, p.batch), dim3(128), 0, st, p, rel, gcells, ngh);
+    launch_sweep32v<false>(p, rel, by, mb, z0, z1, gcells, ngh, st);
 }
 
 void launch_e32v(const P32 &p, int rel, int by, int mb, int z0, int z1, const int *gcells, int nge,
                  cudaStream_t st)
 {
-    launch_sweep32v<true>(p, rel, by, mb, z0, z1, st);
-    if (nge > 0) launch_after(k_general32<true>, dim3((nge + 127) / 128, p.batch), dim3(128), 0, st, p, rel, gcells, nge);
-}
-
-template <bool EF>
-static void launch_sweep32p(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng,
-                            cudaStream_t st)
-{
-    const int n = sweep32f_blocks(p.g.P0 / 4 * p.g.L1, threads);
-    launch_after(k_sweep32f<EF, true, 5>, dim3(n * p.batch, z1 - z0), dim3(threads), 0, st, p, rel, z0);
-    if (ng > 0) launch_after(k_general32<EF>, dim3((ng + 127) / 128, p.batch), dim3(128), 0, st, p, rel, gcells, ng);
+    launch_sweep32v<true>(p, rel, by, mb, z0, z1, gcells, nge, st);
 }
 
 void launch_h32p(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng, cudaStream_t st)
 {
-    launch_sweep32p<false>(p, rel, threads, z0, z1, gcells, ng, st);
+    launch_sweep32f<false, true>(p, rel, threads, z0, z1, gcells, ng, st);
 }
 
 void launch_e32p(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng, cudaStream_t st)
 {
-    launch_sweep32p<true>(p, rel, threads, z0, z1, gcells, ng, st);
+    launch_sweep32f<true, true>(p, rel, threads, z0, z1, gcells, ng, st);
 }
 
 void launch_flush32(const P32 &p, int rel_end, int count, cudaStream_t st)

@@ -1051,3 +1051,21 @@ def test_row_fused_run_of_one_graph_from_the_other_set(built):
             out.append(p.get_fields(0))
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("L,batch", [((36, 9, 40, 2), 1), ((40, 40, 60, 2), 2), ((300, 150, 52, 2), 2)])
+def test_general_cells_in_the_sweep_launch(built, L, batch):
+    """General cells (metal, lossy, PEC: in quads with ordinary, split and other
+    general cells, on monitor and source planes) inside the vectorised sweep's
+    launch and, in a plan of more than 4.5 million cells and excitations, after
+    it: the bits of the one-cell-per-thread sweeps, whole grid and z chunks."""
+    from smatranem_gb300 import workloads as W
+    big = L[0] > 200
+    s = W.random_structure(L, seed=97, pml=(3, 2, 4), metals=0.02, lossy=0.1, pec=0.1, iBc=(-1, 1, 0))
+    pr = W.prepare(s)
+    iBTIin = (6, L[2] - 7, 8, 1)
+    ref = _run_fp32(s, pr, iBTIin, (0, 4, 0, 0, 4), 8, batch=batch)
+    for tuning in [(2, 1, 0, 5, 4)] if big else [(2, 1, 0, 5, 4), (2, 4, 0, 5, 4), (2, 2, 5, 5, 4), (2, 2, 0, 6, 4)]:
+        for rb, gb in zip(ref, _run_fp32(s, pr, iBTIin, tuning, 8, batch=batch)):
+            for a, b in zip(rb, gb):
+                assert np.all(np.isfinite(a)) and np.array_equal(a, b), tuning
