@@ -1010,7 +1010,7 @@ template <bool EF, bool PAD>
 static void launch_sweep32f(const P32 &p, int rel, int threads, int z0, int z1, const int *gcells, int ng, cudaStream_t st)
 {
     const int n = sweep32f_blocks((PAD ? p.g.P0 : p.g.L0) / 4 * p.g.L1, threads) * p.batch;
-    const bool inside = ng > 0 && (long long)p.g.ps * (z1 - z0) * p.batch <= 4500000;
+    const bool inside = ng > 0 && (long long)p.g.ps * (z1 - z0) * p.batch <= 4500000 && z1 - z0 < 65535;
     if (inside) launch_after(k_sweep32f<EF, PAD, 5, true>, dim3(n, z1 - z0 + 1), dim3(threads), 0, st, p, rel, z0, gcells, ng);
     else launch_after(k_sweep32f<EF, PAD, 5, false>, dim3(n, z1 - z0), dim3(threads), 0, st, p, rel, z0, gcells, 0);
     if (ng > 0 && !inside)
