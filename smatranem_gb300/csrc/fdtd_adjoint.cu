@@ -524,7 +524,8 @@ StateView state_view(smat_fdtd_plan *p)
         v.ptr[1] = p->d_E64;
         v.ptr[2] = p->d_Ha64;
         v.ptr[3] = p->d_Ea64;
-        v.bytes[0] = v.bytes[1] = v.bytes[2] = v.bytes[3] = b * 3 * p->n3 * 8;
+        v.bytes[0] = v.bytes[1] = b * 3 * p->n3 * 8;
+        v.bytes[2] = v.bytes[3] = b * 3 * (size_t)(p->lnotn + 1) * 8;
     } else {
         const P32 q = make_p32(p, false);
         v.ptr[0] = q.H;

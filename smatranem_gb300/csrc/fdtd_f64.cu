@@ -60,11 +60,9 @@ __device__ __forceinline__ double ld_coherent(const double *p)
     return v;
 }
 
-template <bool AFTER>
 __device__ __forceinline__ Near load_near(const double *__restrict__ F, int i1, int i2, int o1, int o2)
 {
-    if (AFTER) return Near{ld_coherent(F + i1), ld_coherent(F + i2), ld_coherent(F + i2 + o1), ld_coherent(F + i1 + o2)};
-    return Near{F[i1], F[i2], F[i2 + o1], F[i1 + o2]};
+    return Near{ld_coherent(F + i1), ld_coherent(F + i2), ld_coherent(F + i2 + o1), ld_coherent(F + i1 + o2)};
 }
 
 /* The half curls from them.  pl: the term differentiated along axis a1 ("+"
@@ -150,10 +148,10 @@ __device__ __noinline__ double metal_cell(const P64 &p, int cls, int b, int c, i
     }
     const int a1 = (c + 1) % 3, a2 = (c + 2) % 3;
     double pl, mi;
-    curl_near<false>(load_near<true>((EF ? p.H : p.E) + (long long)b * 3 * n3, a1 * n3 + l, a2 * n3 + l, o[a1], o[a2]), wrap,
+    curl_near<false>(load_near((EF ? p.H : p.E) + (long long)b * 3 * n3, a1 * n3 + l, a2 * n3 + l, o[a1], o[a2]), wrap,
                      s[a1], s[a2], pl, mi);
     const double W = pl + mi;
-    double *x = (EF ? p.Ea : p.Ha) + ((long long)b * 3 + c) * n3 + l;
+    double *x = (EF ? p.Ea : p.Ha) + ((long long)b * 3 + c) * (p.lnotn + 1) + a;
     const double *ca = p.ca + (long long)(EF ? 6 + c : c) * p.lnotn + a;
     double v = *x;
     f += 0.5 * v;
@@ -178,32 +176,31 @@ __device__ __noinline__ double metal_cell(const P64 &p, int cls, int b, int c, i
  * others, row by row.  And latency, of the loads and of the FP64 pipe (67
  * clocks): a thread takes one component of a cell, a block's three warps the
  * three components of 32 cells, which share the loaded lines in L1, so that
- * 39 warps fit an SM where 16 of whole cells did; cells that the host knows
- * to be split issue their aux loads with the others, before the class byte
- * has come back; the aux slots are dense, so that no address is fetched
- * first.  Excitations are fastest in the grid: the coefficients are shared
- * through L2.
+ * 39 warps fit an SM where 16 of whole cells did; a sweep is launched beside the
+ * one before (launch_after) and has its coefficients and the addresses of its
+ * aux slots by the time that one ends; and the aux slots, which fewer cells
+ * have, are asked for before the main ones (after them: the same on large
+ * grids, but 24 x 24 x 40 8.0 us a step instead of 6.0, the dependents falling
+ * into step with one another).  Dense aux slots, which need no addresses, took
+ * 48 bytes a cell and excitation more and gained nothing (119 us a step at
+ * 96^3, now 111).  Excitations are fastest in the grid: the coefficients are
+ * shared through L2.
  *
- * Measured a sweep, against one thread per cell with 32 consecutive x a warp
- * and every operation on the FP64 pipe: 96^3 cube (12-cell PML) 60 us, from
- * 85; 130 x 98 x 81 bend, two excitations, 129 us, from 211 (70 % of the
- * pipe's peak); 24 x 20 x 40 guide 3.2 us, from 5.  Blocks of 32 cells rather
- * than 64 or 128: 3 % and 10 % on the cube, 10 % and 30 % on the guide, whose
- * plane fills 15 of them.  13 resident blocks (48 registers): 10 and 15 are
- * within 7 %, 17 spills.
- *
- * AFTER: launched beside the sweep before (launch_after), with the coefficients
- * loaded before that one has ended. */
-template <bool EF, bool AFTER>
+ * us a step of two sweeps, run after run: 96^3 cube (12-cell PML) 111, 130 x 98
+ * x 81 bend of two excitations 243, 24 x 20 x 40 guide 5.2, where one thread per
+ * cell with 32 consecutive x a warp and every operation on the FP64 pipe took
+ * 170, 422 and 10.  Blocks of 32 cells rather than 64 or 128: 3 % and 10 % on the
+ * cube, 10 % and 30 % on the guide, whose plane fills 15 of them.  13 resident
+ * blocks (48 registers): 10 and 15 are within 7 %. */
+template <bool EF>
 __global__ void __launch_bounds__(96, 13) k_sweep64(const P64 p, const int rel)
 {
     const Geo &g = p.g;
     const int b = blockIdx.x % p.batch, i = blockIdx.x / p.batch * 32 + threadIdx.x;
     const int j2 = blockIdx.y, c = threadIdx.y;
     if (i >= g.pl) return;
-    const int2 od = p.ord[(EF ? g.pl : 0) + i]; /* pixel; 1: wraps along x, 2: along y, 4: split */
+    const int2 od = p.ord[(EF ? g.pl : 0) + i]; /* pixel; 1: wraps along x, 2: along y */
     const int px = od.x, n3 = (int)g.n3, l = px + g.pl * j2;
-    const bool sp = (od.y & 4) | p.smask[j2];
     const bool ex = od.y & 1, ey = od.y & 2, ez = j2 == (EF ? g.L2 - 1 : 0);
     const int sd = EF ? 1 : -1;
     const int ox = ex ? -sd * (g.L0 - 1) : sd, oy = (ey ? -sd * (g.L1 - 1) : sd) * g.L0;
@@ -214,32 +211,37 @@ __global__ void __launch_bounds__(96, 13) k_sweep64(const P64 p, const int rel)
     const Sel s1 = make_sel(g.bc[c == 2 ? 0 : c + 1], w1), s2 = make_sel(g.bc[c == 0 ? 2 : c - 1], w2);
     const int i0 = c * n3 + l, i1 = (c == 2 ? 0 : c + 1) * n3 + l, i2 = (c == 0 ? 2 : c - 1) * n3 + l;
     const long long bo = (long long)b * 3 * n3;
-    double *__restrict__ F = (EF ? p.E : p.H) + bo, *__restrict__ Fa = (EF ? p.Ea : p.Ha) + bo;
-    const double *__restrict__ G = (EF ? p.H : p.E) + bo, *__restrict__ Ga = (EF ? p.Ha : p.Ea) + bo;
+    const int as = p.lnotn + 1;
+    const long long ao = (long long)b * 3 * as;
+    double *__restrict__ F = (EF ? p.E : p.H) + bo, *__restrict__ Fa = (EF ? p.Ea : p.Ha) + ao + (long long)c * as;
+    const double *__restrict__ G = (EF ? p.H : p.E) + bo;
+    const double *__restrict__ Ga1 = (EF ? p.Ha : p.Ea) + ao + (long long)(c == 2 ? 0 : c + 1) * as;
+    const double *__restrict__ Ga2 = (EF ? p.Ha : p.Ea) + ao + (long long)(c == 0 ? 2 : c - 1) * as;
     const double *__restrict__ cm = p.cm + (EF ? 6 : 0) * g.n3, *__restrict__ ca = p.ca + (EF ? 6 + c : c) * (long long)p.lnotn;
     const int fl = p.flags[l], cls = fl & 7;
+    const bool aux = cls == CLS_A || (fl & (EF ? FL_FWD : FL_BWD)); /* the curl takes aux slots in */
     const double A = cm[i0], B = cm[3 * g.n3 + i0];
     double Aa, Ba;
-    auto load_coef = [&]() {
-        const int a = p.addr[l];
+    int a = 0, n1 = 0, n2 = 0; /* aux slots of the cell and of its neighbours along a1, a2 */
+    if (aux) {
+        a = p.addr[l];
+        n1 = p.addr[l + o1];
+        n2 = p.addr[l + o2];
+    }
+    if (cls == CLS_A) {
         Aa = ca[a];
         Ba = ca[3LL * p.lnotn + a];
-    };
-    if (AFTER) {
-        if (sp) load_coef();
-        prior_done();
-        next_may_start();
     }
+    prior_done();
+    next_may_start();
     double f = F[i0];
-    const Near v = load_near<AFTER>(G, i1, i2, o1, o2);
     double fa = 0.0;
     Near va;
-    auto load_aux = [&]() {
-        fa = Fa[i0];
-        if (!AFTER) load_coef();
-        va = load_near<AFTER>(Ga, i1, i2, o1, o2);
-    };
-    if (sp) load_aux();
+    if (aux) {
+        fa = Fa[a];
+        va = Near{ld_coherent(Ga1 + a), ld_coherent(Ga2 + a), ld_coherent(Ga2 + n1), ld_coherent(Ga1 + n2)};
+    }
+    const Near v = load_near(G, i1, i2, o1, o2);
     double pl, mi, pa, ma;
     if (cls == CLS_N) {
         curl_near<EF>(v, w1 | w2, s1, s2, pl, mi);
@@ -249,22 +251,18 @@ __global__ void __launch_bounds__(96, 13) k_sweep64(const P64 p, const int rel)
             W = c == 0 ? W + t : W - t;
         }
         f = amul(A, f) + imul<!EF>(B, W);
-        if (fl & (EF ? FL_FWD : FL_BWD)) {
-            curl_near<EF>(load_near<AFTER>(Ga, i1, i2, o1, o2), w1 | w2, s1, s2, pa, ma);
+        if (aux) {
+            curl_near<EF>(va, w1 | w2, s1, s2, pa, ma);
             f += imul<!EF>(B, pa + ma);
         }
     } else if (cls == CLS_A) {
-        if (!sp) {
-            if (AFTER) load_coef();
-            load_aux();
-        }
         curl_near<EF>(v, w1 | w2, s1, s2, pl, mi);
         curl_near<EF>(va, w1 | w2, s1, s2, pa, ma);
         const double h = amul(A, f) + imul<!EF>(B, pl);
         f = h + imul<!EF>(B, pa);
         const double x = amul(Aa, fa) + imul<!EF>(Ba, mi);
         fa = x + imul<!EF>(Ba, ma);
-        Fa[i0] = fa;
+        Fa[a] = fa;
     } else {
         f = metal_cell<EF>(p, cls, b, c, j2, px, f);
     }
@@ -339,12 +337,7 @@ __global__ void k_maxabs(const void *x, long long n, int is_double, unsigned lon
 template <bool EF> static void launch_sweep64(const P64 &p, int rel, cudaStream_t st)
 {
     const dim3 grid((p.g.pl + 31) / 32 * p.batch, p.g.L2), block(32, 3);
-    /* Small grids: a sweep is launched beside the one before, where the blocks
-     * of both are resident at once (13 a SM).  us a step, one after another /
-     * beside: 24 x 20 x 40 (600 blocks) 9.8 / 8.2, 32 x 24 x 40 (960) 11.8 /
-     * 10.0; 32 x 32 x 32 (1024) 11.8 / 14.2. */
-    if (2LL * grid.x * grid.y <= 13LL * plan::sm_count()) launch_after(k_sweep64<EF, true>, grid, block, 0, st, p, rel);
-    else k_sweep64<EF, false><<<grid, block, 0, st>>>(p, rel);
+    launch_after(k_sweep64<EF>, grid, block, 0, st, p, rel);
 }
 
 void launch_h64(const P64 &p, int rel, cudaStream_t st) { launch_sweep64<false>(p, rel, st); }

@@ -8,7 +8,8 @@
  *
  *   FP64 (bit-identical path, the reference's representation):
  *     H, E   [3][L3D] doubles    main slot (total field of ordinary cells)
- *     Ha, Ea [3][L3D]            aux slot of each non-'n' cell, zero elsewhere
+ *     Ha, Ea [3][Lnotn+1]        aux slot of each non-'n' cell, compact in
+ *                                 address_notn order, then a zero sentinel
  *     coefficients: main [4][3][L3D] (Ah, Bh, Ae, Be), aux [4][3][Lnotn]
  *     flags  [L3D] bytes: cell class + "a neighbour has an aux slot" bits
  *
@@ -83,12 +84,10 @@ struct P64 {
     const double *cm; /* [4][3][n3] */
     const double *ca; /* [4][3][lnotn] */
     double *H, *E;    /* [batch][3][n3] */
-    double *Ha, *Ea;  /* [batch][3][n3], zero where a cell has no aux slot */
+    double *Ha, *Ea;  /* [batch][3][lnotn+1] */
     /* [2][pl]: the order in which the H and the E sweep take the pixels of a
-     * plane, each with what the sweep needs to know of it: 1, 2: its neighbour
-     * along x, y wraps, 4: no cell of its x or of its y is an ordinary one */
+     * plane, each with whether its neighbour along x (1) or y (2) wraps */
     const int2 *ord;
-    const uint8_t *smask; /* [L2]: no cell of the plane is an ordinary one */
     Src s;
     Dft d;
 };

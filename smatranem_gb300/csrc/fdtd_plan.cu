@@ -83,7 +83,6 @@ P64 make_p64(const smat_fdtd_plan *p, bool xp)
     q.flags = p->d_flags;
     q.addr = p->d_addr;
     q.ord = p->d_ord;
-    q.smask = p->d_smask;
     q.cm = p->d_cm;
     q.ca = p->d_ca;
     q.H = p->d_H64;
@@ -459,13 +458,13 @@ int upload_f64(smat_fdtd_plan *p, const double *Ah, const double *Bh, const doub
      * ordinary one) row by row; those whose neighbour in the sweep's direction
      * is such a column, column by column; the others, row by row */
     const int L0 = p->L[0], L1 = p->L[1], L2 = p->L[2];
-    std::vector<uint8_t> sx(L0, 1), sy(L1, 1), sz(L2, 1);
+    std::vector<uint8_t> sx(L0, 1);
     {
         long long l = 0;
         for (int z = 0; z < L2; z++)
             for (int y = 0; y < L1; y++)
                 for (int x = 0; x < L0; x++, l++)
-                    if (p->cont[l] == 'n') sx[x] = sy[y] = sz[z] = 0;
+                    if (p->cont[l] == 'n') sx[x] = 0;
     }
     std::vector<int2> ord;
     ord.reserve(2 * (size_t)p->pl);
@@ -477,7 +476,7 @@ int upload_f64(smat_fdtd_plan *p, const double *Ah, const double *Bh, const doub
         }
         auto put = [&](int x, int y) {
             const int wx = x == (ef ? L0 - 1 : 0), wy = y == (ef ? L1 - 1 : 0);
-            ord.push_back(make_int2(x + L0 * y, wx | wy << 1 | (sx[x] || sy[y]) << 2));
+            ord.push_back(make_int2(x + L0 * y, wx | wy << 1));
         };
         for (int y = 0; y < L1; y++)
             for (int x : cols[0]) put(x, y);
@@ -486,16 +485,15 @@ int upload_f64(smat_fdtd_plan *p, const double *Ah, const double *Bh, const doub
         for (int y = 0; y < L1; y++)
             for (int x : cols[2]) put(x, y);
     }
-    if ((rc = p->alloc(&p->d_ord, ord.size())) || (rc = p->alloc(&p->d_smask, sz.size()))) return rc;
+    if ((rc = p->alloc(&p->d_ord, ord.size()))) return rc;
     CK(p->cpy(p->d_ord, ord.data(), ord.size() * sizeof(int2), cudaMemcpyHostToDevice));
-    CK(p->cpy(p->d_smask, sz.data(), sz.size(), cudaMemcpyHostToDevice));
     if ((rc = p->alloc(&p->d_flags, n3))) return rc;
     if ((rc = p->alloc(&p->d_addr, n3))) return rc;
     if ((rc = p->alloc(&p->d_cm, 12 * (size_t)n3))) return rc;
     if ((rc = p->alloc(&p->d_ca, 12 * (size_t)ln))) return rc;
-    const size_t fs = (size_t)p->batch * 3 * n3;
+    const size_t fs = (size_t)p->batch * 3 * n3, as = (size_t)p->batch * 3 * (ln + 1);
     if ((rc = p->alloc(&p->d_H64, fs)) || (rc = p->alloc(&p->d_E64, fs))) return rc;
-    if ((rc = p->alloc(&p->d_Ha64, fs)) || (rc = p->alloc(&p->d_Ea64, fs))) return rc;
+    if ((rc = p->alloc(&p->d_Ha64, as)) || (rc = p->alloc(&p->d_Ea64, as))) return rc;
     std::vector<double> cm(12 * (size_t)n3), ca(12 * (size_t)ln);
     const double *src[4] = {Ah, Bh, Ae, Be};
     for (int w = 0; w < 4; w++)
@@ -883,17 +881,17 @@ extern "C" int smat_fdtd_set_fields(smat_fdtd_plan *p, int b, const double *H_t,
     smat_clear_error();
     if (!p || !H_t || !E_t || b < 0 || b >= p->batch) return smat_fail(SMAT_EINVAL, "set_fields: bad arguments");
     const long long n3 = p->n3;
+    const int ln = p->lnotn;
     for (int w = 0; w < 2; w++) {
         const double *src = w ? E_t : H_t;
         if (p->precision == SMAT_FP64) {
-            std::vector<double> m(3 * n3), a(3 * n3, 0.0);
-            for (int c = 0; c < 3; c++)
-                for (long long l = 0; l < n3; l++) {
-                    m[c * n3 + l] = src[c + 3 * l];
-                    if (p->cont[l] != 'n') a[c * n3 + l] = src[c + 3 * (n3 + p->addr[l])];
-                }
+            std::vector<double> m(3 * n3), a(3 * (size_t)(ln + 1), 0.0);
+            for (int c = 0; c < 3; c++) {
+                for (long long l = 0; l < n3; l++) m[c * n3 + l] = src[c + 3 * l];
+                for (int x = 0; x <= ln; x++) a[(size_t)c * (ln + 1) + x] = src[c + 3 * (n3 + x)];
+            }
             double *dm = (w ? p->d_E64 : p->d_H64) + (size_t)b * 3 * n3;
-            double *da = (w ? p->d_Ea64 : p->d_Ha64) + (size_t)b * 3 * n3;
+            double *da = (w ? p->d_Ea64 : p->d_Ha64) + (size_t)b * 3 * (ln + 1);
             CK(p->cpy(dm, m.data(), m.size() * 8, cudaMemcpyHostToDevice));
             CK(p->cpy(da, a.data(), a.size() * 8, cudaMemcpyHostToDevice));
             CK(cudaStreamSynchronize(p->stream));
@@ -929,18 +927,15 @@ extern "C" int smat_fdtd_get_fields(smat_fdtd_plan *p, int b, double *H_t, doubl
         double *dst = w ? E_t : H_t;
         if (!dst) continue;
         if (p->precision == SMAT_FP64) {
-            std::vector<double> m(3 * n3), a(3 * n3);
+            std::vector<double> m(3 * n3), a(3 * (size_t)(ln + 1));
             const double *dm = (w ? p->d_E64 : p->d_H64) + (size_t)b * 3 * n3;
-            const double *da = (w ? p->d_Ea64 : p->d_Ha64) + (size_t)b * 3 * n3;
+            const double *da = (w ? p->d_Ea64 : p->d_Ha64) + (size_t)b * 3 * (ln + 1);
             CK(p->cpy(m.data(), dm, m.size() * 8, cudaMemcpyDeviceToHost));
             CK(p->cpy(a.data(), da, a.size() * 8, cudaMemcpyDeviceToHost));
             CK(cudaStreamSynchronize(p->stream));
             for (int c = 0; c < 3; c++) {
-                for (long long l = 0; l < n3; l++) {
-                    dst[c + 3 * l] = m[c * n3 + l];
-                    if (p->cont[l] != 'n') dst[c + 3 * (n3 + p->addr[l])] = a[c * n3 + l];
-                }
-                dst[c + 3 * (n3 + ln)] = 0.0; /* the sentinel */
+                for (long long l = 0; l < n3; l++) dst[c + 3 * l] = m[c * n3 + l];
+                for (int x = 0; x <= ln; x++) dst[c + 3 * (n3 + x)] = a[(size_t)c * (ln + 1) + x];
             }
         } else {
             const long long n3p = p->n3p;
@@ -1452,10 +1447,11 @@ extern "C" int smat_fdtd_check_finite(smat_fdtd_plan *p, int *finite, double *ma
     CK(cudaMemsetAsync(p->d_scratch, 0, 8, p->stream));
     const bool d = p->precision == SMAT_FP64;
     const long long nf = (long long)p->batch * 3 * p->n3p;
+    const long long na = d ? (long long)p->batch * 3 * (p->lnotn + 1) : nf;
     const P32 q = make_p32(p, false);
     const void *arr[4] = {d ? (void *)p->d_H64 : (void *)q.H, d ? (void *)p->d_E64 : (void *)q.E,
                           d ? (void *)p->d_Ha64 : (void *)q.Ha, d ? (void *)p->d_Ea64 : (void *)q.Ea};
-    for (int i = 0; i < 4; i++) launch_maxabs(arr[i], nf, d, p->d_scratch, p->stream);
+    for (int i = 0; i < 4; i++) launch_maxabs(arr[i], i < 2 ? nf : na, d, p->d_scratch, p->stream);
     unsigned long long bits = 0;
     CK(p->cpy(&bits, p->d_scratch, 8, cudaMemcpyDeviceToHost));
     CK(cudaStreamSynchronize(p->stream));
@@ -1502,14 +1498,12 @@ struct StateHeader {
 
 constexpr char STATE_MAGIC[8] = {'S', 'M', 'A', 'T', 'S', 'T', 'A', 'T'};
 
-/* a device array of a plan's state and how the file holds it: as it is;
- * FP64 aux slots, dense on the device, as [batch][3][lnotn + 1]
- * (address_notn order, then a zero); FP32 fields without their rows' padding */
-enum class InFile { same, compact, unpadded };
+/* a device array of a plan's state; padded: FP32 fields, which the file holds
+ * without their rows' padding */
 struct StateArray {
     void *dev;
     size_t bytes;
-    InFile form;
+    bool padded;
 };
 
 /* the device arrays that hold a plan's state, in file order */
@@ -1518,26 +1512,25 @@ std::vector<StateArray> state_arrays(smat_fdtd_plan *p)
     std::vector<StateArray> a;
     const size_t b = (size_t)p->batch, n3 = (size_t)p->n3;
     if (p->precision == SMAT_FP64) {
-        const size_t f = b * 3 * n3 * 8;
-        a.push_back({p->d_H64, f, InFile::same});
-        a.push_back({p->d_E64, f, InFile::same});
-        a.push_back({p->d_Ha64, f, InFile::compact});
-        a.push_back({p->d_Ea64, f, InFile::compact});
+        const size_t main = b * 3 * n3 * 8, aux = b * 3 * ((size_t)p->lnotn + 1) * 8;
+        a.push_back({p->d_H64, main, false});
+        a.push_back({p->d_E64, main, false});
+        a.push_back({p->d_Ha64, aux, false});
+        a.push_back({p->d_Ea64, aux, false});
     } else {
         const P32 q = make_p32(p, false);
         const size_t f = b * 3 * (size_t)p->n3p * 4;
-        for (float *x : {q.H, q.E, q.Ha, q.Ea}) a.push_back({x, f, p->P0 == p->L[0] ? InFile::same : InFile::unpadded});
+        for (float *x : {q.H, q.E, q.Ha, q.Ea}) a.push_back({x, f, p->P0 != p->L[0]});
     }
     if (p->d_acc && p->nq > 0 && p->nfreq > 0)
-        a.push_back({p->d_acc, b * (size_t)p->nfreq * p->nq * 4 * (size_t)p->pl * 16, InFile::same});
+        a.push_back({p->d_acc, b * (size_t)p->nfreq * p->nq * 4 * (size_t)p->pl * 16, false});
     return a;
 }
 
 /* bytes of a state array in the file */
 size_t file_bytes(const smat_fdtd_plan *p, const StateArray &a)
 {
-    if (a.form == InFile::compact) return (size_t)p->batch * 3 * ((size_t)p->lnotn + 1) * 8;
-    return a.form == InFile::unpadded ? (size_t)p->batch * 3 * p->n3 * 4 : a.bytes;
+    return a.padded ? (size_t)p->batch * 3 * p->n3 * 4 : a.bytes;
 }
 
 /* FP32 fields between padded and unpadded rows (padding: 0) */
@@ -1552,24 +1545,6 @@ void rows_pad(const smat_fdtd_plan *p, const float *rows, float *padded)
     const size_t L0 = p->L[0], n = (size_t)p->batch * 3 * p->L[1] * p->L[2];
     memset(padded, 0, n * p->P0 * 4);
     for (size_t r = 0; r < n; r++) memcpy(padded + r * p->P0, rows + r * L0, L0 * 4);
-}
-
-/* the aux slots between their dense and their compact form */
-void aux_compact(const smat_fdtd_plan *p, const double *dense, double *compact)
-{
-    for (size_t r = 0; r < (size_t)p->batch * 3; r++) {
-        double *c = compact + r * ((size_t)p->lnotn + 1);
-        for (long long l = 0; l < p->n3; l++)
-            if (p->cont[l] != 'n') c[p->addr[l]] = dense[r * p->n3 + l];
-        c[p->lnotn] = 0.0;
-    }
-}
-
-void aux_dense(const smat_fdtd_plan *p, const double *compact, double *dense)
-{
-    for (size_t r = 0; r < (size_t)p->batch * 3; r++)
-        for (long long l = 0; l < p->n3; l++)
-            dense[r * p->n3 + l] = p->cont[l] != 'n' ? compact[r * ((size_t)p->lnotn + 1) + p->addr[l]] : 0.0;
 }
 
 void fill_header(const smat_fdtd_plan *p, StateHeader &h)
@@ -1608,10 +1583,11 @@ extern "C" int smat_fdtd_save_state(smat_fdtd_plan *p, const char *path)
             break;
         }
         const size_t n = file_bytes(p, a);
-        if (a.form != InFile::same) file.resize(n);
-        if (a.form == InFile::compact) aux_compact(p, (const double *)buf.data(), (double *)file.data());
-        if (a.form == InFile::unpadded) rows_unpad(p, (const float *)buf.data(), (float *)file.data());
-        if (fwrite(a.form != InFile::same ? file.data() : buf.data(), 1, n, f) != n)
+        if (a.padded) {
+            file.resize(n);
+            rows_unpad(p, (const float *)buf.data(), (float *)file.data());
+        }
+        if (fwrite(a.padded ? file.data() : buf.data(), 1, n, f) != n)
             rc = smat_fail(SMAT_EINVAL, "save_state: write error");
     }
     if (fclose(f) != 0 && !rc) rc = smat_fail(SMAT_EINVAL, "save_state: write error");
@@ -1644,13 +1620,12 @@ extern "C" int smat_fdtd_load_state(smat_fdtd_plan *p, const char *path)
         if (rc) break;
         const size_t n = file_bytes(p, a);
         buf.resize(a.bytes);
-        if (a.form != InFile::same) file.resize(n);
-        if (fread(a.form != InFile::same ? file.data() : buf.data(), 1, n, f) != n) {
+        if (a.padded) file.resize(n);
+        if (fread(a.padded ? file.data() : buf.data(), 1, n, f) != n) {
             rc = smat_fail(SMAT_EINVAL, "load_state: %s is truncated", path);
             break;
         }
-        if (a.form == InFile::compact) aux_dense(p, (const double *)file.data(), (double *)buf.data());
-        if (a.form == InFile::unpadded) rows_pad(p, (const float *)file.data(), (float *)buf.data());
+        if (a.padded) rows_pad(p, (const float *)file.data(), (float *)buf.data());
         p->h2d_bytes += (long long)a.bytes;
         if (cudaMemcpy(a.dev, buf.data(), a.bytes, cudaMemcpyHostToDevice) != cudaSuccess)
             rc = cuda_fail(cudaGetLastError(), "load_state: copy");

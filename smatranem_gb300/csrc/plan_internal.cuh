@@ -90,7 +90,6 @@ struct smat_fdtd_plan {
     uint8_t *d_flags = nullptr;
     int *d_addr = nullptr;
     int2 *d_ord = nullptr; /* [2][pl] pixel order of the two sweeps */
-    uint8_t *d_smask = nullptr;
     double *d_cm = nullptr, *d_ca = nullptr;
     double *d_H64 = nullptr, *d_E64 = nullptr, *d_Ha64 = nullptr, *d_Ea64 = nullptr;
 

@@ -1027,6 +1027,23 @@ def test_fp64_small_grids_beside_one_another(built, L, pml):
             assert np.all(np.isfinite(a)) and np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("batch", [1, 3])
+def test_fp64_plan_holds_aux_slots_of_split_cells_only(built, batch):
+    """Device memory of an FP64 plan: 48 bytes of fields a cell and excitation
+    and 48 more a split cell, beside the coefficients, the sources and the DFT."""
+    f = _fdtd()
+    from smatranem_gb300 import workloads as W
+    L = (40, 36, 50, 1)
+    s = W.random_structure(L, seed=7, pml=(3, 0, 2))
+    pr = W.prepare(s)
+    with f.Plan.create(L, s.iBc, (6, 40, 8, 1), pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma, batch=batch) as p:
+        n, ln, pl = s.n3, pr.lnotn, L[0] * L[1]
+        assert 0 < ln < n // 2
+        fixed = (96 + 1 + 4) * n + 96 * ln + (64 * batch + 32 + 32) * pl  # coefficients, classes, addresses, sources
+        dft = batch * 2 * 4 * pl * (16 + 32 * 8)                          # sums and samples of the reference planes
+        assert p.device_bytes <= fixed + 48 * batch * (n + ln + 1) + dft + 4096
+
+
 def test_row_fused_run_of_one_graph_from_the_other_set(built):
     """A run of exactly 32 steps (one graph) that starts from the second field
     set, before and after a graph exists, as the sweeps."""
