@@ -21,16 +21,19 @@
  *     S pairs per sum, every partial sum is an integer below 2^24 and the FP32
  *     accumulation of the tensor cores is exact.  The pairs (i, l) with the
  *     same i + l = d share the scale 2^(-14-8d) and one TMEM accumulator.
- *   - the d-accumulators are combined exactly in integers, X = sum_d acc_d
- *     256^(S-1-d), rounded once to the nearest double, scaled by
- *     2^(e_r + e_c - 14 - 8(S-1)) (exact), multiplied by alpha and added to C.
- *   Error: the cuts keep 55 bits below each row's (column's) leading bit and
- *   the pairs with i + l >= S are dropped, about 2k * S * 2^(-8S) of |row
- *   max| * |col max| per entry: 2^-47 relative for S = 7 at 2k = 64, the size
- *   of the FP64 product's own rounding bound over that inner size.
+ *   - the accumulators of d < S are combined exactly in integers, X = sum_d
+ *     acc_d 256^(S-1-d), that of d = S to the nearest unit of X; X is rounded
+ *     once to the nearest double, scaled by 2^(e_r + e_c - 14 - 8(S-1))
+ *     (exact), multiplied by alpha and added to C.
+ *   Error: the cuts keep 55 bits below each row's (column's) leading bit, and
+ *     the pairs with i + l > S are dropped: at most 2k (S-2) 2^(-8(S+1)), 2^-55.6
+ *     for S = 7 at 2k = 64, of |row max| * |col max| per entry, less than the
+ *     cuts' own.  (Without the pairs of i + l = S, 2^-53 of it in the mean, the
+ *     layer transfer's S was two to four times as far from the exact one: 1.8e-14
+ *     against 5.4e-15 on a 13 x 11 grating, 3.9e-14 against 1.1e-14 at 24 x 24.)
  *
  * GB300 form.  Output tiles of 128 rows x 16 complex columns, two CTAs of
- * 256 threads per SM (224 TMEM columns each), so that one CTA's epilogue runs
+ * 256 threads per SM (256 TMEM columns each), so that one CTA's epilogue runs
  * beside the other's products.  The slices are written by the two cutting
  * kernels (integer digit extraction: one FP64 multiply and one conversion per
  * value) as images of the shared-memory operand tiles (K-major, no swizzle:
@@ -38,8 +41,8 @@
  * async copies (cp.async.bulk, completion on mbarriers: every B slice at
  * once, the A slices through a ring of three buffers) and issues the
  * tcgen05.mma (kind::f16, bf16 x bf16 -> f32, M = 128, K = 16) of slice i
- * with all the B slices it meets, side by side as N = 32 (S - i) columns, as
- * soon as it has landed; the S accumulators (32 TMEM columns each)
+ * with all the B slices it meets, side by side as up to 32 S columns, as
+ * soon as it has landed; the S + 1 accumulators (32 TMEM columns each)
  * are read back by all eight warps (tcgen05.ld, one row per thread) for an
  * integer epilogue (exact int64 sum of the digit levels, the double assembled
  * from its bits) with one FP64 multiply-add per output: GB300's FP64 pipe
@@ -70,12 +73,12 @@ constexpr int KC = KI / 2;           /* complex inner terms per pass */
 constexpr int AIMG = BM * KI * 2;    /* bytes of an A slice image (16 KB) */
 constexpr int BIMG = BN * KI * 2;    /* bytes of a B slice image (4 KB) */
 constexpr int RING = 3;              /* A slice buffers */
-constexpr int TMEM_COLS = 256;       /* S * BN = 224 columns used: two CTAs per SM fit TMEM */
+constexpr int TMEM_COLS = 256;       /* S + 1 accumulators of BN columns: two CTAs per SM fill TMEM */
 constexpr int CTILE = BM * BNC * 16; /* bytes of a tile of C (32 KB) */
 constexpr int SMEM = RING * AIMG + S * BIMG + CTILE + 8 * (2 * RING + 2) + 16;
 constexpr unsigned WAIT_LIMIT = 1u << 24;
 
-static_assert(S * BN <= TMEM_COLS && S * BN <= 256, "accumulators exceed the TMEM allocation or a product's columns");
+static_assert((S + 1) * BN <= TMEM_COLS && S * BN <= 256, "accumulators exceed the TMEM allocation or a product's columns");
 static_assert(BIMG == BN / 8 * 1024, "the B images continue each other's row groups");
 static_assert(S * KI * 128 * 128 < (1 << 24), "partial sums must stay exact in FP32");
 
@@ -417,17 +420,18 @@ constexpr int MMA_THREADS = 256; /* 8 warps: two per TMEM lane quarter in the ep
  * B slice (one mbarrier) and streams the A slices through a ring of three
  * buffers (full / empty mbarriers per buffer; a buffer is refilled once the
  * products that read it have completed, tcgen05.commit); slice i is multiplied
- * with B_l, l = 0 .. S-1-i, into accumulators i + l in one product of 32 (S - i)
- * columns.  Then the 8 warps read
+ * with B_l, l = 0 .. S-i (S-1 at most), into accumulators i + l in one product of
+ * 32 columns a B slice.  Then the 8 warps read
  * the accumulators back, warp w the TMEM lanes of quarter w % 4 and the
  * complex columns 8 (w / 4) .. + 7.  Bound by a tile's latency (load,
  * products, epilogue; two tiles a SM at a time: 21000 clocks once).  So the
- * loads start before the TMEM allocation; 28 products of up to 224 columns take
- * the place of 112 of 32 (75 clocks each, 8500 in all); a thread's values of C
+ * loads start before the TMEM allocation; 29 products of up to 224 columns take
+ * the place of 136 of 32 (75 clocks each); a thread's values of C
  * come into shared memory beside the products instead of one by one between
  * its stores; and its 16 results are assembled without a branch, so that they
- * overlap.  1210 x 1210 at k = 32: 50 us, 40 with C fetched early, 30 with all
- * of it.  Every wait is bounded: on a timeout the
+ * overlap.  1210 x 1210 at k = 32, without the pairs of i + l = S: 50 us, 40
+ * with C fetched early, 30 with all of it; with them 1 % more on the layer
+ * transfer of a 24 x 24 grating.  Every wait is bounded: on a timeout the
  * CTA records error 1, lets its copies in flight land (bounded) and returns
  * through the same epilogue. */
 __global__ void __launch_bounds__(MMA_THREADS, 2)
@@ -504,12 +508,18 @@ __global__ void __launch_bounds__(MMA_THREADS, 2)
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            /* slice i with B_0 .. B_(S-1-i), whose images lie one after
-             * another as the rows of one operand, into accumulators i .. S-1 */
+            /* slice i with B_0 .. B_(S-i) (at most B_(S-1)), whose images lie
+             * one after another as the rows of one operand, into accumulators
+             * i .. S; slice 1's first product with B_(S-1) is S's first */
+            const int nb = i == 0 ? S : S + 1 - i;
 #pragma unroll
-            for (int ks = 0; ks < KI / 16; ks++)
-                mma_bf16(tmem + (unsigned)(i * BN), op_desc(smem_u32(ring + slot * AIMG + ks * 256)),
-                         op_desc(smem_u32(sB + ks * 256)), instr_desc((S - i) * BN), (i > 0 || ks > 0) ? 1u : 0u);
+            for (int ks = 0; ks < KI / 16; ks++) {
+                const uint64_t a = op_desc(smem_u32(ring + slot * AIMG + ks * 256)), b = op_desc(smem_u32(sB + ks * 256));
+                const bool first = i == 1 && ks == 0;
+                mma_bf16(tmem + (unsigned)(i * BN), a, b, instr_desc((first ? nb - 1 : nb) * BN), (i > 0 || ks > 0) ? 1u : 0u);
+                if (first)
+                    mma_bf16(tmem + (unsigned)(S * BN), a, op_desc(smem_u32(sB + (S - 1) * BIMG + ks * 256)), instr_desc(BN), 0u);
+            }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                              smem_u32(a_empty + slot))
                          : "memory");
@@ -543,8 +553,8 @@ __global__ void __launch_bounds__(MMA_THREADS, 2)
         if (lane == 0) atomicExch(err, 2);
     } else {
         const unsigned lane_base = tmem + ((unsigned)(q * 32) << 16);
-        /* X = sum_d acc_d 256^(S-1-d) exactly: int32 pairs (acc_1, acc_2),
-         * (acc_3, acc_4), (acc_5, acc_6) (each below 2^31), then two int64
+        /* X = sum_d acc_d 256^(S-1-d), exact but for acc_S's last byte: int32 pairs (acc_1, acc_2),
+         * (acc_3, acc_4), (acc_5, acc_6) + acc_7 / 256 (each below 2^31), then two int64
          * halves th = acc_0 2^16 + p12 (below 2^40) and tl = p34 2^16 + p56
          * (below 2^48): X = th 2^32 + tl; value X 2^(er + ec - 62) */
         static_assert(S == 7, "the pairing below is written for 7 slices");
@@ -568,6 +578,9 @@ __global__ void __launch_bounds__(MMA_THREADS, 2)
                     else p56[h][j] = q2;
                 }
             }
+            tmem_ld8(base + (unsigned)(S * BN), v);
+#pragma unroll
+            for (int j = 0; j < 8; j++) p56[h][j] += (__float2int_rn(v[j]) + 128) >> 8;
         }
         /* C += alpha * value; a real alpha (the layer transfer's -1 and 1)
          * gets a loop of its own, so that no element evaluates the complex

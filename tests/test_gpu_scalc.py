@@ -240,6 +240,32 @@ def test_zgemm_results_round_to_nearest(built, m, n, k):
                 assert np.array_equal(got, want), (r, c)
 
 
+@pytest.mark.parametrize("m,n,k", [(128, 16, 32), (130, 17, 31), (257, 33, 64)])
+def test_zgemm_is_within_half_a_unit_and_the_dropped_digits(built, m, n, k):
+    """Entries of 53 bits, which the cut into digits keeps whole: what is left out
+    are the digit pairs i + l >= 8 of 7 x 7, at most 64 2^14 (5 2^-78 + 4 2^-86
+    + 3 2^-94 + ...) of row max times column max a pass, a half unit 2^-63 of it for
+    the last level that is kept, and the rounding to a double, of the result and of
+    each pass into it."""
+    rng = np.random.default_rng(m + n + k)
+    a, b = rng.integers(-2 ** 53, 2 ** 53, (m, k, 2)), rng.integers(-2 ** 53, 2 ** 53, (k, n, 2))
+    A, B = (np.ldexp(x[..., 0].astype(float), -53) + 1j * np.ldexp(x[..., 1].astype(float), -53) for x in (a, b))
+    a[:, 0, 0] = b[0, :, 0] = 2 ** 53 - 1
+    A[:, 0], B[0, :] = 1 - 2.0 ** -53 + 1j * A[:, 0].imag, 1 - 2.0 ** -53 + 1j * B[0, :].imag
+    C = scalc.zgemm(A, B, mode=1)
+    a, b = a.astype(object), b.astype(object)
+    passes = (k + 31) // 32
+    left = passes * 2.0 ** 106 * (64 * (5 * 2.0 ** -64 + 5 * 2.0 ** -72) + 2.0 ** -63)  # in units of 2^-106
+    for r in range(m):
+        for v, want in ((C[r].real, a[r, :, 0] @ b[:, :, 0] - a[r, :, 1] @ b[:, :, 1]),
+                        (C[r].imag, a[r, :, 0] @ b[:, :, 1] + a[r, :, 1] @ b[:, :, 0])):
+            for got, w in zip(v, want):
+                unit = 2.0 ** 106 * np.spacing(max(abs(got), 2.0 ** -53))
+                err = abs(int(got * 2.0 ** 106) - w)
+                # one pass: half a unit of the result; more: of the largest sum on the way too (below 2 k)
+                assert err <= left + unit / 2 + (2.0 ** 106 * np.spacing(2.0 * k) if passes > 1 else 0), (r, err, left)
+
+
 def test_port_matrices_in_either_order(built):
     """Row-major, column-major and strided port matrices, alike or mixed, give
     the same bits."""
