@@ -500,7 +500,15 @@ int smat_scalc_ordered(int L0, int L1, const int BoundC[2], double omega, int nl
                        const double *XiB, int nB, int rowsB, const double *XiT, int nT, int rowsT, int both_ways,
                        double *S, smat_scalc_info *info);
 
-/* No counterpart in the reference: the GPU LU solve behind smat_scalc (zgesv
+/* No counterpart in the reference: the elimination behind smat_scalc on a host
+ * array, for testing.  M: rows x cols complex column-major, [A, F; B, G] with A
+ * n x n; on return [X, X P F; -B X, G - B X P F] with X = A^-1 P^-1, column i of
+ * A^-1 being (X P)[:, perm[i]] = X[:, i].  max_cluster: the largest cluster a
+ * panel runs on (1, 4, 8, 16; 0: the library's choice).  *info = first zero
+ * pivot (1-based) or 0.  Products as smat_dense_mode says. */
+int smat_zsweep(int n, int rows, int cols, double *M, int max_cluster, int *perm, int *info);
+
+/* No counterpart in the reference: a GPU LU solve (zgesv
  * semantics) on host arrays, for testing.  A: n x n, B and X: n x nrhs, all
  * complex column-major; *info = first zero pivot (1-based) or 0. */
 int smat_zgesv(int n, int nrhs, const double *A, const double *B, double *X, int *info);

@@ -509,11 +509,13 @@ __device__ __forceinline__ double2 cfnma(double2 c, double2 a, double2 b) /* c -
     return make_double2(fma(a.y, b.y, fma(-a.x, b.x, c.x)), fma(-a.y, b.x, fma(-a.x, b.y, c.y)));
 }
 
-/* 1 / d, 0 for d = 0: conj(d) / |d|^2, the real reciprocal by the cubic
- * iteration x <- x + x (e + e^2), e = 1 - s x, from the hardware's 20-bit
- * approximation (error e^3 < 2^-57); the FP64 division takes three times as
- * long, on every column's critical path.  |d|^2 outside 2^+-1000: the
- * division, scaled. */
+/* 1 / d, 0 for d = 0: conj(d) / |d|^2, the real reciprocal by one step of the
+ * cubic iteration x <- x (1 + e + e^2), e = 1 - s x (M. Altman, "An optimum cubically convergent
+ * iterative method of inverting a linear bounded operator in Hilbert space",
+ * Pacific J. Math. 10, 1960), from the 20-bit rcp.approx.ftz.f64: error e^3 <
+ * 2^-57.  The FP64 division takes three times as long, on every column's
+ * critical path.  |d|^2 outside 2^+-1000: the division, of d scaled by a power
+ * of two, the scale put back last. */
 __device__ __forceinline__ double2 reciprocal(double2 d)
 {
     const double s = fma(d.x, d.x, d.y * d.y);
@@ -522,8 +524,8 @@ __device__ __forceinline__ double2 reciprocal(double2 d)
         if (d.x == 0.0 && d.y == 0.0) return make_double2(0.0, 0.0);
         const double f = e > 0 ? 0x1p-600 : 0x1p600;
         const double2 v = make_double2(d.x * f, d.y * f);
-        const double r = 1.0 / fma(v.x, v.x, v.y * v.y) * f;
-        return make_double2(v.x * r, -v.y * r);
+        const double r = 1.0 / fma(v.x, v.x, v.y * v.y);
+        return make_double2(v.x * r * f, -v.y * r * f);
     }
     double x;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(s));
@@ -649,7 +651,7 @@ __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int
                 if (lane == 0) {
                     rd[c] = inv;
                     piv[c] = q;
-                    if (rank == 0 && inv.x == 0.0 && inv.y == 0.0 && *info == 0) *info = j + c + 1;
+                    if (rank == 0 && d.x == 0.0 && d.y == 0.0 && *info == 0) *info = j + c + 1;
                 }
             }
         }
@@ -693,16 +695,15 @@ static int gj_width(int n)
     return 0;
 }
 
-static int launch_gj_panel(const double2 *A, int lda, int j, int n, int nb, int w, double2 *lud, int *mv, int *info,
-                           cudaStream_t st)
+static int launch_gj_panel(const double2 *A, int lda, int j, int n, int nb, int w, const SweepWs &ws, int *info, cudaStream_t st)
 {
     /* 16 CTAs for panels of 128 rows and more; fewer rows synchronise fewer */
-    const int m = n - j, cs = m >= 128 ? 16 : m >= 64 ? 8 : m >= 32 ? 4 : 1;
+    const int m = n - j, cs = std::min(ws.max_cs, m >= 128 ? 16 : m >= 64 ? 8 : m >= 32 ? 4 : 1);
     static const bool ready = cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
                               cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GJ_SMEM) == cudaSuccess;
     if (!ready) return smat_fail(SMAT_ECUDA, "k_gj_panel: cluster of 16 CTAs refused");
-    if (launch_after_in(cs, k_gj_panel, dim3(cs), dim3(GJT), gj_panel_smem((m + cs - 1) / cs, w), st, A, lda, j, n, nb, w, lud,
-                        mv, info) != cudaSuccess)
+    if (launch_after_in(cs, k_gj_panel, dim3(cs), dim3(GJT), gj_panel_smem((m + cs - 1) / cs, w), st, A, lda, j, n, nb, w, ws.lud,
+                        ws.mv, info) != cudaSuccess)
         return smat_fail(SMAT_ECUDA, "k_gj_panel launch: %s", cudaGetErrorString(cudaGetLastError()));
     return SMAT_OK;
 }
@@ -720,7 +721,7 @@ int sweep(int n, int rows, int cols, double2 *M, int ld, const SweepWs &w, const
     k_iota<<<(n + 255) / 256, 256, 0, st>>>(w.perm, n);
     for (int j = 0; j < n; j += width) {
         const int nb = std::min(width, n - j);
-        if (int rc = launch_gj_panel(M, ld, j, n, nb, width, w.lud, w.mv, info, st)) return rc;
+        if (int rc = launch_gj_panel(M, ld, j, n, nb, width, w, info, st)) return rc;
         if (int rc = sweep_update(rows, cols, j, nb, M, ld, w, g, st)) return rc;
     }
     return SMAT_OK;
@@ -922,6 +923,44 @@ extern "C" int smat_zgesv(int n, int nrhs, const double *A, const double *B, dou
     cudaFree(dB);
     cudaFree(dp);
     cudaFree(dinfo);
+    if (st) cudaStreamDestroy(st);
+    return rc;
+}
+
+extern "C" int smat_zsweep(int n, int rows, int cols, double *M, int max_cluster, int *perm, int *info_out)
+{
+    using namespace smat::dense;
+    if (n <= 0 || rows < n || cols < n || !M || !perm || !info_out ||
+        (max_cluster != 0 && max_cluster != 1 && max_cluster != 4 && max_cluster != 8 && max_cluster != 16))
+        return smat_fail(SMAT_EINVAL, "smat_zsweep: n = %d, %d x %d, clusters up to %d", n, rows, cols, max_cluster);
+    cudaStream_t st = nullptr;
+    double2 *dM = nullptr;
+    int *dinfo = nullptr;
+    GemmCtx g{0, nullptr, 0, nullptr, 0, -1};
+    SweepWs w{};
+    const size_t bytes = (size_t)rows * cols * sizeof(double2);
+    int rc = SMAT_OK;
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess || cudaMalloc(&dM, bytes) != cudaSuccess ||
+        cudaMalloc(&dinfo, sizeof(int)) != cudaSuccess || cudaMalloc(&w.lud, NBMAX * NBMAX * sizeof(double2)) != cudaSuccess ||
+        cudaMalloc(&w.mv, 2 * NBMAX * sizeof(int)) != cudaSuccess || cudaMalloc(&w.perm, (size_t)n * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&w.prow, (size_t)rows * NBMAX * sizeof(double2)) != cudaSuccess ||
+        cudaMalloc(&w.bcol, (size_t)cols * NBMAX * sizeof(double2)) != cudaSuccess)
+        rc = smat_fail(SMAT_ENOMEM, "smat_zsweep: device allocation");
+    if (max_cluster) w.max_cs = max_cluster;
+    if (!rc) rc = gemm_ctx_alloc(g, rows, cols, st);
+    if (!rc && (cudaMemcpyAsync(dM, M, bytes, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+                cudaMemsetAsync(dinfo, 0, sizeof(int), st) != cudaSuccess))
+        rc = smat_fail(SMAT_ECUDA, "smat_zsweep: upload");
+    if (!rc) rc = sweep(n, rows, cols, dM, rows, w, g, dinfo, st);
+    if (!rc && (cudaMemcpyAsync(M, dM, bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                cudaMemcpyAsync(perm, w.perm, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                cudaMemcpyAsync(info_out, dinfo, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                cudaStreamSynchronize(st) != cudaSuccess))
+        rc = smat_fail(SMAT_ECUDA, "smat_zsweep: %s", cudaGetErrorString(cudaGetLastError()));
+    if (!rc) rc = gemm_ctx_check(g);
+    if (st) cudaStreamSynchronize(st);
+    gemm_ctx_release(g);
+    for (void *p : {(void *)dM, (void *)dinfo, (void *)w.lud, (void *)w.mv, (void *)w.perm, (void *)w.prow, (void *)w.bcol}) cudaFree(p);
     if (st) cudaStreamDestroy(st);
     return rc;
 }

@@ -55,6 +55,7 @@ struct SweepWs {
     double2 *lud;
     int *mv, *perm;
     double2 *prow, *bcol;
+    int max_cs = 16; /* largest cluster of a panel */
 };
 /* The in-place Gauss-Jordan sweep of the leading n x n block A of M (rows x
  * cols, column-major): [A, F; B, G] -> [X, X P F; -B X, G - B X P F], X P =

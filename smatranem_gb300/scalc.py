@@ -27,6 +27,7 @@ def _lib():
         L.smat_scalc_ordered.argtypes = [C.c_int, C.c_int, _P, C.c_double, C.c_int, _P, _P, C.c_int, C.c_int, _P,
                                          C.c_int, C.c_int, C.c_int, _P, _P]
         L.smat_zgesv.argtypes = [C.c_int, C.c_int, _P, _P, _P, _P]
+        L.smat_zsweep.argtypes = [C.c_int, C.c_int, C.c_int, _P, C.c_int, _P, _P]
         L.smat_zgemm.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, _P, _P, C.c_int, _P, C.c_int, _P, C.c_int]
         L.smat_dense_mode.argtypes = [C.c_int]
         L.smat_zgemm_wait_test.argtypes = [_P]
@@ -61,7 +62,7 @@ def smatrix(meds, omega, L0, L1, bc, XiB, nB, XiT, nT, both_ways=True):
 
 
 def zgesv(A, B):
-    """X = A^{-1} B on the GPU (the LU solve behind smatrix); returns (X, info)."""
+    """X = A^{-1} B on the GPU (an LU solve); returns (X, info)."""
     A = np.asfortranarray(np.asarray(A, np.complex128))
     B = np.asarray(B, np.complex128)
     one = B.ndim == 1
@@ -71,6 +72,18 @@ def zgesv(A, B):
     fdtd._check(_lib().smat_zgesv(A.shape[0], B.shape[1], A.ctypes.data_as(_P), B.ctypes.data_as(_P),
                                   X.ctypes.data_as(_P), C.byref(info)))
     return (X[:, 0] if one else np.array(X)), info.value
+
+
+def zsweep(M, n, max_cluster=0):
+    """The elimination behind smatrix: the sweep of the leading n x n block A of
+    M = [A, F; B, G].  Returns (swept M, perm, info): columns perm of A^{-1} are
+    the first n columns of the swept rows."""
+    M = np.array(M, np.complex128, order="F")
+    perm = np.zeros(n, np.int32)
+    info = C.c_int(-1)
+    fdtd._check(_lib().smat_zsweep(int(n), M.shape[0], M.shape[1], M.ctypes.data_as(_P), int(max_cluster),
+                                   perm.ctypes.data_as(_P), C.byref(info)))
+    return M, perm, info.value
 
 
 def dense_mode(mode):

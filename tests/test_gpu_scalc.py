@@ -266,6 +266,108 @@ def test_zgemm_is_within_half_a_unit_and_the_dropped_digits(built, m, n, k):
                 assert err <= left + unit / 2 + (2.0 ** 106 * np.spacing(2.0 * k) if passes > 1 else 0), (r, err, left)
 
 
+# ---- the elimination (smat_zsweep) ----------------------------------------------
+
+
+def _sweep_blocks(A, F, B, G, max_cluster=0):
+    """A^-1, A^-1 F, B A^-1, G - B A^-1 F, perm and info by the sweep."""
+    n = len(A)
+    M, perm, info = scalc.zsweep(np.block([[A, F], [B, G]]), n, max_cluster)
+    back = np.empty(n, int)
+    back[perm] = np.arange(n)
+    return M[:n, :n][:, back], M[:n, n:], -M[n:, :n][:, back], M[n:, n:], perm, info
+
+
+def _pivots(A):
+    """Rows that partial pivoting by |re| + |im| takes, column by column."""
+    A, left, out = A.copy(), np.arange(len(A)), []
+    for c in range(len(A)):
+        p = int(np.argmax(np.abs(A[left, c].real) + np.abs(A[left, c].imag)))
+        out.append(left[p])
+        left = np.delete(left, p)
+        A[left] -= np.outer(A[left, c] / A[out[-1], c], A[out[-1]])
+    return np.array(out)
+
+
+@pytest.mark.parametrize("n,extra", [(1, 0), (5, 3), (31, 1), (33, 40), (64, 0), (130, 9), (257, 300)])
+def test_sweep_matches_numpy(dense, n, extra):
+    """Small diagonals (every column pivots), orders around the panels of 32 and
+    the cluster sizes: every block against numpy, the pivots in the order of
+    partial pivoting."""
+    rng = np.random.default_rng(n)
+    z = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)
+    A, F, B, G = z(n, n), z(n, extra), z(extra, n), z(extra, extra)
+    A[np.arange(n), np.arange(n)] *= 1e-3
+    X, XF, BX, S, perm, info = _sweep_blocks(A, F, B, G)
+    assert info == 0 and np.array_equal(perm, _pivots(A))
+    ref = np.linalg.inv(A)
+    tol = 1e-10 * np.abs(ref).max()
+    assert np.abs(X - ref).max() <= tol
+    assert np.abs(A @ X - np.eye(n)).max() <= 1e-11 * np.abs(A).max() * np.abs(X).max() * n
+    if extra:
+        assert np.abs(XF - ref @ F).max() <= tol * n and np.abs(BX - B @ ref).max() <= tol * n
+        assert np.abs(S - (G - B @ ref @ F)).max() <= tol * n * n
+
+
+@pytest.mark.parametrize("scale", [2.0 ** 900, 2.0 ** -900])
+def test_sweep_of_huge_and_tiny_entries(dense, scale):
+    """Pivots whose square leaves the exponent range are no zero pivots."""
+    rng = np.random.default_rng(3)
+    A = rng.standard_normal((70, 70)) + 1j * rng.standard_normal((70, 70))
+    X, _, _, _, perm, info = _sweep_blocks(A * scale, *(np.zeros(s) for s in ((70, 0), (0, 70), (0, 0))))
+    assert info == 0 and np.array_equal(perm, _pivots(A))
+    ref = np.linalg.inv(A)
+    assert np.abs(X * scale - ref).max() <= 1e-11 * np.abs(ref).max()
+
+
+def test_sweep_pivot_reciprocals(built):
+    """The inverse of a diagonal matrix is its pivots' reciprocals: conj(d) / |d|^2
+    with |d|^2 (two roundings), its reciprocal (one and 2^-57) and a product
+    (one), a relative error of at most 4.5 2^-53 a part, over all exponents at
+    which the result is a normal number."""
+    from fractions import Fraction
+    rng = np.random.default_rng(9)
+    n = 1500
+    d = np.ldexp(rng.uniform(0.5, 1, n), rng.integers(-1021, 1020, n)) * rng.choice([-1, 1], n) \
+        + 1j * np.ldexp(rng.uniform(0.5, 1, n), rng.integers(-1021, 1020, n)) * rng.choice([-1, 1], n)
+    near = np.abs(d.real) * np.ldexp(rng.uniform(0.5, 1, n), rng.integers(-20, 1, n))
+    d = np.where(rng.random(n) < 0.7, d.real + 1j * near, d)  # parts of like size
+    d[:4] = 2.0 ** -812, 2.0 ** 850, 2.0 ** -1021, 2.0 ** 1021
+    X, _, _, _, perm, info = _sweep_blocks(np.diag(d), np.zeros((n, 0)), np.zeros((0, n)), np.zeros((0, 0)))
+    assert info == 0 and np.array_equal(perm, np.arange(n))
+    assert np.array_equal(X, np.diag(np.diag(X)))
+    for v, x in zip(d, np.diag(X)):
+        a, b = Fraction(v.real), Fraction(v.imag)
+        s = a * a + b * b
+        for got, want in ((x.real, a / s), (x.imag, -b / s)):
+            if want == 0 or not Fraction(2) ** -1020 < abs(want) < Fraction(2) ** 1023:
+                continue
+            assert abs(Fraction(float(got)) - want) <= abs(want) * Fraction(9, 2) * Fraction(2) ** -53, v
+
+
+def test_sweep_reports_a_zero_pivot(dense):
+    """A column without a pivot, in the first panel and in a later one."""
+    rng = np.random.default_rng(4)
+    for n, c in ((6, 3), (80, 50), (200, 140)):
+        A = np.triu(rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) + 4 * np.eye(n)
+        A[c, c:] = 0
+        *_, info = _sweep_blocks(A, np.zeros((n, 0)), np.zeros((0, n)), np.zeros((0, 0)))
+        assert info == c + 1
+    A = np.eye(40)
+    A[:, 7] = 0
+    *_, info = _sweep_blocks(A, np.zeros((40, 0)), np.zeros((0, 40)), np.zeros((0, 0)))
+    assert info == 8  # 1-based, as LAPACK's INFO
+
+
+def test_smatrix_of_a_singular_port_is_refused(dense):
+    L0, L1, n = 4, 3, 2
+    NA = 2 * L0 * L1
+    meds = np.random.default_rng(1).uniform(1, 4, (3, 6, L0 * L1)) + 0j
+    with pytest.raises(fdtd.FdtdError) as e:
+        scalc.smatrix(meds, 0.4, L0, L1, (1, 1), np.zeros((2 * NA, 2 * NA)), n, np.eye(2 * NA), n)
+    assert e.value.code == -6
+
+
 def test_port_matrices_in_either_order(built):
     """Row-major, column-major and strided port matrices, alike or mixed, give
     the same bits."""
