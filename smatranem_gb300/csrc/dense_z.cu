@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(PT) k_panel(double2 *A, int lda, int m, int nb
 }
 
 constexpr int NBMAX = 32;
-constexpr size_t GJ_SMEM = 224 * 1024; /* dynamic shared memory of a sweep's panel CTA */
+constexpr size_t GJ_SMEM = 224 * 1024; /* dynamic shared memory of a sweep's panel CTA, at most */
 
 /* X (nb x ncols at X, leading dimension ldx) <- T^{-1} X with T the nb x nb
  * triangle at T (unit lower if lower, else non-unit upper, nb <= 32): one
@@ -534,28 +534,36 @@ __device__ __forceinline__ double2 reciprocal(double2 d)
     return make_double2(d.x * x, -d.y * x);
 }
 
-__host__ __device__ inline size_t gj_panel_smem(int R, int w)
-{
-    return sizeof(double2) * ((size_t)R * (w + 1) + 2 * 16 * NBMAX + (NBMAX + 1) * (NBMAX + 1) + R) + sizeof(int) * ((size_t)R + 64);
-}
+/* shared memory of a panel CTA, and of what it keeps of each of its rows */
+constexpr size_t GJ_FIXED = sizeof(double2) * (2 * 16 * NBMAX + (NBMAX + 1) * (NBMAX + 1)) + sizeof(int) * 64;
+constexpr size_t GJ_ROW = sizeof(double2) * (NBMAX + 2) + sizeof(int);
+/* bytes of a CTA's part of `rows`, R of them: a multiple of 16 */
+__host__ __device__ constexpr size_t gj_part(int R) { return GJ_ROW * ((R + 3) / 4 * 4); }
+static_assert(GJ_FIXED % 16 == 0 && gj_part(1) % 16 == 0, "double2 alignment");
 
-__global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int j, int n, int nb, int w,
-                                                  double2 *__restrict__ lud, int *__restrict__ mv, int *info)
+/* ROWS_IN_L2: a panel whose rows do not fit the cluster's shared memory (more than
+ * 5696 on 16 CTAs) keeps them at `rows` in device memory, each CTA its own part,
+ * which L2 holds: 9 MB at order 16384. */
+template <bool ROWS_IN_L2>
+__global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int j, int n, int nb, double2 *__restrict__ lud,
+                                                  int *__restrict__ mv, int *info, unsigned char *rows)
 {
     prior_done();
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     const int nc = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    const int m = n - j, R = (m + nc - 1) / nc, rbeg = rank * R, rn = max(0, min(m, rbeg + R) - rbeg), S = w + 1;
-    constexpr int LS = NBMAX + 1;
+    const int m = n - j, R = (m + nc - 1) / nc, rbeg = rank * R, rn = max(0, min(m, rbeg + R) - rbeg);
+    constexpr int LS = NBMAX + 1, S = NBMAX + 1;
     extern __shared__ __align__(16) unsigned char psm[];
-    double2 *a = reinterpret_cast<double2 *>(psm);   /* [R][S] this CTA's rows */
-    double2 *cand = a + (size_t)R * S;               /* [2][16][32] candidate rows, by column parity */
-    double2 *lu = cand + 2 * 16 * NBMAX;             /* [32][LS] the pivot rows: D's factors */
-    double2 *rd = lu + NBMAX * LS;                   /* [LS] reciprocals of U's diagonal */
-    double2 *lcol = rd + LS;                         /* [R] multipliers of this column */
-    int *used = reinterpret_cast<int *>(lcol + R);   /* [R] the row is a pivot */
-    int *ckey = used + R, *crow = ckey + 32;         /* [2][16] */
+    /* the rows first: after the candidates a panel of 200 rows takes 80 us, not 73 */
+    double2 *a = reinterpret_cast<double2 *>(psm), *cand = a + (ROWS_IN_L2 ? 0 : (size_t)R * S);
+    if constexpr (ROWS_IN_L2) a = reinterpret_cast<double2 *>(rows + rank * gj_part(R)); /* [R][S] this CTA's rows */
+    /* cand: [2][16][32] candidate rows, by column parity */
+    double2 *lu = cand + 2 * 16 * NBMAX;                             /* [32][LS] the pivot rows: D's factors */
+    double2 *rd = lu + NBMAX * LS;                                   /* [LS] reciprocals of U's diagonal */
+    int *ckey = reinterpret_cast<int *>(rd + LS), *crow = ckey + 32; /* [2][16] */
+    double2 *lcol = ROWS_IN_L2 ? a + (size_t)R * S : rd + LS + 16;   /* [R] multipliers of this column */
+    int *used = reinterpret_cast<int *>(lcol + R);                   /* [R] the row is a pivot */
     __shared__ unsigned wk[GJT / 32];
     __shared__ int wr[GJT / 32], piv[NBMAX];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -685,25 +693,63 @@ __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int
     cl.sync(); /* no CTA leaves while another may still write to it */
 }
 
-/* the panel's width for matrices of order n: 32 columns where the rows of a
- * full-height panel fit the shared memory of 16 CTAs (n up to about 5,500),
- * else 16 or 8 */
-static int gj_width(int n)
+/* the largest cluster of full-sized panel CTAs that the current device runs
+ * (the function attributes are the device's own too) */
+static int gj_clusters()
 {
-    for (int w : {32, 16, 8})
-        if (gj_panel_smem((n + 15) / 16, w) <= GJ_SMEM) return w;
-    return 0;
+    int n = 0;
+    for (auto fn : {k_gj_panel<false>, k_gj_panel<true>})
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GJ_SMEM) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+    for (int cs : {16, 8, 4}) {
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cs;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(cs);
+        cfg.blockDim = dim3(GJT);
+        cfg.dynamicSmemBytes = GJ_SMEM;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, k_gj_panel<false>, &cfg) == cudaSuccess && n > 0) return cs;
+    }
+    cudaGetLastError();
+    return 1;
 }
 
-static int launch_gj_panel(const double2 *A, int lda, int j, int n, int nb, int w, const SweepWs &ws, int *info, cudaStream_t st)
+/* whether the rows of panels of order n on clusters of cs CTAs fit their shared memory */
+static bool gj_fits(int n, int cs) { return GJ_FIXED + GJ_ROW * ((n + cs - 1) / cs) <= GJ_SMEM; }
+
+/* 16 CTAs for panels of 128 rows and more; fewer rows synchronise fewer.
+ * Rows in L2 keep the panel at 32 columns at any order: with panels of 16 and 8
+ * columns in shared memory, the products' inner size of 32 half and three quarters
+ * empty, one direction over two layers took 1.8 s at order 5832 and 17 s at 11552;
+ * now 1.3 and 6.5 (LU, substitutions and product: 3.3 and 19). */
+static int gj_ctas(int m, int max_cs) { return std::min(max_cs, m >= 128 ? 16 : m >= 64 ? 8 : m >= 32 ? 4 : 1); }
+
+int sweep_setup(SweepWs &w, int n, int max_cluster)
 {
-    /* 16 CTAs for panels of 128 rows and more; fewer rows synchronise fewer */
-    const int m = n - j, cs = std::min(ws.max_cs, m >= 128 ? 16 : m >= 64 ? 8 : m >= 32 ? 4 : 1);
-    static const bool ready = cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                              cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GJ_SMEM) == cudaSuccess;
-    if (!ready) return smat_fail(SMAT_ECUDA, "k_gj_panel: cluster of 16 CTAs refused");
-    if (launch_after_in(cs, k_gj_panel, dim3(cs), dim3(GJT), gj_panel_smem((m + cs - 1) / cs, w), st, A, lda, j, n, nb, w, ws.lud,
-                        ws.mv, info) != cudaSuccess)
+    const int most = gj_clusters();
+    if (!most) return smat_fail(SMAT_ECUDA, "sweep: %zu bytes of shared memory refused", GJ_SMEM);
+    w.max_cs = max_cluster ? std::min(most, max_cluster) : most;
+    /* the first panel has the most rows a CTA (those of fewer CTAs, below 128 rows, fit) */
+    const int cs = gj_ctas(n, w.max_cs);
+    w.row_bytes = gj_fits(n, cs) ? 0 : gj_part((n + cs - 1) / cs) * cs;
+    return SMAT_OK;
+}
+
+static int launch_gj_panel(const double2 *A, int lda, int j, int n, int nb, const SweepWs &w, int *info, cudaStream_t st)
+{
+    const int m = n - j, cs = gj_ctas(m, w.max_cs), R = (m + cs - 1) / cs;
+    const bool fits = gj_fits(m, cs);
+    if (!fits && (!w.rows || w.row_bytes < gj_part(R) * cs)) return smat_fail(SMAT_EINVAL, "sweep: no workspace for %d rows", m);
+    const size_t smem = GJ_FIXED + (fits ? GJ_ROW * R : 0);
+    if (launch_after_in(cs, fits ? k_gj_panel<false> : k_gj_panel<true>, dim3(cs), dim3(GJT), smem, st, A, lda, j, n, nb, w.lud,
+                        w.mv, info, w.rows) != cudaSuccess)
         return smat_fail(SMAT_ECUDA, "k_gj_panel launch: %s", cudaGetErrorString(cudaGetLastError()));
     return SMAT_OK;
 }
@@ -716,12 +762,10 @@ __global__ void k_iota(int *p, int n)
 
 int sweep(int n, int rows, int cols, double2 *M, int ld, const SweepWs &w, const GemmCtx &g, int *info, cudaStream_t st)
 {
-    const int width = gj_width(n);
-    if (!width) return smat_fail(SMAT_EINVAL, "sweep: order %d", n);
     k_iota<<<(n + 255) / 256, 256, 0, st>>>(w.perm, n);
-    for (int j = 0; j < n; j += width) {
-        const int nb = std::min(width, n - j);
-        if (int rc = launch_gj_panel(M, ld, j, n, nb, width, w, info, st)) return rc;
+    for (int j = 0; j < n; j += NBMAX) {
+        const int nb = std::min(NBMAX, n - j);
+        if (int rc = launch_gj_panel(M, ld, j, n, nb, w, info, st)) return rc;
         if (int rc = sweep_update(rows, cols, j, nb, M, ld, w, g, st)) return rc;
     }
     return SMAT_OK;
@@ -946,7 +990,8 @@ extern "C" int smat_zsweep(int n, int rows, int cols, double *M, int max_cluster
         cudaMalloc(&w.prow, (size_t)rows * NBMAX * sizeof(double2)) != cudaSuccess ||
         cudaMalloc(&w.bcol, (size_t)cols * NBMAX * sizeof(double2)) != cudaSuccess)
         rc = smat_fail(SMAT_ENOMEM, "smat_zsweep: device allocation");
-    if (max_cluster) w.max_cs = max_cluster;
+    if (!rc) rc = sweep_setup(w, n, max_cluster);
+    if (!rc && w.row_bytes && cudaMalloc(&w.rows, w.row_bytes) != cudaSuccess) rc = smat_fail(SMAT_ENOMEM, "smat_zsweep: device allocation");
     if (!rc) rc = gemm_ctx_alloc(g, rows, cols, st);
     if (!rc && (cudaMemcpyAsync(dM, M, bytes, cudaMemcpyHostToDevice, st) != cudaSuccess ||
                 cudaMemsetAsync(dinfo, 0, sizeof(int), st) != cudaSuccess))
@@ -960,7 +1005,9 @@ extern "C" int smat_zsweep(int n, int rows, int cols, double *M, int max_cluster
     if (!rc) rc = gemm_ctx_check(g);
     if (st) cudaStreamSynchronize(st);
     gemm_ctx_release(g);
-    for (void *p : {(void *)dM, (void *)dinfo, (void *)w.lud, (void *)w.mv, (void *)w.perm, (void *)w.prow, (void *)w.bcol}) cudaFree(p);
+    for (void *p : {(void *)dM, (void *)dinfo, (void *)w.lud, (void *)w.mv, (void *)w.perm, (void *)w.prow, (void *)w.bcol,
+                    (void *)w.rows})
+        cudaFree(p);
     if (st) cudaStreamDestroy(st);
     return rc;
 }

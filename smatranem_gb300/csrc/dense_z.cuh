@@ -55,8 +55,13 @@ struct SweepWs {
     double2 *lud;
     int *mv, *perm;
     double2 *prow, *bcol;
-    int max_cs = 16; /* largest cluster of a panel */
+    int max_cs = 1;       /* largest cluster of a panel */
+    size_t row_bytes = 0; /* of rows: where the panels' rows do not fit shared memory */
+    unsigned char *rows = nullptr;
 };
+/* chooses max_cs on the current device for orders up to n (max_cluster not 0:
+ * at most that) and the size of rows, which the caller allocates */
+int sweep_setup(SweepWs &w, int n, int max_cluster);
 /* The in-place Gauss-Jordan sweep of the leading n x n block A of M (rows x
  * cols, column-major): [A, F; B, G] -> [X, X P F; -B X, G - B X P F], X P =
  * A^-1, (X P)[:, perm[i]] = X[:, i]; *info: first zero pivot, 1-based, or 0.

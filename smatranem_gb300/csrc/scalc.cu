@@ -355,6 +355,8 @@ extern "C" int smat_scalc_ordered(int L0, int L1, const int BoundC[2], double om
     if (!(omega > 0) || !std::isfinite(omega)) return smat_fail(SMAT_EINVAL, "smat_scalc: omega = %g", omega);
     const int Nmax = std::max(nB, nT);
     const size_t cols = (size_t)Nmax + NA, rows = cols + NA;
+    smat::dense::SweepWs form{};
+    RC(smat::dense::sweep_setup(form, NA, 0));
     /* one transfer state per direction: device matrices, stream, product workspace */
     auto setup = [&](Transfer &T) {
         T.NA = NA;
@@ -378,11 +380,13 @@ extern "C" int smat_scalc_ordered(int L0, int L1, const int BoundC[2], double om
         buf(T.M[1], rows * cols);
         buf(T.LP, cols * NA);
         buf(T.out, (size_t)(nB + nT) * (nB + nT));
+        T.w = form;
         buf(T.w.lud, 32 * 32);
         buf(T.w.prow, T.gm.tc ? 0 : rows * 32);
         buf(T.w.bcol, T.gm.tc ? 0 : cols * 32);
         buf(T.w.mv, 64);
         buf(T.w.perm, NA);
+        buf(T.w.rows, T.w.row_bytes);
         buf(T.dinfo, 1);
         if (cudaMalloc(&T.slab, used) != cudaSuccess) {
             cudaGetLastError();

@@ -309,6 +309,23 @@ def test_sweep_matches_numpy(dense, n, extra):
         assert np.abs(S - (G - B @ ref @ F)).max() <= tol * n * n
 
 
+@pytest.mark.parametrize("n,max_cluster", [(300, 1), (356, 1), (357, 1), (700, 1), (1424, 4), (1425, 4), (600, 8),
+                                           (5750, 0)])
+def test_sweep_cluster_sizes(built, n, max_cluster):
+    """Panels on smaller clusters, of more rows than a CTA has threads, and of rows
+    that no longer fit shared memory (order 357 on one CTA, 1425 on four, 5697 on
+    sixteen), against the inverse's definition."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    A[np.arange(n), np.arange(n)] *= 1e-3
+    X, _, _, _, perm, info = _sweep_blocks(A, *(np.zeros(s) for s in ((n, 0), (0, n), (0, 0))), max_cluster)
+    assert info == 0 and np.array_equal(np.sort(perm), np.arange(n))
+    if n < 1000:
+        assert np.array_equal(perm, _pivots(A))
+    v = rng.standard_normal((n, 8))
+    assert np.abs(A @ (X @ v) - v).max() <= 1e-11 * np.abs(A).max() * np.abs(X).max() * n * np.abs(v).max()
+
+
 @pytest.mark.parametrize("scale", [2.0 ** 900, 2.0 ** -900])
 def test_sweep_of_huge_and_tiny_entries(dense, scale):
     """Pivots whose square leaves the exponent range are no zero pivots."""
