@@ -489,20 +489,29 @@ static int launch_panel(double2 *A, int lda, int m, int nb, int row0, int *ipiv,
  *   lud:        [k][r], 32 x 32 (a unit matrix beyond nb): L below the
  *               diagonal, the inverse of U's diagonal on it, U's rows divided
  *               by theirs above it
- * Per column: every thread's largest |re| + |im| among its rows (upper 32 bits
- * of the double: enough to choose a pivot by) by warp and block; each CTA
- * sends its candidate row to all others; one cluster barrier; all CTAs pick
- * the same winner from their own copies.  The rank-1 update of a column's
- * step is split: the thread that owns a row brings the next column up to date
- * at once, for the next pivot, and a candidate row is brought up to date as
- * it is sent; the other columns follow between arriving at the barrier and
- * waiting for it.  The FP64 pipe (20 clocks a warp instruction, whatever its
- * lanes) bounds panels of many rows, latency the others.  So two warps, not all eight, bring the candidate row up to date and send it,
- * which leaves the others free to go on while the stores drain, and the
- * trailing columns are dealt out by element (a row's columns rounded up to a
- * power of two would idle a quarter of the lanes).  32 columns of 200 rows: 73
- * us, 1152 rows 96 us (79 and 111 before). */
+ * Per column: every thread's largest |re| + |im| among its rows by warp and
+ * block, all 64 bits of it; each CTA sends its candidate row to all others; one
+ * cluster barrier; all CTAs pick the same winner from their own copies.  The
+ * rank-1 update of a column's step is split: the thread that owns a row brings
+ * the next column up to date at once, for the next pivot, and a candidate row is
+ * brought up to date as it is sent; the other columns follow between arriving at
+ * the barrier and waiting for it.  The FP64 pipe (20 clocks a warp instruction,
+ * whatever its lanes) bounds panels of many rows, latency the others.  So two
+ * warps, not all eight, bring the candidate row up to date and send it, which
+ * leaves the others free to go on while the stores drain, and the trailing
+ * columns are dealt out by element (a row's columns rounded up to a power of two
+ * would idle a quarter of the lanes).  32 columns of 200 rows: 73 us, 1152 rows
+ * 96 us (79 and 111 before); the lower 32 bits of the keys add 2 us. */
 constexpr int GJT = 256, GJS = 2; /* threads; warps that send */
+
+/* the first lane with the warp's largest key, and that key */
+__device__ __forceinline__ int first_largest(unsigned long long key, unsigned long long &most)
+{
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32)), mine = (unsigned)(key >> 32) == hi ? (unsigned)key : 0u;
+    const unsigned lo = __reduce_max_sync(0xffffffffu, mine);
+    most = (unsigned long long)hi << 32 | lo;
+    return __ffs(__ballot_sync(0xffffffffu, key == most)) - 1;
+}
 
 __device__ __forceinline__ double2 cfnma(double2 c, double2 a, double2 b) /* c - a b, four multiply-adds */
 {
@@ -535,7 +544,7 @@ __device__ __forceinline__ double2 reciprocal(double2 d)
 }
 
 /* shared memory of a panel CTA, and of what it keeps of each of its rows */
-constexpr size_t GJ_FIXED = sizeof(double2) * (2 * 16 * NBMAX + (NBMAX + 1) * (NBMAX + 1)) + sizeof(int) * 64;
+constexpr size_t GJ_FIXED = sizeof(double2) * (2 * 16 * NBMAX + (NBMAX + 1) * (NBMAX + 1)) + 12 * 32;
 constexpr size_t GJ_ROW = sizeof(double2) * (NBMAX + 2) + sizeof(int);
 /* bytes of a CTA's part of `rows`, R of them: a multiple of 16 */
 __host__ __device__ constexpr size_t gj_part(int R) { return GJ_ROW * ((R + 3) / 4 * 4); }
@@ -561,10 +570,11 @@ __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int
     /* cand: [2][16][32] candidate rows, by column parity */
     double2 *lu = cand + 2 * 16 * NBMAX;                             /* [32][LS] the pivot rows: D's factors */
     double2 *rd = lu + NBMAX * LS;                                   /* [LS] reciprocals of U's diagonal */
-    int *ckey = reinterpret_cast<int *>(rd + LS), *crow = ckey + 32; /* [2][16] */
-    double2 *lcol = ROWS_IN_L2 ? a + (size_t)R * S : rd + LS + 16;   /* [R] multipliers of this column */
+    unsigned long long *ckey = reinterpret_cast<unsigned long long *>(rd + LS); /* [2][16] */
+    int *crow = reinterpret_cast<int *>(ckey + 32);                  /* [2][16] */
+    double2 *lcol = ROWS_IN_L2 ? a + (size_t)R * S : rd + LS + 24;   /* [R] multipliers of this column */
     int *used = reinterpret_cast<int *>(lcol + R);                   /* [R] the row is a pivot */
-    __shared__ unsigned wk[GJT / 32];
+    __shared__ unsigned long long wk[GJT / 32];
     __shared__ int wr[GJT / 32], piv[NBMAX];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int t = tid; t < rn * nb; t += GJT) a[(t % rn) * S + t / rn] = A[(j + rbeg + t % rn) + (long long)lda * (j + t / rn)];
@@ -572,10 +582,10 @@ __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int
     for (int t = tid; t < NBMAX * LS; t += GJT) lu[t] = make_double2(0.0, 0.0);
     if (tid < LS) rd[tid] = make_double2(1.0, 0.0);
     cl.sync();
-    unsigned key = 0;
+    unsigned long long key = 0;
     int row = 0;
-    auto consider = [&](int i, double2 v) {
-        const unsigned k = (unsigned)__double2hiint(fabs(v.x) + fabs(v.y)) + 1u;
+    auto consider = [&](int i, double2 v) { /* |re| + |im|, which orders as its bits do, above 0 */
+        const unsigned long long k = (__double_as_longlong(fabs(v.x) + fabs(v.y)) & 0x7fffffffffffffffull) + 1ull;
         if (k > key) {
             key = k;
             row = i;
@@ -586,8 +596,8 @@ __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int
     for (int c = 0; c < nb; c++) {
         const int par = c & 1;
         {
-            const unsigned mk = __reduce_max_sync(0xffffffffu, key);
-            const int src = __ffs(__ballot_sync(0xffffffffu, key == mk)) - 1;
+            unsigned long long mk;
+            const int src = first_largest(key, mk);
             row = __shfl_sync(0xffffffffu, row, src);
             if (lane == 0) {
                 wk[warp] = mk;
@@ -599,9 +609,8 @@ __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int
          * date for itself: more of them would queue for the FP64 pipe) */
         if (warp < GJS && warp < nc) {
             key = lane < GJT / 32 ? wk[lane] : 0;
-            const unsigned mk = __reduce_max_sync(0xffffffffu, key);
-            const int src = __ffs(__ballot_sync(0xffffffffu, key == mk)) - 1;
-            row = wr[src];
+            unsigned long long mk;
+            row = wr[first_largest(key, mk)];
             double2 v = make_double2(0.0, 0.0);
             if (mk && lane < nb) {
                 v = a[row * S + lane];
@@ -610,7 +619,7 @@ __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int
             for (int t = warp; t < nc; t += GJS) {
                 cl.map_shared_rank(cand, t)[(par * 16 + rank) * NBMAX + lane] = v;
                 if (lane == 0) {
-                    cl.map_shared_rank(ckey, t)[par * 16 + rank] = (int)mk;
+                    cl.map_shared_rank(ckey, t)[par * 16 + rank] = mk;
                     cl.map_shared_rank(crow, t)[par * 16 + rank] = rbeg + row;
                 }
             }
@@ -631,9 +640,8 @@ __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int
         }
         cl.barrier_wait();
         __syncthreads();
-        key = lane < nc ? (unsigned)ckey[par * 16 + lane] : 0;
-        const unsigned mk = __reduce_max_sync(0xffffffffu, key);
-        const int win = __ffs(__ballot_sync(0xffffffffu, key == mk)) - 1;
+        unsigned long long mk;
+        const int win = first_largest(lane < nc ? ckey[par * 16 + lane] : 0, mk);
         const int q = crow[par * 16 + win];
         prow = cand + (par * 16 + win) * NBMAX;
         key = 0;

@@ -362,6 +362,18 @@ def test_sweep_pivot_reciprocals(built):
             assert abs(Fraction(float(got)) - want) <= abs(want) * Fraction(9, 2) * Fraction(2) ** -53, v
 
 
+@pytest.mark.parametrize("step", [2.0 ** -30, 2.0 ** -51])
+def test_sweep_pivots_by_all_bits(built, step):
+    """Of two candidates that differ in their last bits the larger is taken: within
+    a warp, in two warps and on two CTAs."""
+    n = 200
+    for r, q in ((3, 9), (9, 3), (1, 190), (190, 1), (100, 101)):
+        A = np.eye(n) * 0.5 + 0j
+        A[r, 0], A[q, 0] = 1.0, 1.0 + step
+        *_, perm, info = _sweep_blocks(A, np.zeros((n, 0)), np.zeros((0, n)), np.zeros((0, 0)))
+        assert info == 0 and perm[0] == q
+
+
 def test_sweep_reports_a_zero_pivot(dense):
     """A column without a pivot, in the first panel and in a later one."""
     rng = np.random.default_rng(4)
