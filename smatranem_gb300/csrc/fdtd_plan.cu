@@ -315,48 +315,74 @@ int check_planes(const smat_fdtd_plan *p, int nq, const int *planes)
     return SMAT_OK;
 }
 
-/* (re)allocate DFT accumulators and the sample ring for nfreq x nq planes */
+/* values of the DFT accumulators and of the sample ring */
+size_t acc_len(const smat_fdtd_plan *p) { return (size_t)p->batch * p->nfreq * p->nq * 4 * p->pl * 2; }
+size_t ring_len(const smat_fdtd_plan *p) { return (size_t)p->batch * RING_K * p->nq * 4 * p->pl; }
+
+void drop_acc(smat_fdtd_plan *p)
+{
+    if (p->d_acc) p->dev_bytes -= (long long)(acc_len(p) * 8);
+    cudaFree(p->d_acc);
+    p->d_acc = nullptr;
+}
+
+void drop_ring(smat_fdtd_plan *p)
+{
+    if (p->d_ring64) p->dev_bytes -= (long long)(ring_len(p) * sizeof(double));
+    if (p->d_ring) p->dev_bytes -= (long long)(ring_len(p) * sizeof(float));
+    cudaFree(p->d_ring);
+    cudaFree(p->d_ring64);
+    p->d_ring = nullptr;
+    p->d_ring64 = nullptr;
+}
+
+/* no DFT: nothing samples and nothing is accumulated */
+void drop_dft(smat_fdtd_plan *p)
+{
+    drop_graph(p);
+    drop_acc(p);
+    drop_ring(p);
+    p->nfreq = p->nq = 0;
+    p->ref_dft = false;
+}
+
+/* no schedule: run refuses */
+void drop_schedule(smat_fdtd_plan *p)
+{
+    cudaFree(p->d_sched);
+    cudaFree(p->d_phase);
+    cudaFree(p->d_phase32);
+    p->d_sched = p->d_phase = nullptr;
+    p->d_phase32 = nullptr;
+    p->nsched = 0;
+}
+
+/* DFT accumulators and the sample ring for nfreq x nq planes, zeroed; where
+ * they do not fit, the plan is left without a DFT */
 int setup_dft(smat_fdtd_plan *p, int nfreq, int nq, const int *planes)
 {
     if (nq > MAX_PLANES) return smat_fail(SMAT_EINVAL, "at most %d monitor planes", MAX_PLANES);
-    int rc;
     for (int q = 0; q < nq; q++)
         if (planes[q] < 0 || planes[q] >= p->L[2])
             return smat_fail(SMAT_EINVAL, "monitor plane %d outside 0..%d", planes[q], p->L[2] - 1);
     drop_graph(p);
-    const size_t acc_n = (size_t)p->batch * nfreq * nq * 4 * p->pl * 2;
-    const size_t ring_n = (size_t)p->batch * RING_K * nq * 4 * p->pl;
-    const size_t old_acc = (size_t)p->batch * p->nfreq * p->nq * 4 * p->pl * 2;
-    const size_t old_ring = (size_t)p->batch * RING_K * p->nq * 4 * p->pl;
-    if (acc_n != old_acc || !p->d_acc) {
-        if (p->d_acc) cudaFree(p->d_acc), p->dev_bytes -= old_acc * 8;
-        p->d_acc = nullptr;
-        if (acc_n) {
-            rc = dalloc(&p->d_acc, acc_n, p->stream);
-            if (rc) return rc;
-            p->dev_bytes += acc_n * 8;
-        }
-    }
-    const bool f64 = p->precision == SMAT_FP64;
-    const size_t rs = f64 ? sizeof(double) : sizeof(float);
-    if (ring_n != old_ring || (!p->d_ring && !p->d_ring64 && ring_n)) {
-        if (p->d_ring || p->d_ring64) {
-            cudaFree(p->d_ring);
-            cudaFree(p->d_ring64);
-            p->dev_bytes -= old_ring * rs;
-        }
-        p->d_ring = nullptr;
-        p->d_ring64 = nullptr;
-        if (ring_n) {
-            rc = f64 ? dalloc(&p->d_ring64, ring_n, p->stream) : dalloc(&p->d_ring, ring_n, p->stream);
-            if (rc) return rc;
-            p->dev_bytes += ring_n * rs;
-        }
-    }
+    if ((size_t)nfreq * nq != (size_t)p->nfreq * p->nq) drop_acc(p);
+    if (nq != p->nq) drop_ring(p);
     p->nfreq = nfreq;
     p->nq = nq;
+    int rc = SMAT_OK;
+    if (p->d_acc) CK(cudaMemsetAsync(p->d_acc, 0, acc_len(p) * 8, p->stream));
+    else if (!(rc = dalloc(&p->d_acc, acc_len(p), p->stream))) p->dev_bytes += (long long)(acc_len(p) * 8);
+    if (!rc && !p->d_ring && !p->d_ring64) {
+        const bool f64 = p->precision == SMAT_FP64;
+        rc = f64 ? dalloc(&p->d_ring64, ring_len(p), p->stream) : dalloc(&p->d_ring, ring_len(p), p->stream);
+        if (!rc) p->dev_bytes += (long long)(ring_len(p) * (f64 ? sizeof(double) : sizeof(float)));
+    }
+    if (rc) {
+        drop_dft(p);
+        return rc;
+    }
     for (int i = 0; i < MAX_PLANES; i++) p->planes[i] = i < nq ? planes[i] : -1;
-    if (p->d_acc) CK(cudaMemsetAsync(p->d_acc, 0, acc_n * 8, p->stream));
     return SMAT_OK;
 }
 
@@ -847,12 +873,8 @@ extern "C" int smat_fdtd_destroy(smat_fdtd_plan *p)
     if (p->stream) cudaStreamSynchronize(p->stream);
     drop_graph(p);
     for (void *a : p->allocations) cudaFree(a);
-    if (p->d_acc) cudaFree(p->d_acc);
-    if (p->d_ring) cudaFree(p->d_ring);
-    if (p->d_ring64) cudaFree(p->d_ring64);
-    if (p->d_sched) cudaFree(p->d_sched);
-    if (p->d_phase) cudaFree(p->d_phase);
-    if (p->d_phase32) cudaFree(p->d_phase32);
+    drop_dft(p);
+    drop_schedule(p);
     if (p->own_stream && p->stream) cudaStreamDestroy(p->stream);
     delete p;
     return SMAT_OK;
@@ -987,22 +1009,14 @@ extern "C" int smat_fdtd_set_source_plane(smat_fdtd_plan *p, int b, int iI, int 
     return SMAT_OK;
 }
 
-extern "C" int smat_fdtd_set_schedule(smat_fdtd_plan *p, int nsteps, const double *src, int nfreq, int nplanes,
-                                      const int *planes, const double *phase)
+/* a schedule's sources and phases to the device */
+static int upload_schedule(smat_fdtd_plan *p, int nsteps, const double *src, const double *phase)
 {
-    smat_clear_error();
-    if (!p || nsteps <= 0 || !src || nfreq < 0 || (nfreq > 0 && (!phase || !planes || nplanes <= 0)))
-        return smat_fail(SMAT_EINVAL, "set_schedule: bad arguments");
-    int rc = setup_dft(p, nfreq, nfreq > 0 ? nplanes : 0, planes);
-    if (rc) return rc;
-    p->ref_dft = false;
-    if (p->d_sched) cudaFree(p->d_sched), p->d_sched = nullptr;
-    if (p->d_phase) cudaFree(p->d_phase), p->d_phase = nullptr;
-    if (p->d_phase32) cudaFree(p->d_phase32), p->d_phase32 = nullptr;
+    int rc;
     if ((rc = dalloc(&p->d_sched, 6 * (size_t)nsteps, p->stream))) return rc;
     CK(p->cpy(p->d_sched, src, 6 * (size_t)nsteps * 8, cudaMemcpyHostToDevice));
-    if (nfreq > 0) {
-        const size_t np = 4 * (size_t)nsteps * nfreq;
+    if (p->nfreq > 0) {
+        const size_t np = 4 * (size_t)nsteps * p->nfreq;
         if ((rc = dalloc(&p->d_phase, np, p->stream))) return rc;
         CK(p->cpy(p->d_phase, phase, np * 8, cudaMemcpyHostToDevice));
         if (p->precision == SMAT_FP32) {
@@ -1022,6 +1036,25 @@ extern "C" int smat_fdtd_set_schedule(smat_fdtd_plan *p, int nsteps, const doubl
             CK(p->cpy(p->d_phase32, ph32.data(), 2 * np * 4, cudaMemcpyHostToDevice));
         }
     }
+    return SMAT_OK;
+}
+
+extern "C" int smat_fdtd_set_schedule(smat_fdtd_plan *p, int nsteps, const double *src, int nfreq, int nplanes,
+                                      const int *planes, const double *phase)
+{
+    smat_clear_error();
+    if (!p || nsteps <= 0 || !src || nfreq < 0 || (nfreq > 0 && (!phase || !planes || nplanes <= 0)))
+        return smat_fail(SMAT_EINVAL, "set_schedule: bad arguments");
+    int rc = setup_dft(p, nfreq, nfreq > 0 ? nplanes : 0, planes);
+    if (rc == SMAT_EINVAL) return rc;
+    drop_schedule(p);
+    if (!rc) rc = upload_schedule(p, nsteps, src, phase);
+    if (rc) { /* neither the old schedule nor half of the new one */
+        drop_schedule(p);
+        drop_dft(p);
+        return rc;
+    }
+    p->ref_dft = false;
     p->nsched = nsteps;
     CK(cudaStreamSynchronize(p->stream));
     return SMAT_OK;

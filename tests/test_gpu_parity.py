@@ -1044,6 +1044,54 @@ def test_fp64_plan_holds_aux_slots_of_split_cells_only(built, batch):
         assert p.device_bytes <= fixed + 48 * batch * (n + ln + 1) + dft + 4096
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("part", ["sums", "phases"])
+def test_schedule_out_of_memory_leaves_no_half_of_it(built, precision, part):
+    """A schedule whose DFT sums (or phases) do not fit the device: the plan has
+    neither it nor the one before, run and get_dft refuse, and the next schedule
+    gives what a fresh plan gives."""
+    f = _fdtd()
+    from smatranem_gb300 import workloads as W
+    L = (48, 40, 30, 1)
+    s = W.random_structure(L, seed=8, pml=(3, 3, 3))
+    pr = W.prepare(s)
+    src, ph = (a[:20] for a in f.cw_schedule(pr.n2pi, (1, 1, 3)))
+    big = np.zeros((1, 600000, 4)) if part == "sums" else np.zeros((1, 1, 4))
+    planes = tuple(range(5, 13)) if part == "sums" else (5,)
+    out = []
+    for fail in (True, False):
+        with f.Plan.create(L, s.iBc, (4, 25, 5, 1), pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma,
+                           precision=precision) as p:
+            p.set_incident(0, *W.random_incident(L[0] * L[1], seed=2))
+            if fail:
+                p.set_schedule(src, planes=(4, 25), phase=ph)
+                hold = []
+                if part == "phases":  # 6 doubles a step and 4 of phases: room for the sources alone
+                    torch = pytest.importorskip("torch")
+                    big = np.zeros((1 << 21, 1, 4))
+                    while True:
+                        free = torch.cuda.mem_get_info()[0]
+                        take = free - (130 << 20)
+                        if take < (4 << 20):
+                            break
+                        hold.append(torch.empty(take, dtype=torch.uint8, device="cuda"))
+                with pytest.raises(f.FdtdError) as e:
+                    p.set_schedule(np.zeros((big.shape[0], 6)), planes=planes, phase=big)
+                assert e.value.code == -3
+                if hold:
+                    hold.clear()
+                    torch.cuda.empty_cache()
+                with pytest.raises(f.FdtdError):
+                    p.run(0, 1)
+                with pytest.raises(f.FdtdError):
+                    p.get_dft(0, 0, 0)
+            p.set_schedule(src, planes=(4, 25), phase=ph)
+            p.run(0, 20)
+            out.append((*p.get_fields(0), p.get_dft(0, 0, 0), p.get_dft(0, 0, 1)))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
 def test_row_fused_run_of_one_graph_from_the_other_set(built):
     """A run of exactly 32 steps (one graph) that starts from the second field
     set, before and after a graph exists, as the sweeps."""
