@@ -598,6 +598,11 @@ int adjoint_run(smat_fdtd_plan *p, const C &coef, int nsteps, int K, int f, int 
     const size_t need = ck_bytes * nseg + 4 * fs * sizeof(T) + rec_n * sizeof(T) * (K + 1) + rec_n * 8;
     size_t fr = 0, tot = 0;
     CK(cudaMemGetInfo(&fr, &tot));
+    if (need > fr / 10 * 9 && p->d_ring64) { /* FP64 plans go without the ring before they refuse */
+        drop_ring(p);
+        drop_graph(p);
+        CK(cudaMemGetInfo(&fr, &tot));
+    }
     if (need > fr / 10 * 9)
         return smat_fail(SMAT_ENOMEM, "adjoint: %zu bytes of checkpoints and adjoint state, %zu free (raise K)", need,
                          fr);

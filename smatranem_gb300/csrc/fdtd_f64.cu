@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(96, 13) k_sweep64(const P64 p, const int rel)
     }
     F[i0] = f;
     const int q = monitor_index64(p.d, j2);
-    if (q >= 0 && c < 2) {
+    if (q >= 0 && c < 2 && p.d.ring64) {
         /* a plane through the PML (allowed for general schedules only; the
          * reference exits, :320) samples the total field main + aux */
         ring64_at(p.d, g.pl, b, *p.s.base + rel, q, (EF ? 2 : 0) + c)[px] = cls == CLS_A ? f + fa : f;
@@ -283,7 +283,9 @@ __global__ void __launch_bounds__(96, 13) k_sweep64(const P64 p, const int rel)
  * accumulators every step, at 1/32 of their traffic and launches.  A thread
  * takes one pixel and component of one plane and excitation and every
  * gridDim.z / batch-th frequency.  96^3 cube, 11 wavelengths, 2 planes: 6.6 us
- * a step (half of it the FP64 pipe's additions), from 32 us. */
+ * a step (half of it the FP64 pipe's additions), from 32 us.  RING false: a plan
+ * without the ring (no room for it), one step. */
+template <bool RING>
 __global__ void __launch_bounds__(128) k_flush64(const P64 p, const int rel_end, const int count)
 {
     const int px = blockIdx.x * 128 + threadIdx.x, q = blockIdx.y >> 2, v = blockIdx.y & 3;
@@ -293,12 +295,18 @@ __global__ void __launch_bounds__(128) k_flush64(const P64 p, const int rel_end,
     if (px >= g.pl) return;
     const int k0 = *p.s.base + rel_end - count;
     const int qs = monitor_index64(d, d.planes[q]); /* the slot the sweeps fill, where a plane is listed twice */
+    double now = 0.0;
+    if (!RING) { /* count is 1: from the fields, as the sweeps sample them */
+        const long long l = px + (long long)g.pl * d.planes[q], a = p.addr[l], as = p.lnotn + 1;
+        now = (v < 2 ? p.H : p.E)[(3LL * b + v % 2) * g.n3 + l];
+        if ((p.flags[l] & 7) == CLS_A) now += (v < 2 ? p.Ha : p.Ea)[(3LL * b + v % 2) * as + a];
+    }
     for (int f = f0; f < d.nfreq; f += nf) {
         double *acc = d.acc + 2 * (((((long long)b * d.nfreq + f) * d.nq + q) * 4 + v) * g.pl + px);
         double re = acc[0], im = acc[1];
 #pragma unroll 4
         for (int s = 0; s < count; s++) {
-            const double x = ring64_at(d, g.pl, b, k0 + s, qs, v)[px];
+            const double x = RING ? ring64_at(d, g.pl, b, k0 + s, qs, v)[px] : now;
             const double *ph = (d.xphase ? d.xphase : d.phase + 4 * ((long long)(k0 + s) * d.nfreq + f)) + (v < 2 ? 0 : 2);
             re += imul(ph[0], x);
             im += imul(ph[1], x);
@@ -352,7 +360,7 @@ void launch_flush64(const P64 &p, int rel_end, int count, cudaStream_t st)
     const int nb = (p.g.pl + 127) / 128, used = nb * p.d.nq * 4 * p.batch;
     int nf = used >= 1824 ? 1 : (1824 + used - 1) / used; /* 152 SMs x 12 blocks */
     if (nf > p.d.nfreq) nf = p.d.nfreq;
-    k_flush64<<<dim3(nb, p.d.nq * 4, p.batch * nf), 128, 0, st>>>(p, rel_end, count);
+    (p.d.ring64 ? k_flush64<true> : k_flush64<false>)<<<dim3(nb, p.d.nq * 4, p.batch * nf), 128, 0, st>>>(p, rel_end, count);
 }
 
 void launch_bump(int *base, int by, cudaStream_t st) { k_bump<<<1, 1, 0, st>>>(base, by); }

@@ -73,7 +73,7 @@ struct Dft {
     double *acc;          /* [batch][nfreq][nq][4][pl] complex */
     int ringK;            /* samples kept per flush */
     float *ring;          /* FP32: [batch][ringK][nq][4][pl] */
-    double *ring64;       /* FP64: the same */
+    double *ring64;       /* FP64: the same; null: no room for it, flushed every step from the fields */
 };
 
 struct P64 {

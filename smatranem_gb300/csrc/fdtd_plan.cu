@@ -163,8 +163,9 @@ void enqueue_steps(smat_fdtd_plan *p, int rel0, int n, bool xp)
         for (int i = 0; i < n; i++) {
             launch_h64(q, rel0 + i, p->stream);
             launch_e64(q, rel0 + i, p->stream);
+            if (!q.d.ring64) launch_flush64(q, rel0 + i + 1, 1, p->stream);
         }
-        launch_flush64(q, rel0 + n, n, p->stream);
+        if (q.d.ring64) launch_flush64(q, rel0 + n, n, p->stream);
     } else if (p->fused == 6) {
         for (int i = 0; i < n; i++) launch_row_step(p, xp, rel0 + i, p->stream);
         launch_flush32(make_p32(p, xp), rel0 + n, n, p->stream);
@@ -357,8 +358,8 @@ void drop_schedule(smat_fdtd_plan *p)
     p->nsched = 0;
 }
 
-/* DFT accumulators and the sample ring for nfreq x nq planes, zeroed; where
- * they do not fit, the plan is left without a DFT */
+/* DFT accumulators for nfreq x nq planes, zeroed; where they do not fit, the
+ * plan is left without a DFT */
 int setup_dft(smat_fdtd_plan *p, int nfreq, int nq, const int *planes)
 {
     if (nq > MAX_PLANES) return smat_fail(SMAT_EINVAL, "at most %d monitor planes", MAX_PLANES);
@@ -373,16 +374,24 @@ int setup_dft(smat_fdtd_plan *p, int nfreq, int nq, const int *planes)
     int rc = SMAT_OK;
     if (p->d_acc) CK(cudaMemsetAsync(p->d_acc, 0, acc_len(p) * 8, p->stream));
     else if (!(rc = dalloc(&p->d_acc, acc_len(p), p->stream))) p->dev_bytes += (long long)(acc_len(p) * 8);
-    if (!rc && !p->d_ring && !p->d_ring64) {
-        const bool f64 = p->precision == SMAT_FP64;
-        rc = f64 ? dalloc(&p->d_ring64, ring_len(p), p->stream) : dalloc(&p->d_ring, ring_len(p), p->stream);
-        if (!rc) p->dev_bytes += (long long)(ring_len(p) * (f64 ? sizeof(double) : sizeof(float)));
-    }
     if (rc) {
         drop_dft(p);
         return rc;
     }
     for (int i = 0; i < MAX_PLANES; i++) p->planes[i] = i < nq ? planes[i] : -1;
+    return SMAT_OK;
+}
+
+/* the sample ring, last of all: an FP64 plan that has no room for it folds each
+ * step's samples in from the fields */
+int setup_ring(smat_fdtd_plan *p)
+{
+    if (p->d_ring || p->d_ring64) return SMAT_OK;
+    const bool f64 = p->precision == SMAT_FP64;
+    int rc = f64 ? dalloc(&p->d_ring64, ring_len(p), p->stream) : dalloc(&p->d_ring, ring_len(p), p->stream);
+    if (!rc) p->dev_bytes += (long long)(ring_len(p) * (f64 ? sizeof(double) : sizeof(float)));
+    if (rc != SMAT_ENOMEM || !f64) return rc;
+    smat_clear_error();
     return SMAT_OK;
 }
 
@@ -408,8 +417,7 @@ int common_alloc(smat_fdtd_plan *p)
     }
     /* the reference DFT: one frequency on planes iB and iT */
     const int pls[2] = {p->iBTIin[0], p->iBTIin[1]};
-    rc = setup_dft(p, 1, 2, pls);
-    if (rc) return rc;
+    if ((rc = setup_dft(p, 1, 2, pls)) || (rc = setup_ring(p))) return rc;
     p->ref_dft = true;
     p->ref_planes_ok = check_planes(p, 2, pls) == SMAT_OK;
     smat_clear_error();
@@ -1049,6 +1057,7 @@ extern "C" int smat_fdtd_set_schedule(smat_fdtd_plan *p, int nsteps, const doubl
     if (rc == SMAT_EINVAL) return rc;
     drop_schedule(p);
     if (!rc) rc = upload_schedule(p, nsteps, src, phase);
+    if (!rc) rc = setup_ring(p);
     if (rc) { /* neither the old schedule nor half of the new one */
         drop_schedule(p);
         drop_dft(p);
@@ -1184,8 +1193,9 @@ extern "C" int smat_fdtd_time_kernels(smat_fdtd_plan *p, int k_begin, int nsteps
         if (p->precision == SMAT_FP64) launch_e64(q64, i, p->stream);
         else if (p->fused != 6 && !(p->szc > 0 && p->szc < p->L[2])) sweep_e(p, q32, i, 0, p->L[2], p->stream);
         CK(cudaEventRecord(ev[2], p->stream));
-        if ((i + 1) % RING_K == 0 || i + 1 == nsteps) {
-            const int cnt = (i + 1) % RING_K == 0 ? RING_K : (i + 1) % RING_K;
+        const bool each = p->precision == SMAT_FP64 && !q64.d.ring64;
+        if (each || (i + 1) % RING_K == 0 || i + 1 == nsteps) {
+            const int cnt = each ? 1 : (i + 1) % RING_K == 0 ? RING_K : (i + 1) % RING_K;
             if (p->precision == SMAT_FP64) launch_flush64(q64, i + 1, cnt, p->stream);
             else launch_flush32(make_p32(p, false), i + 1, cnt, p->stream);
         }

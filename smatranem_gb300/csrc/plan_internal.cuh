@@ -18,7 +18,7 @@
 namespace smat {
 namespace plan {
 
-constexpr int GRAPH_STEPS = 32; /* steps per captured graph (= FP32 ring length) */
+constexpr int GRAPH_STEPS = 32; /* steps per captured graph (= ring length) */
 constexpr int RING_K = 32;
 
 inline int cuda_fail(cudaError_t e, const char *what)
@@ -164,6 +164,7 @@ void enqueue_update(smat_fdtd_plan *p, int rel, cudaStream_t st);
 void launch_row_step(smat_fdtd_plan *p, bool xp, int rel, cudaStream_t st);
 int sm_count();
 void drop_graph(smat_fdtd_plan *p);
+void drop_ring(smat_fdtd_plan *p); /* FP64: the plan goes on without it */
 } // namespace plan
 } // namespace smat
 

@@ -1044,6 +1044,59 @@ def test_fp64_plan_holds_aux_slots_of_split_cells_only(built, batch):
         assert p.device_bytes <= fixed + 48 * batch * (n + ln + 1) + dft + 4096
 
 
+class _Ballast:
+    """Device memory taken until `left` bytes are free."""
+
+    def __init__(self, left):
+        self.torch = pytest.importorskip("torch")
+        self.hold = []
+        while True:
+            take = self.torch.cuda.mem_get_info()[0] - left
+            if take < (4 << 20):
+                break
+            self.hold.append(self.torch.empty(take, dtype=self.torch.uint8, device="cuda"))
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *a):
+        self.hold.clear()
+        self.torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("L,pml", [((64, 60, 40, 1), (3, 0, 3)), ((64, 60, 40, 1), (3, 3, 0))])
+def test_fp64_plan_without_room_for_the_sample_ring(built, L, pml):
+    """An FP64 schedule of eight planes (one of them through the PML, one listed
+    twice) with room for its sums but not for the ring: the same fields and DFT,
+    through graphs, single launches and steps of their own."""
+    f = _fdtd()
+    from smatranem_gb300 import workloads as W
+    s = W.random_structure(L, seed=12, pml=pml, lossy=0.05, pec=0.03)
+    pr = W.prepare(s)
+    src, ph = (a[:70] for a in f.cw_schedule(pr.n2pi, (1, 1, 6)))
+    planes = (1, 5, 9, 9, 20, 25, 30, 36)
+    H0, E0 = W.random_fields(s.n3, pr.lnotn, seed=1, scale=1e-2)
+    ring = 32 * 8 * 4 * L[0] * L[1] * 8
+    out, held = [], []
+    for small in (False, True):
+        with f.Plan.create(L, s.iBc, (4, 36, 5, 1), pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma, pec=s.pec) as p:
+            p.set_fields(0, H0, E0)
+            p.set_incident(0, *W.random_incident(L[0] * L[1], seed=2))
+            if small:
+                # the plan's ring of two planes goes, and leaves less than eight take
+                with _Ballast(ring // 2):
+                    p.set_schedule(src, planes=planes, phase=ph)
+            else:
+                p.set_schedule(src, planes=planes, phase=ph)
+            held.append(p.device_bytes)
+            for k in ((0, 3), (3, 67), (67, 68), (68, 70)):
+                p.run(*k)
+            out.append((*p.get_fields(0), *(p.get_dft(0, 0, q) for q in range(8))))
+    assert held[0] - held[1] == ring
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("part", ["sums", "phases"])
 def test_schedule_out_of_memory_leaves_no_half_of_it(built, precision, part):
@@ -1065,22 +1118,12 @@ def test_schedule_out_of_memory_leaves_no_half_of_it(built, precision, part):
             p.set_incident(0, *W.random_incident(L[0] * L[1], seed=2))
             if fail:
                 p.set_schedule(src, planes=(4, 25), phase=ph)
-                hold = []
                 if part == "phases":  # 6 doubles a step and 4 of phases: room for the sources alone
-                    torch = pytest.importorskip("torch")
                     big = np.zeros((1 << 21, 1, 4))
-                    while True:
-                        free = torch.cuda.mem_get_info()[0]
-                        take = free - (130 << 20)
-                        if take < (4 << 20):
-                            break
-                        hold.append(torch.empty(take, dtype=torch.uint8, device="cuda"))
-                with pytest.raises(f.FdtdError) as e:
-                    p.set_schedule(np.zeros((big.shape[0], 6)), planes=planes, phase=big)
+                with _Ballast(130 << 20 if part == "phases" else 1 << 40):
+                    with pytest.raises(f.FdtdError) as e:
+                        p.set_schedule(np.zeros((big.shape[0], 6)), planes=planes, phase=big)
                 assert e.value.code == -3
-                if hold:
-                    hold.clear()
-                    torch.cuda.empty_cache()
                 with pytest.raises(f.FdtdError):
                     p.run(0, 1)
                 with pytest.raises(f.FdtdError):
