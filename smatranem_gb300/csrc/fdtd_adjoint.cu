@@ -768,8 +768,6 @@ extern "C" int smat_fdtd_adjoint_grad(smat_fdtd_plan *p, int nsteps, int K, int 
         const char *sc = getenv("SMATRAN_ADJOINT_SCALAR");
         p->adj_scalar = sc && sc[0] && sc[0] != '0';
         Coef32 c;
-        c.bh = p->d_bh;
-        c.be = p->d_be;
         c.hrec = p->d_hrec;
         c.erec = p->d_erec;
         c.tab = p->d_tab;
@@ -777,7 +775,13 @@ extern "C" int smat_fdtd_adjoint_grad(smat_fdtd_plan *p, int nsteps, int K, int 
         c.S = p->L[0] + p->L[1] + p->L[2];
         c.s1 = p->L[0];
         c.s2 = p->L[0] + p->L[1];
-        return adjoint_run<float>(p, c, nsteps, K, f, q, ncols, tilXi_cols, bx, grad, grad_c, J);
+        int rc;
+        do {
+            c.bh = p->d_bh;
+            c.be = p->d_be;
+            rc = adjoint_run<float>(p, c, nsteps, K, f, q, ncols, tilXi_cols, bx, grad, grad_c, J);
+        } while (found_room(p, rc));
+        return rc;
     }
     Coef64 c;
     c.flags = p->d_flags;

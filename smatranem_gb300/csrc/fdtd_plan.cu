@@ -750,9 +750,82 @@ int upload_f32(smat_fdtd_plan *p, const smat_fdtd_desc *d, const double *Ah, con
     return SMAT_OK;
 }
 
+/* n rows of FP32 values between padded and unpadded length (padding: 0) */
+void rows_unpad(const smat_fdtd_plan *p, size_t n, const float *padded, float *rows)
+{
+    const size_t L0 = p->L[0];
+    for (size_t r = 0; r < n; r++) memcpy(rows + r * L0, padded + r * p->P0, L0 * 4);
+}
+
+void rows_pad(const smat_fdtd_plan *p, size_t n, const float *rows, float *padded)
+{
+    const size_t L0 = p->L[0];
+    memset(padded, 0, n * p->P0 * 4);
+    for (size_t r = 0; r < n; r++) memcpy(padded + r * p->P0, rows + r * L0, L0 * 4);
+}
+
+/* A plan of padded rows gives the padding's memory back (up to 15 %) where a
+ * schedule or an adjoint lacks it: its arrays go through the host, one by one.
+ * It then runs the one-cell-per-thread sweeps: the same bits. */
+int unpad_plan(smat_fdtd_plan *p)
+{
+    CK(cudaStreamSynchronize(p->stream));
+    drop_graph(p);
+    const size_t rows = (size_t)p->L[1] * p->L[2], b = p->batch;
+    std::vector<std::pair<float **, size_t>> arrays = {{&p->d_bh, 3}, {&p->d_be, 3}};
+    for (float **a : {&p->d_H32, &p->d_E32, &p->d_Ha32, &p->d_Ea32, &p->d_H32b, &p->d_E32b, &p->d_Ha32b, &p->d_Ea32b})
+        arrays.push_back({a, 3 * b});
+    std::vector<float> in(3 * b * rows * p->P0), out(3 * b * rows * p->L[0]);
+    for (auto &[a, comps] : arrays) {
+        const size_t n = comps * rows;
+        CK(cudaMemcpy(in.data(), *a, n * p->P0 * 4, cudaMemcpyDeviceToHost));
+        rows_unpad(p, n, in.data(), out.data());
+        for (void *&x : p->allocations)
+            if (x == *a) {
+                cudaFree(x);
+                x = *a = nullptr;
+                if (int rc = dalloc(a, n * p->L[0], p->stream)) return rc; /* (another thread took it) */
+                x = *a;
+            }
+        p->dev_bytes -= (long long)(n * (p->P0 - p->L[0]) * 4);
+        CK(p->cpy(*a, out.data(), n * p->L[0] * 4, cudaMemcpyHostToDevice));
+        CK(cudaStreamSynchronize(p->stream));
+    }
+    for (auto *gen : {&p->hgen_host, &p->egen_host}) {
+        for (int &l : *gen) l -= l / p->P0 * (p->P0 - p->L[0]);
+        if (!gen->empty())
+            CK(p->cpy(gen == &p->hgen_host ? p->d_hgen : p->d_egen, gen->data(), gen->size() * sizeof(int), cudaMemcpyHostToDevice));
+    }
+    CK(cudaStreamSynchronize(p->stream));
+    p->P0 = p->L[0];
+    p->n3p = p->n3;
+    return SMAT_OK;
+}
+
+/* after a call ran out of memory: whether it may find room now */
+bool found_room(smat_fdtd_plan *p, int rc)
+{
+    if (rc != SMAT_ENOMEM || p->P0 == p->L[0]) return false;
+    if (unpad_plan(p) != SMAT_OK) {
+        drop_schedule(p);
+        drop_dft(p);
+        return false;
+    }
+    smat_clear_error();
+    return true;
+}
+
+/* an FP32 plan whose arrays were lost in unpad_plan runs nothing more */
+bool lost_arrays(const smat_fdtd_plan *p)
+{
+    if (p->precision != SMAT_FP32) return false;
+    for (const float *a : {p->d_bh, p->d_be, p->d_H32, p->d_E32, p->d_Ha32, p->d_Ea32, p->d_H32b, p->d_E32b, p->d_Ha32b, p->d_Ea32b})
+        if (!a) return true;
+    return false;
+}
+
 int finish_create(smat_fdtd_plan *p, int rc, smat_fdtd_plan **out)
 {
-    if (rc == SMAT_OK) rc = common_alloc(p);
     if (rc == SMAT_OK) {
         cudaError_t e = cudaStreamSynchronize(p->stream);
         if (e != cudaSuccess) rc = cuda_fail(e, "plan upload");
@@ -820,10 +893,15 @@ extern "C" int smat_fdtd_create(const smat_fdtd_desc *d, void *stream, smat_fdtd
         for (long long l = 0; l < n3; l++)
             if (d->pec[l])
                 for (int c = 0; c < 3; c++) Ae[c + 3 * l] = Be[c + 3 * l] = 0.0;
-    rc = p->precision == SMAT_FP64 ? upload_f64(p, Ah.get(), Bh.get(), Ae.get(), Be.get())
-                                   : upload_f32(p, d, Ah.get(), Bh.get(), Ae.get(), Be.get());
+    auto upload = [&] {
+        const int r = p->precision == SMAT_FP64 ? upload_f64(p, Ah.get(), Bh.get(), Ae.get(), Be.get())
+                                                : upload_f32(p, d, Ah.get(), Bh.get(), Ae.get(), Be.get());
+        return r ? r : common_alloc(p);
+    };
+    rc = upload();
     if (rc == SMAT_ENOMEM && p->P0 != p->L[0]) { /* no room for the padding: without it */
         cudaStreamSynchronize(p->stream);
+        drop_dft(p);
         for (void *a : p->allocations) cudaFree(a);
         p->allocations.clear();
         p->dev_bytes = 0;
@@ -831,7 +909,7 @@ extern "C" int smat_fdtd_create(const smat_fdtd_desc *d, void *stream, smat_fdtd
         p->P0 = p->L[0];
         p->n3p = p->n3;
         smat_clear_error();
-        rc = upload_f32(p, d, Ah.get(), Bh.get(), Ae.get(), Be.get());
+        rc = upload();
     }
     return finish_create(p, rc, out);
 }
@@ -872,6 +950,7 @@ extern "C" int smat_fdtd_create_from_coeffs(const int L[4], const double *Ah, co
         return smat_fail(SMAT_EINVAL, "Lnotn = %d but %d non-'n' cells", Lnotn, count);
     }
     rc = upload_f64(p, Ah, Bh, Ae, Be);
+    if (!rc) rc = common_alloc(p);
     return finish_create(p, rc, out);
 }
 
@@ -1053,11 +1132,15 @@ extern "C" int smat_fdtd_set_schedule(smat_fdtd_plan *p, int nsteps, const doubl
     smat_clear_error();
     if (!p || nsteps <= 0 || !src || nfreq < 0 || (nfreq > 0 && (!phase || !planes || nplanes <= 0)))
         return smat_fail(SMAT_EINVAL, "set_schedule: bad arguments");
-    int rc = setup_dft(p, nfreq, nfreq > 0 ? nplanes : 0, planes);
-    if (rc == SMAT_EINVAL) return rc;
-    drop_schedule(p);
-    if (!rc) rc = upload_schedule(p, nsteps, src, phase);
-    if (!rc) rc = setup_ring(p);
+    if (lost_arrays(p)) return smat_fail(SMAT_ENOMEM, "set_schedule: the plan's arrays were lost for want of memory");
+    int rc;
+    do {
+        rc = setup_dft(p, nfreq, nfreq > 0 ? nplanes : 0, planes);
+        if (rc == SMAT_EINVAL) return rc;
+        drop_schedule(p);
+        if (!rc) rc = upload_schedule(p, nsteps, src, phase);
+        if (!rc) rc = setup_ring(p);
+    } while (found_room(p, rc));
     if (rc) { /* neither the old schedule nor half of the new one */
         drop_schedule(p);
         drop_dft(p);
@@ -1487,6 +1570,7 @@ extern "C" int smat_fdtd_check_finite(smat_fdtd_plan *p, int *finite, double *ma
 {
     smat_clear_error();
     if (!p) return smat_fail(SMAT_EINVAL, "null plan");
+    if (lost_arrays(p)) return smat_fail(SMAT_ENOMEM, "check_finite: the plan's arrays were lost for want of memory");
     CK(cudaMemsetAsync(p->d_scratch, 0, 8, p->stream));
     const bool d = p->precision == SMAT_FP64;
     const long long nf = (long long)p->batch * 3 * p->n3p;
@@ -1576,20 +1660,6 @@ size_t file_bytes(const smat_fdtd_plan *p, const StateArray &a)
     return a.padded ? (size_t)p->batch * 3 * p->n3 * 4 : a.bytes;
 }
 
-/* FP32 fields between padded and unpadded rows (padding: 0) */
-void rows_unpad(const smat_fdtd_plan *p, const float *padded, float *rows)
-{
-    const size_t L0 = p->L[0], n = (size_t)p->batch * 3 * p->L[1] * p->L[2];
-    for (size_t r = 0; r < n; r++) memcpy(rows + r * L0, padded + r * p->P0, L0 * 4);
-}
-
-void rows_pad(const smat_fdtd_plan *p, const float *rows, float *padded)
-{
-    const size_t L0 = p->L[0], n = (size_t)p->batch * 3 * p->L[1] * p->L[2];
-    memset(padded, 0, n * p->P0 * 4);
-    for (size_t r = 0; r < n; r++) memcpy(padded + r * p->P0, rows + r * L0, L0 * 4);
-}
-
 void fill_header(const smat_fdtd_plan *p, StateHeader &h)
 {
     memset(&h, 0, sizeof h);
@@ -1628,7 +1698,7 @@ extern "C" int smat_fdtd_save_state(smat_fdtd_plan *p, const char *path)
         const size_t n = file_bytes(p, a);
         if (a.padded) {
             file.resize(n);
-            rows_unpad(p, (const float *)buf.data(), (float *)file.data());
+            rows_unpad(p, (size_t)p->batch * 3 * p->L[1] * p->L[2], (const float *)buf.data(), (float *)file.data());
         }
         if (fwrite(a.padded ? file.data() : buf.data(), 1, n, f) != n)
             rc = smat_fail(SMAT_EINVAL, "save_state: write error");
@@ -1668,7 +1738,7 @@ extern "C" int smat_fdtd_load_state(smat_fdtd_plan *p, const char *path)
             rc = smat_fail(SMAT_EINVAL, "load_state: %s is truncated", path);
             break;
         }
-        if (a.padded) rows_pad(p, (const float *)file.data(), (float *)buf.data());
+        if (a.padded) rows_pad(p, (size_t)p->batch * 3 * p->L[1] * p->L[2], (const float *)file.data(), (float *)buf.data());
         p->h2d_bytes += (long long)a.bytes;
         if (cudaMemcpy(a.dev, buf.data(), a.bytes, cudaMemcpyHostToDevice) != cudaSuccess)
             rc = cuda_fail(cudaGetLastError(), "load_state: copy");

@@ -165,6 +165,7 @@ void launch_row_step(smat_fdtd_plan *p, bool xp, int rel, cudaStream_t st);
 int sm_count();
 void drop_graph(smat_fdtd_plan *p);
 void drop_ring(smat_fdtd_plan *p); /* FP64: the plan goes on without it */
+bool found_room(smat_fdtd_plan *p, int rc);
 } // namespace plan
 } // namespace smat
 

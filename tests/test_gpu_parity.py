@@ -954,6 +954,80 @@ def test_padded_rows_adjoint(built, case):
     assert abs(J - sum(o[0] for o in one)) <= 1e-12 * abs(J)
 
 
+class _Ballast:
+    """Device memory taken until `left` bytes are free."""
+
+    def __init__(self, left):
+        self.torch = pytest.importorskip("torch")
+        self.hold = []
+        while True:
+            take = self.torch.cuda.mem_get_info()[0] - left
+            if take < (4 << 20):
+                break
+            self.hold.append(self.torch.empty(take, dtype=self.torch.uint8, device="cuda"))
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *a):
+        self.hold.clear()
+        self.torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("call", ["create", "set_schedule", "adjoint"])
+def test_padded_plan_without_room_for_the_padding(built, call):
+    """A plan of padded rows on a device with room for the rows but not for all of
+    the padding, at creation (anywhere in it), at a schedule with larger DFT sums
+    and at an adjoint: the results of a device with room."""
+    f = _fdtd()
+    from smatranem_gb300 import workloads as W
+    L, batch, iBTIin = (21, 160, 160, 2), 8, (4, 150, 6, 1)
+    s = W.random_structure(L, seed=5, pml=(3, 3, 3), pec=0.0 if call == "adjoint" else 0.02)
+    pr = W.prepare(s)
+    pl, n3 = L[0] * L[1], s.n3
+    padding = 12 * (2 + 8 * batch) * 3 * L[1] * L[2]  # bytes: three cells a row of every array
+    src, ph = (a[:24] for a in f.cw_schedule(pr.n2pi, (1, 1, 3)))
+    ph = ph * (1 + np.arange(17)[None, :, None] / 17)
+    rng = np.random.default_rng(1)
+    col = rng.standard_normal(4 * pl) + 1j * rng.standard_normal(4 * pl)
+
+    def run(small, left=0):
+        """Fields and DFT, or the gradient; `small`: the call with little room."""
+        make = lambda: f.Plan.create(s.L, s.iBc, iBTIin, pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma,
+                                     precision=f.FP32, batch=batch, pec=s.pec)
+        room = lambda name: _Ballast(left) if small and call == name else _Ballast(1 << 50)
+        with room("create"):
+            p = make()
+        with p:
+            size = p.device_bytes
+            for b in range(batch):
+                p.set_incident(b, *W.random_incident(pl, seed=10 + b))
+            with room("set_schedule"):
+                p.set_schedule(src, planes=(4, 150), phase=ph)
+            if call == "adjoint":
+                with room("adjoint"):
+                    J, g, gc = p.adjoint_grad(24, 4, 3, 1, col, (8, 12, 40, 44, 60, 70))
+                return size, p.device_bytes, (np.array(J), np.asarray(g), np.asarray(gc))
+            p.run(0, 24)
+            return size, p.device_bytes, (*p.get_fields(3), p.get_dft(3, 16, 1))
+
+    size, _, want = run(False)
+    if call == "create":
+        lefts = [size - padding + (32 << 20) + (k << 23) for k in range(5)]
+    elif call == "set_schedule":
+        lefts = [20 << 20]  # the sums take 58 MB
+    else:
+        state = 48 * batch * n3
+        lefts = [int((6 * state + 4 * state // 4 + (1 << 20)) / 0.9)]
+    gone = 0
+    for left in lefts:
+        before, after, got = run(True, left)
+        gone += before < size or after < before
+        for a, b in zip(want, got):
+            assert np.array_equal(a, b), left
+    assert gone > 0  # the padding went somewhere
+
+
 @pytest.mark.parametrize("L", [(4, 7, 9, 2), (124, 5, 7, 2), (128, 6, 7, 2), (132, 5, 6, 2), (256, 3, 6, 2)])
 def test_quads_dealt_out_bit_identical(built, L):
     """The vectorised sweeps whose quads go to the threads row after row (L0 not
@@ -1042,26 +1116,6 @@ def test_fp64_plan_holds_aux_slots_of_split_cells_only(built, batch):
         fixed = (96 + 1 + 4) * n + 96 * ln + (64 * batch + 32 + 32) * pl  # coefficients, classes, addresses, sources
         dft = batch * 2 * 4 * pl * (16 + 32 * 8)                          # sums and samples of the reference planes
         assert p.device_bytes <= fixed + 48 * batch * (n + ln + 1) + dft + 4096
-
-
-class _Ballast:
-    """Device memory taken until `left` bytes are free."""
-
-    def __init__(self, left):
-        self.torch = pytest.importorskip("torch")
-        self.hold = []
-        while True:
-            take = self.torch.cuda.mem_get_info()[0] - left
-            if take < (4 << 20):
-                break
-            self.hold.append(self.torch.empty(take, dtype=self.torch.uint8, device="cuda"))
-
-    def __enter__(self):
-        return self
-
-    def __exit__(self, *a):
-        self.hold.clear()
-        self.torch.cuda.empty_cache()
 
 
 @pytest.mark.parametrize("L,pml", [((64, 60, 40, 1), (3, 0, 3)), ((64, 60, 40, 1), (3, 3, 0))])
