@@ -771,16 +771,23 @@ struct Solver {
         return cudaPeekAtLastError() == cudaSuccess ? SMAT_OK : smat_fail(SMAT_ECUDA, "k_mbb launch");
     }
     /* Yn = alpha (mbb maa Yc - c Yc) - beta Yp; W: room for maa Yc where the
-     * stencils run one after the other (one-cell axes, SMATRAN_MODE_ONE_PASS) */
+     * stencils run one after the other (one-cell axes, long layers of a few
+     * columns, SMATRAN_MODE_ONE_PASS) */
     template <class T>
     int product(const T *Yc, const typename nd<T>::type *Yp, T *Yn, T *W, int m, double alpha, double c, double beta,
                 const double *ascale = nullptr)
     {
-        if (!fused()) {
+        const int ntx = (op.L0 + PX - 1) / PX, n16 = ntx * ((op.L1 + 15) / 16);
+        /* Layers of a few columns leave most of a tile empty: where the tiles no
+         * longer all run at once (8 an SM), the launches that k_product saves count
+         * for less.  ms a solve, four launches / one: 8 x 4000 157 / 196, 4 x 4000 98 /
+         * 150, 12 x 4000 166 / 174, but 16 x 4000 212 / 196, and 4 x 2000 40 / 39, 8 x
+         * 1000 22 / 16 */
+        const bool thin = op.L0 < 16 && (long long)n16 * m > 8LL * sms;
+        if (!two_pass || op.L0 < 2 || op.L1 < 2 || thin) {
             int rc = maa(Yc, W, m);
             return rc ? rc : mbb(W, Yc, Yp, Yn, m, alpha, c, beta, ascale);
         }
-        const int ntx = (op.L0 + PX - 1) / PX, n16 = ntx * ((op.L1 + 15) / 16);
         if (n16 * m >= 2 * sms)
             k_product<T, 16><<<dim3(n16, m), 256, 0, st>>>(op, coef(Yc), Yc, Yp, Yn, ld, (T)alpha, (T)c, (T)beta, ascale);
         else
@@ -788,7 +795,6 @@ struct Solver {
                                                                              (T)beta, ascale);
         return cudaPeekAtLastError() == cudaSuccess ? SMAT_OK : smat_fail(SMAT_ECUDA, "k_product launch");
     }
-    bool fused() const { return two_pass && op.L0 > 1 && op.L1 > 1; }
     template <class A, class B> int convert(const A *in, B *out, int m)
     {
         const long long count = n * m;

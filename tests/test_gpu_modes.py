@@ -253,3 +253,16 @@ def test_tiled_product_equals_the_stencils_in_turn(built, L0, L1, bc):
         X = rng.standard_normal((2 * L0 * L1, m))
         want = modes.apply(med, 0.405, L0, L1, bc, 1, modes.apply(med, 0.405, L0, L1, bc, 0, X))
         assert np.array_equal(modes.apply(med, 0.405, L0, L1, bc, 2, X), want)
+
+
+@pytest.mark.parametrize("L0", [2, 15, 16])
+def test_product_of_long_thin_layers(built, L0):
+    """Many columns of a long layer of few cells take the four launches, one column
+    the tiled product: the same bits."""
+    L1 = 700
+    rng = np.random.default_rng(L0)
+    med = rng.uniform(1, 4, (6, L0 * L1)) + 0j
+    X = rng.standard_normal((2 * L0 * L1, 40))
+    Y = modes.apply(med, 0.405, L0, L1, (1, -1), 2, X)
+    for j in (0, 17, 39):
+        assert np.array_equal(Y[:, j], modes.apply(med, 0.405, L0, L1, (1, -1), 2, X[:, j:j + 1])[:, 0])
