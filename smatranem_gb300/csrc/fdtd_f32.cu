@@ -212,14 +212,6 @@ __device__ __forceinline__ void set_el(float4 &v, int i, float x)
 }
 __device__ __forceinline__ float4 scale4(float4 v, float f) { return make_float4(f * v.x, f * v.y, f * v.z, f * v.w); }
 
-/* loads of the other field: CG = true reads through L2 only (ld.global.cg),
- * for data another CTA of the same launch may have written */
-template <bool CG> __device__ __forceinline__ float4 ldG4(const float *p)
-{
-    return CG ? __ldcg(reinterpret_cast<const float4 *>(p)) : *reinterpret_cast<const float4 *>(p);
-}
-template <bool CG> __device__ __forceinline__ float ldG(const float *p) { return CG ? __ldcg(p) : *p; }
-
 /* The loads of one quad row segment (cells x = xr..xr+3 of row j1, plane j2,
  * excitation b; a warp covers 128 consecutive x-cells, lane = threadIdx.x % 32)
  * into q, including the x neighbours by warp shuffle.  False for a row past
@@ -232,7 +224,7 @@ struct QIn {
     bool live, qsplit, pyz;
 };
 
-template <bool EF, bool CG>
+template <bool EF>
 __device__ __forceinline__ bool quad_load(const P32 &p, const int b, const int j1, const int j2, const int xr, QIn &q)
 {
     const Geo &g = p.g;
@@ -267,17 +259,17 @@ __device__ __forceinline__ bool quad_load(const P32 &p, const int b, const int j
     for (int i = 0; i < 3; i++) {
         c[i] = ld4(cf + i * n3 + l);
         out[i] = ld4(F + i * n3 + l);
-        gh[i] = ldG4<CG>(G + i * n3 + l);
+        gh[i] = ld4(G + i * n3 + l);
     }
     if (qsplit) {
 #pragma unroll
         for (int i = 0; i < 3; i++) aux[i] = ld4(Fa + i * n3 + l);
     }
     /* H sweep: Ex, Ez at y-1; Ex, Ey at z-1.  E sweep: Hx, Hz at y+1; Hx, Hy at z+1. */
-    q.gy0 = scale4(ldG4<CG>(G + 0 * n3 + l + oy), fy);
-    q.gy2 = scale4(ldG4<CG>(G + 2 * n3 + l + oy), fy);
-    q.gz0 = scale4(ldG4<CG>(G + 0 * n3 + l + oz), fz);
-    q.gz1 = scale4(ldG4<CG>(G + 1 * n3 + l + oz), fz);
+    q.gy0 = scale4(ld4(G + 0 * n3 + l + oy), fy);
+    q.gy2 = scale4(ld4(G + 2 * n3 + l + oy), fy);
+    q.gz0 = scale4(ld4(G + 0 * n3 + l + oz), fz);
+    q.gz1 = scale4(ld4(G + 1 * n3 + l + oz), fz);
     /* x neighbours: H sweep needs Ey, Ez at x-1; E sweep Hy, Hz at x+1 */
     const unsigned full = 0xffffffffu;
     float &xn1 = q.xn1, &xn2 = q.xn2; /* component 1, 2 of the outer neighbour of the quad */
@@ -288,8 +280,8 @@ __device__ __forceinline__ bool quad_load(const P32 &p, const int b, const int j
             const bool edge = x0 == 0;
             const long long o = edge ? g.L0 - 1 : -1;
             const float f = edge ? (float)g.bc[0] : 1.0f;
-            xn1 = f * ldG<CG>(G + 1 * n3 + l + o);
-            xn2 = f * ldG<CG>(G + 2 * n3 + l + o);
+            xn1 = f * *(G + 1 * n3 + l + o);
+            xn2 = f * *(G + 2 * n3 + l + o);
         }
     } else {
         xn1 = __shfl_down_sync(full, gh[1].x, 1);
@@ -298,8 +290,8 @@ __device__ __forceinline__ bool quad_load(const P32 &p, const int b, const int j
             const bool edge = x0 + 4 == g.L0;
             const long long o = edge ? -(g.L0 - 4) : 4;
             const float f = edge ? (float)g.bc[0] : 1.0f;
-            xn1 = f * ldG<CG>(G + 1 * n3 + l + o);
-            xn2 = f * ldG<CG>(G + 2 * n3 + l + o);
+            xn1 = f * *(G + 1 * n3 + l + o);
+            xn2 = f * *(G + 2 * n3 + l + o);
         }
     }
     return true;
@@ -449,7 +441,7 @@ __device__ __forceinline__ void quad_compute(const P32 &p, const int rel, const 
  * cut off at L0 -- its cells past L0 neither wrap, nor take the source, nor are
  * sampled; lanes that are not in repeat a live quad and store nothing.  GEN:
  * other threads of the launch take the general cells. */
-template <bool EF, bool CG, bool PAD, bool GEN>
+template <bool EF, bool PAD, bool GEN>
 __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const int b, const int j1, const int j2,
                                               const int xr, const bool in)
 {
@@ -486,19 +478,19 @@ __device__ __forceinline__ void sweep32v_quad(const P32 &p, const int rel, const
     for (int i = 0; i < 3; i++) {
         c[i] = ld4(cf + i * n3 + l);
         out[i] = ld4(F + i * n3 + l);
-        gh[i] = ldG4<CG>(G + i * n3 + l);
+        gh[i] = ld4(G + i * n3 + l);
     }
     /* H sweep: Ex, Ez at y-1; Ex, Ey at z-1.  E sweep: Hx, Hz at y+1; Hx, Hy at z+1. */
-    float4 gy0 = ldG4<CG>(G + 0 * n3 + l + oy), gy2 = ldG4<CG>(G + 2 * n3 + l + oy);
-    float4 gz0 = ldG4<CG>(G + 0 * n3 + l + oz), gz1 = ldG4<CG>(G + 1 * n3 + l + oz);
+    float4 gy0 = ld4(G + 0 * n3 + l + oy), gy2 = ld4(G + 2 * n3 + l + oy);
+    float4 gz0 = ld4(G + 0 * n3 + l + oz), gz1 = ld4(G + 1 * n3 + l + oz);
     /* the outer x neighbour (H sweep: Ey, Ez at x-1; E sweep: Hy, Hz at x+1) is
      * the next lane's, or at the end of a warp or row loaded with the others */
     const bool edge = EF ? x0 + 4 == P0 : x0 == 0, own_xn = edge | ((threadIdx.x & 31) == (EF ? 31 : 0));
     float xn1 = 0.0f, xn2 = 0.0f; /* its components 1, 2 */
     if (own_xn) {
         const long long o = EF ? (edge ? -(P0 - 4) : 4) : (edge ? g.L0 - 1 : -1);
-        xn1 = ldG<CG>(G + 1 * n3 + l + o);
-        xn2 = ldG<CG>(G + 2 * n3 + l + o);
+        xn1 = *(G + 1 * n3 + l + o);
+        xn2 = *(G + 2 * n3 + l + o);
     }
     if (qsplit) {
 #pragma unroll
@@ -679,12 +671,12 @@ __global__ void __launch_bounds__(128, MB) k_sweep32v(const P32 p, const int rel
     const int b = blockIdx.y % p.batch;
     const int xr = (blockIdx.x * 32 + threadIdx.x) * 4;
     const int j1 = (blockIdx.y / p.batch) * blockDim.y + threadIdx.y;
-    sweep32v_quad<EF, false, false, false>(p, rel, b, j1, z0 + blockIdx.z, xr, true);
+    sweep32v_quad<EF, false, false>(p, rel, b, j1, z0 + blockIdx.z, xr, true);
 }
 
 /* general cells of the vectorised sweeps: one thread per record cell, after
  * the sweep of the same field or beside it (the quads skip them) */
-template <bool EF, bool CG>
+template <bool EF>
 __device__ __noinline__ void general32_cell(const P32 &p, const int rel, const int b, const long long l)
 {
     const Geo &g = p.g;
@@ -704,7 +696,7 @@ __device__ __noinline__ void general32_cell(const P32 &p, const int rel, const i
     if (r.kind == RK_FROZEN) {
         for (int c = 0; c < 3; c++) main_out[c] = F[c * n3 + l] - Fa[c * n3 + l];
     } else if (stable) {
-        auto get = [&](int c, long long o) { return ldG<CG>(G + c * n3 + l + o) - ldG<CG>(Ga + c * n3 + l + o); };
+        auto get = [&](int c, long long o) { return *(G + c * n3 + l + o) - *(Ga + c * n3 + l + o); };
         float pl[3], mi[3];
         curl32<false>(get, st, pl, mi);
         for (int c = 0; c < 3; c++) {
@@ -719,7 +711,7 @@ __device__ __noinline__ void general32_cell(const P32 &p, const int rel, const i
             Fa[c * n3 + l] = x;
         }
     } else {
-        auto get = [&](int c, long long o) { return ldG<CG>(G + c * n3 + l + o); };
+        auto get = [&](int c, long long o) { return *(G + c * n3 + l + o); };
         float pl[3], mi[3];
         curl32<EF>(get, st, pl, mi);
         if (r.kind == RK_N) {
@@ -770,13 +762,13 @@ __global__ void __launch_bounds__(128, MB) k_sweep32f(const P32 p, const int rel
     prior_done();
     if (GEN && blockIdx.y == 0) {
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncells * p.batch; i += gridDim.x * blockDim.x)
-            general32_cell<EF, false>(p, rel, i % p.batch, cells[i / p.batch]);
+            general32_cell<EF>(p, rel, i % p.batch, cells[i / p.batch]);
         return;
     }
     const int b = blockIdx.x % p.batch, nq = (PAD ? p.g.P0 : p.g.L0) >> 2;
     const int i = blockIdx.x / p.batch * blockDim.x + threadIdx.x, last = nq * p.g.L1 - 1;
     const int u = i <= last ? i : last, j1 = u / nq;
-    sweep32v_quad<EF, false, PAD, GEN>(p, rel, b, j1, z0 + blockIdx.y - GEN, 4 * (u - j1 * nq), i <= last);
+    sweep32v_quad<EF, PAD, GEN>(p, rel, b, j1, z0 + blockIdx.y - GEN, 4 * (u - j1 * nq), i <= last);
 }
 
 template <bool EF>
@@ -785,7 +777,7 @@ __global__ void k_general32(const P32 p, const int rel, const int *cells, int nc
     prior_done();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ncells) return;
-    general32_cell<EF, false>(p, rel, blockIdx.y, cells[i]);
+    general32_cell<EF>(p, rel, blockIdx.y, cells[i]);
 }
 
 /* ---------------------------------------------------------------------------
@@ -812,7 +804,7 @@ __global__ void __launch_bounds__(128, 5) k_group32v(const int rel)
         const int z = local / per, t = local - z * per, b = t % p.batch;
         const int i = t / p.batch * 32 * c_group.by + 32 * threadIdx.y + threadIdx.x, last = nq * p.g.L1 - 1;
         const int u = i <= last ? i : last, j1 = u / nq;
-        sweep32v_quad<EF, false, false, false>(p, rel, b, j1, z, 4 * (u - j1 * nq), i <= last);
+        sweep32v_quad<EF, false, false>(p, rel, b, j1, z, 4 * (u - j1 * nq), i <= last);
         return;
     }
     const int nxb = (nq + 31) / 32;
@@ -821,7 +813,7 @@ __global__ void __launch_bounds__(128, 5) k_group32v(const int rel)
     const int yb = t % nyb, z = t / nyb;
     const int b = yb % p.batch;
     const int j1 = (yb / p.batch) * blockDim.y + threadIdx.y;
-    sweep32v_quad<EF, false, false, false>(p, rel, b, j1, z, (xb * 32 + threadIdx.x) * 4, true);
+    sweep32v_quad<EF, false, false>(p, rel, b, j1, z, (xb * 32 + threadIdx.x) * 4, true);
 }
 
 template <bool EF>
@@ -834,7 +826,7 @@ __global__ void k_group_general32(const int rel)
     while (m + 1 < c_group.n && i >= gb[m + 1]) m++;
     const int ng = EF ? c_group.negen[m] : c_group.nhgen[m];
     const int local = i - gb[m];
-    general32_cell<EF, false>(c_group.p[m], rel, local / ng, (EF ? c_group.egen[m] : c_group.hgen[m])[local % ng]);
+    general32_cell<EF>(c_group.p[m], rel, local / ng, (EF ? c_group.egen[m] : c_group.hgen[m])[local % ng]);
 }
 
 /* the member table for the steps that follow on stream st (from pinned host
@@ -993,8 +985,8 @@ __global__ void __launch_bounds__(128, MB) k_sweep32v2(const P32 p, const int re
     const int za = z0 + 2 * blockIdx.z;
     const bool two = za + 1 < z1;
     QIn qa, qb;
-    if (!quad_load<EF, false>(p, b, j1, za, xr, qa)) return;
-    if (two) quad_load<EF, false>(p, b, j1, za + 1, xr, qb);
+    if (!quad_load<EF>(p, b, j1, za, xr, qa)) return;
+    if (two) quad_load<EF>(p, b, j1, za + 1, xr, qb);
     quad_compute<EF>(p, rel, b, j1, za, qa);
     if (two) quad_compute<EF>(p, rel, b, j1, za + 1, qb);
 }

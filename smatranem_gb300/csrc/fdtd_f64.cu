@@ -358,7 +358,8 @@ void launch_flush64(const P64 &p, int rel_end, int count, cudaStream_t st)
 {
     if (p.d.nfreq <= 0 || p.d.nq <= 0 || count <= 0) return;
     const int nb = (p.g.pl + 127) / 128, used = nb * p.d.nq * 4 * p.batch;
-    int nf = used >= 1824 ? 1 : (1824 + used - 1) / used; /* 152 SMs x 12 blocks */
+    const int fill = 12 * plan::sm_count(); /* 12 blocks an SM */
+    int nf = used >= fill ? 1 : (fill + used - 1) / used;
     if (nf > p.d.nfreq) nf = p.d.nfreq;
     (p.d.ring64 ? k_flush64<true> : k_flush64<false>)<<<dim3(nb, p.d.nq * 4, p.batch * nf), 128, 0, st>>>(p, rel_end, count);
 }
