@@ -750,18 +750,14 @@ int upload_f32(smat_fdtd_plan *p, const smat_fdtd_desc *d, const double *Ah, con
     return SMAT_OK;
 }
 
-/* n rows of FP32 values between padded and unpadded length (padding: 0) */
-void rows_unpad(const smat_fdtd_plan *p, size_t n, const float *padded, float *rows)
+/* n rows of a device array of FP32 values, which may be padded, to the host (the
+ * other way it is the host that pads: such a copy takes half as long again) */
+cudaError_t read_rows(smat_fdtd_plan *p, void *dst, const void *src, size_t n)
 {
-    const size_t L0 = p->L[0];
-    for (size_t r = 0; r < n; r++) memcpy(rows + r * L0, padded + r * p->P0, L0 * 4);
-}
-
-void rows_pad(const smat_fdtd_plan *p, size_t n, const float *rows, float *padded)
-{
-    const size_t L0 = p->L[0];
-    memset(padded, 0, n * p->P0 * 4);
-    for (size_t r = 0; r < n; r++) memcpy(padded + r * p->P0, rows + r * L0, L0 * 4);
+    const size_t row = (size_t)p->L[0] * 4, pitch = (size_t)p->P0 * 4;
+    if (row == pitch) return p->cpy(dst, src, n * row, cudaMemcpyDeviceToHost);
+    p->d2h_bytes += (long long)(n * row);
+    return cudaMemcpy2DAsync(dst, row, src, pitch, row, n, cudaMemcpyDeviceToHost, p->stream);
 }
 
 /* A plan of padded rows gives the padding's memory back (up to 15 %) where a
@@ -775,11 +771,11 @@ int unpad_plan(smat_fdtd_plan *p)
     std::vector<std::pair<float **, size_t>> arrays = {{&p->d_bh, 3}, {&p->d_be, 3}};
     for (float **a : {&p->d_H32, &p->d_E32, &p->d_Ha32, &p->d_Ea32, &p->d_H32b, &p->d_E32b, &p->d_Ha32b, &p->d_Ea32b})
         arrays.push_back({a, 3 * b});
-    std::vector<float> in(3 * b * rows * p->P0), out(3 * b * rows * p->L[0]);
+    std::vector<float> out(3 * b * rows * p->L[0]);
     for (auto &[a, comps] : arrays) {
         const size_t n = comps * rows;
-        CK(cudaMemcpy(in.data(), *a, n * p->P0 * 4, cudaMemcpyDeviceToHost));
-        rows_unpad(p, n, in.data(), out.data());
+        CK(read_rows(p, out.data(), *a, n));
+        CK(cudaStreamSynchronize(p->stream));
         for (void *&x : p->allocations)
             if (x == *a) {
                 cudaFree(x);
@@ -979,12 +975,6 @@ extern "C" int smat_fdtd_info(const smat_fdtd_plan *p, int L[4], int *Lnotn, int
 
 extern "C" long long smat_fdtd_device_bytes(const smat_fdtd_plan *p) { return p ? p->dev_bytes : 0; }
 
-/* cell l of the grid in a device array */
-static long long device_cell(const smat_fdtd_plan *p, long long l)
-{
-    return p->P0 == p->L[0] ? l : l + l / p->L[0] * (p->P0 - p->L[0]);
-}
-
 extern "C" int smat_fdtd_set_fields(smat_fdtd_plan *p, int b, const double *H_t, const double *E_t)
 {
     smat_clear_error();
@@ -1005,21 +995,22 @@ extern "C" int smat_fdtd_set_fields(smat_fdtd_plan *p, int b, const double *H_t,
             CK(p->cpy(da, a.data(), a.size() * 8, cudaMemcpyHostToDevice));
             CK(cudaStreamSynchronize(p->stream));
         } else {
-            const long long n3p = p->n3p;
-            std::vector<float> t(3 * n3p, 0.0f), a(3 * n3p, 0.0f);
+            const size_t rows = 3 * (size_t)p->L[1] * p->L[2], n = rows * p->P0, at = b * n;
+            std::unique_ptr<float[]> t(new float[n]), a(new float[n]);
+            size_t ld = 0;
             for (int c = 0; c < 3; c++)
-                for (long long l = 0; l < n3; l++) {
-                    const long long ld = c * n3p + device_cell(p, l);
-                    double main = src[c + 3 * l], ax = 0.0;
-                    if (p->cont[l] != 'n') ax = src[c + 3 * (n3 + p->addr[l])];
-                    t[ld] = (float)(main + ax);
-                    a[ld] = (float)ax;
+                for (long long l = 0; l < n3;) {
+                    for (int x = 0; x < p->L[0]; x++, l++, ld++) {
+                        double main = src[c + 3 * l], ax = 0.0;
+                        if (p->cont[l] != 'n') ax = src[c + 3 * (n3 + p->addr[l])];
+                        t[ld] = (float)(main + ax);
+                        a[ld] = (float)ax;
+                    }
+                    for (int x = p->L[0]; x < p->P0; x++, ld++) t[ld] = a[ld] = 0.0f;
                 }
             const P32 q = make_p32(p, false);
-            float *dt = (w ? q.E : q.H) + (size_t)b * 3 * n3p;
-            float *da = (w ? q.Ea : q.Ha) + (size_t)b * 3 * n3p;
-            CK(p->cpy(dt, t.data(), t.size() * 4, cudaMemcpyHostToDevice));
-            CK(p->cpy(da, a.data(), a.size() * 4, cudaMemcpyHostToDevice));
+            CK(p->cpy((w ? q.E : q.H) + at, t.get(), n * 4, cudaMemcpyHostToDevice));
+            CK(p->cpy((w ? q.Ea : q.Ha) + at, a.get(), n * 4, cudaMemcpyHostToDevice));
             CK(cudaStreamSynchronize(p->stream));
         }
     }
@@ -1047,23 +1038,20 @@ extern "C" int smat_fdtd_get_fields(smat_fdtd_plan *p, int b, double *H_t, doubl
                 for (int x = 0; x <= ln; x++) dst[c + 3 * (n3 + x)] = a[(size_t)c * (ln + 1) + x];
             }
         } else {
-            const long long n3p = p->n3p;
-            std::vector<float> t(3 * n3p), a(3 * n3p);
+            std::vector<float> t(3 * n3), a(3 * n3);
             const P32 q = make_p32(p, false);
-            const float *dt = (w ? q.E : q.H) + (size_t)b * 3 * n3p;
-            const float *da = (w ? q.Ea : q.Ha) + (size_t)b * 3 * n3p;
-            CK(p->cpy(t.data(), dt, t.size() * 4, cudaMemcpyDeviceToHost));
-            CK(p->cpy(a.data(), da, a.size() * 4, cudaMemcpyDeviceToHost));
+            const size_t rows = 3 * (size_t)p->L[1] * p->L[2], at = b * rows * p->P0;
+            CK(read_rows(p, t.data(), (w ? q.E : q.H) + at, rows));
+            CK(read_rows(p, a.data(), (w ? q.Ea : q.Ha) + at, rows));
             CK(cudaStreamSynchronize(p->stream));
             memset(dst, 0, sizeof(double) * 3 * (size_t)(n3 + ln + 1));
             for (int c = 0; c < 3; c++)
                 for (long long l = 0; l < n3; l++) {
-                    const long long ld = c * n3p + device_cell(p, l);
                     if (p->cont[l] == 'n') {
-                        dst[c + 3 * l] = t[ld];
+                        dst[c + 3 * l] = t[c * n3 + l];
                     } else {
-                        const float ax = a[ld];
-                        dst[c + 3 * l] = (double)(t[ld] - ax);
+                        const float ax = a[c * n3 + l];
+                        dst[c + 3 * l] = (double)(t[c * n3 + l] - ax);
                         dst[c + 3 * (n3 + p->addr[l])] = ax;
                     }
                 }
@@ -1625,12 +1613,11 @@ struct StateHeader {
 
 constexpr char STATE_MAGIC[8] = {'S', 'M', 'A', 'T', 'S', 'T', 'A', 'T'};
 
-/* a device array of a plan's state; padded: FP32 fields, which the file holds
- * without their rows' padding */
+/* a device array of a plan's state, its bytes in the file, and for FP32 fields
+ * their rows, which the file holds without padding (else 0) */
 struct StateArray {
     void *dev;
-    size_t bytes;
-    bool padded;
+    size_t bytes, rows;
 };
 
 /* the device arrays that hold a plan's state, in file order */
@@ -1640,24 +1627,17 @@ std::vector<StateArray> state_arrays(smat_fdtd_plan *p)
     const size_t b = (size_t)p->batch, n3 = (size_t)p->n3;
     if (p->precision == SMAT_FP64) {
         const size_t main = b * 3 * n3 * 8, aux = b * 3 * ((size_t)p->lnotn + 1) * 8;
-        a.push_back({p->d_H64, main, false});
-        a.push_back({p->d_E64, main, false});
-        a.push_back({p->d_Ha64, aux, false});
-        a.push_back({p->d_Ea64, aux, false});
+        a.push_back({p->d_H64, main, 0});
+        a.push_back({p->d_E64, main, 0});
+        a.push_back({p->d_Ha64, aux, 0});
+        a.push_back({p->d_Ea64, aux, 0});
     } else {
         const P32 q = make_p32(p, false);
-        const size_t f = b * 3 * (size_t)p->n3p * 4;
-        for (float *x : {q.H, q.E, q.Ha, q.Ea}) a.push_back({x, f, p->P0 != p->L[0]});
+        for (float *x : {q.H, q.E, q.Ha, q.Ea}) a.push_back({x, b * 3 * n3 * 4, b * 3 * p->L[1] * p->L[2]});
     }
     if (p->d_acc && p->nq > 0 && p->nfreq > 0)
-        a.push_back({p->d_acc, b * (size_t)p->nfreq * p->nq * 4 * (size_t)p->pl * 16, false});
+        a.push_back({p->d_acc, b * (size_t)p->nfreq * p->nq * 4 * (size_t)p->pl * 16, 0});
     return a;
-}
-
-/* bytes of a state array in the file */
-size_t file_bytes(const smat_fdtd_plan *p, const StateArray &a)
-{
-    return a.padded ? (size_t)p->batch * 3 * p->n3 * 4 : a.bytes;
 }
 
 void fill_header(const smat_fdtd_plan *p, StateHeader &h)
@@ -1686,22 +1666,17 @@ extern "C" int smat_fdtd_save_state(smat_fdtd_plan *p, const char *path)
     FILE *f = fopen(path, "wb");
     if (!f) return smat_fail(SMAT_EINVAL, "save_state: cannot open %s", path);
     int rc = fwrite(&h, sizeof h, 1, f) == 1 ? SMAT_OK : smat_fail(SMAT_EINVAL, "save_state: write error");
-    std::vector<char> buf, file;
+    std::vector<char> buf;
     for (const auto &a : state_arrays(p)) {
         if (rc) break;
         buf.resize(a.bytes);
-        p->d2h_bytes += (long long)a.bytes;
-        if (cudaMemcpy(buf.data(), a.dev, a.bytes, cudaMemcpyDeviceToHost) != cudaSuccess) {
-            rc = cuda_fail(cudaGetLastError(), "save_state: copy");
+        cudaError_t e = a.rows ? read_rows(p, buf.data(), a.dev, a.rows) : p->cpy(buf.data(), a.dev, a.bytes, cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
+        if (e != cudaSuccess) {
+            rc = cuda_fail(e, "save_state: copy");
             break;
         }
-        const size_t n = file_bytes(p, a);
-        if (a.padded) {
-            file.resize(n);
-            rows_unpad(p, (size_t)p->batch * 3 * p->L[1] * p->L[2], (const float *)buf.data(), (float *)file.data());
-        }
-        if (fwrite(a.padded ? file.data() : buf.data(), 1, n, f) != n)
-            rc = smat_fail(SMAT_EINVAL, "save_state: write error");
+        if (fwrite(buf.data(), 1, a.bytes, f) != a.bytes) rc = smat_fail(SMAT_EINVAL, "save_state: write error");
     }
     if (fclose(f) != 0 && !rc) rc = smat_fail(SMAT_EINVAL, "save_state: write error");
     return rc;
@@ -1728,20 +1703,25 @@ extern "C" int smat_fdtd_load_state(smat_fdtd_plan *p, const char *path)
     /* FP32: into the field set it was saved from, so that a run continues with
      * the same set parity (and so the same grouping of the DFT ring's sums) */
     if (!rc && p->precision == SMAT_FP32) p->cur = h.cur;
-    std::vector<char> buf, file;
+    std::vector<char> buf;
     for (const auto &a : state_arrays(p)) {
         if (rc) break;
-        const size_t n = file_bytes(p, a);
         buf.resize(a.bytes);
-        if (a.padded) file.resize(n);
-        if (fread(a.padded ? file.data() : buf.data(), 1, n, f) != n) {
+        if (fread(buf.data(), 1, a.bytes, f) != a.bytes) {
             rc = smat_fail(SMAT_EINVAL, "load_state: %s is truncated", path);
             break;
         }
-        if (a.padded) rows_pad(p, (size_t)p->batch * 3 * p->L[1] * p->L[2], (const float *)file.data(), (float *)buf.data());
-        p->h2d_bytes += (long long)a.bytes;
-        if (cudaMemcpy(a.dev, buf.data(), a.bytes, cudaMemcpyHostToDevice) != cudaSuccess)
-            rc = cuda_fail(cudaGetLastError(), "load_state: copy");
+        /* padded rows by way of the other field set, which plans of padded rows
+         * have no other use for */
+        const bool padded = a.rows && p->P0 != p->L[0];
+        void *to = padded ? (p->cur ? p->d_H32 : p->d_H32b) : a.dev;
+        cudaError_t e = p->cpy(to, buf.data(), a.bytes, cudaMemcpyHostToDevice);
+        if (padded && e == cudaSuccess) {
+            const size_t row = (size_t)p->L[0] * 4;
+            e = cudaMemcpy2DAsync(a.dev, (size_t)p->P0 * 4, to, row, row, a.rows, cudaMemcpyDeviceToDevice, p->stream);
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
+        if (e != cudaSuccess) rc = cuda_fail(e, "load_state: copy");
     }
     if (!rc && fgetc(f) != EOF) rc = smat_fail(SMAT_EINVAL, "load_state: %s has trailing data", path);
     fclose(f);
