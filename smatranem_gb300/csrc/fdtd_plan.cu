@@ -494,11 +494,15 @@ int upload_f64(smat_fdtd_plan *p, const double *Ah, const double *Bh, const doub
     const int L0 = p->L[0], L1 = p->L[1], L2 = p->L[2];
     std::vector<uint8_t> sx(L0, 1);
     {
-        long long l = 0;
-        for (int z = 0; z < L2; z++)
-            for (int y = 0; y < L1; y++)
-                for (int x = 0; x < L0; x++, l++)
-                    if (p->cont[l] == 'n') sx[x] = 0;
+        std::vector<int> left(L0); /* the columns without an ordinary cell so far */
+        for (int x = 0; x < L0; x++) left[x] = x;
+        for (long long l = 0; l < n3 && !left.empty(); l += L0) {
+            size_t n = 0;
+            for (int x : left)
+                if (p->cont[l + x] == 'n') sx[x] = 0;
+                else left[n++] = x;
+            left.resize(n);
+        }
     }
     std::vector<int2> ord;
     ord.reserve(2 * (size_t)p->pl);
@@ -519,10 +523,14 @@ int upload_f64(smat_fdtd_plan *p, const double *Ah, const double *Bh, const doub
         for (int y = 0; y < L1; y++)
             for (int x : cols[2]) put(x, y);
     }
-    if ((rc = p->alloc(&p->d_ord, ord.size()))) return rc;
+    /* classes, addresses and the pixel order in one allocation (a fifth of a small
+     * plan's creation is its allocations) */
+    int2 *tables = nullptr;
+    if ((rc = p->alloc(&tables, ord.size() + (size_t)(n3 + 1) / 2 + (size_t)(n3 + 7) / 8))) return rc;
+    p->d_ord = tables;
+    p->d_addr = reinterpret_cast<int *>(tables + ord.size());
+    p->d_flags = reinterpret_cast<uint8_t *>(tables + ord.size() + (n3 + 1) / 2);
     CK(p->cpy(p->d_ord, ord.data(), ord.size() * sizeof(int2), cudaMemcpyHostToDevice));
-    if ((rc = p->alloc(&p->d_flags, n3))) return rc;
-    if ((rc = p->alloc(&p->d_addr, n3))) return rc;
     if ((rc = p->alloc(&p->d_cm, 12 * (size_t)n3))) return rc;
     if ((rc = p->alloc(&p->d_ca, 12 * (size_t)ln))) return rc;
     const size_t fs = (size_t)p->batch * 3 * n3, as = (size_t)p->batch * 3 * (ln + 1);
