@@ -444,14 +444,16 @@ int validate_common(const int L[4], const int iBc[3], const int iBTIin[4], int b
 
 /* FP32 rows of L0 % 4 != 0 cells are padded for the vectorised sweeps, which
  * a few warps' worth of quads cannot keep busy: small plans run the
- * one-cell-per-thread sweeps.  The two meet near 220000 cells (us a step, one
- * cell per thread / padded: 131 x 40 x 40 14.7 / 15.8, 33 x 60 x 60 of two
- * excitations 19.8 / 16.0, 131 x 117 x 103 of two 138 / 83, 321 x 200 x 150
- * 320 / 205).  Rows under 20 cells would grow by more than 15 %. */
+ * one-cell-per-thread sweeps.  Those cost 6 us a step and 19 ns a thousand lanes
+ * (rows rounded up to whole warps); the two meet near 400000 lanes (us a step,
+ * one cell per thread / padded: 63 x 63 x 63 254000 lanes 10.7 / 13.1, 250 x 50 x
+ * 30 384000 12.2 / 13.7, 71 x 65 x 65 406000 13.3 / 13.1, 33 x 60 x 60 of two
+ * excitations 461000 14.9 / 13.1, 81 x 81 x 81 630000 17.9 / 15.0, 131 x 117 x 103
+ * of two 138 / 83).  Rows under 20 cells would grow by more than 15 %. */
 bool padded_rows(const int L[4], int batch)
 {
-    const long long n = (L[0] + 3LL) / 4 * 4 * L[1] * L[2];
-    return L[0] % 4 != 0 && L[0] >= 20 && n * batch >= 220000 && n < (1LL << 31) / 3;
+    const long long rows = (long long)L[1] * L[2], n = (L[0] + 3LL) / 4 * 4 * rows;
+    return L[0] % 4 != 0 && L[0] >= 20 && (L[0] + 31LL) / 32 * 32 * rows * batch >= 400000 && n < (1LL << 31) / 3;
 }
 
 smat_fdtd_plan *new_plan(const int L[4], const int iBc[3], const int iBTIin[4], int precision, int batch,

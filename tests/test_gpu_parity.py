@@ -1028,6 +1028,41 @@ def test_padded_plan_without_room_for_the_padding(built, call):
     assert gone > 0  # the padding went somewhere
 
 
+@pytest.mark.parametrize("case", range(len(PADDED_CASES)))
+def test_padded_rows_of_larger_plans(built, case, tmp_path):
+    """The same comparison and the adjoint's at 48 excitations, more than 400000
+    lanes, from which on rows are padded: more device memory than 48 plans of one
+    excitation hold in fields, the same bits (the gradient, summed in another
+    order: 1e-12)."""
+    f = _fdtd()
+    from smatranem_gb300 import workloads as W
+    _, ref = _padded_setup(case, 1)
+    for kw in ({}, dict(tuning=(0, 4, 3, 0, 4)), dict(path=str(tmp_path / "padded"), resume=True)):
+        _, got = _padded_setup(case, 48, **kw)
+        for a, b in zip(ref, got):
+            assert np.array_equal(a, b), kw
+    L, seed, kw, iBTIin = PADDED_CASES[case]
+    s, pr = _padded_structure(L, seed, {k: v for k, v in kw.items() if k not in ("metals", "pec", "lossy", "lossy_pml")})
+    src, ph = f.cw_schedule(pr.n2pi, (1, 1, 3))
+    pl = L[0] * L[1]
+    rng = np.random.default_rng(seed)
+    cols = rng.standard_normal(4 * pl) + 1j * rng.standard_normal(4 * pl)
+
+    def run(batch):
+        with f.Plan.create(s.L, s.iBc, iBTIin, pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma, precision=f.FP32,
+                           batch=batch) as p:
+            if batch > 1:
+                fields = 8 * 3 * 4 * batch * s.n3
+                assert p.device_bytes > fields * ((L[0] + 3) // 4 * 4) / L[0]
+            for b in range(batch):
+                p.set_incident(b, *W.random_incident(pl, seed=100))
+            p.set_schedule(src, planes=(iBTIin[0], iBTIin[1], 0), phase=ph)
+            return p.adjoint_grad(12, 5, 0, 0, cols, (8, 12, 3, 6, 12, 16))[:2]
+
+    (J, g), (J1, g1) = run(48), run(1)
+    assert _relerr(np.asarray(g), 48 * np.asarray(g1)) < 1e-12 and abs(J - 48 * J1) <= 1e-12 * abs(J)
+
+
 @pytest.mark.parametrize("L", [(4, 7, 9, 2), (124, 5, 7, 2), (128, 6, 7, 2), (132, 5, 6, 2), (256, 3, 6, 2)])
 def test_quads_dealt_out_bit_identical(built, L):
     """The vectorised sweeps whose quads go to the threads row after row (L0 not
