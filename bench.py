@@ -1085,7 +1085,7 @@ def config_scalc(L0=32, L1=32, nl=10, steps=2, dense="both", cpu=True):
         "s_per_smatrix": best, "runs": nruns, "solves": solves,
         "fp64_tflops": flops / best / 1e12,
         "products": "FP64-accurate complex products on the tensor cores (7 bf16 slices per operand, Ozaki scheme, "
-                    "tcgen05.mma); LU panels and triangle blocks in FP64",
+                    "tcgen05.mma); sweep panels and triangle blocks in FP64",
         "fp64_kernel": None if best64 is None else {"s_per_smatrix": best64, "fp64_tflops": flops / best64 / 1e12,
                                                     "speedup_tensor_cores": best64 / best},
         "s_max_abs_diff_vs_fp64_kernel": None if S64 is None else float(np.abs(S - S64).max()),

@@ -142,7 +142,8 @@ int smat_fdtd_get_fields(smat_fdtd_plan *plan, int b, double *H_t, double *E_t);
 /* Checkpoint and resume.  No counterpart in the reference (its FDTD state is
  * never written).  save_state writes the plan's state -- the fields and aux
  * slots of every excitation and the running-DFT accumulators -- to a binary
- * file, exactly as held on the device; load_state restores it into a plan of
+ * file, value for value as held on the device (FP32 rows without the padding
+ * they may have there); load_state restores it into a plan of
  * the same grid, precision, batch, split-cell count and DFT setup (refused
  * with SMAT_EINVAL otherwise), after which run(k, ...) continues from step k
  * with the bits an uninterrupted run would give (FP32: with the same launch
@@ -351,8 +352,7 @@ int smat_fdtd_copy_bytes(const smat_fdtd_plan *plan, long long *h2d, long long *
 int smat_fdtd_check_finite(smat_fdtd_plan *plan, int *finite, double *max_abs);
 
 /* Average device time per launch (ms) of the H sweep, the E sweep and the
- * per-step DFT work (FP64: the DFT kernel; FP32: the ring flush amortised over
- * its steps), measured with CUDA events on the plan's stream over steps
+ * per-step DFT work (the ring's flush, amortised over its steps), measured with CUDA events on the plan's stream over steps
  * [k_begin, k_begin+nsteps) of the schedule.  The steps are really taken. */
 int smat_fdtd_time_kernels(smat_fdtd_plan *plan, int k_begin, int nsteps, double ms[3]);
 

@@ -9,16 +9,17 @@
 
 namespace smat {
 
-/* Kernels of a step (of the FDTD loop, or of a sweep of the layer transfer) follow one another as programmatic dependents
- * (launch_after): one is set up while the one before ends and waits for its
- * results in prior_done, which every thread that touches fields, the ring or
- * the step counter calls first (half a microsecond a launch: 14.1 -> 12.6 us
- * for a step of two sweeps at 48^3 cells, 21.0 -> 20.0 at 100^3, 71.9 -> 71.4
- * at 160 x 160 x 120).  What the kernel before writes is read through coherent
- * loads (no const __restrict__: such loads may count on data that stands still for
- * the whole kernel).  After next_may_start in every block the next kernel may
- * run up to its own prior_done beside this one -- index arithmetic and loads of
- * what no launch of a run changes (coefficients, masks, orders, records). */
+/* Kernels of a step (of the FDTD loop, or of a sweep of the layer transfer)
+ * follow one another as programmatic dependents (launch_after): one is set up
+ * while the one before ends and waits for its results in prior_done, which every
+ * thread that touches fields, the ring or the step counter calls first (most of
+ * a microsecond a launch: 14.1 -> 12.8 us for a step of two FP32 sweeps at 48^3
+ * cells, 21.0 -> 20.0 at 100^3, 71.9 -> 71.4 at 160 x 160 x 120).  What the kernel
+ * before writes is read through coherent loads (no const __restrict__: such loads
+ * may count on data that stands still for the whole kernel).  After
+ * next_may_start in every block the next kernel may run up to its own prior_done
+ * beside this one: index arithmetic and loads of what no launch of a run changes
+ * (coefficients, addresses, orders, records). */
 __device__ __forceinline__ void prior_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>

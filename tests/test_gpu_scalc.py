@@ -1,8 +1,9 @@
 """GPU layer-transfer S matrix (smat_scalc) against the reference S-matrix
 program (Smat/Scalc.c).
 
-* the LU solve behind it (smat_zgesv) against numpy on random, pivoting-heavy
-  and singular systems (block sizes straddling the 32-column panels);
+* the elimination behind it (smat_zsweep) and the LU solve (smat_zgesv) against
+  numpy on random, pivoting-heavy and singular systems (block sizes straddling
+  the 32-column panels, every cluster size, all exponents);
 * the S matrix against the stock Scalc's own output on its fixtures
   (tests/golden/scalc_*.npz) and against the oracle restatement on larger
   seeded structures (lossy inner layers, every BoundC);
@@ -180,7 +181,7 @@ def test_sweep_sizes_match_oracle(built, L0, L1, bc, layers, n, mode):
     """The Gauss-Jordan sweeps at orders around their blocks of 32 columns and
     their cluster sizes (NA = 2, 30, 32, 66, 144) and from one port mode to all
     of them, on lossy random layers between dense random port matrices: the
-    restatement's S within 1e-9 of its largest entry, the start's LU path's own
+    restatement's S within 1e-9 of its largest entry, an LU form's own
     spread on such ports being under 1e-10; twice the same bits."""
     rng = np.random.default_rng(L0 * 31 + L1)
     NA = 2 * L0 * L1
@@ -264,6 +265,35 @@ def test_zgemm_is_within_half_a_unit_and_the_dropped_digits(built, m, n, k):
                 err = abs(int(got * 2.0 ** 106) - w)
                 # one pass: half a unit of the result; more: of the largest sum on the way too (below 2 k)
                 assert err <= left + unit / 2 + (2.0 ** 106 * np.spacing(2.0 * k) if passes > 1 else 0), (r, err, left)
+
+
+@pytest.mark.parametrize("L0,L1,layers", [(6, 5, 6), (10, 8, 10), (13, 11, 6)])
+def test_gratings_to_the_last_digits(dense, L0, L1, layers):
+    """S of gratings between plane-wave ports against the restatement (LAPACK):
+    2 * layers eliminations of order NA a direction, each of relative error NA
+    2^-53 at most on either side, at entries of S up to 1."""
+    om = 0.405
+    _, Xi, nr = W.plane_wave_basis(L0, L1, omega=om)
+    meds = W.grating_layers(L0, L1, layers, seed=3)
+    ref = SO.smatrix(list(meds), om, L0, L1, (1, 1), Xi, nr, Xi, nr)
+    S, _ = scalc.smatrix(meds, om, L0, L1, (1, 1), Xi, nr, Xi, nr)
+    assert np.abs(S - ref).max() <= 2 * 2 * layers * 2 * L0 * L1 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("L0,L1,bc,layers,n", [(1, 1, (0, 0), 2, 1), (3, 5, (1, 0), 3, 4), (4, 4, (1, 1), 2, 32),
+                                               (3, 11, (0, 1), 3, 7), (8, 9, (1, -1), 4, 3)])
+def test_random_ports_as_close_as_an_lu(dense, L0, L1, bc, layers, n):
+    """Dense random port matrices, at the bound that an LU form keeps: 1e-10 of
+    the largest entry."""
+    rng = np.random.default_rng(L0 * 31 + L1)
+    NA = 2 * L0 * L1
+    n = min(n, NA)
+    meds = rng.uniform(1, 4, (layers, 6, L0 * L1)) + 0j
+    meds[1:-1] += 0.1j * rng.uniform(0, 1, meds[1:-1].shape)
+    Xi = [rng.standard_normal((2 * NA, 2 * NA)) + 1j * rng.standard_normal((2 * NA, 2 * NA)) for _ in range(2)]
+    want = SO.smatrix(list(meds), 0.4, L0, L1, bc, Xi[0], n, Xi[1], n)
+    got, _ = scalc.smatrix(meds, 0.4, L0, L1, bc, Xi[0], n, Xi[1], n)
+    assert np.abs(got - want).max() <= 1e-10 * np.abs(want).max()
 
 
 # ---- the elimination (smat_zsweep) ----------------------------------------------
