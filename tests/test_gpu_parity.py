@@ -1186,6 +1186,36 @@ def test_fp64_plan_without_room_for_the_sample_ring(built, L, pml):
         assert np.array_equal(a, b)
 
 
+def test_fp64_adjoint_takes_the_sample_rings_room(built):
+    """An FP64 adjoint whose checkpoints fit the device without the ring of eight
+    planes only: the gradient of a device with room, and the plan runs on."""
+    f = _fdtd()
+    from smatranem_gb300 import workloads as W
+    L, nsteps, K = (64, 60, 40, 1), 12, 3
+    s = W.random_structure(L, seed=12, pml=(3, 3, 3))
+    pr = W.prepare(s)
+    src, ph = (a[:nsteps] for a in f.cw_schedule(pr.n2pi, (1, 1, 6)))
+    pl = L[0] * L[1]
+    rng = np.random.default_rng(2)
+    col = rng.standard_normal(4 * pl) + 1j * rng.standard_normal(4 * pl)
+    ring = 32 * 8 * 4 * pl * 8
+    box = (20, 24, 20, 24, 12, 16)
+    need = 48 * (s.n3 + pr.lnotn + 1) * (nsteps // K) + 96 * s.n3 + 64 * 24 * (K + 2)
+    out = []
+    for left in (1 << 50, int(need / 0.9) - ring // 2):
+        with f.Plan.create(L, s.iBc, (4, 36, 5, 1), pr.invtau_R, pr.invtau_I, pr.mu, pr.epsi, pr.sigma) as p:
+            p.set_incident(0, *W.random_incident(pl, seed=2))
+            p.set_schedule(src, planes=(4, 5, 9, 10, 20, 25, 30, 36), phase=ph)
+            held = p.device_bytes
+            with _Ballast(left):
+                J, g, gc = p.adjoint_grad(nsteps, K, 0, 7, col, box)
+            assert held - p.device_bytes == (ring if out else 0)
+            p.run(0, nsteps)
+            out.append((np.array(J), np.asarray(g), np.asarray(gc), *p.get_fields(0), p.get_dft(0, 0, 7)))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("part", ["sums", "phases"])
 def test_schedule_out_of_memory_leaves_no_half_of_it(built, precision, part):
