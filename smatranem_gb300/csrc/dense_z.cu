@@ -519,12 +519,12 @@ __device__ __forceinline__ double2 cfnma(double2 c, double2 a, double2 b) /* c -
 }
 
 /* 1 / d, 0 for d = 0: conj(d) / |d|^2, the real reciprocal by one step of the
- * cubic iteration x <- x (1 + e + e^2), e = 1 - s x (M. Altman, "An optimum cubically convergent
- * iterative method of inverting a linear bounded operator in Hilbert space",
- * Pacific J. Math. 10, 1960), from the 20-bit rcp.approx.ftz.f64: error e^3 <
- * 2^-57.  The FP64 division takes three times as long, on every column's
- * critical path.  |d|^2 outside 2^+-1000: the division, of d scaled by a power
- * of two, the scale put back last. */
+ * cubic iteration x <- x (1 + e + e^2), e = 1 - s x (M. Altman, "An optimum
+ * cubically convergent iterative method of inverting a linear bounded operator
+ * in Hilbert space", Pacific J. Math. 10, 1960), from the 20-bit
+ * rcp.approx.ftz.f64: error e^3 < 2^-57.  The FP64 division takes three times as
+ * long, on every column's critical path.  |d|^2 outside 2^+-1000: the division,
+ * of d scaled by a power of two, the scale put back last. */
 __device__ __forceinline__ double2 reciprocal(double2 d)
 {
     const double s = fma(d.x, d.x, d.y * d.y);
@@ -552,7 +552,10 @@ static_assert(GJ_FIXED % 16 == 0 && gj_part(1) % 16 == 0, "double2 alignment");
 
 /* ROWS_IN_L2: a panel whose rows do not fit the cluster's shared memory (more than
  * 5696 on 16 CTAs) keeps them at `rows` in device memory, each CTA its own part,
- * which L2 holds: 9 MB at order 16384. */
+ * which L2 holds: 9 MB at order 16384.  So the panel has 32 columns at any order:
+ * with 16 or 8 columns in shared memory, the products' inner size of 32 half or
+ * three quarters empty, one direction over two layers took 1.8 s at order 5832 and
+ * 17 s at 11552; now 1.3 and 6.4 (LU, substitutions and product: 3.3 and 19). */
 template <bool ROWS_IN_L2>
 __global__ void __launch_bounds__(GJT) k_gj_panel(const double2 *A, int lda, int j, int n, int nb, double2 *__restrict__ lud,
                                                   int *__restrict__ mv, int *info, unsigned char *rows)
@@ -732,11 +735,7 @@ static int gj_clusters()
 /* whether the rows of panels of order n on clusters of cs CTAs fit their shared memory */
 static bool gj_fits(int n, int cs) { return GJ_FIXED + GJ_ROW * ((n + cs - 1) / cs) <= GJ_SMEM; }
 
-/* 16 CTAs for panels of 128 rows and more; fewer rows synchronise fewer.
- * Rows in L2 keep the panel at 32 columns at any order: with panels of 16 and 8
- * columns in shared memory, the products' inner size of 32 half and three quarters
- * empty, one direction over two layers took 1.8 s at order 5832 and 17 s at 11552;
- * now 1.3 and 6.5 (LU, substitutions and product: 3.3 and 19). */
+/* 16 CTAs for panels of 128 rows and more; fewer rows synchronise fewer */
 static int gj_ctas(int m, int max_cs) { return std::min(max_cs, m >= 128 ? 16 : m >= 64 ? 8 : m >= 32 ? 4 : 1); }
 
 int sweep_setup(SweepWs &w, int n, int max_cluster)
